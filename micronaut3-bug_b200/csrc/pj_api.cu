@@ -22,18 +22,16 @@
 #include "petjson.h"
 #include "pj_kernels.cuh"
 #include "pj_array_kernels.cuh"
-#include "pj_stream_kernel.cuh"
+#include "pj_item.cuh"
 
 using namespace pj;
 
-/* the four instantiations of the tile kernel live in objects of their own (pj_tile_inst.cu) */
+/* the four instantiations of the parse kernel live in objects of their own (pj_tile_inst.cu) */
 namespace pj {
-cudaError_t tile_init_1(const Schema*); cudaError_t tile_launch_1(const TileArgs*, unsigned, cudaStream_t);
-cudaError_t tile_init_2(const Schema*); cudaError_t tile_launch_2(const TileArgs*, unsigned, cudaStream_t);
-cudaError_t tile_init_3(const Schema*); cudaError_t tile_launch_3(const TileArgs*, unsigned, cudaStream_t);
-cudaError_t tile_init_4(const Schema*); cudaError_t tile_launch_4(const TileArgs*, unsigned, cudaStream_t);
-cudaError_t stream_launch_1(const StreamArgs*, unsigned, cudaStream_t); cudaError_t stream_launch_2(const StreamArgs*, unsigned, cudaStream_t);
-cudaError_t stream_launch_3(const StreamArgs*, unsigned, cudaStream_t); cudaError_t stream_launch_4(const StreamArgs*, unsigned, cudaStream_t);
+cudaError_t item_init_1(const Schema*); cudaError_t item_launch_1(const ItemArgs*, cudaStream_t);
+cudaError_t item_init_2(const Schema*); cudaError_t item_launch_2(const ItemArgs*, cudaStream_t);
+cudaError_t item_init_3(const Schema*); cudaError_t item_launch_3(const ItemArgs*, cudaStream_t);
+cudaError_t item_init_4(const Schema*); cudaError_t item_launch_4(const ItemArgs*, cudaStream_t);
 }
 
 namespace {
@@ -269,33 +267,45 @@ pj_status finish_columns(pj_ctx* c, uint32_t schema, uint64_t len, const ParsePl
   return PJ_OK;
 }
 
-/* Tile size of the stream kernel: about 104 records per tile of 128 threads, from the bytes per record the context
- * saw in its earlier calls on the schema (before the first one: from the benchmark distributions). The result of a
- * call does not depend on it. */
-uint32_t pick_tile_bytes(const pj_ctx* c, uint32_t schema) {
-  uint64_t tb;
-  if (c->tile_bytes_opt) tb = c->tile_bytes_opt;
-  else {
-    static const double dflt[5] = {0, 300, 125, 190, 220};
-    const double avg = c->avg_rec_bytes[schema] > 0 ? c->avg_rec_bytes[schema] : dflt[schema];
-    tb = (uint64_t)(avg * (ST_THREADS * 13 / 16));
+/* How a call's input is cut into tiles. The result of a call does not depend on it. */
+struct TileShape { uint32_t tile_bytes, win_bytes, str_ratio, row_cap; };
+uint32_t item_stride(uint32_t schema) {
+  return schema == PJ_SCHEMA_PET ? ItStride<1>::n : (schema == PJ_SCHEMA_ORDER ? ItStride<2>::n : (schema == PJ_SCHEMA_USER ? ItStride<3>::n : ItStride<4>::n));
+}
+TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
+  static const double dflt[5] = {0, 300, 146, 190, 230};
+  static constexpr uint32_t BUDGET = 69 * 1024; /* dynamic shared memory that lets three blocks share an SM */
+  const double avg = c->avg_rec_bytes[schema] > 0 ? c->avg_rec_bytes[schema] : dflt[schema];
+  TileShape t;
+  /* room behind the tile for its last records: 13 average records reach the longest ones of a skewed distribution */
+  uint32_t slack = (uint32_t)(avg * 13);
+  slack = (slack < 4096 ? 4096u : (slack > 28672 ? 28672u : slack)) & ~15u;
+  t.str_ratio = 43; /* a string per six bytes */
+  uint64_t tile = (uint64_t)(avg * 190); /* at most 256 records */
+  if (tile > 32768) tile = 32768;
+  if (len / 296 < tile) { tile = len / 296; if (tile < 4096) tile = 4096; t.str_ratio = 128; } /* few tiles: one for every SM's two halves, and room enough */
+  if (c->tile_bytes_opt) { tile = c->tile_bytes_opt; if (tile < ST_MIN_TILE_BYTES) tile = ST_MIN_TILE_BYTES; if (tile > 32768) tile = 32768; }
+  for (;;) {
+    t.tile_bytes = (uint32_t)(tile & ~31ull);
+    if (t.tile_bytes < ST_MIN_TILE_BYTES) t.tile_bytes = ST_MIN_TILE_BYTES;
+    t.win_bytes = t.tile_bytes + slack;
+    const double recs = (double)t.tile_bytes / avg * 1.4 + 40;
+    t.row_cap = recs > 272 ? 272u : (uint32_t)recs;
+    if (t.str_ratio > 100 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_ratio, t.row_cap, item_stride(schema)).total <= BUDGET) return t;
+    tile -= 1024;
   }
-  tb &= ~15ull;
-  if (tb < ST_MIN_TILE_BYTES) tb = ST_MIN_TILE_BYTES;
-  if (tb > ST_MAX_TILE_BYTES) tb = ST_MAX_TILE_BYTES;
-  return (uint32_t)tb;
 }
 
-cudaError_t stream_launch(uint32_t schema, const StreamArgs* a, unsigned grid, cudaStream_t s) {
+cudaError_t item_launch(uint32_t schema, const ItemArgs* a, cudaStream_t s) {
   switch (schema) {
-    case PJ_SCHEMA_PET: return stream_launch_1(a, grid, s);
-    case PJ_SCHEMA_ORDER: return stream_launch_2(a, grid, s);
-    case PJ_SCHEMA_USER: return stream_launch_3(a, grid, s);
-    default: return stream_launch_4(a, grid, s);
+    case PJ_SCHEMA_PET: return item_launch_1(a, s);
+    case PJ_SCHEMA_ORDER: return item_launch_2(a, s);
+    case PJ_SCHEMA_USER: return item_launch_3(a, s);
+    default: return item_launch_4(a, s);
   }
 }
 
-/* NDJSON: one launch of k_parse_stream per piece. Host buffers of a whole stream are parsed in pieces cut after line
+/* NDJSON: one launch of k_parse_items per piece. Host buffers of a whole stream are parsed in pieces cut after line
  * feeds, so that the copy of piece p+1 to the device, the kernel of piece p and the copy of the columns of piece p-1
  * back run at the same time on three streams. Every launch is enqueued before the host waits for anything: a piece
  * starts where the piece before it ended, which it reads from that piece's totals ON THE DEVICE (StreamArgs.prev). */
@@ -362,27 +372,29 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     }
   }
 
-  const uint32_t tile_bytes = pick_tile_bytes(c, schema);
+  uint64_t longest = 0;
+  for (int p = 0; p < np; ++p) longest = cut[p + 1] - cut[p] > longest ? cut[p + 1] - cut[p] : longest;
+  const TileShape shape = pick_tile_shape(c, schema, longest);
   /* look-back states: one buffer per piece, so that no launch waits for the one before it to be read back */
   uint64_t nt[MAX_PIECES], nt_total = 0;
   for (int p = 0; p < np; ++p) {
     const uint8_t* pin = d_in ? d_in + cut[p] : d_in;
     const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(pin) & 15u);
-    nt[p] = stream_tiles(mis, cut[p + 1] - cut[p], 1u, tile_bytes); /* at least one tile: it closes the offset columns */
+    nt[p] = stream_tiles(mis, cut[p + 1] - cut[p], 1u, shape.tile_bytes); /* at least one tile: it closes the offset columns */
     if (nt[p] >= (1ull << 31)) return set_err(c, PJ_ERR_TOO_LARGE, "pj_parse: too many tiles");
     nt_total += nt[p];
   }
-  { pj_status st = ensure(c, &c->tiles, nt_total * sizeof(StreamTile) + (size_t)np * 256 + 256); if (st) return st; }
-  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * sizeof(StreamTile) + (size_t)np * 256, c->stream));
+  { pj_status st = ensure(c, &c->tiles, nt_total * sizeof(ItemTile) + (size_t)np * 256 + 256); if (st) return st; }
+  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * sizeof(ItemTile) + (size_t)np * 256, c->stream));
   PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult) * np, c->stream));
   if (c->stall_once) { /* test hook: tickets start at 1, tile 0 is never processed, the waits for it run out */
     c->stall_once = false;
     for (int p = 0; p < np; ++p) PJ_CUDA(c, cudaMemsetAsync((uint8_t*)c->tiles.p + (size_t)p * 256, 1, 1, c->stream));
   }
-  c->stats.tile_records = ST_THREADS;
+  c->stats.tile_records = IT_THREADS;
   uint64_t tiles_at = 0;
   for (int p = 0; p < np; ++p) {
-    StreamArgs sa;
+    ItemArgs sa;
     memset(&sa, 0, sizeof sa);
     const uint64_t plen = cut[p + 1] - cut[p];
     sa.in = d_in ? d_in + cut[p] : d_in;
@@ -396,11 +408,12 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
       sa.is_first = p == 0 ? (uint32_t)is_first : 0u;
       sa.is_last = (is_last && sl == rest) ? 1u : 0u;
     }
-    sa.tile_bytes = tile_bytes; sa.ntiles = (uint32_t)nt[p];
+    sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_ratio = shape.str_ratio; sa.row_cap = shape.row_cap;
+    sa.ntiles = (uint32_t)nt[p];
     sa.spin_limit_ns = c->spin_ns;
     sa.opts = c->opt_flags;
     sa.ticket = (uint32_t*)((uint8_t*)c->tiles.p + (size_t)p * 256);
-    sa.tiles = (StreamTile*)((uint8_t*)c->tiles.p + (size_t)np * 256) + tiles_at;
+    sa.tiles = (ItemTile*)((uint8_t*)c->tiles.p + (size_t)np * 256) + tiles_at;
     tiles_at += nt[p];
     sa.res = c->d_res + p;
     sa.prev = p ? c->d_res + p - 1 : nullptr;
@@ -410,7 +423,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     sa.cols = pp.dcols;
     if (pipe) PJ_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_in[p], 0));
     PJ_CUDA(c, cudaEventRecord(c->ev_k0[p], c->stream));
-    PJ_CUDA(c, stream_launch(schema, &sa, (unsigned)nt[p], c->stream));
+    PJ_CUDA(c, item_launch(schema, &sa, c->stream));
     PJ_CUDA(c, cudaEventRecord(c->ev_k1[p], c->stream));
     PJ_CUDA(c, cudaMemcpyAsync(c->h_res + p, c->d_res + p, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
     PJ_CUDA(c, cudaEventRecord(c->ev_done[p], c->stream));
@@ -430,9 +443,9 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     if (cudaEventElapsedTime(&ms, c->ev_k0[p], c->ev_k1[p]) == cudaSuccess) { c->stats.stage_ms[2] += ms; c->stats.device_ms += ms; }
     n_fast += r.n_fast; n_errors += r.n_errors;
     for (int k = 0; k < 4; ++k) c->stats.phase_cycles[k] += r.phase_cycles[k];
-    c->stats.lookback_polls += r.lookback_polls; c->stats.lookback_rounds += r.lookback_rounds;
     c->stats.wide_records += r.n_wide; c->stats.wide_fast_records += r.n_wide_fast;
     c->stats.wide_cycles[0] += r.wide_cycles[0]; c->stats.wide_cycles[1] += r.wide_cycles[1];
+    c->stats.lookback_polls += r.lookback_polls; c->stats.lookback_rounds += r.lookback_rounds;
     if (r.timeout) return set_err(c, PJ_ERR_TIMEOUT, "pj_parse: a bounded device-side wait ran out");
     if (r.over) over = true;
     const uint64_t rows_new = r.n_records;
@@ -467,8 +480,8 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   return PJ_OK;
 }
 
-/* Array framing: the record index of pj_array_kernels.cuh (extent of every element), then the tile kernel over
- * tiles of TILE_THREADS records. */
+/* Array framing: the separator bitmap of pj_array_kernels.cuh, then the parse kernel with it in the place of the line
+ * feeds. */
 pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t len, uint32_t in_kind, pj_columns* out) {
   ParsePlan pp;
   { pj_status st = plan_columns(c, schema, out, len, true, &pp); if (st) return st; }
@@ -481,84 +494,58 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
     PJ_CUDA(c, cudaMemcpyAsync(c->in_stage.p, in, len, cudaMemcpyHostToDevice, c->stream));
     c->stats.h2d_bytes += len;
   }
-  const uint64_t cap_all = pp.rec_cap;
   const uint64_t nwords = (len + 63) >> 6;
   const uint64_t atiles = nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1;
   const size_t off_fn = align_up((atiles + 1) * 4, 256);
   const size_t off_tin = align_up(off_fn + atiles * sizeof(ArrFn), 256);
   const size_t off_sep = align_up(off_tin + atiles * sizeof(ArrState), 256);
-  const size_t off_rend = align_up(off_sep + (nwords + 1) * 8, 256);
-  const size_t off_rblank = align_up(off_rend + cap_all * 8, 256);
-  { pj_status st = ensure(c, &c->scratch, off_rblank + cap_all + 256); if (st) return st; }
-  uint32_t* d_tile = (uint32_t*)c->scratch.p;
-  uint64_t* d_rec_end = (uint64_t*)((uint8_t*)c->scratch.p + off_rend);
-  uint8_t* d_rec_blank = (uint8_t*)c->scratch.p + off_rblank;
-  uint32_t slot_lo, slot_hi;
-  slot_range(schema, &slot_lo, &slot_hi);
+  const size_t off_end = align_up(off_sep + (nwords + 1) * 8, 256);
+  { pj_status st = ensure(c, &c->scratch, off_end + 256); if (st) return st; }
 
   PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult), c->stream));
   Stage stage(c);
   ArrArgs aa;
   aa.in = d_in; aa.len = len; aa.nwords = nwords;
   aa.tile_fn = (ArrFn*)((uint8_t*)c->scratch.p + off_fn); aa.tile_in = (ArrState*)((uint8_t*)c->scratch.p + off_tin);
-  aa.sep = (uint64_t*)((uint8_t*)c->scratch.p + off_sep); aa.tile_cnt = d_tile;
-  aa.rec_start = (uint64_t*)pp.dcols.ptr[PJ_COL_REC_START]; aa.rec_end = d_rec_end; aa.rec_blank = d_rec_blank;
-  aa.cap = cap_all; aa.goff = 0; aa.ntiles = (uint32_t)atiles; aa.res = c->d_res;
+  aa.sep = (uint64_t*)((uint8_t*)c->scratch.p + off_sep); aa.tile_cnt = nullptr;
+  aa.rec_start = nullptr; aa.rec_end = nullptr; aa.rec_blank = nullptr;
+  aa.cap = 0; aa.goff = 0; aa.ntiles = (uint32_t)atiles; aa.res = c->d_res;
   /* the two running minima start at "none" */
   PJ_CUDA(c, cudaMemsetAsync(&c->d_res->doc_err_off, 0xFF, sizeof(unsigned long long), c->stream));
   PJ_CUDA(c, cudaMemsetAsync(&c->d_res->first_opener, 0xFF, sizeof(unsigned long long), c->stream));
   k_arr_summary<<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
   k_arr_scan_tiles<<<1, 32, 0, c->stream>>>(aa);
   k_arr_mark<<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-  k_arr_records<false><<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-  k_scan_single<uint32_t><<<1, 1024, 0, c->stream>>>(d_tile, atiles, &c->d_res->n_records);
-  k_arr_records<true><<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-  count_launch(c, 0, 6);
+  count_launch(c, 0, 3);
   PJ_CUDA(c, cudaGetLastError());
   stage.next();
 
-  /* the tile kernel needs the record count to size its grid */
-  PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
-  PJ_CUDA(c, cudaStreamSynchronize(c->stream));
-  const uint64_t N0 = c->h_res->n_records;
   uint64_t total[NSLOT];
   for (uint32_t k = 0; k < NSLOT; ++k) total[k] = 0;
-  if (N0 > cap_all) {
-    out->schema = schema; out->n_records = N0; out->n_errors = 0;
-    for (int i = 0; i < pp.nrc; ++i) out->col[pp.rcols[i]].count = N0;
-    return set_err(c, PJ_ERR_CAPACITY, "pj_parse: %llu records, per-record buffers hold %llu", (unsigned long long)N0, (unsigned long long)cap_all);
-  }
-  TileArgs ta;
-  memset(&ta, 0, sizeof ta);
-  ta.in = d_in; ta.limit = len; ta.goff = 0; ta.n_records = N0;
-  ta.lf_ws = 1u; ta.open_end = 0u; ta.schema = schema; ta.slot_lo = slot_lo; ta.slot_hi = slot_hi;
-  ta.win_bytes = TILE_WIN_BYTES; ta.tape_cap = TILE_TAPE_CAP;
-  ta.tile_recs = TILE_THREADS;
-  const uint64_t ntiles = N0 ? (N0 + TILE_THREADS - 1) / TILE_THREADS : 1;
-  ta.ntiles = (uint32_t)ntiles;
-  ta.spin_limit_ns = c->spin_ns;
-  ta.opts = c->opt_flags;
-  c->stats.tile_records = TILE_THREADS; c->stats.tiles += (uint32_t)ntiles;
-  ta.rec_end = d_rec_end; ta.rec_blank = d_rec_blank;
-  { pj_status st = ensure(c, &c->tiles, ntiles * sizeof(TileState) + 256); if (st) return st; }
-  ta.ticket = (uint32_t*)c->tiles.p;
-  ta.tiles = (TileState*)((uint8_t*)c->tiles.p + 128);
-  ta.res = c->d_res;
-  for (uint32_t k = 0; k < NSLOT; ++k) { ta.slot_cap[k] = pp.slot_cap[k]; ta.slot_base[k] = 0; }
-  ta.plan = pp.plan;
-  ta.cols = pp.dcols;
-  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, ntiles * sizeof(TileState) + 128, c->stream));
-  const uint32_t one = 1;
-  PJ_CUDA(c, cudaMemcpyAsync(&c->d_res->ok, &one, sizeof one, cudaMemcpyHostToDevice, c->stream));
+  ItemArgs sa;
+  memset(&sa, 0, sizeof sa);
+  const TileShape shape = pick_tile_shape(c, schema, len);
+  sa.in = d_in; sa.len = len; sa.limit = len;
+  sa.is_first = 1; sa.is_last = 1;
+  sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_ratio = shape.str_ratio; sa.row_cap = shape.row_cap;
+  sa.ntiles = (uint32_t)stream_tiles((uint32_t)(reinterpret_cast<uintptr_t>(d_in) & 15u), len, 1u, shape.tile_bytes);
+  sa.spin_limit_ns = c->spin_ns;
+  sa.opts = c->opt_flags;
+  sa.sep = aa.sep;
+  c->stats.tile_records = IT_THREADS; c->stats.tiles += sa.ntiles;
+  { pj_status st = ensure(c, &c->tiles, sa.ntiles * sizeof(ItemTile) + 512); if (st) return st; }
+  sa.ticket = (uint32_t*)c->tiles.p;
+  sa.tiles = (ItemTile*)((uint8_t*)c->tiles.p + 256);
+  sa.res = c->d_res;
+  for (uint32_t k = 0; k < NSLOT; ++k) sa.slot_cap[k] = pp.slot_cap[k];
+  sa.rec_cap = pp.rec_cap;
+  sa.plan = pp.plan;
+  sa.cols = pp.dcols;
+  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, sa.ntiles * sizeof(ItemTile) + 256, c->stream));
   stage.next(); /* stage 1: set-up */
-  switch (schema) {
-    case PJ_SCHEMA_PET: PJ_CUDA(c, tile_launch_1(&ta, (unsigned)ntiles, c->stream)); break;
-    case PJ_SCHEMA_ORDER: PJ_CUDA(c, tile_launch_2(&ta, (unsigned)ntiles, c->stream)); break;
-    case PJ_SCHEMA_USER: PJ_CUDA(c, tile_launch_3(&ta, (unsigned)ntiles, c->stream)); break;
-    default: PJ_CUDA(c, tile_launch_4(&ta, (unsigned)ntiles, c->stream)); break;
-  }
+  PJ_CUDA(c, item_launch(schema, &sa, c->stream));
   count_launch(c, 2);
-  stage.next(); /* stage 2: the tile kernel */
+  stage.next(); /* stage 2: the parse kernel */
   PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   PJ_CUDA(c, cudaGetLastError());
@@ -574,7 +561,8 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   out->doc_err_kind = 0; out->doc_err_off = 0;
   if (r.doc_err_off != ~0ull) { out->doc_err_kind = PJ_E_SYNTAX; out->doc_err_off = r.doc_err_off; }
   else if (r.first_opener == ~0ull || r.arr_final_s || r.arr_final_d != 0) { out->doc_err_kind = PJ_E_EOF; out->doc_err_off = len; }
-  const pj_status st = finish_columns(c, schema, len, pp, r.n_records, r.n_errors, total, !r.ok, out);
+  const pj_status st = finish_columns(c, schema, len, pp, r.n_records, r.n_errors, total, r.over != 0, out);
+  if (!st && r.n_records > 1000 && !c->tile_bytes_opt) c->avg_rec_bytes[schema] = (double)len / (double)r.n_records;
   if (st) return st;
   if (host_out) {
     for (int i = 0; i < pp.nneed; ++i) {
@@ -679,18 +667,15 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   for (auto& ev : c->ev_k1) { e = cudaEventCreate(&ev); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
   for (auto& ev : c->ev_done) { e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
   build_schema(&c->schema);
-  e = tile_init_1(&c->schema);
-  if (e == cudaSuccess) e = tile_init_2(&c->schema);
-  if (e == cudaSuccess) e = tile_init_3(&c->schema);
-  if (e == cudaSuccess) e = tile_init_4(&c->schema);
+  e = item_init_1(&c->schema);
+  if (e == cudaSuccess) e = item_init_2(&c->schema);
+  if (e == cudaSuccess) e = item_init_3(&c->schema);
+  if (e == cudaSuccess) e = item_init_4(&c->schema);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, WTILE_SMEM_BYTES);
 #ifdef PJ_WT_CARVEOUT
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile, cudaFuncAttributePreferredSharedMemoryCarveout, PJ_WT_CARVEOUT);
 #endif
   if (e != cudaSuccess) return fail_create(e, "cudaFuncSetAttribute");
-  build_schema(&c->schema);
-  e = cudaMemcpyToSymbol(c_schema, &c->schema, sizeof(Schema));
-  if (e != cudaSuccess) return fail_create(e, "cudaMemcpyToSymbol");
   *out = c;
   return PJ_OK;
 }

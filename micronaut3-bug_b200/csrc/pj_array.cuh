@@ -152,7 +152,7 @@ PJ_HD ArrState fn_apply(const ArrFn& f, ArrState in) {
  * `ws [ ... ] ws` (doc_bit, 64 = none) and the lowest opener (opener_bit, 64 = none). */
 struct WordMarks {
   uint64_t sep;
-  uint32_t doc_bit, opener_bit;
+  uint32_t doc_bit, opener_bit, n_openers;
 };
 PJ_HD WordMarks mark_word(const WordMasks& m, const WordEval& e, int32_t depth_in) {
   WordMarks r;
@@ -188,6 +188,7 @@ PJ_HD WordMarks mark_word(const WordMasks& m, const WordEval& e, int32_t depth_i
   r.sep = sep;
   r.doc_bit = bad ? ctz64a(bad) : 64u;
   r.opener_bit = openers ? ctz64a(openers) : 64u;
+  r.n_openers = popc64(openers);
   return r;
 }
 

@@ -148,7 +148,10 @@ static __global__ void __launch_bounds__(ARR_THREADS) k_arr_mark(const __grid_co
   const WordMarks k = mark_word(m, e, in.d);
   a.sep[w] = k.sep;
   if (k.doc_bit < 64) atomicMin(&a.res->doc_err_off, (unsigned long long)((w << 6) + k.doc_bit));
-  if (k.opener_bit < 64) atomicMin(&a.res->first_opener, (unsigned long long)((w << 6) + k.opener_bit));
+  if (k.opener_bit < 64) {
+    atomicMin(&a.res->first_opener, (unsigned long long)((w << 6) + k.opener_bit));
+    atomicAdd(&a.res->n_openers, k.n_openers);
+  }
 }
 
 template <bool WRITE>

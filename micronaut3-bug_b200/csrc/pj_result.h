@@ -1,0 +1,36 @@
+/*
+ * pj_result.h — the block of counters and flags the kernels leave for the host.
+ */
+#ifndef PJ_RESULT_H
+#define PJ_RESULT_H
+
+#include "pj_schema.h"
+
+namespace pj {
+
+/* Written by the kernels, read back by the host once per call. */
+struct DevResult {
+  unsigned long long n_records;
+  unsigned long long n_errors;
+  unsigned long long total[NSLOT];
+  unsigned long long out_bytes; /* writer: JSON bytes */
+  unsigned long long doc_err_off;
+  uint32_t doc_err_kind;
+  uint32_t ok;      /* every output fits its buffer */
+  uint32_t over;    /* stream kernel: some output does not fit its buffer */
+  uint32_t timeout; /* a bounded wait ran out */
+  uint32_t needs_escape; /* writer: some string byte of the columns has to be escaped (k_arena_flags) */
+  unsigned long long n_fast;  /* records decoded by the speculative pass alone */
+  unsigned long long phase_cycles[4]; /* tile kernel, summed over blocks: staging, tokenising, look-back, emit */
+  unsigned long long lookback_polls, lookback_rounds;
+  unsigned long long n_wide;       /* records walked by a whole warp */
+  unsigned long long n_wide_fast;  /* of those, finished by the word-at-a-time tokeniser (the rest: the exact parser) */
+  unsigned long long wide_cycles[2]; /* cycles the blocks spent in the warps' size pass / emit pass, summed over blocks */
+  uint32_t n_openers;              /* array framing: `[` at depth 0 (a clean document has one) */
+  unsigned long long first_opener; /* array framing: offset of the first `[` at depth 0 */
+  uint32_t arr_final_s;            /* array framing: the input ends inside a string */
+  int32_t arr_final_d;             /* array framing: nesting depth at the end of the input */
+};
+
+}  // namespace pj
+#endif

@@ -42,15 +42,15 @@ struct StreamGeom {
   uint32_t copy_bytes; /* multiple of 16: what the bulk copy brings */
   uint32_t to_limit;   /* the window reaches the end of the readable bytes */
 };
-PJ_HD StreamGeom stream_geom(uint32_t mis, uint64_t len, uint64_t limit, uint32_t tile_bytes, uint32_t tile) {
+PJ_HD StreamGeom stream_geom(uint32_t mis, uint64_t len, uint64_t limit, uint32_t tile_bytes, uint32_t tile, uint32_t win_bytes = ST_WIN_BYTES) {
   StreamGeom g;
   g.mis = mis;
   g.v0 = (uint64_t)tile * tile_bytes;
   g.vlimit = limit + mis;
   const uint64_t vlen = len + mis; /* line feeds below it are the shard's own */
   const uint64_t left = g.vlimit > g.v0 ? g.vlimit - g.v0 : 0;
-  g.hi_valid = left < ST_WIN_BYTES ? (uint32_t)left : ST_WIN_BYTES;
-  g.to_limit = left <= ST_WIN_BYTES;
+  g.hi_valid = left < win_bytes ? (uint32_t)left : win_bytes;
+  g.to_limit = left <= win_bytes;
   g.copy_bytes = (g.hi_valid + 15u) & ~15u;
   g.lo_valid = tile == 0 ? mis : 0;
   const uint64_t own = vlen > g.v0 ? vlen - g.v0 : 0;
