@@ -268,30 +268,32 @@ pj_status finish_columns(pj_ctx* c, uint32_t schema, uint64_t len, const ParsePl
 }
 
 /* How a call's input is cut into tiles. The result of a call does not depend on it. */
-struct TileShape { uint32_t tile_bytes, win_bytes, str_ratio, row_cap; };
+struct TileShape { uint32_t tile_bytes, win_bytes, str_words, row_cap; };
 uint32_t item_stride(uint32_t schema) {
   return schema == PJ_SCHEMA_PET ? ItStride<1>::n : (schema == PJ_SCHEMA_ORDER ? ItStride<2>::n : (schema == PJ_SCHEMA_USER ? ItStride<3>::n : ItStride<4>::n));
 }
 TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   static const double dflt[5] = {0, 300, 146, 190, 230};
-  static constexpr uint32_t BUDGET = 69 * 1024; /* dynamic shared memory that lets three blocks share an SM */
+  /* dynamic shared memory that lets IT_BLOCKS blocks share an SM (228 KB, 1 KB of which every block costs) */
+  static constexpr uint32_t BUDGET = (228u * 1024u) / IT_BLOCKS - 1024u - (uint32_t)sizeof(ItemShared) - 256u;
   const double avg = c->avg_rec_bytes[schema] > 0 ? c->avg_rec_bytes[schema] : dflt[schema];
   TileShape t;
   /* room behind the tile for its last records: 13 average records reach the longest ones of a skewed distribution */
   uint32_t slack = (uint32_t)(avg * 13);
   slack = (slack < 4096 ? 4096u : (slack > 28672 ? 28672u : slack)) & ~15u;
-  t.str_ratio = 43; /* a string per six bytes */
+  uint32_t per_word = 8; /* window bytes per word for strings */
   uint64_t tile = (uint64_t)(avg * 190); /* at most 256 records */
   if (tile > 32768) tile = 32768;
-  if (len / 296 < tile) { tile = len / 296; if (tile < 4096) tile = 4096; t.str_ratio = 128; } /* few tiles: one for every SM's two halves, and room enough */
+  if (len / 296 < tile) { tile = len / 296; if (tile < 4096) tile = 4096; per_word = 2; } /* few tiles: one for every SM's two halves, and room enough */
   if (c->tile_bytes_opt) { tile = c->tile_bytes_opt; if (tile < ST_MIN_TILE_BYTES) tile = ST_MIN_TILE_BYTES; if (tile > 32768) tile = 32768; }
   for (;;) {
     t.tile_bytes = (uint32_t)(tile & ~31ull);
     if (t.tile_bytes < ST_MIN_TILE_BYTES) t.tile_bytes = ST_MIN_TILE_BYTES;
     t.win_bytes = t.tile_bytes + slack;
+    t.str_words = t.win_bytes / per_word;
     const double recs = (double)t.tile_bytes / avg * 1.4 + 40;
     t.row_cap = recs > 272 ? 272u : (uint32_t)recs;
-    if (t.str_ratio > 100 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_ratio, t.row_cap, item_stride(schema)).total <= BUDGET) return t;
+    if (per_word == 2 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_words, t.row_cap, item_stride(schema)).total <= BUDGET) return t;
     tile -= 1024;
   }
 }
@@ -408,7 +410,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
       sa.is_first = p == 0 ? (uint32_t)is_first : 0u;
       sa.is_last = (is_last && sl == rest) ? 1u : 0u;
     }
-    sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_ratio = shape.str_ratio; sa.row_cap = shape.row_cap;
+    sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_words = shape.str_words; sa.row_cap = shape.row_cap;
     sa.ntiles = (uint32_t)nt[p];
     sa.spin_limit_ns = c->spin_ns;
     sa.opts = c->opt_flags;
@@ -527,7 +529,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   const TileShape shape = pick_tile_shape(c, schema, len);
   sa.in = d_in; sa.len = len; sa.limit = len;
   sa.is_first = 1; sa.is_last = 1;
-  sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_ratio = shape.str_ratio; sa.row_cap = shape.row_cap;
+  sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_words = shape.str_words; sa.row_cap = shape.row_cap;
   sa.ntiles = (uint32_t)stream_tiles((uint32_t)(reinterpret_cast<uintptr_t>(d_in) & 15u), len, 1u, shape.tile_bytes);
   sa.spin_limit_ns = c->spin_ns;
   sa.opts = c->opt_flags;

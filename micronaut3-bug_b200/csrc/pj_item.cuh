@@ -1,30 +1,29 @@
 /*
  * pj_item.cuh — k_parse_items<SCHEMA>: JSON records to typed columns in one kernel and one pass over HBM, with the work
- * spread over STRINGS instead of records.
+ * spread over bytes, strings and fields instead of records.
  *
- * One thread block = one tile of the input, staged in shared memory by one bulk copy. Its warps take equal byte ranges
- * of the tile; a warp owns the records whose preceding separator (the line feed; in array framing a bit of the
- * separator bitmap) lies in its range, and follows its last one to its end.
+ * One thread block = one tile of the input, staged in shared memory by one bulk copy. A tile owns the lines (in array
+ * framing: the extents) whose preceding separator lies in it and follows its last one to its end. The steps:
  *
- *  1. item_index: 32 bytes per lane and step. Byte-parallel masks of quotes and control characters give the positions
- *     of all quotes of the warp's records in order: string k = (open, close). Backslashes, bytes beyond ASCII and control
- *     characters take extra work only in the steps that hold one; strings with escapes are decoded in place.
- *  2. item_tokens: 32 strings per step, one per lane: a string and the gap behind it, up to the next string. The
- *     punctuation of a gap alone tells where in the record it stands (`}],` closes an element, its list and is
- *     followed by a key of the root; `,` and `:` leave the place as it is), so the object a string lies in is the one
- *     the nearest telling gap before it left: one ballot and one shuffle instead of a walk. Keys are looked up in a
- *     hash table, and the REFERENCE to the key's value goes to its place in the record's row. Nothing is parsed here and
- *     no lane waits for a longer record.
- *  3. item_values: one record (or list element) per lane: the references of a property are decoded by 32 lanes that all
- *     do the same (integers, enums, date-times), then what is required is checked.
- *  4. Counts per record are added up, ONE decoupled look-back over the earlier tiles gives the tile's place in every
- *     column and arena, and the columns are written.
+ *  1. item_index: 32 bytes per thread. Byte-parallel masks of quotes and control characters give the positions of all
+ *     quotes of the tile in order: string k = (open, close); and the lines: first byte and first string. Backslashes, bytes
+ *     beyond ASCII and control characters take extra work only where they are; strings with escapes are decoded in place.
+ *  2. item_walk: one line per thread. A record as a serialiser writes it is walked property by property; every string's end
+ *     is known, so nothing is scanned, and nothing is decoded either: REFERENCES to the values' text go to the line's row.
+ *  3. item_pack: the lines the walk did not recognise (blanks, another order of keys, null, errors), 32 strings at a time,
+ *     a string and the gap behind it per lane. The punctuation of a gap alone tells where in the record it stands (`}],`
+ *     closes an element, its list and is followed by a key of the root; `,` and `:` leave the place as it is), so the object a
+ *     string lies in is what the nearest telling gap before it left: one ballot and one shuffle instead of a walk. Keys are
+ *     looked up in a hash table.
+ *  4. item_value: groups of 32 lines and one field: the references are decoded by lanes that all do the same.
+ *  5. Counts per record are added up, ONE decoupled look-back over the earlier tiles gives the tile's place in every
+ *     column and arena, and the columns are written, again by groups of 32 lines.
  *
  * The steps detect every deviation from a valid record of the model; the common failures (wrong JSON type, unknown
  * literal, bad date-time, missing property, record ending inside a string) are reported with the exact parser's kind
  * and offset, because the smallest offset of a record's deviations is its first failure. Any other deviation sends the
- * record to the exact parser (pj_core.cuh); should that one accept the record (unknown keys with nested values, repeated keys,
- * ...), or does the tile not fit the shared memory laid out for it (a record longer than the window, many more records
+ * record to the exact parser (pj_core.cuh); should that one accept the record (unknown keys with nested values, repeated
+ * keys, ...), or does the tile not fit the shared memory laid out for it (a record longer than the window, many more lines
  * or strings than its bytes suggest), the block walks the tile with the exact parser alone (item_slow_tile).
  */
 #ifndef PJ_ITEM_CUH
@@ -40,19 +39,23 @@
 
 namespace pj {
 
+#ifndef PJ_IT_BLOCKS
+#define PJ_IT_BLOCKS 3 /* resident blocks per SM the kernel is compiled for */
+#endif
+static constexpr uint32_t IT_BLOCKS = PJ_IT_BLOCKS;
 static constexpr uint32_t IT_THREADS = 256;
 static constexpr uint32_t IT_WARPS = IT_THREADS / 32;
-static constexpr uint32_t IT_STEP = 1024;        /* bytes a warp indexes per step */
-static constexpr uint32_t IT_FRONT = 32;         /* bytes before the window that may be read (and mean nothing) */
-static constexpr uint32_t IT_PAD = IT_STEP + 64; /* ... and behind it */
-static constexpr uint32_t IT_MAX_RECS = 256;     /* records per tile */
-static constexpr uint32_t IT_RCHUNKS = IT_MAX_RECS / 32;
-static constexpr uint32_t IT_MAX_UNITS = 64;     /* groups of 32 list elements per tile and list */
-static constexpr uint32_t IT_MAX_STRS = 1024;    /* strings per warp */
-static constexpr uint32_t IT_MAX_WIN = 65536 - 64; /* window offsets are 16-bit */
-static constexpr uint32_t IT_ARR_SEP = 0x1E;     /* what the separators of array framing are replaced with in the window */
-
+static constexpr uint32_t IT_STEP = IT_THREADS * 32; /* bytes the block indexes per step */
+static constexpr uint32_t IT_FRONT = 32;             /* bytes before the window that may be read (and mean nothing) */
+static constexpr uint32_t IT_PAD = 64;               /* ... and behind it */
+static constexpr uint32_t IT_MAX_LINES = IT_THREADS; /* lines per tile */
+static constexpr uint32_t IT_MAX_STRS = 4096;        /* strings per tile */
+static constexpr uint32_t IT_MAX_SPECIAL = 1024;     /* strings per tile that need a closer look */
+static constexpr uint32_t IT_MAX_WIN = 65536 - 64;   /* window offsets are 16-bit */
+static constexpr uint32_t IT_SHORT = 8;              /* a list of up to this many elements is its line's lane's, a longer one the warp's */
 static constexpr uint32_t IT_MAX_DYN_SMEM = 200 * 1024; /* dynamic shared memory of a block */
+static constexpr uint32_t IT_NONE = 0xFFFFFFFFu;
+
 static constexpr uint32_t IT_NLB = 16;    /* look-back counters: the NSLOT counters and the record count */
 static constexpr uint32_t IT_REC = NSLOT; /* number of the record counter */
 static_assert(NSLOT + 1 == IT_NLB, "one more than counters");
@@ -69,9 +72,9 @@ struct ItemArgs {
   uint64_t len, limit, goff;
   uint32_t is_first, is_last;
   uint32_t tile_bytes, ntiles;
-  uint32_t win_bytes;  /* bytes staged per tile: the tile and what its last records may need behind it */
-  uint32_t str_ratio;  /* 32-bit words for strings per 256 bytes of text */
-  uint32_t row_cap;    /* record rows in shared memory */
+  uint32_t win_bytes;  /* bytes staged per tile: the tile and what its last record may need behind it */
+  uint32_t str_words;  /* 32-bit words for strings */
+  uint32_t row_cap;    /* rows of lines */
   uint32_t opts;       /* PJ_OPT_* bits that change a rule */
   unsigned long long spin_limit_ns;
   const uint64_t* sep; /* array framing: one bit per input byte, set for `[`, the commas and `]` that delimit records; else null */
@@ -93,44 +96,39 @@ struct ItemSlots {
   static constexpr uint32_t mask = ((hi > lo ? ((1u << hi) - (1u << lo)) : 0u)) | (1u << IT_REC);
   static constexpr uint32_t count = (hi > lo ? hi - lo : 0u) + 1u;
   static constexpr uint32_t nagg = (count + 2u) / 3u;
-  /* position of slot k among the used ones */
-  static PJ_CX uint32_t pos(uint32_t k) { return k == IT_REC ? count - 1u : k - lo; }
   static constexpr bool lists = SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED;
 };
 static_assert((ItemSlots<PJ_SCHEMA_MIXED>::nagg) <= 6, "packed totals fit");
 
 /* shared memory of a tile: what the dynamic part holds, from a 16-byte aligned base */
 struct ItemLayout { uint32_t win, strs, rows, total; };
-PJ_HD ItemLayout item_layout(uint32_t win_bytes, uint32_t str_ratio, uint32_t row_cap, uint32_t stride) {
+PJ_HD ItemLayout item_layout(uint32_t win_bytes, uint32_t str_words, uint32_t row_cap, uint32_t stride) {
   ItemLayout l;
   l.win = IT_FRONT;
   l.strs = (l.win + win_bytes + IT_PAD + 15u) & ~15u;
-  l.rows = l.strs + ((((win_bytes + 64u) * str_ratio) >> 8) + 2u * IT_WARPS + 4u) * 4u;
-  l.rows = (l.rows + 15u) & ~15u;
+  l.rows = (l.strs + str_words * 4u + 15u) & ~15u;
   l.total = l.rows + row_cap * stride * 4u;
   return l;
 }
 
-/* what a warp leaves about its range */
-struct ItemWarp {
-  uint32_t nstr, nterm, start, stop; /* strings, separators that end a line, first line, last separator */
-  uint32_t str0, words;              /* first of its words for strings, how many there are */
-  uint32_t nrec, nphoto, ntag;
-  uint32_t odd;                      /* bit 0: special strings, bit 1: records that end inside a string */
-  uint32_t row0;                     /* first row */
-};
 struct ItemShared {
   __align__(16) uint32_t key[IT_SLOTS][8];
-  uint32_t field[3][IT_SLOTS];
   __align__(16) ItGapEntry gap[IG_SLOTS];
-  ItemWarp w[IT_WARPS];
-  uint32_t special[IT_WARPS][IT_MAX_STRS / 32]; /* per string: it holds a backslash, a control character or a byte beyond ASCII ... */
-  uint32_t broken[IT_WARPS][IT_MAX_STRS / 32];  /* ... and is not a valid one */
-  uint16_t todo[IT_WARPS][64];
-  uint32_t csum[IT_NLB][IT_RCHUNKS]; /* record-level counters: sums per 32 records, then exclusive prefixes */
-  uint32_t usum[2][IT_MAX_UNITS];    /* string bytes per 32 list elements (list of strings, list of objects), then exclusive prefixes */
+  uint32_t field[3][IT_SLOTS];
+  uint32_t line[IT_MAX_LINES + 1];         /* window offset of a line's first byte | strings before it << 16 */
+  uint32_t special[IT_MAX_STRS / 32];      /* per string: it holds a backslash, a control character or a byte beyond ASCII ... */
+  uint32_t broken[IT_MAX_STRS / 32];       /* ... and is not a valid one */
+  uint32_t oddline[IT_MAX_LINES / 32];     /* lines with a string that was decoded in place or is not valid */
+  uint32_t oddmask[IT_WARPS];              /* lines the walk did not recognise */
+  uint16_t special_list[IT_MAX_SPECIAL];
+  uint8_t perm[IT_THREADS], cls[4][IT_WARPS]; /* mixed streams: lines by model */
+  uint32_t csum[IT_NLB][IT_WARPS];         /* counters: sums per 32 lines, then exclusive prefixes */
   uint32_t tot[IT_NLB], base[IT_NLB];
-  uint32_t ok, slow, bad, tile, next;
+  uint32_t wsum[2][IT_WARPS], wmin[3][IT_WARPS];
+  uint32_t nspecial, odd;                  /* odd: some record ends inside a string */
+  uint32_t nstr, nline, stop;              /* strings, lines, last separator */
+  uint32_t free_word;                      /* first free word behind the strings */
+  uint32_t ok, slow, tile, next, viol;
   unsigned long long mbar;
 };
 
@@ -268,6 +266,11 @@ __device__ __forceinline__ uint32_t item_mask32(const uint32_t* w, F f) {
   for (int k = 0; k < 4; ++k) m |= item_gather(f(w[2 * k]), f(w[2 * k + 1])) << (8 * k);
   return m;
 }
+__device__ __forceinline__ uint32_t item_mask_of(const uint32_t* f) {
+  const uint32_t g0 = __dp4a(f[1], 0x80402010u, __dp4a(f[0], 0x08040201u, 0u)), g1 = __dp4a(f[3], 0x80402010u, __dp4a(f[2], 0x08040201u, 0u));
+  const uint32_t g2 = __dp4a(f[5], 0x80402010u, __dp4a(f[4], 0x08040201u, 0u)), g3 = __dp4a(f[7], 0x80402010u, __dp4a(f[6], 0x08040201u, 0u));
+  return ((g0 + (g1 << 8)) >> 7) | ((g2 + (g3 << 8)) << 9); /* multiples of 128 below 2^15 each */
+}
 __device__ __forceinline__ uint32_t item_prefix_xor(uint32_t x) {
   x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8; x ^= x << 16;
   return x;
@@ -282,147 +285,165 @@ __device__ __forceinline__ uint32_t item_escaped(uint32_t bs, uint32_t carry) {
   return (even ^ (sum << 1)) & follows;
 }
 
-/* Positions of the quotes of the records this warp owns. False: the tile does not fit (or cannot be told apart this
- * way), the block has to take the other road. */
-template <bool ARR>
-__device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t warp, uint32_t lane, uint32_t tile) {
-  const uint32_t span = (((a.tile_bytes + IT_WARPS - 1) / IT_WARPS) + 31u) & ~31u;
-  const uint32_t lo = warp * span;
-  uint32_t hi = lo + span;
-  if (hi > g.own_end) hi = g.own_end;
-  bool started = !ARR && tile == 0 && warp == 0 && a.is_first && a.limit > 0;
-  uint32_t start = g.mis, stop = 0, nq = 0, nterm = 0, ecarry = 0;
-  bool done = false, fine = true;
-  uint32_t odd_bits = 0;
-  ItemWarp& W = sh.w[warp];
-  if (lane == 0) { W.nstr = 0; W.nterm = 0; W.start = 0; W.stop = 0; W.str0 = 0; W.words = 0; W.row0 = 0; W.nrec = 0; W.nphoto = 0; W.ntag = 0; W.odd = 0; }
-  if (!started && lo >= hi) return true;
+/* The strings and lines the tile owns. False (for every thread): the tile does not fit, the block has to take the other road.
+ * CAREFUL: some record ends inside a string; its separator then counts as the string's closing quote. */
+template <bool ARR, bool CAREFUL>
+__device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t tid, uint32_t tile) {
+  const uint32_t lane = tid & 31, warp = tid >> 5;
+  bool started = !ARR && tile == 0 && a.is_first && a.limit > 0, done = false, fine = true;
+  uint32_t start = g.mis, stop = 0, nq = 0, nline = 0, step = 0;
   const int32_t end_valid = (int32_t)g.hi_valid + (g.to_limit ? 1 : 0); /* the end of the input counts as a separator */
-  const uint32_t lt = (1u << lane) - 1u;
-  uint16_t* q16 = nullptr;
-  uint32_t str0 = 0, words = 0;
-  for (uint32_t o = lo; !done; o += IT_STEP) {
-    if ((int32_t)o >= end_valid) { fine = !started; break; } /* its last record runs out of the window */
-    if (!started && o >= hi) break;
-    const int32_t p0 = (int32_t)(o + 32u * lane);
+  uint16_t* q16 = reinterpret_cast<uint16_t*>(strs);
+  if (tid == 0 && started) sh.line[0] = start;
+  for (uint32_t o = 0; !done; o += IT_STEP, ++step) {
+    if ((int32_t)o >= end_valid) { fine = !started; break; } /* the last record runs out of the window */
+    if (!started && o >= g.own_end) break;
+    const int32_t p0 = (int32_t)(o + 32u * tid);
     uint32_t w[8];
-    {
+    if (p0 < end_valid) {
       const uint4* src = reinterpret_cast<const uint4*>(win + p0);
       const uint4 x = src[0], y = src[1];
       w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w; w[4] = y.x; w[5] = y.y; w[6] = y.z; w[7] = y.w;
-    }
-    const uint32_t vm = item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
-    uint32_t q = item_mask32(w, [](uint32_t x) { return ~((((x ^ 0x22222222u) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u; }) & vm;
-    uint32_t c = item_mask32(w, [](uint32_t x) { return ~(((x & 0x7F7F7F7Fu) + 0x60606060u) | x) & 0x80808080u; }) & vm;
-    uint32_t sp = 0; /* bit 7 of a byte set: some word has a backslash or a byte beyond ASCII there */
+    } else {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) sp |= ~(((w[k] ^ 0x5C5C5C5Cu) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w[k];
-    const bool has_sp = (sp & 0x80808080u) != 0;
-    /* separators */
-    uint32_t t = 0;
+      for (int k = 0; k < 8; ++k) w[k] = 0x41414141u;
+    }
+    /* Bytes below 0x23 are few: of them, bit 5 tells the printable ones from the control characters, and of the printable
+       ones ( space ! " ) bit 1 tells the quotes. Or-ed up over the words: backslashes, bytes beyond ASCII. */
+    uint32_t fq[8], fc[8], bs = 0, hb = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t x = w[k];
+      const uint32_t low = ~(((x & 0x7F7F7F7Fu) + 0x5D5D5D5Du) | x) & 0x80808080u;
+      const uint32_t printable = low & (x << 2);
+      fq[k] = printable & (x << 6);
+      fc[k] = low & ~(x << 2);
+      bs |= ~(((x ^ 0x5C5C5C5Cu) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu);
+      hb |= x;
+    }
+    uint32_t q = item_mask_of(fq);
+    const bool has_sp = ((bs | hb) & 0x80808080u) != 0;
+    uint32_t c = 0, t = 0; /* control characters, separators */
+    if (fc[0] | fc[1] | fc[2] | fc[3] | fc[4] | fc[5] | fc[6] | fc[7]) c = item_mask_of(fc);
+    const bool edge = !started || o + IT_STEP > g.own_end || (int32_t)(o + IT_STEP) > end_valid || o < g.lo_valid;
+    if (edge) {
+      const uint32_t vm = item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
+      q &= vm; c &= vm;
+    }
     if (ARR) {
-      const int64_t bit = (int64_t)g.v0 + p0 - (int64_t)g.mis; /* input offset of the lane's first byte */
+      const int64_t bit = (int64_t)g.v0 + p0 - (int64_t)g.mis; /* input offset of the thread's first byte */
       const int64_t nwords32 = (int64_t)((a.len + 31) >> 5);
       const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.sep);
       const int64_t i0 = bit >> 5; /* floor: the first tile may begin a few bytes before the input */
       const uint32_t b0 = i0 >= 0 && i0 < nwords32 ? sw[i0] : 0u, b1 = i0 + 1 >= 0 && i0 + 1 < nwords32 ? sw[i0 + 1] : 0u;
-      t = __funnelshift_r(b0, b1, (uint32_t)(bit & 31)) & vm;
+      t = __funnelshift_r(b0, b1, (uint32_t)(bit & 31)) & item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
       if (g.to_limit && (int32_t)g.hi_valid >= p0 && (int32_t)g.hi_valid < p0 + 32) t |= 1u << (g.hi_valid - (uint32_t)p0);
-      for (uint32_t m = t; m; m &= m - 1u) win[p0 + __ffs((int)m) - 1] = (uint8_t)IT_ARR_SEP;
-      c |= t; /* all of them count as control characters from here on */
     } else {
       for (uint32_t m = c; m; m &= m - 1u) {
         const uint32_t b = (uint32_t)__ffs((int)m) - 1u;
         if (win[p0 + b] == '\n') t |= 1u << b;
       }
     }
-    if (!started) {
-      const uint32_t cand = t & item_low((int32_t)hi - p0);
-      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cand != 0);
-      if (!bal) continue;
-      start = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)cand), __ffs((int)bal) - 1); /* behind the separator */
-      started = true;
+    uint32_t act = 0xFFFFFFFFu;
+    if (edge) { /* where the first own line begins and the last one ends */
+      const uint32_t own = item_low((int32_t)g.own_end - p0);
+      const uint32_t c0 = t & own, c1 = t & ~own;
+      const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, c0 != 0), b1 = __ballot_sync(0xFFFFFFFFu, c1 != 0);
+      const uint32_t m0 = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)c0), b0 ? __ffs((int)b0) - 1 : 0); /* behind the separator */
+      const uint32_t m1 = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)c1) - 1u, b1 ? __ffs((int)b1) - 1 : 0);
+      if (lane == 0) { sh.wmin[0][warp] = b0 ? m0 : IT_NONE; sh.wmin[1][warp] = b1 ? m1 : IT_NONE; }
+      __syncthreads();
+      uint32_t x0 = IT_NONE, x1 = IT_NONE;
+#pragma unroll
+      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t y0 = sh.wmin[0][k], y1 = sh.wmin[1][k]; x0 = y0 < x0 ? y0 : x0; x1 = y1 < x1 ? y1 : x1; }
+      if (!started && x0 != IT_NONE) { started = true; start = x0; if (tid == 0) sh.line[0] = start; }
+      if (!started) { __syncthreads(); continue; }
+      act = ~item_low((int32_t)start - p0);
+      if (x1 != IT_NONE) { stop = x1; done = true; act &= item_low((int32_t)stop + 1 - p0); }
+      t &= act; q &= act;
     }
-    if (!q16) {
-      str0 = ((start * a.str_ratio) >> 8) + 2u * warp;
-      q16 = reinterpret_cast<uint16_t*>(strs + str0);
-    }
-    uint32_t act = ~item_low((int32_t)start - p0);
-    {
-      const uint32_t cand = t & act & ~item_low((int32_t)hi - p0);
-      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cand != 0);
-      if (bal) {
-        stop = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)cand) - 1u, __ffs((int)bal) - 1);
-        done = true;
-        act &= item_low((int32_t)stop + 1 - p0);
-      }
-    }
-    t &= act; q &= act;
     const uint32_t ctl = c & act & ~t;
     uint32_t B = 0, H = 0;
-    const bool any_sp = __any_sync(0xFFFFFFFFu, has_sp);
-    if (any_sp) {
-      B = item_mask32(w, [](uint32_t x) { return item_eq4(x, 0x5C5C5C5Cu); }) & vm;
+    const bool warp_sp = __any_sync(0xFFFFFFFFu, has_sp || (lane == 0 && p0 > 0 && p0 <= end_valid && win[p0 - 1] == '\\'));
+    if (warp_sp) {
+      B = item_mask32(w, [](uint32_t x) { return item_eq4(x, 0x5C5C5C5Cu); });
       H = item_mask32(w, [](uint32_t x) { return x & 0x80808080u; }) & act;
-      if (__any_sync(0xFFFFFFFFu, B != 0) || ecarry) {
-        if (__any_sync(0xFFFFFFFFu, B == 0xFFFFFFFFu)) { fine = false; break; }
-        const uint32_t cout = (uint32_t)__clz((int)~B) & 1u; /* parity of the run of backslashes that ends the 32 bytes */
-        uint32_t cin = __shfl_up_sync(0xFFFFFFFFu, cout, 1);
-        if (lane == 0) cin = ecarry;
-        q &= ~item_escaped(B, cin);
-        ecarry = __shfl_sync(0xFFFFFFFFu, cout, 31);
+      if (edge) B &= item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
+      /* is the first byte escaped? An odd run of backslashes ends before it (looked at only where there is one) */
+      uint32_t cin = 0;
+      {
+        int32_t r = p0 - 1;
+        while (r >= (int32_t)g.lo_valid && r < end_valid && win[r] == '\\' && p0 - 1 - r < 4096) --r;
+        cin = (uint32_t)(p0 - 1 - r) & 1u;
+        if (p0 - 1 - r >= 4096) sh.slow = 1;
       }
+      q &= ~item_escaped(B, cin);
       B &= act;
-    } else if (ecarry) { if (lane == 0) q &= ~1u; ecarry = 0; }
-    /* order of the quotes; a record that ends inside a string gets its separator as the closing quote */
-    uint32_t ex, total;
-    for (;;) {
-      const uint32_t n = (uint32_t)__popc(q);
-      const uint32_t inc = warp_incl_scan(n);
-      ex = inc - n;
-      total = __shfl_sync(0xFFFFFFFFu, inc, 31);
-      uint32_t odd = 0;
-      for (uint32_t m = t & ~q; m; m &= m - 1u) { /* separators this lane sees with a string open */
-        const uint32_t low = (m & (0u - m)) - 1u;
-        if ((nq + ex + (uint32_t)__popc(q & low)) & 1u) { odd = m & (0u - m); break; }
-      }
-      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, odd != 0);
-      if (!bal) break;
-      if ((int)lane == __ffs((int)bal) - 1) q |= odd;
-      odd_bits |= 2u;
     }
-    /* strings that need a closer look */
-    if (__any_sync(0xFFFFFFFFu, (B | H | ctl) != 0)) {
-      odd_bits |= 1u;
-      const uint32_t instr = item_prefix_xor(q) ^ (((nq + ex) & 1u) ? 0xFFFFFFFFu : 0u);
-      for (uint32_t m = (B | H | ctl) & instr; m; m &= m - 1u) {
-        const uint32_t k = (nq + ex + (uint32_t)__popc(q & ((m & (0u - m)) - 1u))) >> 1;
-        if (k < IT_MAX_STRS) atomicOr(&sh.special[warp][k >> 5], 1u << (k & 31u));
+    /* order of the quotes (low half) and separators (high half) */
+    uint32_t at, total;
+    for (uint32_t round = 0;; ++round) {
+      const uint32_t n = (uint32_t)__popc(q) | ((uint32_t)__popc(t) << 16);
+      const uint32_t inc = warp_incl_scan(n);
+      uint32_t* ws = sh.wsum[CAREFUL ? 0 : (step & 1u)];
+      if (lane == 31) ws[warp] = inc;
+      __syncthreads();
+      at = inc - n; total = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t x = ws[k]; if (k < warp) at += x; total += x; }
+      uint32_t odd = 0;
+      for (uint32_t m = t & ~q; m; m &= m - 1u) { /* separators this thread sees with a string open */
+        const uint32_t low = (m & (0u - m)) - 1u;
+        if ((nq + (at & 0xFFFFu) + (uint32_t)__popc(q & low)) & 1u) { odd = m & (0u - m); break; }
       }
-      if (ARR) { /* a raw separator byte of our own choice in the text */
-        bool raw = false;
-        for (uint32_t m = ctl; m; m &= m - 1u) raw = raw || win[p0 + __ffs((int)m) - 1] == IT_ARR_SEP;
-        if (__any_sync(0xFFFFFFFFu, raw)) { fine = false; break; }
+      if (!CAREFUL) { if (odd) sh.viol = 1; break; }
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, odd != 0);
+      const uint32_t mine = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)odd), bal ? __ffs((int)bal) - 1 : 0);
+      if (lane == 0) sh.wmin[2][warp] = bal ? mine : IT_NONE;
+      __syncthreads();
+      uint32_t first = IT_NONE;
+#pragma unroll
+      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t y = sh.wmin[2][k]; first = y < first ? y : first; }
+      if (first == IT_NONE) break;
+      if (odd && (uint32_t)p0 + (uint32_t)__ffs((int)odd) == first) q |= odd;
+      __syncthreads();
+    }
+    const uint32_t q0 = nq + (at & 0xFFFFu); /* number of this thread's first quote */
+    /* strings that need a closer look */
+    if ((B | H | ctl) != 0) {
+      const uint32_t instr = item_prefix_xor(q) ^ ((q0 & 1u) ? 0xFFFFFFFFu : 0u);
+      for (uint32_t m = (B | H | ctl) & instr; m; m &= m - 1u) {
+        const uint32_t k = (q0 + (uint32_t)__popc(q & ((m & (0u - m)) - 1u))) >> 1;
+        if (k < IT_MAX_STRS) {
+          const uint32_t bit = 1u << (k & 31u);
+          if (!(atomicOr(&sh.special[k >> 5], bit) & bit)) {
+            const uint32_t i = atomicAdd(&sh.nspecial, 1u);
+            if (i < IT_MAX_SPECIAL) sh.special_list[i] = (uint16_t)k;
+          }
+        }
       }
     }
     {
-      const uint32_t upto = done ? stop + 1u : o + IT_STEP; /* the words of the bytes seen so far: ranges never share one */
-      words = ((upto * a.str_ratio) >> 8) + 2u * warp + 2u - str0;
-      if ((nq + total) / 2u + 1u > words || (nq + total) / 2u >= IT_MAX_STRS) { fine = false; break; }
-      uint32_t i = nq + ex;
-      for (uint32_t m = q; m; m &= m - 1u) q16[i++] = (uint16_t)((uint32_t)p0 + (uint32_t)__ffs((int)m) - 1u);
-    }
-    nq += total;
-    nterm += __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(t));
-  }
-  if (!fine) return false;
-  if (started && done) {
-    if (lane == 0) {
-      W.nstr = nq >> 1; W.nterm = nterm; W.start = start; W.stop = stop; W.str0 = str0; W.words = words; W.odd = odd_bits;
-      strs[str0 + (nq >> 1)] = (stop + 1u) | ((stop + 1u) << 16);
+      const uint32_t n = nq + (total & 0xFFFFu), nl = nline + (total >> 16);
+      if (n / 2u + 2u > a.str_words || n / 2u >= IT_MAX_STRS || nl > IT_MAX_LINES || nl > a.row_cap) { fine = false; break; }
+      uint16_t* d = q16 + q0;
+      for (uint32_t m = q; m; m &= m - 1u) *d++ = (uint16_t)((uint32_t)p0 + (uint32_t)__ffs((int)m) - 1u);
+      uint32_t i = nline + (at >> 16) + 1u;
+      for (uint32_t m = t; m; m &= m - 1u, ++i) { /* the line behind every separator */
+        const uint32_t bit = m & (0u - m);
+        sh.line[i] = ((uint32_t)p0 + (uint32_t)__ffs((int)m)) | (((q0 + (uint32_t)__popc(q & (bit | (bit - 1u)))) >> 1) << 16);
+      }
+      nq = n; nline = nl;
     }
   }
-  return true;
+  if (tid == 0) {
+    const bool any = fine && started && done;
+    sh.nstr = any ? nq >> 1 : 0u; sh.nline = any ? nline : 0u; sh.stop = stop;
+    sh.free_word = (any ? nq >> 1 : 0u) + 1u;
+    if (any) strs[nq >> 1] = (stop + 1u) | ((stop + 1u) << 16);
+    if (CAREFUL) sh.odd = 1;
+  }
+  return fine;
 }
 
 /* One string that holds a backslash, a control character or a byte beyond ASCII: decoded in place (the decoded text is
@@ -496,342 +517,26 @@ static __device__ __noinline__ bool item_decode_string(uint8_t* win, uint32_t op
   }
   return true;
 }
-/* the strings of a warp that item_index() marked, 32 at a time */
-__device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t warp, uint32_t lane) {
-  if (!(sh.w[warp].odd & 1u)) return;
-  const uint32_t nstr = sh.w[warp].nstr;
-  uint32_t* pairs = strs + sh.w[warp].str0;
-  const uint32_t nw = (nstr + 31u) >> 5; /* <= 32 */
-  const uint32_t mine = lane < nw ? sh.special[warp][lane] : 0u;
-  if (!__any_sync(0xFFFFFFFFu, mine != 0)) return;
-  uint32_t have = 0;
-  for (uint32_t k = 0; k < nw; ++k) {
-    const uint32_t bits = __shfl_sync(0xFFFFFFFFu, mine, (int)k);
-    if ((bits >> lane) & 1u) sh.todo[warp][have + (uint32_t)__popc(bits & ((1u << lane) - 1u))] = (uint16_t)(32u * k + lane);
-    have += (uint32_t)__popc(bits);
-    __syncwarp();
-    if (have >= 32u || k + 1 == nw) {
-      uint32_t at = 0;
-      while (have - at >= 32u || (k + 1 == nw && at < have)) {
-        const uint32_t n = have - at < 32u ? have - at : 32u;
-        if (lane < n) {
-          const uint32_t s = sh.todo[warp][at + lane];
-          const uint32_t pr = pairs[s];
-          uint32_t nc, moved;
-          if (!item_decode_string(win, pr & 0xFFFFu, pr >> 16, a.opts, &nc, &moved)) atomicOr(&sh.broken[warp][s >> 5], 1u << (s & 31u));
-          else pairs[s] = (pr & 0xFFFFu) | (nc << 16);
-          if (!moved) atomicAnd(&sh.special[warp][s >> 5], ~(1u << (s & 31u))); /* plain after all: positions are the input's */
-        }
-        at += n;
-      }
-      __syncwarp();
-      const uint32_t rest = have - at;
-      const uint32_t keep = lane < rest ? sh.todo[warp][at + lane] : 0u;
-      __syncwarp();
-      if (lane < rest) sh.todo[warp][lane] = (uint16_t)keep;
-      have = rest;
-      __syncwarp();
-    }
+/* The strings item_index() marked, one per thread. */
+__device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh, uint8_t* win, uint32_t* pairs, uint32_t tid) {
+  for (uint32_t i = tid; i < sh.nspecial; i += IT_THREADS) {
+    const uint32_t k = sh.special_list[i], pr = pairs[k];
+    uint32_t nc, moved;
+    const bool ok = item_decode_string(win, pr & 0xFFFFu, pr >> 16, a.opts, &nc, &moved);
+    if (ok) pairs[k] = (pr & 0xFFFFu) | (nc << 16);
+    if (ok && !moved) { atomicAnd(&sh.special[k >> 5], ~(1u << (k & 31u))); continue; } /* plain after all: positions are the input's */
+    if (!ok) atomicOr(&sh.broken[k >> 5], 1u << (k & 31u));
+    uint32_t lo = 0, hi = sh.nline; /* its line: the last one that begins at or before it and has a string */
+    while (lo + 1u < hi) { const uint32_t mid = (lo + hi) >> 1; if (sh.line[mid] >> 16 <= k) lo = mid; else hi = mid; }
+    atomicOr(&sh.oddline[lo >> 5], 1u << (lo & 31u));
   }
 }
 
-/* ---- 2. tokens ------------------------------------------------------------------------------------------------ */
 __device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
   Win w;
   w.s = win; w.w0 = 0;
   return wpeek4(w, p);
 }
-__device__ __forceinline__ void item_error(uint32_t* row, uint32_t pos, uint32_t kind) { atomicMin(&row[IW_ERR], (pos << 8) | kind); }
-/* A scalar token that belongs to no property: only what is cheap to see as valid (integers, literals) passes. */
-static __device__ __noinline__ bool item_plain_scalar(const uint8_t* win, uint32_t s, uint32_t n) {
-  if (n == 4 && (item_peek4(win, s) == 0x65757274u || item_peek4(win, s) == 0x6C6C756Eu)) return true;
-  if (n == 5 && win[s] == 'f' && item_peek4(win, s + 1) == 0x65736C61u) return true;
-  uint32_t i = win[s] == '-' ? 1u : 0u;
-  if (i >= n || (win[s + i] == '0' && i + 1 < n)) return false;
-  for (; i < n; ++i) if (win[s + i] - (uint32_t)'0' > 9u) return false;
-  return true;
-}
-
-/* A gap as the tables know it, and the places in it that matter. */
-struct ItemView {
-  uint32_t desc;              /* ItGap, 0: not one of the texts */
-  uint32_t vpos, vend;        /* first byte of the value behind the colon, end of a number or literal */
-  uint32_t last_sep, nsep;    /* the separator that ends the record: its last byte, how many there are (blank lines) */
-  uint32_t clpos;             /* the record's closing brace */
-};
-template <bool ARR>
-__device__ __forceinline__ bool item_blank(uint32_t x) { return x == ' ' || x == '\t' || x == '\r' || (ARR && x == '\n'); }
-template <bool ARR>
-__device__ __forceinline__ uint32_t item_gap_find(const ItemShared& sh, uint32_t lo, uint32_t hi, uint32_t len) {
-  const ItGapEntry e = sh.gap[it_gap_hash(lo, hi, ARR)];
-  return e.lo == lo && e.hi == hi && e.len == len ? e.desc : 0u;
-}
-/* A gap with blanks: its text is put together byte by byte, numbers and literals are skipped. */
-template <bool ARR>
-__device__ __forceinline__ void item_gap_spaced(const ItemShared& sh, const uint8_t* win, uint32_t from, uint32_t b, ItemView& v) {
-  constexpr uint32_t T = ARR ? IT_ARR_SEP : (uint32_t)'\n';
-  Win w;
-  w.s = win; w.w0 = 0;
-  uint64_t text = 0;
-  uint32_t n = 0, p = from, brace = 0, last = 0;
-  v.nsep = 0; v.vpos = b; v.vend = 0; v.last_sep = 0; v.clpos = 0;
-  while (p < b && n <= 8) {
-    uint32_t c = win[p];
-    if (item_blank<ARR>(c)) { ++p; continue; }
-    if (n == 1) v.vpos = p;
-    if (c - (uint32_t)'0' <= 9u || c == '-' || (c | 0x20u) - (uint32_t)'a' <= 25u) {
-      ++p;
-      for (;;) {
-        const uint64_t m = swar_nondigit(wpeek8(w, p));
-        if (!m) { p += 8; continue; }
-        p += ctz64(m) >> 3;
-        const uint32_t x = win[p];
-        if ((x | 0x20u) - (uint32_t)'a' <= 25u || x == '.' || x == '+' || x == '-') { ++p; continue; }
-        break;
-      }
-      v.vend = p;
-      c = '0';
-    } else {
-      if (c == '}') brace = p;
-      if (c == T) {
-        v.last_sep = p; ++v.nsep;
-        if (last == T) { ++p; continue; } /* a blank line */
-        v.clpos = brace;
-      }
-      ++p;
-    }
-    last = c;
-    if (n < 8) text |= (uint64_t)c << (8 * n);
-    ++n;
-  }
-  v.desc = n <= 8 && p == b ? item_gap_find<ARR>(sh, (uint32_t)text, (uint32_t)(text >> 32), n) : 0u;
-}
-template <int SCHEMA, bool ARR>
-__device__ __forceinline__ bool item_tokens(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, uint32_t* strs, uint32_t* rows, uint32_t warp, uint32_t lane) {
-  constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
-  constexpr uint32_t T = ARR ? IT_ARR_SEP : (uint32_t)'\n';
-  ItemWarp& W = sh.w[warp];
-  const uint32_t nstr = W.nstr, start = W.start, stop = W.stop, row0 = W.row0, odd = W.odd;
-  uint32_t* pairs = strs + W.str0;
-  uint32_t* photo_end = pairs + W.words; /* list strings are kept from the end of the warp's words downwards */
-  const uint32_t lt = (1u << lane) - 1u, le = (2u << lane) - 1u; /* lane 31: 2 << 31 wraps to 0, so all ones */
-  if (W.nterm == 0) return true;
-  for (uint32_t k = lane; k < W.nterm; k += 32) { rows[(row0 + k) * STRIDE + IW_FLAGS] = 0; rows[(row0 + k) * STRIDE + IW_ERR] = IE_NONE; }
-  bool slow = false;
-  if (nstr == 0) { /* no string at all: blank lines, or records for the other road */
-    uint32_t seen = 0, seps = 0;
-    for (uint32_t p = start + lane; p <= stop; p += 32) {
-      const uint32_t x = win[p];
-      if (x == T) seps += p < g.hi_valid; else if (!item_blank<ARR>(x)) seen = 1;
-    }
-    seps = __reduce_add_sync(0xFFFFFFFFu, seps);
-    return !__any_sync(0xFFFFFFFFu, seen != 0) && !(ARR && seps) && (ARR || a.is_last || stop < g.hi_valid);
-  }
-  uint32_t seps = 0; /* separators met */
-  __syncwarp();
-  /* what precedes the first string: blank lines and an opening brace */
-  {
-    uint32_t err = 0, first = start, bad = 0, n = 0;
-    if (lane == 0) {
-      uint32_t p = start, brace = 0;
-      const uint32_t e = pairs[0] & 0xFFFFu;
-      for (; p < e; ++p) {
-        const uint32_t x = win[p];
-        if (x == T && !ARR && !brace) { if (err) bad = 1; first = p + 1u; ++n; }
-        else if (x == T) bad = 1;
-        else if (x == '{' && !brace && !err) brace = 1;
-        else if (!item_blank<ARR>(x)) err = 1;
-      }
-      if (!brace) err = 1;
-      reinterpret_cast<uint16_t*>(&rows[row0 * STRIDE + IW_POS])[0] = (uint16_t)first;
-      if (err) item_error(&rows[row0 * STRIDE], first, IE_REFUSED);
-    }
-    slow = __any_sync(0xFFFFFFFFu, bad != 0);
-    seps = n; /* of lane 0 */
-  }
-  uint32_t st = IS_ROOT, rec = 0, nP = 0, nT = 0, pk = 0;
-  for (uint32_t k0 = 0; k0 < nstr; k0 += 32) {
-    const uint32_t k = k0 + lane;
-    const bool live = k < nstr;
-    const uint32_t pr = pairs[live ? k : nstr], nx = pairs[live ? k + 1u : nstr];
-    const uint32_t open = pr & 0xFFFFu, close = pr >> 16, b = nx & 0xFFFFu;
-    const bool trunc = (odd & 2u) && live && win[close] == T;
-    const uint32_t from = trunc ? close : close + 1u;
-    __syncwarp(); /* every lane has its pairs: what lies before k0 + 32 may be overwritten */
-
-    /* ---- the gap behind the string ---- */
-    ItemView v;
-    v.vpos = b; v.vend = 0;
-    {
-      /* without blanks: the bytes themselves, or `:0` and what follows the number (found from the gap's end) */
-      Win w;
-      w.s = win; w.w0 = 0;
-      const uint32_t n = b - from;
-      const uint64_t h = wpeek8(w, from);
-      uint32_t lo = (uint32_t)h, hi = (uint32_t)(h >> 32);
-      const uint32_t c0 = lo & 0xFFu, c1 = (lo >> 8) & 0xFFu;
-      if (n < 8u) {
-        const uint64_t m = (1ull << (8u * n)) - 1ull;
-        lo &= (uint32_t)m; hi &= (uint32_t)(m >> 32);
-      }
-      uint32_t len = n;
-      bool fits = n <= 8u;
-      if (c0 == ':' && n > 1u) v.vpos = from + 1u;
-      if (c0 == ':' && n > 2u && (c1 - (uint32_t)'0' <= 9u || c1 == '-' || c1 - (uint32_t)'a' <= 25u)) {
-        const uint64_t t = wpeek8(w, b - 8u);
-        const uint32_t tl = (uint32_t)t, th = (uint32_t)(t >> 32);
-        /* bytes 0x30-0x3F and 0x60-0x6F: digits, and the letters a literal ends with */
-        const uint32_t ah = (th ^ 0x30303030u) & 0xF0F0F0F0u, bh = (th ^ 0x60606060u) & 0xF0F0F0F0u;
-        const uint32_t al = (tl ^ 0x30303030u) & 0xF0F0F0F0u, bl = (tl ^ 0x60606060u) & 0xF0F0F0F0u;
-        const uint32_t zh = (~((ah & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | ah) | ~((bh & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | bh)) & 0x80808080u;
-        const uint32_t zl = (~((al & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | al) | ~((bl & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | bl)) & 0x80808080u;
-        const uint32_t tail = zh ? (uint32_t)__clz((int)zh) >> 3 : 4u + ((uint32_t)__clz((int)zl) >> 3); /* bytes behind the last of them */
-        v.vend = b - tail;
-        fits = tail >= 1u && tail <= 6u;
-        len = tail + 2u;
-        const uint64_t x = (t >> (8u * (8u - (fits ? tail : 1u)))) << 16;
-        lo = (uint32_t)x | (uint32_t)':' | ((uint32_t)'0' << 8); hi = (uint32_t)(x >> 32);
-      }
-      v.desc = fits ? item_gap_find<ARR>(sh, lo, hi, len) : 0u;
-      const uint32_t brace = (v.desc & ItGap::BRACE) ? 1u : 0u;
-      v.last_sep = b - 1u - brace; v.clpos = v.last_sep - 1u;
-      v.nsep = (v.desc & ItGap::ENDS) ? 1u : 0u;
-    }
-    bool next_bad = false;
-    if (live && v.desc == 0 && !trunc) {
-      item_gap_spaced<ARR>(sh, win, from, b, v);
-      /* Blank lines between records are none. But in array framing an extent without a value is a record (only the end of the
-         input follows the closing bracket), and so is a blank line that the readable bytes cut off. */
-      if (v.desc && v.nsep > 1u) slow = slow || (ARR ? !(v.nsep == 2u && v.last_sep >= g.hi_valid) : (v.last_sep >= g.hi_valid && !a.is_last));
-    }
-    if (live && v.desc && (v.desc & ItGap::ENDS)) {
-      if (!(v.desc & ItGap::BRACE) != (k + 1u == nstr)) v.desc = 0; /* a brace opens the next record, if there is one */
-      if (!a.is_last && v.last_sep >= g.hi_valid) v.desc = 0;       /* the readable bytes end here, the stream does not */
-    }
-    const bool ok = live && v.desc != 0;
-    if (live && !ok) { /* a record that ends inside this string, or no valid record: they have to be kept apart all the same */
-      uint32_t n = 0;
-      for (uint32_t p = from; p < b; ++p) if (win[p] == T) { ++n; v.last_sep = p; }
-      if (n > 1u) slow = true;
-      v.nsep = n; v.vend = 0; v.clpos = 0;
-      if (n && k + 1u != nstr) { /* does the next record begin as it should? */
-        uint32_t p = v.last_sep + 1u;
-        while (p < b && item_blank<ARR>(win[p])) ++p;
-        next_bad = true;
-        if (win[p] == '{') { ++p; while (p < b && item_blank<ARR>(win[p])) ++p; next_bad = p != b; }
-      }
-      /* trunc: nothing may stand between the string and its separator; the gap begins with it */
-      v.desc = ItGap::make(IV_NONE, 15, IS_ROOT, n != 0, n != 0, false, false, false);
-    }
-    const uint32_t d = v.desc, vk = ItGap::vk(d);
-    const bool telling = live && (d & ItGap::TELLS), ends = live && (d & ItGap::ENDS), newelem = live && (d & ItGap::ELEM);
-    bool iskey = live && (d & ItGap::KEY);
-
-    /* ---- the object the string lies in: what the nearest telling gap before it left ---- */
-    const uint32_t NI = __ballot_sync(0xFFFFFFFFu, telling);
-    const uint32_t pm = NI & lt;
-    const uint32_t from_lane = __shfl_sync(0xFFFFFFFFu, ItGap::out(d), pm ? 31 - __clz((int)pm) : 0);
-    const uint32_t s = pm ? from_lane : st;
-    const uint32_t RN = __ballot_sync(0xFFFFFFFFu, ends);
-    const uint32_t myrec = rec + (uint32_t)__popc(RN & lt);
-    const uint32_t PK = __ballot_sync(0xFFFFFFFFu, iskey && vk == IV_STR);
-    const bool isval = lane ? (PK >> (lane - 1)) & 1u : pk != 0;
-    const bool iselem = live && !isval && s == IS_LIST && !iskey;
-    const uint32_t EL = __ballot_sync(0xFFFFFFFFu, iselem);
-    const uint32_t NE = __ballot_sync(0xFFFFFFFFu, newelem);
-    const bool inrow = live && myrec < W.nterm; /* always: every record ends at a separator of its own */
-    uint32_t* row = rows + (row0 + (inrow ? myrec : 0u)) * STRIDE;
-    const uint32_t need = ItGap::need(d);
-    const bool role_ok = isval ? !iskey : (s == IS_LIST ? !iskey : (iskey || trunc));
-    if (inrow) {
-      if (trunc) { item_error(row, close, (!a.is_last && close >= g.hi_valid) ? IE_REFUSED : (uint32_t)PJ_E_EOF); if (!role_ok) item_error(row, open, IE_REFUSED); }
-      else if (!ok || !role_ok || !(need == 15u || need == s)) { item_error(row, close, IE_REFUSED); iskey = false; }
-      if (odd & 1u) {
-        if (((sh.special[warp][k >> 5] | sh.broken[warp][k >> 5]) >> (k & 31u)) & 1u) {
-          atomicOr(&row[IW_FLAGS], IF_MOVED);
-          if ((sh.broken[warp][k >> 5] >> (k & 31u)) & 1u) item_error(row, open - 1u, IE_REFUSED); /* before anything its text is judged by */
-        }
-      }
-      if (ends) { /* the record's last string */
-        reinterpret_cast<uint16_t*>(&row[IW_POS])[1] = (uint16_t)v.clpos;
-        row[IW_CUM] = (nP + (uint32_t)__popc(EL & le)) | ((nT + (uint32_t)__popc(NE & le)) << 16);
-        if (k + 1u != nstr && myrec + 1u < W.nterm) {
-          reinterpret_cast<uint16_t*>(&row[STRIDE + IW_POS])[0] = (uint16_t)(v.last_sep + 1u);
-          if (next_bad) item_error(row + STRIDE, v.last_sep + 1u, IE_REFUSED);
-        }
-      }
-      if (iselem) {
-        const uint32_t i = nP + (uint32_t)__popc(EL & lt);
-        if (nstr + 1u + i < W.words) photo_end[-(int32_t)i - 1] = (open + 1u) | ((close - open - 1u) << 16);
-        else slow = true;
-      }
-    } else iskey = false;
-    if (NE) {
-      if (newelem) {
-        const uint32_t t = nT + (uint32_t)__popc(NE & lt);
-        if (3u * t + 3u <= k0 + 32u && 3u * t + 3u <= nstr) {
-          pairs[3u * t] = 0; pairs[3u * t + 1] = 0; pairs[3u * t + 2] = (row0 + myrec) << 16;
-        } else slow = true;
-      }
-      __syncwarp();
-    }
-    /* ---- keys ---- */
-    if (iskey && !slow) {
-      const uint32_t n = close - open - 1u;
-      const uint32_t* kw = reinterpret_cast<const uint32_t*>(win) + ((open + 1u) >> 2);
-      const uint32_t ksh = ((open + 1u) & 3u) * 8u;
-      const uint32_t y0 = kw[0], y1 = kw[1], y2 = kw[2], y3 = kw[3], y4 = kw[4];
-      const uint32_t x0 = __funnelshift_r(y0, y1, ksh), x1 = __funnelshift_r(y1, y2, ksh), x2 = __funnelshift_r(y2, y3, ksh), x3 = __funnelshift_r(y3, y4, ksh);
-      const uint32_t slot = it_hash(x0 & 0xFFFFu, n, IT_MUL);
-      const uint4 kt = *reinterpret_cast<const uint4*>(&sh.key[slot][0]), km = *reinterpret_cast<const uint4*>(&sh.key[slot][4]);
-      uint32_t f = sh.field[s == IS_ROOT ? 0 : (s == IS_CHILD ? 1 : 2)][slot];
-      if ((((x0 ^ kt.x) & km.x) | ((x1 ^ kt.y) & km.y) | ((x2 ^ kt.z) & km.z) | ((x3 ^ kt.w) & km.w)) != 0 || n < 2u || n > 15u) f = 0;
-      const uint32_t vlen = v.vend - v.vpos;
-      if (!f) {
-        if (!(vk == IV_STR || (vk == IV_SCALAR && item_plain_scalar(win, v.vpos, vlen)))) item_error(row, close, IE_REFUSED);
-      } else {
-        const uint32_t kind = ItField::kind(f), vclose = nx >> 16;
-        const bool null = vk == IV_SCALAR && vlen == 4u && item_peek4(win, v.vpos) == 0x6C6C756Eu;
-        bool good = ((ItField::allowed(f) >> vk) & 1u) != 0;
-        const uint32_t len = vk == IV_STR ? vclose - b - 1u : vlen;
-        uint32_t ref = (vk == IV_STR ? b + 1u : v.vpos) | (len << 16);
-        if ((vk == IV_STR || vk == IV_SCALAR) && len >= 0x8000u) slow = true;
-        if (!good && !null) {
-          const uint32_t at = vk == IV_STR ? b : v.vpos, x = win[at];
-          if ((a.opts & PJ_OPT_COERCE_SCALARS) && ((vk == IV_STR && (kind == K_I64 || kind == K_I32 || kind == K_BOOL)) || (vk == IV_SCALAR && kind == K_STR))) {
-            if (vk == IV_STR) ref |= 0x80000000u;
-            else if (!item_plain_scalar(win, at, vlen)) item_error(row, at, IE_REFUSED);
-            good = true;
-          } else if ((kind == K_LIST_STR && vk == IV_ELEM) || (kind == K_LIST_OBJ && vk == IV_LIST) || (vk == IV_SCALAR && !(x == '-' || x - (uint32_t)'0' <= 9u || x == 't' || x == 'f')))
-            item_error(row, close, IE_REFUSED);
-          else item_error(row, at, PJ_E_TYPE);
-        }
-        if ((odd & 2u) && vk == IV_STR && win[vclose] == T) good = false; /* cut off: it reports that itself */
-        const uint32_t bit = 1u << ItField::bit(f), word = ItField::word(f);
-        if (s == IS_ELEM) {
-          const uint32_t t = nT + (uint32_t)__popc(NE & lt) - 1u;
-          const uint32_t old = atomicOr(&pairs[3u * t + 2u], bit | (good && !null ? bit << 4 : 0u));
-          if (old & bit) item_error(row, close, IE_REFUSED); /* repeated key */
-          if (good && !null) pairs[3u * t + word] = ref;
-        } else {
-          const uint32_t nm = SCHEMA == PJ_SCHEMA_MIXED && s == IS_ROOT ? (~ItField::models(f) & 7u) << IF_NOTMODEL : 0u;
-          const uint32_t old = atomicOr(&row[IW_FLAGS], bit | nm | (good && !null ? bit << IF_PRESENT : 0u));
-          if (old & bit) item_error(row, close, IE_REFUSED);
-          if (good && !null && kind <= K_DATETIME) row[word] = ref;
-        }
-      }
-    }
-    seps += v.nsep;
-    st = NI ? __shfl_sync(0xFFFFFFFFu, ItGap::out(d), 31 - __clz((int)NI)) : st;
-    rec += (uint32_t)__popc(RN); nP += (uint32_t)__popc(EL); nT += (uint32_t)__popc(NE);
-    pk = (PK >> 31) & 1u;
-    if (__any_sync(0xFFFFFFFFu, slow)) return false;
-  }
-  if (lane == 0) { W.nrec = rec; W.nphoto = nP; W.ntag = nT; }
-  return __reduce_add_sync(0xFFFFFFFFu, seps) == W.nterm; /* none was taken for part of a number */
-}
-
-/* ---- 3. values ------------------------------------------------------------------------------------------------ */
 /* -?(0|[1-9][0-9]*) in the n bytes at pos, within int64 / int32. Read from its end, eight digits at a time. */
 __device__ __forceinline__ bool item_int(const uint8_t* win, uint32_t pos, uint32_t n, bool is64, int64_t* out) {
   Win w;
@@ -871,6 +576,548 @@ __device__ __forceinline__ bool item_int(const uint8_t* win, uint32_t pos, uint3
 __device__ __forceinline__ bool item_true(const uint8_t* win, uint32_t pos, uint32_t n) { return n == 4 && item_peek4(win, pos) == 0x65757274u; }
 __device__ __forceinline__ bool item_false(const uint8_t* win, uint32_t pos, uint32_t n) { return n == 5 && win[pos] == 'f' && item_peek4(win, pos + 1) == 0x65736C61u; }
 
+__device__ __forceinline__ void item_error(uint32_t* row, uint32_t pos, uint32_t kind) { atomicMin(&row[IW_ERR], (pos << 8) | kind); }
+/* A scalar token that belongs to no property: only what is cheap to see as valid (integers, literals) passes. */
+static __device__ __noinline__ bool item_plain_scalar(const uint8_t* win, uint32_t s, uint32_t n) {
+  if (n == 4 && (item_peek4(win, s) == 0x65757274u || item_peek4(win, s) == 0x6C6C756Eu)) return true;
+  if (n == 5 && win[s] == 'f' && item_peek4(win, s + 1) == 0x65736C61u) return true;
+  uint32_t i = win[s] == '-' ? 1u : 0u;
+  if (i >= n || (win[s + i] == '0' && i + 1 < n)) return false;
+  for (; i < n; ++i) if (win[s + i] - (uint32_t)'0' > 9u) return false;
+  return true;
+}
+
+template <int E>
+PJ_CX int it_string_field() { /* the one string property of a flat object */
+  int at = -1;
+  for (int i = 0; i < CObj<E>::N; ++i) if (CObj<E>::f[i].kind == K_STR) at = i;
+  return at;
+}
+/* ---- 2. the walk ------------------------------------------------------------------------------------------------
+ * Records as a serialiser writes them: no blanks, properties in model order, any of the root's missing, embedded objects and
+ * those of lists whole, no null, no escapes. One line per thread, every string's end known from the index; references to the
+ * values' text go to the row. The first deviation ends a line's walk, and item_pack() looks at it. */
+struct ItemWalk {
+  const uint8_t* win;
+  const uint32_t* pairs;
+  uint32_t p;            /* at the brace or comma before the next member, or at the closing brace */
+  uint32_t k, kend, sep; /* next string, end of the line's strings, its separator */
+  bool ok;
+};
+/* is `"name":` of property I at p? */
+template <int OBJ, int I>
+__device__ __forceinline__ bool item_at_key(const uint8_t* win, uint32_t p) {
+  constexpr uint32_t n = FK<OBJ, I>::pat_len;
+  constexpr uint64_t t0 = FK<OBJ, I>::pat0, t1 = FK<OBJ, I>::pat1;
+  const uint32_t* a = reinterpret_cast<const uint32_t*>(win) + (p >> 2);
+  const uint32_t s = (p & 3u) * 8u;
+  const uint32_t y0 = a[0], y1 = a[1];
+  uint32_t d = __funnelshift_r(y0, y1, s) ^ (uint32_t)t0;
+  if constexpr (n < 4) d &= (1u << (8 * (n & 3u))) - 1u;
+  if constexpr (n > 4) {
+    const uint32_t y2 = a[2];
+    const uint32_t x = __funnelshift_r(y1, y2, s) ^ (uint32_t)(t0 >> 32);
+    d |= n >= 8 ? x : x & ((1u << (8 * (n & 3u))) - 1u);
+    if constexpr (n > 8) {
+      const uint32_t y3 = a[3];
+      const uint32_t z = __funnelshift_r(y2, y3, s) ^ (uint32_t)t1;
+      d |= n >= 12 ? z : z & ((1u << (8 * (n & 3u))) - 1u);
+      if constexpr (n > 12) {
+        const uint32_t v = __funnelshift_r(y3, a[4], s) ^ (uint32_t)(t1 >> 32);
+        d |= n >= 16 ? v : v & ((1u << (8 * (n & 3u))) - 1u);
+      }
+    }
+  }
+  return d == 0;
+}
+/* the flat object E at position at: `{"a":1,"b":"c"}`, all of its properties; references to its values in ref[]; returns the
+ * position behind its brace */
+template <int E, int I = 0>
+__device__ __forceinline__ uint32_t item_walk_flat(ItemWalk& f, uint32_t at, uint32_t* ref) {
+  if constexpr (I == 0) f.ok = f.ok && f.win[at] == '{';
+  if constexpr (I < CObj<E>::N) {
+    constexpr uint32_t kind = CObj<E>::f[I].kind;
+    static_assert(kind == K_I64 || kind == K_I32 || kind == K_STR, "flat objects: integers and strings");
+    f.ok = f.ok && item_at_key<E, I>(f.win, at + 1u);
+    const uint32_t v = at + 1u + FK<E, I>::pat_len;
+    f.k++;
+    const uint32_t nx = f.pairs[f.k < f.kend ? f.k : f.kend];
+    uint32_t end;
+    if constexpr (kind == K_STR) {
+      f.ok = f.ok && f.k < f.kend && (nx & 0xFFFFu) == v;
+      end = (nx >> 16) + 1u;
+      ref[I] = (v + 1u) | ((end - v - 2u) << 16);
+      f.ok = f.ok && end - v < 0x1000u; /* a length that fits its row */
+      f.k++;
+    } else {
+      static_assert(I + 1 < CObj<E>::N, "an integer is followed by another property");
+      end = (nx & 0xFFFFu) - 1u; /* the comma before the next key */
+      f.ok = f.ok && f.k < f.kend && end > v && end - v < 32u;
+      ref[I] = v | ((end - v) << 16);
+    }
+    f.ok = f.ok && f.win[f.ok ? end : at] == (I + 1 < CObj<E>::N ? ',' : '}');
+    return item_walk_flat<E, I + 1>(f, end, ref);
+  } else return at + 1u;
+}
+template <int OBJ, int CH, int J = 0>
+__device__ __forceinline__ void item_walk_child(uint32_t* row, const uint32_t* ref) {
+  if constexpr (J < CObj<CH>::N) {
+    row[ItModel<OBJ>::child_word + it_flat_word<CH>(J)] = ref[J];
+    item_walk_child<OBJ, CH, J + 1>(row, ref);
+  }
+}
+struct ItemLists { uint32_t k_str, n_str, k_obj, n_obj, bytes; };
+/* the members of root OBJ from property I on, each tried once, in model order */
+template <int OBJ, int I>
+__device__ __forceinline__ void item_walk_members(ItemWalk& f, uint32_t* row, uint32_t& flags, ItemLists& l) {
+  if constexpr (I < CObj<OBJ>::N) {
+    constexpr uint32_t kind = CObj<OBJ>::f[I].kind, word = it_root_word<OBJ>(I);
+    if (f.ok && f.k < f.kend && item_at_key<OBJ, I>(f.win, f.p + 1u)) {
+      const uint32_t v = f.p + 1u + FK<OBJ, I>::pat_len;
+      f.k++;
+      const bool more = f.k < f.kend; /* strings follow: the next key, or the value */
+      const uint32_t nx = f.pairs[more ? f.k : f.kend];
+      uint32_t end = v; /* behind the value */
+      if constexpr (kind == K_I64 || kind == K_I32 || kind == K_BOOL) {
+        end = more ? (nx & 0xFFFFu) - 1u : f.sep - 1u;
+        f.ok = end > v && end - v < 32u;
+        row[word] = v | ((end - v) << 16);
+      } else if constexpr (kind == K_STR || kind == K_ENUM || kind == K_DATETIME) {
+        end = (nx >> 16) + 1u;
+        f.ok = more && (nx & 0xFFFFu) == v && end - v <= 0x8000u;
+        f.k++;
+        row[word] = (v + 1u) | ((end - v - 2u) << 16);
+      } else if constexpr (kind == K_OBJ) {
+        constexpr int CH = CObj<OBJ>::f[I].child;
+        uint32_t ref[8];
+        end = item_walk_flat<CH>(f, v, ref);
+        item_walk_child<OBJ, CH>(row, ref);
+        flags |= ((1u << CObj<CH>::N) - 1u) << (IF_PRESENT + IB_CHILD);
+      } else { /* a list */
+        f.ok = f.win[v] == '[';
+        uint32_t n = 0;
+        const uint32_t k0 = f.k;
+        bool go = f.ok && f.win[v + 1u] != ']';
+        end = v + (go ? 1u : 2u);
+        while (go) {
+          uint32_t behind;
+          if constexpr (kind == K_LIST_STR) {
+            const uint32_t pr = f.pairs[f.k < f.kend ? f.k : f.kend];
+            f.k++;
+            behind = (pr >> 16) + 1u;
+            f.ok = f.k <= f.kend && (pr & 0xFFFFu) == end && behind - end < 0x8000u;
+            l.bytes += behind - end - 2u;
+          } else {
+            uint32_t ref[8];
+            behind = item_walk_flat<CObj<OBJ>::f[I].child>(f, end, ref);
+            l.bytes += ref[it_string_field<CObj<OBJ>::f[I].child>()] & 0xFFFF0000u;
+          }
+          ++n;
+          const uint32_t x = f.win[f.ok ? behind : end];
+          end = behind + 1u;
+          go = f.ok && x == ',';
+          f.ok = f.ok && (x == ',' || x == ']');
+        }
+        if constexpr (kind == K_LIST_STR) { l.k_str = k0; l.n_str = n; } else { l.k_obj = k0; l.n_obj = n; }
+      }
+      flags |= 1u << (IF_PRESENT + I);
+      const uint32_t x = f.win[f.ok ? end : f.p];
+      f.ok = f.ok && (x == ',' || (x == '}' && end + 1u == f.sep));
+      f.p = f.ok ? end : f.p;
+    }
+    item_walk_members<OBJ, I + 1>(f, row, flags, l);
+  }
+}
+template <int SCHEMA>
+__device__ __forceinline__ ItemWalk item_walk_open(const ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t i) {
+  const uint32_t me = sh.line[i], next = sh.line[i + 1u];
+  ItemWalk f;
+  f.win = win; f.pairs = pairs;
+  f.p = me & 0xFFFFu; f.k = me >> 16; f.kend = next >> 16; f.sep = (next & 0xFFFFu) - 1u;
+  f.ok = true;
+  return f;
+}
+template <bool ARR>
+__device__ __forceinline__ bool item_blank(uint32_t x) { return x == ' ' || x == '\t' || x == '\r' || (ARR && x == '\n'); }
+/* One line: its row, or IF_ODD there. */
+template <int SCHEMA, bool ARR>
+__device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t i, uint32_t type) {
+  constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
+  ItemWalk f = item_walk_open<SCHEMA>(sh, win, pairs, i);
+  uint32_t* row = rows + i * STRIDE;
+  const uint32_t start = f.p;
+  uint32_t flags = 0, err = IE_NONE;
+  ItemLists l;
+  l.k_str = l.n_str = l.k_obj = l.n_obj = l.bytes = 0;
+  const bool cut = f.sep >= g.hi_valid && !a.is_last; /* the readable bytes end here, the stream does not */
+  if (f.k == f.kend) { /* no string */
+    uint32_t p = start;
+    while (p < f.sep && item_blank<ARR>(win[p])) ++p;
+    if (p < f.sep || cut) { flags = IF_RECORD; err = (start << 8) | IE_REFUSED; } /* for the exact parser */
+    else if (ARR && !(i + 1u == sh.nline && f.sep >= g.hi_valid)) sh.slow = 1; /* an extent without a value (what follows the closing bracket is none) */
+    f.p = start;
+  } else {
+    f.ok = win[start] == '{' && !cut && !((sh.oddline[i >> 5] >> (i & 31u)) & 1u);
+    if constexpr (SCHEMA != PJ_SCHEMA_MIXED) item_walk_members<RootOf<SCHEMA>::obj, 0>(f, row, flags, l);
+    else {
+      if (type == PJ_TYPE_PET) { item_walk_members<OBJ_PET, 0>(f, row, flags, l); flags |= 6u << IF_NOTMODEL; }
+      else if (type == PJ_TYPE_ORDER) { item_walk_members<OBJ_ORDER, 0>(f, row, flags, l); flags |= 5u << IF_NOTMODEL; }
+      else if (type == PJ_TYPE_USER) { item_walk_members<OBJ_USER, 0>(f, row, flags, l); flags |= 3u << IF_NOTMODEL; }
+      else f.ok = false;
+    }
+    f.ok = f.ok && f.k == f.kend && win[f.p] == '}' && f.p + 1u == f.sep;
+    flags = IF_RECORD | (f.ok ? flags : IF_ODD);
+  }
+  row[IW_FLAGS] = flags; row[IW_ERR] = err; row[IW_POS] = start | (f.p << 16);
+  if constexpr (ItemSlots<SCHEMA>::lists) {
+    row[IW_LIST] = l.k_str | (l.n_str << 16);
+    if (SCHEMA == PJ_SCHEMA_PET || type == PJ_TYPE_PET) { row[ItWords<OBJ_PET>::n] = l.k_obj | (l.n_obj << 16); row[ItWords<OBJ_PET>::n + 1u] = l.bytes; }
+  }
+}
+static_assert(ItStride<PJ_SCHEMA_PET>::n >= ItWords<OBJ_PET>::n + 2u && ItStride<PJ_SCHEMA_MIXED>::n >= ItWords<OBJ_PET>::n + 2u, "two words behind a Pet's for its lists");
+static_assert(CObj<OBJ_TAG>::N == 2 && CObj<OBJ_TAG>::f[0].kind == K_I64 && CObj<OBJ_TAG>::f[1].kind == K_STR, "list elements: an integer and a string");
+
+/* All lines: one per thread, in order, or, in a stream of several models, sorted by the model the key behind `id` decides,
+ * so that a warp walks one model. */
+template <int SCHEMA, bool ARR>
+__device__ __forceinline__ void item_walk(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t tid) {
+  const uint32_t lane = tid & 31, warp = tid >> 5, nline = sh.nline;
+  uint32_t i = tid, type = 0;
+  if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+    uint32_t cls = 4; /* threads without a line go last */
+    if (tid < nline) {
+      const ItemWalk f = item_walk_open<SCHEMA>(sh, win, pairs, tid);
+      cls = 3; /* no idea */
+      if (f.k + 1u < f.kend) {
+        const uint32_t x = item_peek4(win, (f.pairs[f.k + 1u] & 0xFFFFu) + 1u), c0 = x & 0xFFu, c1 = (x >> 8) & 0xFFu;
+        cls = c0 == 'c' || c0 == 'n' ? 0u : (c0 == 'p' && c1 == 'e' ? 1u : (c0 == 'u' ? 2u : 3u));
+      }
+    }
+    uint32_t rank = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cls == k);
+      if (lane == 0) sh.cls[k][warp] = (uint8_t)__popc(bal);
+      if (cls == k) rank = (uint32_t)__popc(bal & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    uint32_t at = 0, ends[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+#pragma unroll
+      for (uint32_t q = 0; q < IT_WARPS; ++q) {
+        if (cls == k && q == warp) rank += at;
+        at += sh.cls[k][q];
+      }
+      ends[k] = at;
+    }
+    if (cls < 4) sh.perm[rank] = (uint8_t)tid;
+    __syncthreads();
+    type = tid < ends[0] ? (uint32_t)PJ_TYPE_PET : (tid < ends[1] ? (uint32_t)PJ_TYPE_ORDER : (tid < ends[2] ? (uint32_t)PJ_TYPE_USER : (uint32_t)PJ_TYPE_NONE));
+    if (tid < nline) i = sh.perm[tid];
+  }
+  if (tid < nline) item_walk_line<SCHEMA, ARR>(a, g, sh, win, pairs, rows, i, type);
+}
+
+/* ---- 3. strings and gaps ------------------------------------------------------------------------------------------ */
+/* A gap as the tables know it, and the places in it that matter. */
+struct ItemView {
+  uint32_t desc;       /* ItGap, 0: not one of the texts */
+  uint32_t vpos, vend; /* first byte of the value behind the colon, end of a number or literal */
+  uint32_t clpos;      /* the record's closing brace */
+};
+__device__ __forceinline__ uint32_t item_gap_find(const ItemShared& sh, uint32_t lo, uint32_t hi, uint32_t len) {
+  const ItGapEntry e = sh.gap[it_gap_hash(lo, hi)];
+  return e.lo == lo && e.hi == hi && e.len == len ? e.desc : 0u;
+}
+/* [from, b) with blanks: its text is put together byte by byte, numbers and literals are skipped. */
+template <bool ARR>
+__device__ __forceinline__ void item_gap_spaced(const ItemShared& sh, const uint8_t* win, uint32_t from, uint32_t b, ItemView& v) {
+  Win w;
+  w.s = win; w.w0 = 0;
+  uint32_t lo = 0, hi = 0, n = 0, p = from;
+  v.vpos = b; v.vend = 0; v.clpos = b;
+  while (p < b && n <= 8u) {
+    uint32_t c = win[p];
+    if (item_blank<ARR>(c)) { ++p; continue; }
+    if (n == 1u) v.vpos = p;
+    if (c - (uint32_t)'0' <= 9u || c == '-' || (c | 0x20u) - (uint32_t)'a' <= 25u) {
+      ++p;
+      for (;;) {
+        const uint64_t m = swar_nondigit(wpeek8(w, p));
+        if (!m) { p += 8; if (p > b) break; continue; }
+        p += ctz64(m) >> 3;
+        const uint32_t x = win[p];
+        if ((x | 0x20u) - (uint32_t)'a' <= 25u || x == '.' || x == '+' || x == '-') { ++p; continue; }
+        break;
+      }
+      v.vend = p;
+      c = '0';
+    } else {
+      if (c == '}') v.clpos = p;
+      ++p;
+    }
+    if (n < 4u) lo |= c << (8u * n); else if (n < 8u) hi |= c << (8u * (n - 4u));
+    ++n;
+  }
+  v.desc = n <= 8u && p == b ? item_gap_find(sh, lo, hi, n) : 0u;
+}
+
+/* Lines [i0, i0 + n), each with a string, by a warp: together at most 32 strings, or one line with more. Returns false when
+ * the tile has to take the other road. */
+template <int SCHEMA, bool ARR>
+__device__ __noinline__ bool item_pack(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t i0, uint32_t n) {
+  constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
+  constexpr uint32_t LW = ItWords<OBJ_PET>::n; /* the word of the list of objects, then that of the bytes */
+  constexpr int E = OBJ_TAG, ES = it_string_field<E>();
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t lt = (1u << lane) - 1u, le = (2u << lane) - 1u; /* lane 31: 2 << 31 wraps to 0, so all ones */
+  const uint32_t nstr = sh.nstr;
+  const bool special = sh.nspecial != 0, truncs = sh.odd != 0;
+  const uint32_t k_lo = sh.line[i0] >> 16, k_hi = sh.line[i0 + n] >> 16;
+  const bool single = k_hi - k_lo > 32u;
+  /* rows start empty */
+  uint32_t first_bit = 0;
+  if (lane < n) {
+    const uint32_t me = sh.line[i0 + lane];
+    uint32_t* row = rows + (i0 + lane) * STRIDE;
+    row[IW_FLAGS] = IF_RECORD | IF_ROWS; row[IW_ERR] = IE_NONE; row[IW_POS] = me & 0xFFFFu;
+    if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[LW] = 0; row[LW + 1u] = 0; }
+    first_bit = 1u << (((me >> 16) - k_lo) & 31u);
+  }
+  const uint32_t FS = single ? 1u : __reduce_or_sync(0xFFFFFFFFu, first_bit); /* lanes with the first string of a line */
+  __syncwarp();
+  bool slow = false;
+  uint32_t st = IS_ROOT, pk = 0, rows_at = 0, rows_end = 0, nT = 0, nP = 0;
+  for (uint32_t k0 = k_lo; k0 < k_hi; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    const bool live = k < k_hi;
+    const bool first_group = k0 == k_lo;
+    const uint32_t pr = pairs[live ? k : nstr], nx = pairs[live ? k + 1u : nstr];
+    const uint32_t open = pr & 0xFFFFu, close = pr >> 16;
+    const uint32_t ln = single ? i0 : i0 + (uint32_t)__popc(FS & le) - 1u; /* this lane's line */
+    const bool first = single ? k == k_lo : live && ((FS >> lane) & 1u);
+    const uint32_t line_end = live ? sh.line[ln + 1u] : 0u;
+    const uint32_t sep = (line_end & 0xFFFFu) - 1u;
+    const bool last = live && k + 1u == line_end >> 16;
+    const uint32_t b = last ? sep : nx & 0xFFFFu; /* end of the gap: the next string, or the line's separator */
+    uint32_t* row = rows + (live ? ln : i0) * STRIDE;
+    const bool trunc = truncs && live && close == sep;
+    const uint32_t from = trunc ? sep : close + 1u;
+
+    /* ---- the gap behind the string ---- */
+    ItemView v;
+    v.vpos = b; v.vend = 0; v.clpos = b - 1u;
+    {
+      /* without blanks: the bytes themselves, or `:0` and what follows the number (found from the gap's end) */
+      const uint32_t len0 = b - from;
+      const uint32_t* hp = reinterpret_cast<const uint32_t*>(win) + (from >> 2);
+      const uint32_t hs = (from & 3u) * 8u, h0 = hp[0], h1 = hp[1], h2 = hp[2];
+      uint32_t lo = __funnelshift_r(h0, h1, hs), hi = __funnelshift_r(h1, h2, hs), len = len0;
+      const uint32_t c0 = lo & 0xFFu, c1 = (lo >> 8) & 0xFFu;
+      bool fits = len0 <= 8u;
+      hi = len0 <= 4u ? 0u : (len0 < 8u ? hi & ((1u << (8u * (len0 & 3u))) - 1u) : hi);
+      lo = len0 < 4u ? lo & ((1u << (8u * len0)) - 1u) : lo;
+      if (c0 == ':' && len0 > 1u) v.vpos = from + 1u;
+      if (c0 == ':' && len0 > 2u && (c1 - (uint32_t)'0' <= 9u || c1 == '-' || c1 - (uint32_t)'a' <= 25u)) {
+        const uint32_t* tp = reinterpret_cast<const uint32_t*>(win) + ((b - 4u) >> 2);
+        const uint32_t ts = (b & 3u) * 8u;
+        const uint32_t th = __funnelshift_r(tp[0], tp[1], ts); /* the last four bytes */
+        /* bytes 0x30-0x3F and 0x60-0x6F: digits, and the letters a literal ends with */
+        const uint32_t x3 = (th ^ 0x30303030u) & 0xF0F0F0F0u, x6 = (th ^ 0x60606060u) & 0xF0F0F0F0u;
+        const uint32_t z = ~((((x3 & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x3) & (((x6 & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x6)) & 0x80808080u;
+        const uint32_t tail = (uint32_t)__clz((int)z) >> 3; /* bytes behind the last of them; 4: none of the four is one */
+        v.vend = b - tail;
+        fits = tail <= 3u && (tail >= 1u);
+        len = tail + 2u;
+        const uint32_t t = fits ? th >> (32u - 8u * tail) : 0u;
+        lo = (t << 16) | (uint32_t)':' | ((uint32_t)'0' << 8); hi = t >> 16;
+      }
+      v.desc = fits ? item_gap_find(sh, lo, hi, len) : 0u;
+    }
+    if (live && v.desc == 0 && !trunc) item_gap_spaced<ARR>(sh, win, from, b, v);
+    if (live && v.desc != 0 && last != ((v.desc & ItGap::ENDS) != 0)) v.desc = 0;
+    const bool ok = live && v.desc != 0;
+    const uint32_t d = ok ? v.desc : ItGap::make(IV_NONE, 15, IS_ROOT, false, false, false, false), vk = ItGap::vk(d);
+    const bool telling = live && ((d & ItGap::TELLS) || last), newelem = live && (d & ItGap::ELEM);
+    bool iskey = live && (d & ItGap::KEY);
+
+    /* ---- the object the string lies in: what the nearest telling gap before it left ---- */
+    const uint32_t NI = __ballot_sync(0xFFFFFFFFu, telling);
+    const uint32_t pm = NI & lt;
+    const uint32_t out = last ? (uint32_t)IS_ROOT : ItGap::out(d);
+    const uint32_t from_lane = __shfl_sync(0xFFFFFFFFu, out, pm ? 31 - __clz((int)pm) : 0);
+    const uint32_t s = pm ? from_lane : st;
+    const uint32_t PK = __ballot_sync(0xFFFFFFFFu, iskey && vk == IV_STR);
+    const bool isval = !first && (lane ? (PK >> (lane - 1)) & 1u : pk != 0);
+    const bool iselem = live && !isval && s == IS_LIST && !iskey;
+    const uint32_t need = ItGap::need(d);
+    const bool role_ok = isval ? !iskey : (s == IS_LIST ? !iskey : (iskey || trunc));
+    if (live) {
+      if (first) { /* blanks, a brace, blanks */
+        const uint32_t at = sh.line[ln] & 0xFFFFu;
+        bool good = win[at] == '{' && open == at + 1u;
+        if (!good) {
+          uint32_t p = at;
+          while (p < open && item_blank<ARR>(win[p])) ++p;
+          if (p < open && win[p] == '{') { ++p; while (p < open && item_blank<ARR>(win[p])) ++p; good = p == open; }
+        }
+        if (!good || (sep >= g.hi_valid && !a.is_last)) item_error(row, at, IE_REFUSED);
+      }
+      if (trunc) { item_error(row, close, (uint32_t)PJ_E_EOF); if (!role_ok) item_error(row, open, IE_REFUSED); }
+      else if (!ok || !role_ok || !(need == 15u || need == s)) { item_error(row, close, IE_REFUSED); iskey = false; }
+      if (last) reinterpret_cast<uint16_t*>(&row[IW_POS])[1] = (uint16_t)v.clpos;
+      if (special) {
+        if (((sh.special[k >> 5] | sh.broken[k >> 5]) >> (k & 31u)) & 1u) {
+          atomicOr(&row[IW_FLAGS], IF_MOVED);
+          if ((sh.broken[k >> 5] >> (k & 31u)) & 1u) item_error(row, open - 1u, IE_REFUSED); /* before anything its text is judged by */
+        }
+      }
+    }
+    uint32_t NE = 0, erow = 0;
+    if constexpr (ItemSlots<SCHEMA>::lists) {
+      const uint32_t EL = __ballot_sync(0xFFFFFFFFu, iselem);
+      NE = __ballot_sync(0xFFFFFFFFu, newelem);
+      if (EL | NE) {
+        /* lanes of this lane's line */
+        const uint32_t lo = single ? 0u : 31u - (uint32_t)__clz((int)(FS & le)), up = single ? 0u : FS & ~le;
+        const uint32_t mine = (up ? (up & (0u - up)) - 1u : 0xFFFFFFFFu) & ~((1u << lo) - 1u);
+        if (iselem) {
+          if (close - open > 0x8000u) slow = true;
+          atomicAdd(&row[LW + 1u], close - open - 1u);
+          if (!single) { if (!(EL & mine & lt)) row[IW_LIST] = k | ((uint32_t)__popc(EL & mine) << 16); }
+          else if (nP == 0 && !(EL & lt)) row[IW_LIST] = k;
+        }
+        if (NE) {
+          /* rows of the elements: of a pack, all at once; of a long line, room for as many as its strings can make */
+          const uint32_t want = single ? 3u * ((k_hi - k0 + 1u) / 2u + 1u) : 3u * (uint32_t)__popc(NE);
+          if (!single || rows_end == 0) {
+            if (lane == 0) rows_at = atomicAdd(&sh.free_word, want);
+            rows_at = __shfl_sync(0xFFFFFFFFu, rows_at, 0);
+            rows_end = rows_at + want;
+            if (rows_end > a.str_words) slow = true;
+          }
+          if (newelem) {
+            const uint32_t r = rows_at + 3u * (nT + (uint32_t)__popc(NE & lt));
+            if (r + 3u > rows_end) slow = true;
+            if (!slow) { pairs[r] = 0; pairs[r + 1u] = 0; pairs[r + 2u] = 0; }
+            if (!single) { if (!(NE & mine & lt)) row[LW] = r | ((uint32_t)__popc(NE & mine) << 16); }
+            else if (nT == 0 && !(NE & lt)) row[LW] = r;
+          }
+          slow = __any_sync(0xFFFFFFFFu, slow); /* (and every row is empty before a key writes to it) */
+        }
+      }
+      erow = rows_at + 3u * (nT + (uint32_t)__popc(NE & lt) - 1u);
+      nP += (uint32_t)__popc(EL);
+    }
+    /* ---- keys ---- */
+    if (iskey && !slow) {
+      const uint32_t len = close - open - 1u;
+      const uint32_t* kw = reinterpret_cast<const uint32_t*>(win) + ((open + 1u) >> 2);
+      const uint32_t ksh = ((open + 1u) & 3u) * 8u;
+      const uint32_t y0 = kw[0], y1 = kw[1], y2 = kw[2], y3 = kw[3], y4 = kw[4];
+      const uint32_t x0 = __funnelshift_r(y0, y1, ksh), x1 = __funnelshift_r(y1, y2, ksh), x2 = __funnelshift_r(y2, y3, ksh), x3 = __funnelshift_r(y3, y4, ksh);
+      const uint32_t slot = it_hash(x0 & 0xFFFFu, len, IT_MUL);
+      const uint4 kt = *reinterpret_cast<const uint4*>(&sh.key[slot][0]), km = *reinterpret_cast<const uint4*>(&sh.key[slot][4]);
+      uint32_t f = sh.field[s == IS_ROOT ? 0 : (s == IS_CHILD ? 1 : 2)][slot];
+      if ((((x0 ^ kt.x) & km.x) | ((x1 ^ kt.y) & km.y) | ((x2 ^ kt.z) & km.z) | ((x3 ^ kt.w) & km.w)) != 0 || len < 2u || len > 15u) f = 0;
+      const uint32_t vlen = v.vend - v.vpos;
+      if (!f) {
+        if (!(vk == IV_STR || (vk == IV_SCALAR && item_plain_scalar(win, v.vpos, vlen)))) item_error(row, close, IE_REFUSED);
+      } else {
+        const uint32_t kind = ItField::kind(f), vclose = nx >> 16;
+        const bool null = vk == IV_SCALAR && vlen == 4u && item_peek4(win, v.vpos) == 0x6C6C756Eu;
+        bool good = ((ItField::allowed(f) >> vk) & 1u) != 0;
+        const uint32_t n_val = vk == IV_STR ? vclose - b - 1u : vlen;
+        uint32_t ref = (vk == IV_STR ? b + 1u : v.vpos) | (n_val << 16);
+        if ((vk == IV_STR || vk == IV_SCALAR) && n_val >= 0x8000u) slow = true;
+        if (!good && !null) {
+          const uint32_t at = vk == IV_STR ? b : v.vpos, x = win[at];
+          if ((a.opts & PJ_OPT_COERCE_SCALARS) && ((vk == IV_STR && (kind == K_I64 || kind == K_I32 || kind == K_BOOL)) || (vk == IV_SCALAR && kind == K_STR))) {
+            if (vk == IV_STR) ref |= 0x80000000u;
+            else if (!item_plain_scalar(win, at, vlen)) item_error(row, at, IE_REFUSED);
+            good = true;
+          } else if ((kind == K_LIST_STR && vk == IV_ELEM) || (kind == K_LIST_OBJ && vk == IV_LIST) || (vk == IV_SCALAR && !(x == '-' || x - (uint32_t)'0' <= 9u || x == 't' || x == 'f')))
+            item_error(row, close, IE_REFUSED);
+          else item_error(row, at, PJ_E_TYPE);
+        }
+        if (truncs && vk == IV_STR && vclose == (sh.line[ln + 1u] & 0xFFFFu) - 1u) good = false; /* cut off: it reports that itself */
+        const uint32_t bit = 1u << ItField::bit(f), word = ItField::word(f);
+        const bool keep = good && !null;
+        if (s == IS_ELEM) {
+          /* integers are decoded here, a string's reference is kept (twelve bits of length) */
+          uint32_t w2 = bit << 30 | (keep ? bit << 28 : 0u);
+          if (keep && kind == K_STR) {
+            if (n_val >= 0x1000u) slow = true;
+            w2 |= ref & 0x0FFFFFFFu;
+            atomicAdd(&row[LW + 1u], n_val << 16);
+          } else if (keep) {
+            int64_t val = 0;
+            const uint32_t at = ref & 0xFFFFu;
+            if (!item_int(win, at, n_val, kind == K_I64, &val)) {
+              const uint32_t x = win[at];
+              item_error(row, ref >> 31 ? at - 1u : at, (!(ref >> 31) && (x == 't' || x == 'f')) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
+            }
+            if (!slow) { pairs[erow] = (uint32_t)(uint64_t)val; pairs[erow + 1u] = (uint32_t)((uint64_t)val >> 32); }
+          }
+          if (!slow) { if ((atomicOr(&pairs[erow + 2u], w2) >> 30) & bit) item_error(row, close, IE_REFUSED); } /* repeated key */
+        } else {
+          const uint32_t nm = SCHEMA == PJ_SCHEMA_MIXED && s == IS_ROOT ? (~ItField::models(f) & 7u) << IF_NOTMODEL : 0u;
+          const uint32_t old = atomicOr(&row[IW_FLAGS], bit | nm | (keep ? bit << IF_PRESENT : 0u));
+          if (old & bit) item_error(row, close, IE_REFUSED);
+          if (keep && kind <= K_DATETIME) row[word] = ref;
+        }
+      }
+    }
+    nT += (uint32_t)__popc(NE);
+    st = NI ? __shfl_sync(0xFFFFFFFFu, out, 31 - __clz((int)NI)) : st;
+    pk = (PK >> 31) & 1u;
+    if (__any_sync(0xFFFFFFFFu, slow)) return false;
+  }
+  if constexpr (ItemSlots<SCHEMA>::lists) {
+    if (single && lane == 0) { uint32_t* row = rows + i0 * STRIDE; row[IW_LIST] |= nP << 16; row[LW] |= nT << 16; }
+  }
+  __syncwarp();
+  return true;
+}
+/* The lines the walk did not recognise: each by a warp when they are few, otherwise all lines of the tile, several to a
+ * step. */
+template <int SCHEMA, bool ARR>
+__device__ __forceinline__ void item_packs(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t nodd) {
+  const uint32_t lane = threadIdx.x & 31u, nline = sh.nline;
+  const bool few = nodd * 4u <= nline;
+  for (;;) {
+    uint32_t x = 0;
+    if (lane == 0) x = atomicAdd(&sh.next, few ? 1u : 4u);
+    x = __shfl_sync(0xFFFFFFFFu, x, 0);
+    if (x >= (few ? nodd : nline)) return;
+    uint32_t i = x, end = x + 4u < nline ? x + 4u : nline;
+    if (few) { /* line number x of the odd ones */
+      uint32_t at = 0;
+      i = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < IT_WARPS; ++k) {
+        const uint32_t m = sh.oddmask[k], n = (uint32_t)__popc(m);
+        if (x >= at && x < at + n) {
+          const bool hit = (uint32_t)__popc(m & ((1u << lane) - 1u)) == x - at && ((m >> lane) & 1u);
+          i = 32u * k + (uint32_t)__ffs((int)__ballot_sync(0xFFFFFFFFu, hit)) - 1u;
+        }
+        at += n;
+      }
+      end = i + 1u;
+    }
+    while (i < end) {
+      const uint32_t k0 = sh.line[i] >> 16;
+      if (sh.line[i + 1u] >> 16 == k0) { ++i; continue; } /* no string: the walk has dealt with it */
+      uint32_t n = 1;
+      while (i + n < end && (sh.line[i + n + 1u] >> 16) - k0 <= 32u && sh.line[i + n + 1u] >> 16 != sh.line[i + n] >> 16) ++n;
+      if (!item_pack<SCHEMA, ARR>(a, g, sh, win, pairs, rows, i, n)) { sh.slow = 1; return; }
+      i += n;
+    }
+  }
+}
+
+/* ---- 4. values ------------------------------------------------------------------------------------------------ */
 /* The integers, of any model, one after the other: word | bit << 8 | int64 << 16; 0 = no more. */
 template <int OBJ>
 PJ_CX uint32_t it_int_field(uint32_t nth) {
@@ -900,59 +1147,6 @@ PJ_CX uint32_t it_int_all(uint32_t nth) { /* the embedded object's come after th
 }
 template <int OBJ, uint32_t NTH> struct ItInt { static constexpr uint32_t v = it_int_all<OBJ, ItModel<OBJ>::child>(NTH); };
 
-/* the properties of OBJ that are neither integers nor plain strings */
-template <int OBJ, int I = 0>
-__device__ __forceinline__ void item_other_values(const ItemArgs& a, const uint8_t* win, uint32_t* row, uint32_t& flags) {
-  if constexpr (I < CObj<OBJ>::N) {
-    constexpr uint32_t kind = CObj<OBJ>::f[I].kind, word = it_root_word<OBJ>(I), bit = 1u << (IF_PRESENT + I);
-    if constexpr (kind == K_ENUM || kind == K_BOOL || kind == K_DATETIME) {
-      if (flags & bit) {
-        const uint32_t ref = row[word], pos = ref & 0xFFFFu, n = (ref >> 16) & 0x7FFFu;
-        Win w;
-        w.s = win; w.w0 = 0;
-        if constexpr (kind == K_ENUM) {
-          int e = -1;
-          if (n <= 14) {
-            const uint64_t x = wpeek8(w, pos), y = wpeek8(w, pos + 8);
-            const uint64_t lo = n >= 8 ? x : (n ? x & (~0ull >> (64 - 8 * n)) : 0);
-            const uint64_t hi = n > 8 ? y & (~0ull >> (64 - 8 * (n - 8))) : 0;
-            e = match_enum<CObj<OBJ>::f[I].child>(n, lo, hi);
-          }
-          if (e >= 0) row[word] = (uint32_t)e;
-          else if (a.opts & PJ_OPT_ENUM_UNKNOWN_AS_NULL) flags &= ~bit;
-          else item_error(row, pos - 1u, PJ_E_ENUM);
-        } else if constexpr (kind == K_BOOL) {
-          if (item_true(win, pos, n)) row[word] = 1;
-          else if (item_false(win, pos, n)) row[word] = 0;
-          else {
-            const uint32_t x = win[pos];
-            item_error(row, pos, (!(ref >> 31) && (x == '-' || x - (uint32_t)'0' <= 9u)) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
-          }
-        } else {
-          int64_t ep = 0; int32_t ns = 0, of = 0;
-          if (fast_datetime(w, pos, n, &ep, &ns, &of)) { row[word] = (uint32_t)(uint64_t)ep; row[word + 1] = (uint32_t)((uint64_t)ep >> 32); row[word + 2] = (uint32_t)ns; row[word + 3] = (uint32_t)of; }
-          else item_error(row, pos - 1u, PJ_E_DATETIME);
-        }
-      }
-    }
-    item_other_values<OBJ, I + 1>(a, win, row, flags);
-  }
-}
-__device__ __forceinline__ void item_int_value(const ItemArgs& a, const uint8_t* win, uint32_t* row, uint32_t flags, uint32_t desc) {
-  const uint32_t word = desc & 255u, bit = (desc >> 8) & 255u;
-  if (desc && ((flags >> (IF_PRESENT + bit)) & 1u)) {
-    const bool is64 = (desc >> 16) & 1u;
-    const uint32_t ref = row[word], pos = ref & 0xFFFFu, n = (ref >> 16) & 0x7FFFu;
-    int64_t v;
-    if (item_int(win, pos, n, is64, &v)) {
-      row[word] = (uint32_t)(uint64_t)v;
-      if (is64) row[word + 1] = (uint32_t)((uint64_t)v >> 32);
-    } else {
-      const uint32_t x = win[pos];
-      item_error(row, ref >> 31 ? pos - 1u : pos, (!(ref >> 31) && (x == 't' || x == 'f')) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
-    }
-  }
-}
 /* Model of a row: PJ_TYPE_*, 0 when the keys do not tell (mixed streams). */
 template <int SCHEMA>
 __device__ __forceinline__ uint32_t item_type(uint32_t flags) {
@@ -962,77 +1156,114 @@ __device__ __forceinline__ uint32_t item_type(uint32_t flags) {
     return m == 1u ? (uint32_t)PJ_TYPE_PET : (m == 2u ? (uint32_t)PJ_TYPE_ORDER : (m == 4u ? (uint32_t)PJ_TYPE_USER : (uint32_t)PJ_TYPE_NONE));
   }
 }
-template <int OBJ>
-__device__ __forceinline__ void item_finish_values(const ItemArgs& a, const uint8_t* win, uint32_t* row, uint32_t& flags) {
-  item_other_values<OBJ>(a, win, row, flags);
-  if (row[IW_ERR] == IE_NONE && ((flags >> IF_PRESENT) & CObj<OBJ>::required) != (uint32_t)CObj<OBJ>::required) item_error(row, row[IW_POS] >> 16, PJ_E_REQUIRED);
+/* The values of one field (or of the integer number V) of 32 lines, a line per lane. */
+enum { VU_INT0 = 0, VU_INT1 = 1, VU_INT2 = 2, VU_ENUM = 3, VU_BOOL = 4, VU_DATE = 5, VU_ELEM = 6, VU_COUNT = 7 };
+template <int SCHEMA> struct ItemValueUnits {
+  static constexpr uint32_t mask = SCHEMA == PJ_SCHEMA_PET ? (1u << VU_ELEM) | (1u << VU_INT0) | (1u << VU_INT1) | (1u << VU_ENUM)
+                                   : (SCHEMA == PJ_SCHEMA_ORDER ? 0x3Fu : (SCHEMA == PJ_SCHEMA_USER ? (1u << VU_INT0) | (1u << VU_INT1) : 0x7Fu));
+};
+static_assert(ItInt<OBJ_PET, 2>::v == 0 && ItInt<OBJ_ORDER, 3>::v == 0 && ItInt<OBJ_USER, 2>::v == 0, "integers per model");
+template <int OBJ, uint32_t KIND>
+__device__ __forceinline__ uint32_t item_kind_field() { /* word | bit << 8 of the property of this kind */
+  constexpr int i = it_find<OBJ>(KIND);
+  if constexpr (i < 0) return 0;
+  else return it_root_word<OBJ>(i) | ((uint32_t)i << 8);
 }
-/* one record per lane (live: it has one) */
+template <int SCHEMA, uint32_t KIND>
+__device__ __forceinline__ uint32_t item_field_of(uint32_t type) {
+  if constexpr (SCHEMA == PJ_SCHEMA_PET) return item_kind_field<OBJ_PET, KIND>();
+  else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) return item_kind_field<OBJ_ORDER, KIND>();
+  else if constexpr (SCHEMA == PJ_SCHEMA_USER) return item_kind_field<OBJ_USER, KIND>();
+  else return type == PJ_TYPE_PET ? item_kind_field<OBJ_PET, KIND>() : (type == PJ_TYPE_ORDER ? item_kind_field<OBJ_ORDER, KIND>() : item_kind_field<OBJ_USER, KIND>());
+}
+template <int SCHEMA, uint32_t NTH>
+__device__ __forceinline__ uint32_t item_int_of(uint32_t type) {
+  if constexpr (SCHEMA == PJ_SCHEMA_PET) return ItInt<OBJ_PET, NTH>::v;
+  else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) return ItInt<OBJ_ORDER, NTH>::v;
+  else if constexpr (SCHEMA == PJ_SCHEMA_USER) return ItInt<OBJ_USER, NTH>::v;
+  else return type == PJ_TYPE_PET ? ItInt<OBJ_PET, NTH>::v : (type == PJ_TYPE_ORDER ? ItInt<OBJ_ORDER, NTH>::v : ItInt<OBJ_USER, NTH>::v);
+}
+/* Element j of a list of objects as the walk left it (three strings: a key, a key, a value) into its row of three words. */
+__device__ __forceinline__ void item_elem_row(const uint8_t* win, uint32_t* e, uint32_t* row) {
+  const uint32_t p0 = e[0], p1 = e[1], p2 = e[2];
+  const uint32_t at = (p0 >> 16) + 2u, n = (p1 & 0xFFFFu) - 1u - at;
+  int64_t val = 0;
+  if (!item_int(win, at, n, true, &val)) { const uint32_t x = win[at]; item_error(row, at, (x == 't' || x == 'f') ? (uint32_t)PJ_E_TYPE : IE_REFUSED); }
+  e[0] = (uint32_t)(uint64_t)val; e[1] = (uint32_t)((uint64_t)val >> 32);
+  e[2] = ((p2 & 0xFFFFu) + 1u) | (((p2 >> 16) - (p2 & 0xFFFFu) - 1u) << 16) | 0xF0000000u;
+}
 template <int SCHEMA>
-__device__ __forceinline__ void item_record_values(const ItemArgs& a, const uint8_t* win, uint32_t* row, bool live) {
-  if (!live || (row[IW_ERR] != IE_NONE && (row[IW_ERR] & 0xFFu) == IE_REFUSED)) return; /* the exact parser will look at it */
-  uint32_t flags = row[IW_FLAGS];
+__device__ __forceinline__ void item_value(const ItemArgs& a, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t* row, bool live, uint32_t unit) {
+  const uint32_t flags = live ? row[IW_FLAGS] : 0u;
+  const bool rec = (flags & IF_RECORD) && !(row[IW_ERR] != IE_NONE && (row[IW_ERR] & 0xFFu) == IE_REFUSED); /* (refused: the exact parser looks at it) */
   const uint32_t type = item_type<SCHEMA>(flags);
-  if (SCHEMA == PJ_SCHEMA_MIXED) {
-    if (type == PJ_TYPE_NONE) { item_error(row, 0, IE_REFUSED); return; }
-    if (flags & (1u << (IF_PRESENT + IB_SHARED))) flags |= type == PJ_TYPE_PET ? 1u << (IF_PRESENT + it_find<OBJ_PET>(K_ENUM)) : 1u << (IF_PRESENT + it_find<OBJ_ORDER>(K_ENUM));
-  }
-#pragma unroll
-  for (uint32_t s = 0; s < 3; ++s) {
-    uint32_t desc;
-    const uint32_t dp = s == 0 ? ItInt<OBJ_PET, 0>::v : (s == 1 ? ItInt<OBJ_PET, 1>::v : ItInt<OBJ_PET, 2>::v);
-    const uint32_t dn = s == 0 ? ItInt<OBJ_ORDER, 0>::v : (s == 1 ? ItInt<OBJ_ORDER, 1>::v : ItInt<OBJ_ORDER, 2>::v);
-    const uint32_t du = s == 0 ? ItInt<OBJ_USER, 0>::v : (s == 1 ? ItInt<OBJ_USER, 1>::v : ItInt<OBJ_USER, 2>::v);
-    if constexpr (SCHEMA == PJ_SCHEMA_PET) desc = dp;
-    else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) desc = dn;
-    else if constexpr (SCHEMA == PJ_SCHEMA_USER) desc = du;
-    else desc = type == PJ_TYPE_PET ? dp : (type == PJ_TYPE_ORDER ? dn : du);
-    item_int_value(a, win, row, flags, desc);
-  }
-  static_assert(ItInt<OBJ_PET, 3>::v == 0 && ItInt<OBJ_ORDER, 3>::v == 0 && ItInt<OBJ_USER, 3>::v == 0, "three integers at most");
-  if constexpr (SCHEMA == PJ_SCHEMA_PET) item_finish_values<OBJ_PET>(a, win, row, flags);
-  else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) item_finish_values<OBJ_ORDER>(a, win, row, flags);
-  else if constexpr (SCHEMA == PJ_SCHEMA_USER) item_finish_values<OBJ_USER>(a, win, row, flags);
-  else {
-    if (type == PJ_TYPE_PET) item_finish_values<OBJ_PET>(a, win, row, flags);
-    else if (type == PJ_TYPE_ORDER) item_finish_values<OBJ_ORDER>(a, win, row, flags);
-    else item_finish_values<OBJ_USER>(a, win, row, flags);
-  }
-  row[IW_FLAGS] = flags;
-}
-/* one list element (three words at e) per lane: are its integers integers? */
-template <int E, int I = 0>
-__device__ __forceinline__ void item_element_values(const ItemArgs& a, const uint8_t* win, const uint32_t* e, uint32_t* row) {
-  if constexpr (I < CObj<E>::N) {
-    static_assert(CObj<E>::N <= 2 && (CObj<E>::f[I].kind == K_I64 || CObj<E>::f[I].kind == K_I32 || CObj<E>::f[I].kind == K_STR), "elements: two integers or strings");
-    if constexpr (CObj<E>::f[I].kind != K_STR) {
-      if ((e[2] >> (4 + I)) & 1u) {
-        const uint32_t ref = e[I], pos = ref & 0xFFFFu;
-        int64_t v;
-        if (!item_int(win, pos, (ref >> 16) & 0x7FFFu, CObj<E>::f[I].kind == K_I64, &v)) {
-          const uint32_t x = win[pos];
-          item_error(row, ref >> 31 ? pos - 1u : pos, (!(ref >> 31) && (x == 't' || x == 'f')) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
-        }
+  Win w;
+  w.s = win; w.w0 = 0;
+  if (unit <= VU_INT2) {
+    const uint32_t desc = unit == VU_INT0 ? item_int_of<SCHEMA, 0>(type) : (unit == VU_INT1 ? item_int_of<SCHEMA, 1>(type) : item_int_of<SCHEMA, 2>(type));
+    const uint32_t word = desc & 255u, bit = (desc >> 8) & 255u;
+    if (rec && desc && ((flags >> (IF_PRESENT + bit)) & 1u)) {
+      const bool is64 = (desc >> 16) & 1u;
+      const uint32_t ref = row[word], pos = ref & 0xFFFFu;
+      int64_t v = 0;
+      if (!item_int(win, pos, (ref >> 16) & 0x7FFFu, is64, &v)) {
+        const uint32_t x = win[pos];
+        item_error(row, ref >> 31 ? pos - 1u : pos, (!(ref >> 31) && (x == 't' || x == 'f')) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
       }
+      row[word] = (uint32_t)(uint64_t)v;
+      if (is64) row[word + 1] = (uint32_t)((uint64_t)v >> 32);
     }
-    item_element_values<E, I + 1>(a, win, e, row);
+  } else if (unit == VU_ENUM) {
+    uint32_t desc = item_field_of<SCHEMA, K_ENUM>(type), bit = desc >> 8;
+    if (SCHEMA == PJ_SCHEMA_MIXED && (flags & IF_ROWS)) { /* its key is one of two models' */
+      bit = IB_SHARED;
+      if (rec && type != PJ_TYPE_NONE && ((flags >> (IF_PRESENT + IB_SHARED)) & 1u)) atomicOr(&row[IW_FLAGS], 1u << (IF_PRESENT + (desc >> 8)));
+    }
+    if (rec && desc && ((flags >> (IF_PRESENT + bit)) & 1u)) {
+      const uint32_t word = desc & 255u, ref = row[word], pos = ref & 0xFFFFu, n = (ref >> 16) & 0x7FFFu;
+      int e = -1;
+      if (n <= 14) {
+        const uint64_t x = wpeek8(w, pos), y = wpeek8(w, pos + 8);
+        const uint64_t lo = n >= 8 ? x : (n ? x & (~0ull >> (64 - 8 * n)) : 0);
+        const uint64_t hi = n > 8 ? y & (~0ull >> (64 - 8 * (n - 8))) : 0;
+        if (SCHEMA == PJ_SCHEMA_PET || (SCHEMA == PJ_SCHEMA_MIXED && type == PJ_TYPE_PET)) e = match_enum<0>(n, lo, hi);
+        else e = match_enum<1>(n, lo, hi);
+      }
+      if (e >= 0) row[word] = (uint32_t)e;
+      else if (a.opts & PJ_OPT_ENUM_UNKNOWN_AS_NULL) atomicAnd(&row[IW_FLAGS], ~(1u << (IF_PRESENT + (desc >> 8))));
+      else item_error(row, pos - 1u, PJ_E_ENUM);
+    }
+  } else if (unit == VU_BOOL) {
+    const uint32_t desc = item_field_of<SCHEMA, K_BOOL>(type);
+    if (rec && desc && ((flags >> (IF_PRESENT + (desc >> 8))) & 1u)) {
+      const uint32_t word = desc & 255u, ref = row[word], pos = ref & 0xFFFFu, n = (ref >> 16) & 0x7FFFu;
+      if (item_true(win, pos, n)) row[word] = 1;
+      else if (item_false(win, pos, n)) row[word] = 0;
+      else { const uint32_t x = win[pos]; item_error(row, pos, (!(ref >> 31) && (x == '-' || x - (uint32_t)'0' <= 9u)) ? (uint32_t)PJ_E_TYPE : IE_REFUSED); }
+    }
+  } else if (unit == VU_DATE) {
+    const uint32_t desc = item_field_of<SCHEMA, K_DATETIME>(type);
+    if (rec && desc && ((flags >> (IF_PRESENT + (desc >> 8))) & 1u)) {
+      const uint32_t word = desc & 255u, ref = row[word], pos = ref & 0xFFFFu;
+      int64_t ep = 0; int32_t ns = 0, of = 0;
+      if (fast_datetime(w, pos, (ref >> 16) & 0x7FFFu, &ep, &ns, &of)) {
+        row[word] = (uint32_t)(uint64_t)ep; row[word + 1] = (uint32_t)((uint64_t)ep >> 32); row[word + 2] = (uint32_t)ns; row[word + 3] = (uint32_t)of;
+      } else item_error(row, pos - 1u, PJ_E_DATETIME);
+    }
+  } else if constexpr (ItemSlots<SCHEMA>::lists) { /* elements of lists of objects that the walk found */
+    const bool mine = rec && type == PJ_TYPE_PET && !(flags & IF_ROWS);
+    const uint32_t l = mine ? row[ItWords<OBJ_PET>::n] : 0u, n = l >> 16;
+    uint32_t* e = pairs + (l & 0xFFFFu);
+    if (n <= IT_SHORT) for (uint32_t j = 0; j < n; ++j) item_elem_row(win, e + 3u * j, row);
+    for (uint32_t big = __ballot_sync(0xFFFFFFFFu, n > IT_SHORT); big; big &= big - 1u) {
+      const int src = __ffs((int)big) - 1;
+      const uint32_t bl = __shfl_sync(0xFFFFFFFFu, l, src), r = __shfl_sync(0xFFFFFFFFu, (uint32_t)(row - rows), src);
+      for (uint32_t j = threadIdx.x & 31u; j < bl >> 16; j += 32) item_elem_row(win, pairs + (bl & 0xFFFFu) + 3u * j, rows + r);
+    }
   }
 }
 
-/* Group u of 32 list elements: which warp's (*w) and its first element (*j0). counts: elements per warp. */
-template <class C>
-__device__ __forceinline__ void item_unit(uint32_t u, C count_of, uint32_t* w, uint32_t* j0) {
-  uint32_t at = 0, ww = 0, jj = 0;
-#pragma unroll
-  for (uint32_t k = 0; k < IT_WARPS; ++k) {
-    const uint32_t n = (count_of(k) + 31u) >> 5;
-    if (u >= at && u < at + n) { ww = k; jj = (u - at) * 32u; }
-    at += n;
-  }
-  *w = ww; *j0 = jj;
-}
-
-/* ---- 4. emission ------------------------------------------------------------------------------------------------ */
+/* ---- 5. emission ------------------------------------------------------------------------------------------------ */
 /* n bytes at window offset pos to dst (any alignment): whole words of dst, odd bytes at both ends */
 __device__ __forceinline__ void item_copy(uint8_t* dst, const uint8_t* win, uint32_t pos, uint32_t n) {
   uint32_t h = (0u - (uint32_t)reinterpret_cast<uintptr_t>(dst)) & 3u;
@@ -1059,65 +1290,129 @@ __device__ __forceinline__ void item_copy(uint8_t* dst, const uint8_t* win, uint
     if (t > 2) e[2] = (uint8_t)(last >> 16);
   }
 }
-/* string column (offsets at col, bytes at col + 1) of 32 rows: lane = row; start0: where the 32 rows' bytes start */
-__device__ __forceinline__ void item_emit_string(const ItemArgs& a, uint32_t col, const uint8_t* win, bool has_row, uint64_t row_out, uint32_t ref, bool present, uint32_t start0) {
-  const uint32_t n = present ? (ref >> 16) & 0x7FFFu : 0u;
-  const uint32_t at = start0 + warp_incl_scan(n) - n;
-  if (has_row) colp<uint32_t>(&a.cols, col)[row_out] = at;
-  if (n) item_copy(colp<uint8_t>(&a.cols, col + 1) + at, win, ref & 0xFFFFu, n);
-}
-/* the columns of flat object or root OBJ at row_out: WORD0 / BIT0 = where its properties stand in the row */
+/* The place of a model root's row among 32 lines and what a lane needs to write it. */
+struct ItemOut {
+  const uint8_t* win;
+  const uint32_t* row;
+  uint32_t flags, chunk;
+  bool has_row;
+  uint64_t at; /* row of the model's table */
+};
+/* fixed-width columns of root or embedded object OBJ */
 template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
-__device__ __forceinline__ void item_emit_fields(const ItemArgs& a, ItemShared& sh, const uint8_t* win, const uint32_t* row, bool has_row, uint32_t flags, uint64_t row_out, uint32_t chunk,
-                                                 uint32_t nP, uint32_t nT) {
-  if constexpr (I == 0) {
-    if (has_row) colp<uint8_t>(&a.cols, CObj<OBJ>::present_col)[row_out] = (uint8_t)((flags >> (IF_PRESENT + BIT0)) & ((1u << CObj<OBJ>::N) - 1u));
+__device__ __forceinline__ void item_emit_fixed(const ItemArgs& a, const ItemOut& o) {
+  if constexpr (I == 0) colp<uint8_t>(&a.cols, CObj<OBJ>::present_col)[o.at] = (uint8_t)((o.flags >> (IF_PRESENT + BIT0)) & ((1u << CObj<OBJ>::N) - 1u));
+  if constexpr (I < CObj<OBJ>::N) {
+    constexpr uint32_t kind = CObj<OBJ>::f[I].kind, col = CObj<OBJ>::f[I].col;
+    constexpr uint32_t word = ROOT ? it_root_word<OBJ>(I) : WORD0 + it_flat_word<OBJ>(I);
+    const bool pr = (o.flags >> (IF_PRESENT + BIT0 + I)) & 1u;
+    const uint32_t* row = o.row;
+    if constexpr (kind == K_I64) colp<int64_t>(&a.cols, col)[o.at] = pr ? (int64_t)((uint64_t)row[word] | ((uint64_t)row[word + 1] << 32)) : 0;
+    else if constexpr (kind == K_I32) colp<int32_t>(&a.cols, col)[o.at] = pr ? (int32_t)row[word] : 0;
+    else if constexpr (kind == K_BOOL || kind == K_ENUM) colp<uint8_t>(&a.cols, col)[o.at] = pr ? (uint8_t)row[word] : (kind == K_ENUM ? 255 : 0);
+    else if constexpr (kind == K_DATETIME) {
+      colp<int64_t>(&a.cols, col)[o.at] = pr ? (int64_t)((uint64_t)row[word] | ((uint64_t)row[word + 1] << 32)) : 0;
+      colp<int32_t>(&a.cols, col + 1)[o.at] = pr ? (int32_t)row[word + 2] : 0;
+      colp<int32_t>(&a.cols, col + 2)[o.at] = pr ? (int32_t)row[word + 3] : 0;
+    } else if constexpr (kind == K_OBJ) item_emit_fixed<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, o);
+    item_emit_fixed<OBJ, ROOT, WORD0, BIT0, I + 1>(a, o);
   }
+}
+/* string columns of root or embedded object OBJ (every lane of the warp calls this) */
+template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
+__device__ __forceinline__ void item_emit_strings(const ItemArgs& a, const ItemShared& sh, const ItemOut& o) {
   if constexpr (I < CObj<OBJ>::N) {
     constexpr uint32_t kind = CObj<OBJ>::f[I].kind, col = CObj<OBJ>::f[I].col, slot = CObj<OBJ>::f[I].cnt;
     constexpr uint32_t word = ROOT ? it_root_word<OBJ>(I) : WORD0 + it_flat_word<OBJ>(I);
-    const bool pr = (flags >> (IF_PRESENT + BIT0 + I)) & 1u;
-    if constexpr (kind == K_I64) {
-      if (has_row) colp<int64_t>(&a.cols, col)[row_out] = pr ? (int64_t)((uint64_t)row[word] | ((uint64_t)row[word + 1] << 32)) : 0;
-    } else if constexpr (kind == K_I32) {
-      if (has_row) colp<int32_t>(&a.cols, col)[row_out] = pr ? (int32_t)row[word] : 0;
-    } else if constexpr (kind == K_BOOL || kind == K_ENUM) {
-      if (has_row) colp<uint8_t>(&a.cols, col)[row_out] = pr ? (uint8_t)row[word] : (kind == K_ENUM ? 255 : 0);
-    } else if constexpr (kind == K_DATETIME) {
-      if (has_row) {
-        colp<int64_t>(&a.cols, col)[row_out] = pr ? (int64_t)((uint64_t)row[word] | ((uint64_t)row[word + 1] << 32)) : 0;
-        colp<int32_t>(&a.cols, col + 1)[row_out] = pr ? (int32_t)row[word + 2] : 0;
-        colp<int32_t>(&a.cols, col + 2)[row_out] = pr ? (int32_t)row[word + 3] : 0;
-      }
-    } else if constexpr (kind == K_STR) {
-      item_emit_string(a, col, win, has_row, row_out, row[word], pr && has_row, sh.base[slot] + sh.csum[slot][chunk]);
-    } else if constexpr (kind == K_OBJ) {
-      /* absent: its own bits are clear as well */
-      item_emit_fields<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, win, row, has_row, flags, row_out, chunk, nP, nT);
-    } else {
-      const uint32_t n = kind == K_LIST_STR ? nP : nT;
-      const uint32_t at = sh.base[slot] + sh.csum[slot][chunk] + warp_incl_scan(n) - n;
-      if (has_row) colp<uint32_t>(&a.cols, col)[row_out] = at;
-    }
-    item_emit_fields<OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, win, row, has_row, flags, row_out, chunk, nP, nT);
+    if constexpr (kind == K_STR) {
+      const bool pr = o.has_row && ((o.flags >> (IF_PRESENT + BIT0 + I)) & 1u);
+      const uint32_t ref = o.row[word], n = pr ? (ref >> 16) & 0x7FFFu : 0u;
+      const uint32_t at = sh.base[slot] + sh.csum[slot][o.chunk] + warp_incl_scan(n) - n;
+      if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at;
+      if (n) item_copy(colp<uint8_t>(&a.cols, col + 1) + at, o.win, ref & 0xFFFFu, n);
+    } else if constexpr (kind == K_OBJ) item_emit_strings<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
+    item_emit_strings<OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
   }
 }
-
-/* bytes of the row's strings per slot, added up over the warp into csum[slot][chunk] */
+/* bytes of the lines' strings per slot, added up over the warp into csum[slot][chunk] */
 template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
-__device__ __forceinline__ void item_sum_fields(ItemShared& sh, const uint32_t* row, bool mine, uint32_t flags, uint32_t chunk, uint32_t lane, uint32_t nP, uint32_t nT) {
+__device__ __forceinline__ void item_sum_strings(ItemShared& sh, const uint32_t* row, bool mine, uint32_t flags, uint32_t chunk, uint32_t lane) {
   if constexpr (I < CObj<OBJ>::N) {
     constexpr uint32_t kind = CObj<OBJ>::f[I].kind, slot = CObj<OBJ>::f[I].cnt;
     if constexpr (kind == K_STR) {
       constexpr uint32_t word = ROOT ? it_root_word<OBJ>(I) : WORD0 + it_flat_word<OBJ>(I);
       const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, mine && ((flags >> (IF_PRESENT + BIT0 + I)) & 1u) ? (row[word] >> 16) & 0x7FFFu : 0u);
       if (lane == 0) sh.csum[slot][chunk] = s;
-    } else if constexpr (kind == K_OBJ) item_sum_fields<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(sh, row, mine, flags, chunk, lane, nP, nT);
-    else if constexpr (kind == K_LIST_STR || kind == K_LIST_OBJ) {
-      const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, mine ? (kind == K_LIST_STR ? nP : nT) : 0u);
-      if (lane == 0) sh.csum[slot][chunk] = s;
+    } else if constexpr (kind == K_OBJ) item_sum_strings<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(sh, row, mine, flags, chunk, lane);
+    item_sum_strings<OBJ, ROOT, WORD0, BIT0, I + 1>(sh, row, mine, flags, chunk, lane);
+  }
+}
+/* one element of a list of strings: number r of the child table, its bytes at `at` */
+__device__ __forceinline__ void item_emit_list_str(const ItemArgs& a, uint32_t col, const uint8_t* win, uint32_t pr, uint64_t r, uint32_t at) {
+  colp<uint32_t>(&a.cols, col + 1)[r] = at;
+  item_copy(colp<uint8_t>(&a.cols, col + 2) + at, win, (pr & 0xFFFFu) + 1u, (pr >> 16) - (pr & 0xFFFFu) - 1u);
+}
+/* one element of a list of objects (three words at e) */
+template <int E, int I = 0>
+__device__ __forceinline__ void item_emit_elem(const ItemArgs& a, const uint8_t* win, const uint32_t* e, uint64_t r, uint32_t at) {
+  if constexpr (I == 0) colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((e[2] >> 28) & 3u);
+  if constexpr (I < CObj<E>::N) {
+    constexpr uint32_t kind = CObj<E>::f[I].kind, col = CObj<E>::f[I].col;
+    const bool pr = (e[2] >> (28 + I)) & 1u;
+    if constexpr (kind == K_STR) {
+      colp<uint32_t>(&a.cols, col)[r] = at;
+      if (pr) item_copy(colp<uint8_t>(&a.cols, col + 1) + at, win, e[2] & 0xFFFFu, (e[2] >> 16) & 0xFFFu);
+    } else colp<int64_t>(&a.cols, col)[r] = pr ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
+    item_emit_elem<E, I + 1>(a, win, e, r, at);
+  }
+}
+/* the lists of 32 lines, a line per lane; long lists by the whole warp */
+template <bool OBJS>
+__device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemShared& sh, const ItemOut& o, const uint32_t* pairs, bool mine) {
+  constexpr int F = OBJS ? ItModel<OBJ_PET>::ei : ItModel<OBJ_PET>::li;
+  constexpr int E = OBJ_TAG;
+  constexpr uint32_t col = CObj<OBJ_PET>::f[F].col, slot = CObj<OBJ_PET>::f[F].cnt;
+  constexpr uint32_t bslot = OBJS ? CObj<E>::f[it_string_field<E>()].cnt : slot + 1u;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t l = mine ? o.row[OBJS ? ItWords<OBJ_PET>::n : (uint32_t)IW_LIST] : 0u, bw = mine ? o.row[ItWords<OBJ_PET>::n + 1u] : 0u;
+  const uint32_t n = l >> 16, bytes = OBJS ? bw >> 16 : bw & 0xFFFFu;
+  const uint32_t inc = warp_incl_scan(n | (bytes << 16)); /* of 32 lines: below 2^16 both */
+  const uint64_t r0 = (uint64_t)sh.base[slot] + sh.csum[slot][o.chunk] + (inc & 0xFFFFu) - n;
+  const uint32_t at0 = sh.base[bslot] + sh.csum[bslot][o.chunk] + (inc >> 16) - bytes;
+  if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = (uint32_t)r0;
+  if (n <= IT_SHORT) {
+    uint32_t at = at0;
+    for (uint32_t j = 0; j < n; ++j) {
+      if constexpr (OBJS) {
+        const uint32_t* e = pairs + (l & 0xFFFFu) + 3u * j;
+        item_emit_elem<E>(a, o.win, e, r0 + j, at);
+        at += (e[2] >> (28 + it_string_field<E>())) & 1u ? (e[2] >> 16) & 0xFFFu : 0u;
+      } else {
+        const uint32_t pr = pairs[(l & 0xFFFFu) + j];
+        item_emit_list_str(a, col, o.win, pr, r0 + j, at);
+        at += (pr >> 16) - (pr & 0xFFFFu) - 1u;
+      }
     }
-    item_sum_fields<OBJ, ROOT, WORD0, BIT0, I + 1>(sh, row, mine, flags, chunk, lane, nP, nT);
+  }
+  for (uint32_t big = __ballot_sync(0xFFFFFFFFu, n > IT_SHORT); big; big &= big - 1u) {
+    const int src = __ffs((int)big) - 1;
+    const uint32_t bl = __shfl_sync(0xFFFFFFFFu, l, src), br = __shfl_sync(0xFFFFFFFFu, (uint32_t)r0, src);
+    uint32_t at = __shfl_sync(0xFFFFFFFFu, at0, src);
+    for (uint32_t j0 = 0; j0 < bl >> 16; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      const bool has = j < bl >> 16;
+      uint32_t x = 0, len = 0;
+      if (has) {
+        if constexpr (OBJS) { x = pairs[(bl & 0xFFFFu) + 3u * j + 2u]; len = (x >> (28 + it_string_field<E>())) & 1u ? (x >> 16) & 0xFFFu : 0u; }
+        else { x = pairs[(bl & 0xFFFFu) + j]; len = (x >> 16) - (x & 0xFFFFu) - 1u; }
+      }
+      const uint32_t sc = warp_incl_scan(len);
+      if (has) {
+        if constexpr (OBJS) item_emit_elem<E>(a, o.win, pairs + (bl & 0xFFFFu) + 3u * j, (uint64_t)br + j, at + sc - len);
+        else item_emit_list_str(a, col, o.win, x, (uint64_t)br + j, at + sc - len);
+      }
+      at += __shfl_sync(0xFFFFFFFFu, sc, 31);
+    }
   }
 }
 
@@ -1234,302 +1529,178 @@ __device__ __noinline__ void item_slow_tile(const ItemArgs& a, const StreamGeom&
 }
 
 /* ---- a tile ------------------------------------------------------------------------------------------------------ */
-/* Record i of the tile: which warp's (its first record is *first) and its row. */
-__device__ __forceinline__ uint32_t item_row_of(const ItemShared& sh, uint32_t i, uint32_t* first) {
-  uint32_t at = 0, row = 0;
-  *first = 0;
-#pragma unroll
-  for (uint32_t k = 0; k < IT_WARPS; ++k) {
-    const uint32_t n = sh.w[k].nrec;
-    if (i >= at && i < at + n) { row = sh.w[k].row0 + (i - at); *first = at; }
-    at += n;
-  }
-  return row;
-}
-/* The place in the tile's part of a child table of list element j of warp w, whose record has the row `row`: the elements of
- * failed records take none. T: the list of objects. */
-template <bool TAGS>
-__device__ __forceinline__ uint32_t item_child_place(const ItemShared& sh, const uint32_t* rows, uint32_t stride, uint32_t w, uint32_t row, uint32_t j, uint32_t slot) {
-  uint32_t rec = row - sh.w[w].row0;
-#pragma unroll
-  for (uint32_t k = 0; k < IT_WARPS; ++k) if (k < w) rec += sh.w[k].nrec;
-  const uint32_t d = rows[row * stride + IW_ERR];
-  return sh.csum[slot][rec >> 5] + j + (uint32_t)(int32_t)(int16_t)(TAGS ? d >> 16 : d & 0xFFFFu);
-}
-/* row of the record that holds list string j of warp w: the first whose running count is above j */
-__device__ __forceinline__ uint32_t item_photo_row(const ItemShared& sh, const uint32_t* rows, uint32_t stride, uint32_t w, uint32_t j) {
-  uint32_t lo = 0, hi = sh.w[w].nrec - 1u;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if ((rows[(sh.w[w].row0 + mid) * stride + IW_CUM] & 0xFFFFu) > j) hi = mid; else lo = mid + 1u;
-  }
-  return sh.w[w].row0 + lo;
-}
-static constexpr uint32_t IF_BAD = 1u << 31; /* IW_FLAGS of a failed record: the rest is its error offset */
-
-/* one list element (three words at e) per lane: its columns at row `at` of the child table */
-template <int E, int I = 0>
-__device__ __forceinline__ void item_emit_element(const ItemArgs& a, const uint8_t* win, const uint32_t* e, bool good, uint64_t at, uint32_t start0) {
-  if constexpr (I == 0) { if (good) colp<uint8_t>(&a.cols, CObj<E>::present_col)[at] = (uint8_t)((e[2] >> 4) & ((1u << CObj<E>::N) - 1u)); }
-  if constexpr (I < CObj<E>::N) {
-    constexpr uint32_t kind = CObj<E>::f[I].kind, col = CObj<E>::f[I].col;
-    const bool pr = good && ((e[2] >> (4 + I)) & 1u);
-    if constexpr (kind == K_STR) item_emit_string(a, col, win, good, at, e[I], pr, start0);
-    else {
-      int64_t v = 0;
-      if (pr) item_int(win, e[I] & 0xFFFFu, (e[I] >> 16) & 0x7FFFu, kind == K_I64, &v);
-      if (good) { if constexpr (kind == K_I64) colp<int64_t>(&a.cols, col)[at] = v; else colp<int32_t>(&a.cols, col)[at] = (int32_t)v; }
-    }
-    item_emit_element<E, I + 1>(a, win, e, good, at, start0);
-  }
-}
-template <int E>
-PJ_CX int it_string_field() {
-  int at = -1;
-  for (int i = 0; i < CObj<E>::N; ++i) if (CObj<E>::f[i].kind == K_STR) at = i;
-  return at;
-}
-
-/* Steps 2 to 4 of a tile whose index stands. False: the other road (no barrier is left open, nothing was published). */
+/* Steps 2 to 5 of a tile whose index stands. False (for every thread): the other road; nothing was published. */
 template <int SCHEMA, bool ARR>
-__device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t* rows, uint32_t tile, uint32_t tid, long long* ck) {
+__device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t tile, uint32_t tid, long long* ck) {
   using SL = ItemSlots<SCHEMA>;
   constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
-  static_assert(IT_RCHUNKS == IT_WARPS, "one group of 32 records per warp");
-  const uint32_t lane = tid & 31, warp = tid >> 5;
-  /* rows are handed out by the separators each warp met */
-  {
-    uint32_t at = 0, all = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t n = sh.w[k].nterm; if (k < warp) at += n; all += n; }
-    if (all > a.row_cap) return false; /* the same for every thread */
-    if (lane == 0) sh.w[warp].row0 = at;
-    __syncwarp();
-  }
-  item_specials(a, sh, win, strs, warp, lane);
-  __syncwarp();
-  if (!item_tokens<SCHEMA, ARR>(a, g, sh, win, strs, rows, warp, lane)) sh.slow = 1;
-  __syncthreads();
-  if (sh.slow) return false;
-  ck[2] = clock64();
-  uint32_t nrec = 0, nu0 = 0, nu1 = 0;
-#pragma unroll
-  for (uint32_t k = 0; k < IT_WARPS; ++k) { nrec += sh.w[k].nrec; nu0 += (sh.w[k].nphoto + 31u) >> 5; nu1 += (sh.w[k].ntag + 31u) >> 5; }
-  if (nrec > IT_MAX_RECS || nu0 > IT_MAX_UNITS || nu1 > IT_MAX_UNITS) return false;
-  const uint32_t nchunk = (nrec + 31u) >> 5;
+  constexpr uint32_t LW = ItWords<OBJ_PET>::n;
   constexpr int E = OBJ_TAG;
   constexpr uint32_t PCNT = CObj<OBJ_PET>::f[ItModel<OBJ_PET>::li].cnt, TCNT = CObj<OBJ_PET>::f[ItModel<OBJ_PET>::ei].cnt;
-  constexpr uint32_t PCOL = CObj<OBJ_PET>::f[ItModel<OBJ_PET>::li].col;
+  constexpr uint32_t TBYTES = CObj<E>::f[it_string_field<E>()].cnt;
   static_assert(ItModel<OBJ_PET>::elem == OBJ_TAG && ItModel<OBJ_ORDER>::elem < 0 && ItModel<OBJ_USER>::elem < 0 && ItModel<OBJ_ORDER>::li < 0 && ItModel<OBJ_USER>::li < 0, "lists are Pet's");
-  constexpr int ES = it_string_field<E>();
-  constexpr uint32_t ESLOT = CObj<E>::f[ES].cnt; /* arena of the elements' strings */
-  auto photos = [&](uint32_t k) { return sh.w[k].nphoto; };
-  auto tags = [&](uint32_t k) { return sh.w[k].ntag; };
-  auto photo_ref = [&](uint32_t w, uint32_t j) { return strs[sh.w[w].str0 + sh.w[w].words - 1u - j]; };
-  auto tag_row = [&](uint32_t w, uint32_t j) { return strs + sh.w[w].str0 + 3u * j; };
+  const uint32_t lane = tid & 31, warp = tid >> 5;
+  const uint32_t nline = sh.nline, nchunk = (nline + 31u) >> 5;
+  if (sh.nspecial) {
+    if (sh.nspecial > IT_MAX_SPECIAL) return false;
+    item_specials(a, sh, win, pairs, tid);
+    __syncthreads();
+  }
+  item_walk<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid);
+  if (SCHEMA == PJ_SCHEMA_MIXED) __syncthreads(); /* the lines were walked in another order */
+  uint32_t* row = rows + (tid < nline ? tid : 0u) * STRIDE; /* from here on a thread has the line of its number */
+  {
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, tid < nline && (row[IW_FLAGS] & IF_ODD));
+    if (lane == 0) sh.oddmask[warp] = m;
+  }
+  if (__syncthreads_or((int)sh.slow)) return false;
+  ck[2] = clock64();
+  {
+    uint32_t nodd = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
+    if (nodd) {
+      item_packs<SCHEMA, ARR>(a, g, sh, win, pairs, rows, nodd);
+      if (__syncthreads_or((int)sh.slow)) return false;
+    }
+  }
+  ck[7] = clock64();
 
-  /* this warp's 32 records */
-  const uint32_t i = warp * 32u + lane;
-  const bool live = i < nrec;
-  uint32_t first_of_warp;
-  const uint32_t r = item_row_of(sh, i, &first_of_warp);
-  uint32_t* row = rows + r * STRIDE;
-
-  /* ---- values; list elements are taken from the last warp on, the records from the first ---- */
-  if (warp < nchunk) item_record_values<SCHEMA>(a, win, row, live);
-  if constexpr (SL::lists) {
-    for (uint32_t u = IT_WARPS - 1u - warp; u < nu1 + nu0; u += IT_WARPS) {
-      uint32_t w, j0, n = 0;
-      if (u < nu1) {
-        item_unit(u, tags, &w, &j0);
-        const uint32_t j = j0 + lane;
-        if (j < sh.w[w].ntag) {
-          const uint32_t* e = tag_row(w, j);
-          item_element_values<E>(a, win, e, rows + (e[2] >> 16) * STRIDE);
-          if ((e[2] >> (4 + ES)) & 1u) n = (e[ES] >> 16) & 0x7FFFu;
-        }
-      } else {
-        item_unit(u - nu1, photos, &w, &j0);
-        const uint32_t j = j0 + lane;
-        if (j < sh.w[w].nphoto) n = photo_ref(w, j) >> 16;
+  /* ---- values: fields x groups of 32 lines ---- */
+  {
+    uint32_t u = 0;
+#pragma unroll 1
+    for (int v = VU_COUNT - 1; v >= 0; --v) {
+      if (!((ItemValueUnits<SCHEMA>::mask >> v) & 1u)) continue;
+      for (uint32_t c = 0; c < nchunk; ++c, ++u) {
+        if ((u & (IT_WARPS - 1u)) != warp) continue;
+        const uint32_t i = c * 32u + lane;
+        item_value<SCHEMA>(a, win, pairs, rows, rows + (i < nline ? i : 0u) * STRIDE, i < nline, (uint32_t)v);
       }
-      n = __reduce_add_sync(0xFFFFFFFFu, n);
-      if (lane == 0) { if (u < nu1) sh.usum[1][u] = n; else sh.usum[0][u - nu1] = n; }
     }
   }
   __syncthreads();
 
-  ck[7] = clock64();
   /* ---- verdicts and sums ---- */
-  uint32_t nP = 0, nT = 0, type = PJ_TYPE_NONE;
-  bool good = false;
   if (warp < nchunk) {
-    const uint32_t e = live ? row[IW_ERR] : IE_NONE;
-    uint32_t flags = live ? row[IW_FLAGS] : 0u;
-    good = live && e == IE_NONE;
-    if constexpr (SL::lists) { /* list lengths: the running counts less those of the warp's record before */
-      if (live) {
-        const uint32_t cum = row[IW_CUM], prev = i != first_of_warp ? rows[(r - 1u) * STRIDE + IW_CUM] : 0u;
-        nP = (cum & 0xFFFFu) - (prev & 0xFFFFu); nT = (cum >> 16) - (prev >> 16);
-        if (!good && (nP | nT)) { /* the elements of a failed record count for nothing */
-          uint32_t w = 0, u0 = 0, u1 = 0, at = 0;
-#pragma unroll
-          for (uint32_t k = 0; k < IT_WARPS; ++k) if (r >= sh.w[k].row0 && sh.w[k].nrec && r < sh.w[k].row0 + sh.w[k].nrec) w = k;
-          for (uint32_t k = 0; k < w; ++k) { u0 += (sh.w[k].nphoto + 31u) >> 5; u1 += (sh.w[k].ntag + 31u) >> 5; }
-          for (at = prev & 0xFFFFu; at < (cum & 0xFFFFu); ++at) atomicSub(&sh.usum[0][u0 + (at >> 5)], photo_ref(w, at) >> 16);
-          for (at = prev >> 16; at < (cum >> 16); ++at) {
-            const uint32_t* t = tag_row(w, at);
-            if ((t[2] >> (4 + ES)) & 1u) atomicSub(&sh.usum[1][u1 + (at >> 5)], (t[ES] >> 16) & 0x7FFFu);
-          }
-          nP = 0; nT = 0;
-        }
+    uint32_t flags = tid < nline ? row[IW_FLAGS] : 0u;
+    const bool rec = (flags & IF_RECORD) != 0;
+    uint32_t e = rec ? row[IW_ERR] : IE_NONE;
+    uint32_t type = item_type<SCHEMA>(flags);
+    if (rec && e == IE_NONE) { /* required properties; is the model known? */
+      if (SCHEMA == PJ_SCHEMA_MIXED && type == PJ_TYPE_NONE) e = IE_REFUSED;
+      else {
+        const uint32_t req = type == PJ_TYPE_PET ? (uint32_t)CObj<OBJ_PET>::required : (type == PJ_TYPE_ORDER ? (uint32_t)CObj<OBJ_ORDER>::required : (uint32_t)CObj<OBJ_USER>::required);
+        if (((flags >> IF_PRESENT) & req) != req) e = ((row[IW_POS] >> 16) << 8) | (uint32_t)PJ_E_REQUIRED;
       }
     }
-    if (live && !good) {
-      sh.bad = 1;
+    const bool good = rec && e == IE_NONE;
+    if (rec && !good) {
       uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
       if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
         const uint64_t s0 = g.v0 + (row[IW_POS] & 0xFFFFu) - g.mis;
-        uint64_t limit = a.limit;
-        if (ARR) { uint64_t p = s0; while (p < a.len && !((a.sep[p >> 6] >> (p & 63)) & 1u)) ++p; limit = p; }
-        item_exact<SCHEMA>(a, s0, limit, &kind, &off);
-        if (!kind) sh.slow = 1; /* a valid record of a kind the fast steps do not know */
+        item_exact<SCHEMA>(a, s0, ARR ? g.v0 + (sh.line[tid + 1u] & 0xFFFFu) - 1u - g.mis : a.limit, &kind, &off);
+        if (!kind) sh.slow = 1; /* a valid record of a kind the other steps do not know */
       }
-      row[IW_ERR] = kind; row[IW_FLAGS] = IF_BAD | off;
-      flags = 0;
+      flags = IF_BAD | IF_RECORD | off;
+      row[IW_FLAGS] = flags; row[IW_ERR] = kind;
     }
-    if (good) type = item_type<SCHEMA>(flags);
-    const uint32_t bl = __ballot_sync(0xFFFFFFFFu, live);
-    if (lane == 0) sh.csum[IT_REC][warp] = (uint32_t)__popc(bl);
+    if (!good) type = PJ_TYPE_NONE;
+    const uint32_t br = __ballot_sync(0xFFFFFFFFu, rec);
+    if (lane == 0) sh.csum[IT_REC][warp] = (uint32_t)__popc(br);
     if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
       const uint32_t bp = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_PET), bo = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_ORDER), bu = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_USER);
       if (lane == 0) { sh.csum[SLOT_ROWS_PET][warp] = (uint32_t)__popc(bp); sh.csum[SLOT_ROWS_ORD][warp] = (uint32_t)__popc(bo); sh.csum[SLOT_ROWS_USR][warp] = (uint32_t)__popc(bu); }
     }
     if constexpr (SL::lists) {
-      item_sum_fields<OBJ_PET, true, 0u, 0u>(sh, row, type == PJ_TYPE_PET, flags, warp, lane, nP, nT);
-      /* from an element's number in its warp to its place behind the group's first */
-      const uint32_t exP = warp_incl_scan(nP) - nP, exT = warp_incl_scan(nT) - nT;
-      if (good) {
-        const uint32_t prev = i != first_of_warp ? rows[(r - 1u) * STRIDE + IW_CUM] : 0u;
-        row[IW_ERR] = ((exP - (prev & 0xFFFFu)) & 0xFFFFu) | ((exT - (prev >> 16)) << 16);
-      }
+      const bool pet = type == PJ_TYPE_PET;
+      item_sum_strings<OBJ_PET, true, 0u, 0u>(sh, row, pet, flags, warp, lane);
+      const uint32_t n0 = __reduce_add_sync(0xFFFFFFFFu, pet ? row[IW_LIST] >> 16 : 0u), n1 = __reduce_add_sync(0xFFFFFFFFu, pet ? row[LW] >> 16 : 0u);
+      const uint32_t b0 = __reduce_add_sync(0xFFFFFFFFu, pet ? row[LW + 1u] & 0xFFFFu : 0u), b1 = __reduce_add_sync(0xFFFFFFFFu, pet ? row[LW + 1u] >> 16 : 0u);
+      if (lane == 0) { sh.csum[PCNT][warp] = n0; sh.csum[TCNT][warp] = n1; sh.csum[PCNT + 1u][warp] = b0; sh.csum[TBYTES][warp] = b1; }
     }
-    if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) item_sum_fields<OBJ_USER, true, 0u, 0u>(sh, row, type == PJ_TYPE_USER, flags, warp, lane, 0u, 0u);
+    if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) item_sum_strings<OBJ_USER, true, 0u, 0u>(sh, row, type == PJ_TYPE_USER, flags, warp, lane);
   }
-  __syncthreads();
-  if (sh.slow) return false;
+  if (__syncthreads_or((int)sh.slow)) return false;
   ck[3] = clock64();
 
   /* ---- where everything of the tile goes ---- */
   if (warp == 0) {
 #pragma unroll
-    for (uint32_t k0 = 0; k0 < IT_NLB; k0 += 4) { /* four counters a time, eight groups of records each */
+    for (uint32_t k0 = 0; k0 < IT_NLB; k0 += 4) { /* four counters a time, eight groups of lines each */
       if (!((SL::mask >> k0) & 15u)) continue;
       const uint32_t k = k0 + (lane >> 3), c = lane & 7u;
-      const bool bytes = SL::lists && (k == PCNT + 1u || k == ESLOT); /* come from the groups of list elements */
-      uint32_t v = (((SL::mask >> k) & 1u) && !bytes && c < nchunk) ? sh.csum[k][c] : 0u;
+      const bool used = (SL::mask >> k) & 1u;
+      const uint32_t v = used && c < nchunk ? sh.csum[k][c] : 0u;
       uint32_t inc = v;
 #pragma unroll
       for (int d = 1; d < 8; d <<= 1) { const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, d, 8); if (c >= (uint32_t)d) inc += x; }
-      if (((SL::mask >> k) & 1u) && !bytes) { sh.csum[k][c] = inc - v; if (c == 7) sh.tot[k] = inc; }
-    }
-    if constexpr (SL::lists) {
-#pragma unroll
-      for (uint32_t l = 0; l < 2; ++l) {
-        const uint32_t n = l ? nu1 : nu0;
-        const uint32_t v0 = 2 * lane < n ? sh.usum[l][2 * lane] : 0u, v1 = 2 * lane + 1 < n ? sh.usum[l][2 * lane + 1] : 0u;
-        const uint32_t inc = warp_incl_scan(v0 + v1);
-        __syncwarp();
-        sh.usum[l][2 * lane] = inc - v0 - v1; sh.usum[l][2 * lane + 1] = inc - v1;
-        if (lane == 31) sh.tot[l ? ESLOT : PCNT + 1u] = inc;
-      }
+      if (used) { sh.csum[k][c] = inc - v; if (c == 7) sh.tot[k] = inc; }
     }
     __syncwarp();
     item_resolve<SCHEMA>(a, sh, tile, lane);
+    if (lane == 0) sh.next = 0;
   }
   __syncthreads();
   ck[4] = clock64();
   if (!sh.ok) return true;
 
-  /* ---- emission ---- */
-  if (warp < nchunk) {
-    const uint64_t rec = (uint64_t)sh.base[IT_REC] + i; /* chunk starts are multiples of 32 records */
-    const uint32_t flags = good ? row[IW_FLAGS] : 0u;
-    const uint32_t bg = __ballot_sync(0xFFFFFFFFu, good), bl = __ballot_sync(0xFFFFFFFFu, live);
-    if (lane == 0) {
-      if (bl != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(bl & ~bg));
-      if (bg) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg));
-    }
-    if (live) {
-      colp<uint64_t>(&a.cols, PJ_COL_REC_START)[rec] = a.goff + g.v0 + (row[IW_POS] & 0xFFFFu) - g.mis;
-      colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[rec] = good ? 0 : (uint8_t)row[IW_ERR];
-      colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[rec] = good ? 0u : row[IW_FLAGS] & ~IF_BAD;
-    }
-    if constexpr (SCHEMA == PJ_SCHEMA_PET) item_emit_fields<OBJ_PET, true, 0u, 0u>(a, sh, win, row, live, flags, rec, warp, nP, nT);
-    else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) item_emit_fields<OBJ_ORDER, true, 0u, 0u>(a, sh, win, row, live, flags, rec, warp, 0u, 0u);
-    else if constexpr (SCHEMA == PJ_SCHEMA_USER) item_emit_fields<OBJ_USER, true, 0u, 0u>(a, sh, win, row, live, flags, rec, warp, 0u, 0u);
-    else {
-      const uint32_t lt = (1u << lane) - 1u;
-      const uint32_t bp = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_PET), bo = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_ORDER), bu = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_USER);
+  /* ---- emission: four kinds of columns x groups of 32 lines ---- */
+  for (uint32_t u = warp; u < 4u * nchunk; u += IT_WARPS) {
+    /* the kinds cost differently, so that a warp does not get the same one every time */
+    const uint32_t what = u / nchunk, c = u - what * nchunk, i = c * 32u + lane;
+    const uint32_t* r = rows + (i < nline ? i : 0u) * STRIDE;
+    ItemOut o;
+    o.win = win; o.row = r; o.chunk = c;
+    const uint32_t f = i < nline ? r[IW_FLAGS] : 0u;
+    const bool rec = (f & IF_RECORD) != 0, good = rec && !(f & IF_BAD);
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t br = __ballot_sync(0xFFFFFFFFu, rec);
+    const uint64_t n = (uint64_t)sh.base[IT_REC] + sh.csum[IT_REC][c] + (uint32_t)__popc(br & lt);
+    const uint32_t type = good ? item_type<SCHEMA>(f) : (uint32_t)PJ_TYPE_NONE;
+    o.flags = good ? f : 0u;
+    o.at = n;
+    uint32_t bp = 0, bo = 0, bu = 0;
+    if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+      bp = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_PET); bo = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_ORDER); bu = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_USER);
       const uint32_t mine = type == PJ_TYPE_PET ? bp : (type == PJ_TYPE_ORDER ? bo : bu);
       const uint32_t slot = type == PJ_TYPE_PET ? SLOT_ROWS_PET : (type == PJ_TYPE_ORDER ? SLOT_ROWS_ORD : SLOT_ROWS_USR);
-      const uint32_t out = sh.base[slot] + sh.csum[slot][warp] + (uint32_t)__popc(mine & lt);
-      if (live) {
-        colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[rec] = (uint8_t)type;
-        colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[rec] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : out;
-      }
-      if (bp) item_emit_fields<OBJ_PET, true, 0u, 0u>(a, sh, win, row, type == PJ_TYPE_PET, type == PJ_TYPE_PET ? flags : 0u, out, warp, type == PJ_TYPE_PET ? nP : 0u, type == PJ_TYPE_PET ? nT : 0u);
-      if (bo) item_emit_fields<OBJ_ORDER, true, 0u, 0u>(a, sh, win, row, type == PJ_TYPE_ORDER, type == PJ_TYPE_ORDER ? flags : 0u, out, warp, 0u, 0u);
-      if (bu) item_emit_fields<OBJ_USER, true, 0u, 0u>(a, sh, win, row, type == PJ_TYPE_USER, type == PJ_TYPE_USER ? flags : 0u, out, warp, 0u, 0u);
+      o.at = sh.base[slot] + sh.csum[slot][c] + (uint32_t)__popc(mine & lt);
     }
-  }
-  if constexpr (SL::lists) {
-    const bool bad = sh.bad != 0;
-    for (;;) { /* groups of list elements go to whoever is free */
-      uint32_t u = 0;
-      if (lane == 0) u = atomicAdd(&sh.next, 1u);
-      u = __shfl_sync(0xFFFFFFFFu, u, 0);
-      if (u >= nu0 + nu1) break;
-      uint32_t w, j0;
-      if (u < nu0) {
-        item_unit(u, photos, &w, &j0);
-        const uint32_t j = j0 + lane;
-        const bool has = j < sh.w[w].nphoto;
-        bool ok = has;
-        uint32_t at = 0, ref = 0;
-        if (has) {
-          ref = photo_ref(w, j);
-          if (bad) {
-            const uint32_t pr = item_photo_row(sh, rows, STRIDE, w, j);
-            ok = !(rows[pr * STRIDE + IW_FLAGS] & IF_BAD);
-            if (ok) at = item_child_place<false>(sh, rows, STRIDE, w, pr, j, PCNT);
-          } else {
-            at = j;
-#pragma unroll
-            for (uint32_t k = 0; k < IT_WARPS; ++k) if (k < w) at += sh.w[k].nphoto;
-          }
-        }
-        item_emit_string(a, PCOL + 1u, win, ok, (uint64_t)sh.base[PCNT] + at, ref, ok, sh.base[PCNT + 1u] + sh.usum[0][u]);
-      } else {
-        item_unit(u - nu0, tags, &w, &j0);
-        const uint32_t j = j0 + lane;
-        const bool has = j < sh.w[w].ntag;
-        bool ok = has;
-        uint32_t at = 0;
-        const uint32_t* e = tag_row(w, has ? j : j0);
-        if (has) {
-          const uint32_t pr = e[2] >> 16;
-          if (bad) {
-            ok = !(rows[pr * STRIDE + IW_FLAGS] & IF_BAD);
-            if (ok) at = item_child_place<true>(sh, rows, STRIDE, w, pr, j, TCNT);
-          } else {
-            at = j;
-#pragma unroll
-            for (uint32_t k = 0; k < IT_WARPS; ++k) if (k < w) at += sh.w[k].ntag;
-          }
-        }
-        item_emit_element<E>(a, win, e, ok, (uint64_t)sh.base[TCNT] + at, sh.base[ESLOT] + sh.usum[1][u - nu0]);
+    if (what == 3u) {
+      const uint32_t bg = __ballot_sync(0xFFFFFFFFu, good);
+      if (lane == 0) {
+        if (br != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(br & ~bg));
+        if (bg) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg));
       }
+      if (rec) {
+        colp<uint64_t>(&a.cols, PJ_COL_REC_START)[n] = a.goff + g.v0 + (r[IW_POS] & 0xFFFFu) - g.mis;
+        colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[n] = good ? 0 : (uint8_t)r[IW_ERR];
+        colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[n] = good ? 0u : f & ~(IF_BAD | IF_RECORD);
+        if constexpr (SCHEMA == PJ_SCHEMA_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
+        else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
+        else if constexpr (SCHEMA == PJ_SCHEMA_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
+        else {
+          colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[n] = (uint8_t)type;
+          colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[n] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : (uint32_t)o.at;
+          if (type == PJ_TYPE_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
+          else if (type == PJ_TYPE_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
+          else if (type == PJ_TYPE_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
+        }
+      }
+    } else if (what == 2u) {
+      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings<OBJ_PET, true, 0u, 0u>(a, sh, o); }
+      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings<OBJ_USER, true, 0u, 0u>(a, sh, o); }
+      else if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+        o.has_row = type == PJ_TYPE_PET;
+        if (bp) item_emit_strings<OBJ_PET, true, 0u, 0u>(a, sh, o);
+        o.has_row = type == PJ_TYPE_USER;
+        if (bu) item_emit_strings<OBJ_USER, true, 0u, 0u>(a, sh, o);
+      }
+    } else if constexpr (SL::lists) {
+      const bool pet = type == PJ_TYPE_PET;
+      o.has_row = SCHEMA == PJ_SCHEMA_PET ? rec : pet;
+      if (SCHEMA == PJ_SCHEMA_PET || bp) { if (what == 0u) item_emit_lists<false>(a, sh, o, pairs, pet); else item_emit_lists<true>(a, sh, o, pairs, pet); }
     }
   }
   if (tile == a.ntiles - 1) item_close_offsets(a, sh, tid);
@@ -1538,20 +1709,34 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
 
 template <int SCHEMA> struct ItTablesOf { static constexpr ItTables t = it_tables(SCHEMA); };
 template <int SCHEMA> __device__ const ItTables d_item_tables = ItTablesOf<SCHEMA>::t;
-template <bool ARR> struct ItGapTableOf { static constexpr ItGapTable t = it_gap_table(ARR ? IT_ARR_SEP : (uint32_t)'\n'); };
-template <bool ARR> __device__ const ItGapTable d_gap_table = ItGapTableOf<ARR>::t;
+struct ItGapTableOf { static constexpr ItGapTable t = it_gap_table(); };
+static __device__ const ItGapTable d_gap_table = ItGapTableOf::t;
+
+template <int SCHEMA, bool ARR>
+__device__ __forceinline__ bool item_try(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t* rows, uint32_t tile, uint32_t tid, long long* ck) {
+  bool fine = item_index<ARR, false>(a, g, sh, win, strs, tid, tile);
+  if (__syncthreads_or(fine && sh.viol)) { /* some record ends inside a string */
+    for (uint32_t k = tid; k < IT_MAX_STRS / 32; k += IT_THREADS) { sh.special[k] = 0; sh.broken[k] = 0; }
+    if (tid == 0) sh.nspecial = 0;
+    __syncthreads();
+    fine = item_index<ARR, true>(a, g, sh, win, strs, tid, tile);
+  }
+  if (__syncthreads_or(!fine || sh.slow)) return false; /* (decided together: what a warp that goes on may set there comes too late) */
+  ck[6] = clock64();
+  return item_tile<SCHEMA, ARR>(a, g, sh, win, strs, rows, tile, tid, ck);
+}
 
 template <int SCHEMA>
-__global__ void __launch_bounds__(IT_THREADS, 3) k_parse_items(const __grid_constant__ ItemArgs a) {
+__global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __grid_constant__ ItemArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) ItemShared sh;
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const ItemLayout lay = item_layout(a.win_bytes, a.str_ratio, a.row_cap, ItStride<SCHEMA>::n);
+  const uint32_t tid = threadIdx.x;
+  const ItemLayout lay = item_layout(a.win_bytes, a.str_words, a.row_cap, ItStride<SCHEMA>::n);
   uint8_t* win = smem + lay.win;
   uint32_t* strs = reinterpret_cast<uint32_t*>(smem + lay.strs);
   uint32_t* rows = reinterpret_cast<uint32_t*>(smem + lay.rows);
 
-  if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); mbar_init(&sh.mbar, 1); sh.slow = 0; sh.bad = 0; sh.next = 0; }
+  if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); mbar_init(&sh.mbar, 1); sh.slow = 0; sh.next = 0; sh.viol = 0; sh.odd = 0; sh.nspecial = 0; }
   __syncthreads();
   const uint32_t tile = sh.tile;
   if (tile >= a.ntiles) return;
@@ -1565,11 +1750,9 @@ __global__ void __launch_bounds__(IT_THREADS, 3) k_parse_items(const __grid_cons
   if (g.copy_bytes && tid == 0) { mbar_expect_tx(&sh.mbar, g.copy_bytes); bulk_g2s(win, a.in - mis + g.v0, g.copy_bytes, &sh.mbar); }
   for (uint32_t k = tid; k < IT_SLOTS * 8; k += IT_THREADS) (&sh.key[0][0])[k] = (&d_item_tables<SCHEMA>.key[0][0])[k];
   for (uint32_t k = tid; k < IT_SLOTS * 3; k += IT_THREADS) (&sh.field[0][0])[k] = (&d_item_tables<SCHEMA>.field[0][0])[k];
-  {
-    const uint32_t* gt = reinterpret_cast<const uint32_t*>(a.sep ? d_gap_table<true>.e : d_gap_table<false>.e);
-    for (uint32_t k = tid; k < IG_SLOTS * 4; k += IT_THREADS) reinterpret_cast<uint32_t*>(sh.gap)[k] = gt[k];
-  }
-  for (uint32_t k = tid; k < IT_WARPS * IT_MAX_STRS / 32; k += IT_THREADS) { (&sh.special[0][0])[k] = 0; (&sh.broken[0][0])[k] = 0; }
+  for (uint32_t k = tid; k < IG_SLOTS * 4; k += IT_THREADS) reinterpret_cast<uint32_t*>(sh.gap)[k] = reinterpret_cast<const uint32_t*>(d_gap_table.e)[k];
+  for (uint32_t k = tid; k < IT_MAX_STRS / 32; k += IT_THREADS) { sh.special[k] = 0; sh.broken[k] = 0; }
+  if (tid < IT_MAX_LINES / 32) sh.oddline[tid] = 0;
   int stage_failed = 0;
   if (g.copy_bytes) stage_failed = !mbar_wait_bounded(&sh.mbar, 0, a.spin_limit_ns);
   if (__syncthreads_or(stage_failed)) { /* the block gives up together: the results of the call are void */
@@ -1581,26 +1764,14 @@ __global__ void __launch_bounds__(IT_THREADS, 3) k_parse_items(const __grid_cons
     }
     return;
   }
-  if (tid < 64) win[g.hi_valid + tid] = '\n';
+  if (tid < 48) win[g.hi_valid + tid] = '\n';
   __syncthreads();
   ck[1] = clock64();
 
   bool done = false;
-  if (a.sep) {
-    /* a document that is not one clean array is left to the other road */
-    const bool clean = a.res->doc_err_off == ~0ull && a.res->n_openers == 1u && !a.res->arr_final_s && a.res->arr_final_d == 0;
-    if (clean) {
-      if (!item_index<true>(a, g, sh, win, strs, warp, lane, tile)) sh.slow = 1;
-      __syncthreads();
-      ck[6] = clock64();
-      if (!sh.slow) done = item_tile<SCHEMA, true>(a, g, sh, win, strs, rows, tile, tid, ck);
-    }
-  } else {
-    if (!item_index<false>(a, g, sh, win, strs, warp, lane, tile)) sh.slow = 1;
-    __syncthreads();
-    ck[6] = clock64();
-    if (!sh.slow) done = item_tile<SCHEMA, false>(a, g, sh, win, strs, rows, tile, tid, ck);
-  }
+  if (a.sep) { /* a document that is not one clean array is left to the other road */
+    if (a.res->doc_err_off == ~0ull && a.res->n_openers == 1u && !a.res->arr_final_s && a.res->arr_final_d == 0) done = item_try<SCHEMA, true>(a, g, sh, win, strs, rows, tile, tid, ck);
+  } else done = item_try<SCHEMA, false>(a, g, sh, win, strs, rows, tile, tid, ck);
   if (!done) {
     __syncthreads();
     item_slow_tile<SCHEMA>(a, g, sh, tile, tid);

@@ -3,13 +3,13 @@
  * of pj_schema.h: where a record's values stand in its row of shared memory, the hash table of property names and
  * what a property name means in which object.
  *
- * Rows. Every record of a tile has one row of 32-bit words. Words 0-3 are the row's own (flags, first failure, start
- * and closing brace, running list counts); then follow property 0 (`id`, the one property the models share by name,
+ * Rows. Every line of a tile has one row of 32-bit words. Words 0-3 are the row's own (flags, first failure, first byte and
+ * closing brace, list of strings); then follow property 0 (`id`, the one property the models share by name,
  * kind and position), the enums, the other properties and those of the embedded object. While a record is tokenised a
  * word holds a reference to the value's text (ItemRef); int64 takes two words, a date-time four, because the decoded
  * value replaces the reference.
  *
- * Elements of a list of objects have rows of three words: one per property (at most two) and a flag word.
+ * An element of a list of objects is three words: the two of its integer and one for its string and flags (ItElem).
  */
 #ifndef PJ_ITEM_TABLES_H
 #define PJ_ITEM_TABLES_H
@@ -28,11 +28,14 @@ namespace pj {
 enum { IS_ROOT = 0, IS_CHILD = 1, IS_LIST = 2, IS_ELEM = 3 };
 /* what follows the colon of a key: a string, a number or literal, `{"`, `["`, `[{"`, `{}`, `[]` */
 enum { IV_NONE = 0, IV_STR = 1, IV_SCALAR = 2, IV_OBJ = 3, IV_LIST = 4, IV_ELEM = 5, IV_EOBJ = 6, IV_ELIST = 7 };
-/* words of a record's row */
-enum { IW_FLAGS = 0, IW_ERR = 1, IW_POS = 2, IW_CUM = 3, IW_FIELDS = 4 };
+/* words of a record's row; where a model has lists two more stand behind its fields: the list of objects (like IW_LIST: first
+ * string or row | length << 16) and the bytes of both lists' strings (list of strings | list of objects << 16) */
+enum { IW_FLAGS = 0, IW_ERR = 1, IW_POS = 2, IW_LIST = 3, IW_FIELDS = 4 };
 /* IW_FLAGS: bits 0-11 keys met, 12-23 values present, 24-26 models the record cannot be (mixed streams), 27: the text of a
- * string was decoded in place (positions in the window are not the input's any more) */
-static constexpr uint32_t IF_SEEN = 0, IF_PRESENT = 12, IF_NOTMODEL = 24, IF_MOVED = 1u << 27;
+ * string was decoded in place (positions in the window are not the input's any more), 28: the line is a record, 29: the walk
+ * did not recognise it, 30: the list of objects has rows of its own (else it is read off its strings), 31: the record failed
+ * (the rest then is the failure's offset) */
+static constexpr uint32_t IF_PRESENT = 12, IF_NOTMODEL = 24, IF_MOVED = 1u << 27, IF_RECORD = 1u << 28, IF_ODD = 1u << 29, IF_ROWS = 1u << 30, IF_BAD = 1u << 31;
 static constexpr uint32_t IB_CHILD = 8;  /* first bit of the embedded object's properties */
 static constexpr uint32_t IB_SHARED = 10; /* a property of several models at different places of theirs (mixed streams) */
 /* IW_ERR: window offset << 8 | kind of the first failure in reading order; kind 0xFF: the exact parser has to say */
@@ -91,9 +94,9 @@ PJ_CX uint32_t it_max(uint32_t a, uint32_t b) { return a > b ? a : b; }
 /* words per row of a schema; odd, so that a warp that walks 32 rows meets 32 banks */
 template <int SCHEMA>
 struct ItStride {
-  static constexpr uint32_t raw = SCHEMA == PJ_SCHEMA_PET ? ItWords<OBJ_PET>::n
+  static constexpr uint32_t raw = SCHEMA == PJ_SCHEMA_PET ? ItWords<OBJ_PET>::n + 2u
                                   : (SCHEMA == PJ_SCHEMA_ORDER ? ItWords<OBJ_ORDER>::n
-                                     : (SCHEMA == PJ_SCHEMA_USER ? ItWords<OBJ_USER>::n : it_max(ItWords<OBJ_PET>::n, it_max(ItWords<OBJ_ORDER>::n, ItWords<OBJ_USER>::n))));
+                                     : (SCHEMA == PJ_SCHEMA_USER ? ItWords<OBJ_USER>::n : it_max(ItWords<OBJ_PET>::n + 2u, it_max(ItWords<OBJ_ORDER>::n, ItWords<OBJ_USER>::n))));
   static constexpr uint32_t n = raw | 1u;
 };
 
@@ -203,62 +206,58 @@ PJ_CX ItTables it_tables(int schema) {
   return t;
 }
 /* ---- gaps --------------------------------------------------------------------------------------------------------
- * What stands between two strings, without blanks and with '0' for a number or a literal, is one of 36 texts of at most
- * eight bytes in every valid record. Each tells what the string before it is (a key and the kind of its value, or a value),
- * in which object the string must lie and which one the next lies in. */
+ * What stands between two strings of a record, or behind its last one, without blanks and with '0' for a number or a literal,
+ * is one of 26 texts of at most eight bytes in every valid record. Each tells what the string before it is (a key and the kind
+ * of its value, or a value), in which object that string must lie and which one the next lies in. */
 struct ItGap {
-  /* bits 0-2 IV_*, 3-6 object the gap needs (15: any), 7-8 object it leads to, 9: it tells the object at all, 10: a record
-     ends, 11: an element of a list of objects begins, 12: the string before is a key, 13: valid, 14: ends with a brace */
-  static PJ_CX uint32_t make(uint32_t vk, uint32_t need, uint32_t out, bool telling, bool ends, bool elem, bool key, bool brace) {
-    return vk | (need << 3) | (out << 7) | ((telling ? 1u : 0u) << 9) | ((ends ? 1u : 0u) << 10) | ((elem ? 1u : 0u) << 11) | ((key ? 1u : 0u) << 12) | (1u << 13) | ((brace ? 1u : 0u) << 14);
+  /* bits 0-2 IV_*, 3-6 object the gap needs (15: any), 7-8 object it leads to, 9: it tells the object at all, 10: the record
+     ends, 11: an element of a list of objects begins, 12: the string before is a key, 13: valid */
+  static PJ_CX uint32_t make(uint32_t vk, uint32_t need, uint32_t out, bool telling, bool ends, bool elem, bool key) {
+    return vk | (need << 3) | (out << 7) | ((telling ? 1u : 0u) << 9) | ((ends ? 1u : 0u) << 10) | ((elem ? 1u : 0u) << 11) | ((key ? 1u : 0u) << 12) | (1u << 13);
   }
-  static constexpr uint32_t TELLS = 1u << 9, ENDS = 1u << 10, ELEM = 1u << 11, KEY = 1u << 12, VALID = 1u << 13, BRACE = 1u << 14;
+  static constexpr uint32_t TELLS = 1u << 9, ENDS = 1u << 10, ELEM = 1u << 11, KEY = 1u << 12;
   static PJ_CX uint32_t vk(uint32_t d) { return d & 7u; }
   static PJ_CX uint32_t need(uint32_t d) { return (d >> 3) & 15u; }
   static PJ_CX uint32_t out(uint32_t d) { return (d >> 7) & 3u; }
 };
-static constexpr uint32_t IG_SLOTS = 64;
+static constexpr uint32_t IG_SLOTS = 32;
 struct ItGapEntry { uint32_t lo, hi, desc, len; };
 struct ItGapTable { ItGapEntry e[IG_SLOTS]; bool ok; };
-/* multipliers without a collision among the 36 texts, for records that end with a line feed and with the array separator */
-PJ_CX uint32_t it_gap_hash(uint32_t lo, uint32_t hi, bool arr) { return (arr ? lo * 0xB4D1A147u + hi * 0xAB0D6DF3u : lo * 0xA32D7C7Fu + hi * 0x780EC42Fu) >> 26; }
-PJ_CX void it_gap_add(ItGapTable& t, const char* head, const char* tail, uint32_t sep, uint32_t desc) {
+/* multipliers without a collision among the 26 texts, found by search */
+PJ_CX uint32_t it_gap_hash(uint32_t lo, uint32_t hi) { return (lo * 0x3ED35535u + hi * 0x43D40BE5u) >> 27; }
+PJ_CX void it_gap_add(ItGapTable& t, const char* head, const char* tail, uint32_t desc) {
   uint32_t w[2] = {0, 0};
   uint32_t n = 0;
   for (int part = 0; part < 2; ++part)
-    for (const char* p = part ? tail : head; *p; ++p, ++n) w[n >> 2] |= (*p == 'L' ? sep : (uint32_t)(uint8_t)*p) << (8 * (n & 3));
-  ItGapEntry& e = t.e[it_gap_hash(w[0], w[1], sep != '\n')];
+    for (const char* p = part ? tail : head; *p; ++p, ++n) w[n >> 2] |= (uint32_t)(uint8_t)*p << (8 * (n & 3));
+  ItGapEntry& e = t.e[it_gap_hash(w[0], w[1])];
   t.ok = t.ok && e.desc == 0 && n <= 8;
   e.lo = w[0]; e.hi = w[1]; e.desc = desc; e.len = n;
 }
-PJ_CX ItGapTable it_gap_table(uint32_t sep) {
+PJ_CX ItGapTable it_gap_table() {
   ItGapTable t{};
   t.ok = true;
-  it_gap_add(t, ":", "", sep, ItGap::make(IV_STR, 15, 0, false, false, false, true, false));
-  it_gap_add(t, ":{", "", sep, ItGap::make(IV_OBJ, IS_ROOT, IS_CHILD, true, false, false, true, true));
-  it_gap_add(t, ":[", "", sep, ItGap::make(IV_LIST, IS_ROOT, IS_LIST, true, false, false, true, false));
-  it_gap_add(t, ":[{", "", sep, ItGap::make(IV_ELEM, IS_ROOT, IS_ELEM, true, false, true, true, true));
+  it_gap_add(t, ":", "", ItGap::make(IV_STR, 15, 0, false, false, false, true));
+  it_gap_add(t, ":{", "", ItGap::make(IV_OBJ, IS_ROOT, IS_CHILD, true, false, false, true));
+  it_gap_add(t, ":[", "", ItGap::make(IV_LIST, IS_ROOT, IS_LIST, true, false, false, true));
+  it_gap_add(t, ":[{", "", ItGap::make(IV_ELEM, IS_ROOT, IS_ELEM, true, false, true, true));
   for (uint32_t h = 0; h < 4; ++h) {
     const char* const heads[4] = {"", ":0", ":[]", ":{}"};
     const uint32_t vk = h == 0 ? IV_NONE : (h == 1 ? IV_SCALAR : (h == 2 ? IV_ELIST : IV_EOBJ));
-    it_gap_add(t, heads[h], ",", sep, ItGap::make(vk, 15, 0, false, false, false, h != 0, false));
-    it_gap_add(t, heads[h], "}L{", sep, ItGap::make(vk, IS_ROOT, IS_ROOT, true, true, false, h != 0, true));
-    it_gap_add(t, heads[h], "}L", sep, ItGap::make(vk, IS_ROOT, IS_ROOT, true, true, false, h != 0, false));
+    it_gap_add(t, heads[h], ",", ItGap::make(vk, 15, 0, false, false, false, h != 0));
+    it_gap_add(t, heads[h], "}", ItGap::make(vk, IS_ROOT, IS_ROOT, true, true, false, h != 0));
     if (h > 1) continue; /* empty containers stand in the root only */
-    it_gap_add(t, heads[h], "},", sep, ItGap::make(vk, IS_CHILD, IS_ROOT, true, false, false, h != 0, false));
-    it_gap_add(t, heads[h], "],", sep, ItGap::make(vk, IS_LIST, IS_ROOT, true, false, false, h != 0, false));
-    it_gap_add(t, heads[h], "}],", sep, ItGap::make(vk, IS_ELEM, IS_ROOT, true, false, false, h != 0, false));
-    it_gap_add(t, heads[h], "},{", sep, ItGap::make(vk, IS_ELEM, IS_ELEM, true, false, true, h != 0, true));
-    it_gap_add(t, heads[h], "}}L{", sep, ItGap::make(vk, IS_CHILD, IS_ROOT, true, true, false, h != 0, true));
-    it_gap_add(t, heads[h], "]}L{", sep, ItGap::make(vk, IS_LIST, IS_ROOT, true, true, false, h != 0, true));
-    it_gap_add(t, heads[h], "}]}L{", sep, ItGap::make(vk, IS_ELEM, IS_ROOT, true, true, false, h != 0, true));
-    it_gap_add(t, heads[h], "}}L", sep, ItGap::make(vk, IS_CHILD, IS_ROOT, true, true, false, h != 0, false));
-    it_gap_add(t, heads[h], "]}L", sep, ItGap::make(vk, IS_LIST, IS_ROOT, true, true, false, h != 0, false));
-    it_gap_add(t, heads[h], "}]}L", sep, ItGap::make(vk, IS_ELEM, IS_ROOT, true, true, false, h != 0, false));
+    it_gap_add(t, heads[h], "},", ItGap::make(vk, IS_CHILD, IS_ROOT, true, false, false, h != 0));
+    it_gap_add(t, heads[h], "],", ItGap::make(vk, IS_LIST, IS_ROOT, true, false, false, h != 0));
+    it_gap_add(t, heads[h], "}],", ItGap::make(vk, IS_ELEM, IS_ROOT, true, false, false, h != 0));
+    it_gap_add(t, heads[h], "},{", ItGap::make(vk, IS_ELEM, IS_ELEM, true, false, true, h != 0));
+    it_gap_add(t, heads[h], "}}", ItGap::make(vk, IS_CHILD, IS_ROOT, true, true, false, h != 0));
+    it_gap_add(t, heads[h], "]}", ItGap::make(vk, IS_LIST, IS_ROOT, true, true, false, h != 0));
+    it_gap_add(t, heads[h], "}]}", ItGap::make(vk, IS_ELEM, IS_ROOT, true, true, false, h != 0));
   }
   return t;
 }
-static_assert(it_gap_table('\n').ok && it_gap_table(0x1E).ok, "gap texts hash without collisions");
+static_assert(it_gap_table().ok, "gap texts hash without collisions");
 
 static_assert(it_root_word<OBJ_PET>(0) == it_root_word<OBJ_ORDER>(0) && it_root_word<OBJ_PET>(0) == it_root_word<OBJ_USER>(0), "id at one place");
 static_assert(it_root_word<OBJ_PET>(5) == it_root_word<OBJ_ORDER>(4), "status at one place");

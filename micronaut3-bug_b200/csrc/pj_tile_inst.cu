@@ -22,7 +22,7 @@ cudaError_t PJ_CAT(item_init_, PJ_TILE_SCHEMA)(const Schema* s) {
   return e;
 }
 cudaError_t PJ_CAT(item_launch_, PJ_TILE_SCHEMA)(const ItemArgs* a, cudaStream_t stream) {
-  const ItemLayout l = item_layout(a->win_bytes, a->str_ratio, a->row_cap, ItStride<PJ_TILE_SCHEMA>::n);
+  const ItemLayout l = item_layout(a->win_bytes, a->str_words, a->row_cap, ItStride<PJ_TILE_SCHEMA>::n);
   k_parse_items<PJ_TILE_SCHEMA><<<a->ntiles, IT_THREADS, l.total, stream>>>(*a);
   return cudaGetLastError();
 }
