@@ -281,20 +281,23 @@ TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   /* room behind the tile for its last records: 13 average records reach the longest ones of a skewed distribution */
   uint32_t slack = (uint32_t)(avg * 13);
   slack = (slack < 4096 ? 4096u : (slack > 28672 ? 28672u : slack)) & ~15u;
-  uint32_t per_word = 8; /* window bytes per word for strings */
-  uint64_t tile = (uint64_t)(avg * 190); /* at most 256 records */
-  if (tile > 32768) tile = 32768;
-  if (len / 296 < tile) { tile = len / 296; if (tile < 4096) tile = 4096; per_word = 2; } /* few tiles: one for every SM's two halves, and room enough */
+  uint32_t per_word = 9; /* window bytes per word for strings */
+  /* what the block indexes in one step, or so that most tiles have fewer than three quarters of the lines they may have */
+  uint64_t tile = IT_STEP - (uint64_t)(2 * avg), few = (uint64_t)(avg * (IT_MAX_LINES * 47 / 64));
+  if (avg * 4 > IT_STEP) tile = IT_STEP / 2;
+  if (tile > few) tile = few;
+  /* few tiles: one for every block that can be resident, and room enough */
+  if (len / (148 * IT_BLOCKS) < tile) { tile = len / (148 * IT_BLOCKS); if (tile < 4096) tile = 4096; per_word = 2; }
   if (c->tile_bytes_opt) { tile = c->tile_bytes_opt; if (tile < ST_MIN_TILE_BYTES) tile = ST_MIN_TILE_BYTES; if (tile > 32768) tile = 32768; }
   for (;;) {
     t.tile_bytes = (uint32_t)(tile & ~31ull);
     if (t.tile_bytes < ST_MIN_TILE_BYTES) t.tile_bytes = ST_MIN_TILE_BYTES;
     t.win_bytes = t.tile_bytes + slack;
     t.str_words = t.win_bytes / per_word;
-    const double recs = (double)t.tile_bytes / avg * 1.4 + 40;
-    t.row_cap = recs > 272 ? 272u : (uint32_t)recs;
+    const double recs = (double)t.tile_bytes / avg * 1.3 + 24;
+    t.row_cap = recs > IT_MAX_LINES ? IT_MAX_LINES : (uint32_t)recs;
     if (per_word == 2 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_words, t.row_cap, item_stride(schema)).total <= BUDGET) return t;
-    tile -= 1024;
+    tile -= 512;
   }
 }
 

@@ -40,19 +40,22 @@
 namespace pj {
 
 #ifndef PJ_IT_BLOCKS
-#define PJ_IT_BLOCKS 3 /* resident blocks per SM the kernel is compiled for */
+#define PJ_IT_BLOCKS 5 /* resident blocks per SM the kernel is compiled for */
 #endif
 static constexpr uint32_t IT_BLOCKS = PJ_IT_BLOCKS;
-static constexpr uint32_t IT_THREADS = 256;
+static constexpr uint32_t IT_THREADS = 128;
 static constexpr uint32_t IT_WARPS = IT_THREADS / 32;
-static constexpr uint32_t IT_STEP = IT_THREADS * 32; /* bytes the block indexes per step */
+static constexpr uint32_t IT_BLK = 9;                /* 16-byte blocks a thread indexes per step: odd, so that a warp's 128-bit loads are free of bank conflicts */
+static constexpr uint32_t IT_SPAN = IT_BLK * 16;
+static constexpr uint32_t IT_SPANW = (IT_SPAN + 31) / 32;
+static constexpr uint32_t IT_STEP = IT_THREADS * IT_SPAN; /* bytes the block indexes per step */
 static constexpr uint32_t IT_FRONT = 32;             /* bytes before the window that may be read (and mean nothing) */
-static constexpr uint32_t IT_PAD = 64;               /* ... and behind it */
+static constexpr uint32_t IT_PAD = IT_SPAN + 16;               /* ... and behind it */
 static constexpr uint32_t IT_MAX_LINES = IT_THREADS; /* lines per tile */
 static constexpr uint32_t IT_MAX_STRS = 4096;        /* strings per tile */
-static constexpr uint32_t IT_MAX_SPECIAL = 1024;     /* strings per tile that need a closer look */
+static constexpr uint32_t IT_MAX_SPECIAL = 512;     /* strings per tile that need a closer look */
 static constexpr uint32_t IT_MAX_WIN = 65536 - 64;   /* window offsets are 16-bit */
-static constexpr uint32_t IT_SHORT = 8;              /* a list of up to this many elements is its line's lane's, a longer one the warp's */
+static constexpr uint32_t IT_STAGE = 256;            /* words of a warp to put strings together in */
 static constexpr uint32_t IT_MAX_DYN_SMEM = 200 * 1024; /* dynamic shared memory of a block */
 static constexpr uint32_t IT_NONE = 0xFFFFFFFFu;
 
@@ -112,19 +115,25 @@ PJ_HD ItemLayout item_layout(uint32_t win_bytes, uint32_t str_words, uint32_t ro
 }
 
 struct ItemShared {
-  __align__(16) uint32_t key[IT_SLOTS][8];
-  __align__(16) ItGapEntry gap[IG_SLOTS];
-  uint32_t field[3][IT_SLOTS];
+  union { /* what reads the input, and what writes the columns */
+    struct {
+      __align__(16) uint32_t key[IT_SLOTS][8];
+      __align__(16) ItGapEntry gap[IG_SLOTS];
+      uint32_t field[3][IT_SLOTS];
+      uint32_t special[IT_MAX_STRS / 32]; /* per string: it holds a backslash, a control character or a byte beyond ASCII ... */
+      uint32_t broken[IT_MAX_STRS / 32];  /* ... and is not a valid one */
+      uint16_t special_list[IT_MAX_SPECIAL];
+    };
+    uint32_t stage[IT_WARPS][IT_STAGE];
+  };
   uint32_t line[IT_MAX_LINES + 1];         /* window offset of a line's first byte | strings before it << 16 */
-  uint32_t special[IT_MAX_STRS / 32];      /* per string: it holds a backslash, a control character or a byte beyond ASCII ... */
-  uint32_t broken[IT_MAX_STRS / 32];       /* ... and is not a valid one */
   uint32_t oddline[IT_MAX_LINES / 32];     /* lines with a string that was decoded in place or is not valid */
   uint32_t oddmask[IT_WARPS];              /* lines the walk did not recognise */
-  uint16_t special_list[IT_MAX_SPECIAL];
+  uint8_t owner[IT_WARPS][32];
   uint8_t perm[IT_THREADS], cls[4][IT_WARPS]; /* mixed streams: lines by model */
   uint32_t csum[IT_NLB][IT_WARPS];         /* counters: sums per 32 lines, then exclusive prefixes */
   uint32_t tot[IT_NLB], base[IT_NLB];
-  uint32_t wsum[2][IT_WARPS], wmin[3][IT_WARPS];
+  uint32_t wsum[IT_WARPS], wmin[3][IT_WARPS];
   uint32_t nspecial, odd;                  /* odd: some record ends inside a string */
   uint32_t nstr, nline, stop;              /* strings, lines, last separator */
   uint32_t free_word;                      /* first free word behind the strings */
@@ -257,181 +266,206 @@ __device__ __forceinline__ void item_close_offsets(const ItemArgs& a, const Item
 __device__ __forceinline__ uint32_t item_low(int32_t n) { return n <= 0 ? 0u : (n >= 32 ? 0xFFFFFFFFu : ((1u << n) - 1u)); }
 /* 0x80 in every byte of w that equals c (c repeated), exactly */
 __device__ __forceinline__ uint32_t item_eq4(uint32_t w, uint32_t c) { return ~((((w ^ c) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | (w ^ c)) & 0x80808080u; }
-/* the eight flags (0x80 per byte) of two words as bits, times 128, added to acc */
-__device__ __forceinline__ uint32_t item_gather(uint32_t f0, uint32_t f1) { return __dp4a(f1, 0x80402010u, __dp4a(f0, 0x08040201u, 0u)) >> 7; }
-template <class F>
-__device__ __forceinline__ uint32_t item_mask32(const uint32_t* w, F f) {
-  uint32_t m = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) m |= item_gather(f(w[2 * k]), f(w[2 * k + 1])) << (8 * k);
-  return m;
-}
-__device__ __forceinline__ uint32_t item_mask_of(const uint32_t* f) {
-  const uint32_t g0 = __dp4a(f[1], 0x80402010u, __dp4a(f[0], 0x08040201u, 0u)), g1 = __dp4a(f[3], 0x80402010u, __dp4a(f[2], 0x08040201u, 0u));
-  const uint32_t g2 = __dp4a(f[5], 0x80402010u, __dp4a(f[4], 0x08040201u, 0u)), g3 = __dp4a(f[7], 0x80402010u, __dp4a(f[6], 0x08040201u, 0u));
-  return ((g0 + (g1 << 8)) >> 7) | ((g2 + (g3 << 8)) << 9); /* multiples of 128 below 2^15 each */
+/* 0x80 per byte of four words as 16 bits */
+__device__ __forceinline__ uint32_t item_gather16(uint32_t f0, uint32_t f1, uint32_t f2, uint32_t f3) {
+  return (__dp4a(f1, 0x80402010u, __dp4a(f0, 0x08040201u, 0u)) + (__dp4a(f3, 0x80402010u, __dp4a(f2, 0x08040201u, 0u)) << 8)) >> 7;
 }
 __device__ __forceinline__ uint32_t item_prefix_xor(uint32_t x) {
   x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8; x ^= x << 16;
   return x;
 }
-/* bytes escaped by an odd run of backslashes (32 bytes; carry: the first byte is escaped) */
-__device__ __forceinline__ uint32_t item_escaped(uint32_t bs, uint32_t carry) {
-  const uint32_t even = 0x55555555u;
-  bs &= ~carry;
-  const uint32_t follows = (bs << 1) | carry;
-  const uint32_t odd_starts = bs & ~even & ~follows;
-  const uint32_t sum = odd_starts + bs;
-  return (even ^ (sum << 1)) & follows;
-}
-
 /* The strings and lines the tile owns. False (for every thread): the tile does not fit, the block has to take the other road.
  * CAREFUL: some record ends inside a string; its separator then counts as the string's closing quote. */
 template <bool ARR, bool CAREFUL>
 __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t tid, uint32_t tile) {
   const uint32_t lane = tid & 31, warp = tid >> 5;
   bool started = !ARR && tile == 0 && a.is_first && a.limit > 0, done = false, fine = true;
-  uint32_t start = g.mis, stop = 0, nq = 0, nline = 0, step = 0;
-  const int32_t end_valid = (int32_t)g.hi_valid + (g.to_limit ? 1 : 0); /* the end of the input counts as a separator */
+  uint32_t start = g.mis, stop = 0, nq = 0, nline = 0;
+  const int32_t end_valid = (int32_t)g.hi_valid + (g.to_limit ? 1 : 0), lo_valid = (int32_t)g.lo_valid; /* the end of the input counts as a separator */
   uint16_t* q16 = reinterpret_cast<uint16_t*>(strs);
   if (tid == 0 && started) sh.line[0] = start;
-  for (uint32_t o = 0; !done; o += IT_STEP, ++step) {
+  for (uint32_t o = 0; !done; o += IT_STEP) {
     if ((int32_t)o >= end_valid) { fine = !started; break; } /* the last record runs out of the window */
     if (!started && o >= g.own_end) break;
-    const int32_t p0 = (int32_t)(o + 32u * tid);
-    uint32_t w[8];
+    const int32_t p0 = (int32_t)(o + IT_SPAN * tid);
+    /* quotes, separators, control characters (later: all that takes a closer look), a bit per byte of the thread's */
+    uint32_t q[IT_SPANW], t[IT_SPANW], c[IT_SPANW];
+    uint32_t bs = 0, hb = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < IT_SPANW; ++i) q[i] = t[i] = c[i] = 0;
+    const uint4* src = reinterpret_cast<const uint4*>(win + p0);
     if (p0 < end_valid) {
-      const uint4* src = reinterpret_cast<const uint4*>(win + p0);
-      const uint4 x = src[0], y = src[1];
-      w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w; w[4] = y.x; w[5] = y.y; w[6] = y.z; w[7] = y.w;
-    } else {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) w[k] = 0x41414141u;
-    }
-    /* Bytes below 0x23 are few: of them, bit 5 tells the printable ones from the control characters, and of the printable
-       ones ( space ! " ) bit 1 tells the quotes. Or-ed up over the words: backslashes, bytes beyond ASCII. */
-    uint32_t fq[8], fc[8], bs = 0, hb = 0;
+      for (uint32_t b = 0; b < IT_BLK; ++b) {
+        const uint4 v = src[b];
+        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+        /* Bytes below 0x23 are few: of them, bit 5 tells the printable ones from the control characters, and of the printable
+           ones ( space ! " ) bit 1 tells the quotes. Or-ed up over the words: backslashes, bytes beyond ASCII. */
+        uint32_t fq[4], fc[4];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t x = w[k];
-      const uint32_t low = ~(((x & 0x7F7F7F7Fu) + 0x5D5D5D5Du) | x) & 0x80808080u;
-      const uint32_t printable = low & (x << 2);
-      fq[k] = printable & (x << 6);
-      fc[k] = low & ~(x << 2);
-      bs |= ~(((x ^ 0x5C5C5C5Cu) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu);
-      hb |= x;
-    }
-    uint32_t q = item_mask_of(fq);
-    const bool has_sp = ((bs | hb) & 0x80808080u) != 0;
-    uint32_t c = 0, t = 0; /* control characters, separators */
-    if (fc[0] | fc[1] | fc[2] | fc[3] | fc[4] | fc[5] | fc[6] | fc[7]) c = item_mask_of(fc);
-    const bool edge = !started || o + IT_STEP > g.own_end || (int32_t)(o + IT_STEP) > end_valid || o < g.lo_valid;
-    if (edge) {
-      const uint32_t vm = item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
-      q &= vm; c &= vm;
-    }
-    if (ARR) {
-      const int64_t bit = (int64_t)g.v0 + p0 - (int64_t)g.mis; /* input offset of the thread's first byte */
-      const int64_t nwords32 = (int64_t)((a.len + 31) >> 5);
-      const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.sep);
-      const int64_t i0 = bit >> 5; /* floor: the first tile may begin a few bytes before the input */
-      const uint32_t b0 = i0 >= 0 && i0 < nwords32 ? sw[i0] : 0u, b1 = i0 + 1 >= 0 && i0 + 1 < nwords32 ? sw[i0 + 1] : 0u;
-      t = __funnelshift_r(b0, b1, (uint32_t)(bit & 31)) & item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
-      if (g.to_limit && (int32_t)g.hi_valid >= p0 && (int32_t)g.hi_valid < p0 + 32) t |= 1u << (g.hi_valid - (uint32_t)p0);
-    } else {
-      for (uint32_t m = c; m; m &= m - 1u) {
-        const uint32_t b = (uint32_t)__ffs((int)m) - 1u;
-        if (win[p0 + b] == '\n') t |= 1u << b;
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t low = ~(((x[k] & 0x7F7F7F7Fu) + 0x5D5D5D5Du) | x[k]) & 0x80808080u;
+          fq[k] = low & (x[k] << 2) & (x[k] << 6);
+          fc[k] = low & ~(x[k] << 2);
+          bs |= ~(((x[k] ^ 0x5C5C5C5Cu) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu);
+          hb |= x[k];
+        }
+        q[b >> 1] |= item_gather16(fq[0], fq[1], fq[2], fq[3]) << (16u * (b & 1u));
+        c[b >> 1] |= item_gather16(fc[0], fc[1], fc[2], fc[3]) << (16u * (b & 1u));
+      }
+      if (p0 < lo_valid || p0 + (int32_t)IT_SPAN > end_valid) {
+#pragma unroll
+        for (uint32_t i = 0; i < IT_SPANW; ++i) {
+          const int32_t p = p0 + (int32_t)(32u * i);
+          const uint32_t vm = item_low(end_valid - p) & ~item_low(lo_valid - p);
+          q[i] &= vm; c[i] &= vm;
+        }
+      }
+      if (ARR) {
+        const int64_t bit = (int64_t)g.v0 + p0 - (int64_t)g.mis; /* input offset of the thread's first byte */
+        const int64_t nwords32 = (int64_t)((a.len + 31) >> 5);
+        const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.sep);
+        const int64_t i0 = bit >> 5; /* floor: the first tile may begin a few bytes before the input */
+        uint32_t b0 = i0 >= 0 && i0 < nwords32 ? sw[i0] : 0u;
+#pragma unroll
+        for (uint32_t i = 0; i < IT_SPANW; ++i) {
+          const int64_t n = i0 + 1 + (int64_t)i;
+          const uint32_t b1 = n >= 0 && n < nwords32 ? sw[n] : 0u;
+          const int32_t p = p0 + (int32_t)(32u * i);
+          const int32_t room = p0 + (int32_t)IT_SPAN < end_valid ? p0 + (int32_t)IT_SPAN : end_valid;
+          t[i] = __funnelshift_r(b0, b1, (uint32_t)(bit & 31)) & item_low(room - p) & ~item_low(lo_valid - p);
+          if (g.to_limit && (int32_t)g.hi_valid >= p && (int32_t)g.hi_valid < p + 32 && (int32_t)g.hi_valid < room) t[i] |= 1u << (g.hi_valid - (uint32_t)p);
+          c[i] &= ~t[i];
+          b0 = b1;
+        }
+      } else {
+#pragma unroll
+        for (uint32_t i = 0; i < IT_SPANW; ++i) {
+          for (uint32_t m = c[i]; m; m &= m - 1u) {
+            const uint32_t b = (uint32_t)__ffs((int)m) - 1u;
+            if (win[p0 + (int32_t)(32u * i + b)] == '\n') t[i] |= 1u << b;
+          }
+          c[i] &= ~t[i];
+        }
       }
     }
-    uint32_t act = 0xFFFFFFFFu;
-    if (edge) { /* where the first own line begins and the last one ends */
-      const uint32_t own = item_low((int32_t)g.own_end - p0);
-      const uint32_t c0 = t & own, c1 = t & ~own;
-      const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, c0 != 0), b1 = __ballot_sync(0xFFFFFFFFu, c1 != 0);
-      const uint32_t m0 = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)c0), b0 ? __ffs((int)b0) - 1 : 0); /* behind the separator */
-      const uint32_t m1 = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)c1) - 1u, b1 ? __ffs((int)b1) - 1 : 0);
-      if (lane == 0) { sh.wmin[0][warp] = b0 ? m0 : IT_NONE; sh.wmin[1][warp] = b1 ? m1 : IT_NONE; }
+    /* Escaped quotes, and the bytes that make a string one to decode. A quote is escaped when an odd run of backslashes ends
+       before it. */
+    const bool my_sp = p0 < end_valid && (((bs | hb) & 0x80808080u) != 0 || (p0 > lo_valid && win[p0 - 1] == '\\'));
+    if (__any_sync(0xFFFFFFFFu, my_sp)) {
+      if (my_sp) {
+#pragma unroll
+        for (uint32_t b = 0; b < IT_BLK; ++b) {
+          const uint4 v = src[b];
+          const uint32_t B = item_gather16(item_eq4(v.x, 0x5C5C5C5Cu), item_eq4(v.y, 0x5C5C5C5Cu), item_eq4(v.z, 0x5C5C5C5Cu), item_eq4(v.w, 0x5C5C5C5Cu));
+          const uint32_t H = item_gather16(v.x & 0x80808080u, v.y & 0x80808080u, v.z & 0x80808080u, v.w & 0x80808080u);
+          const int32_t p = p0 + (int32_t)(16u * b);
+          const uint32_t before = p > lo_valid && win[p - 1] == '\\' ? 1u : 0u;
+          for (uint32_t m = (q[b >> 1] >> (16u * (b & 1u))) & ((B << 1) | before) & 0xFFFFu; m; m &= m - 1u) {
+            const int32_t at = p + __ffs((int)m) - 1;
+            int32_t r = at - 1;
+            while (r >= lo_valid && win[r] == '\\' && at - r < 4096) --r;
+            if (at - r >= 4096) sh.slow = 1;
+            if ((at - 1 - r) & 1) q[b >> 1] &= ~((m & (0u - m)) << (16u * (b & 1u)));
+          }
+          c[b >> 1] |= (B | H) << (16u * (b & 1u)); /* (only those inside a string will count) */
+        }
+      }
+    }
+    /* where the first own line begins and the last one ends */
+    {
+      uint32_t m0 = IT_NONE, m1 = IT_NONE;
+#pragma unroll
+      for (int i = (int)IT_SPANW - 1; i >= 0; --i) {
+        const int32_t p = p0 + 32 * i;
+        const uint32_t own = item_low((int32_t)g.own_end - p), t0 = t[i] & own, t1 = t[i] & ~own;
+        if (t0) m0 = (uint32_t)(p + __ffs((int)t0)); /* behind the separator */
+        if (t1) m1 = (uint32_t)(p + __ffs((int)t1) - 1);
+      }
+      m0 = __reduce_min_sync(0xFFFFFFFFu, m0); m1 = __reduce_min_sync(0xFFFFFFFFu, m1);
+      if (lane == 0) { sh.wmin[0][warp] = m0; sh.wmin[1][warp] = m1; }
       __syncthreads();
       uint32_t x0 = IT_NONE, x1 = IT_NONE;
 #pragma unroll
       for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t y0 = sh.wmin[0][k], y1 = sh.wmin[1][k]; x0 = y0 < x0 ? y0 : x0; x1 = y1 < x1 ? y1 : x1; }
       if (!started && x0 != IT_NONE) { started = true; start = x0; if (tid == 0) sh.line[0] = start; }
       if (!started) { __syncthreads(); continue; }
-      act = ~item_low((int32_t)start - p0);
-      if (x1 != IT_NONE) { stop = x1; done = true; act &= item_low((int32_t)stop + 1 - p0); }
-      t &= act; q &= act;
-    }
-    const uint32_t ctl = c & act & ~t;
-    uint32_t B = 0, H = 0;
-    const bool warp_sp = __any_sync(0xFFFFFFFFu, has_sp || (lane == 0 && p0 > 0 && p0 <= end_valid && win[p0 - 1] == '\\'));
-    if (warp_sp) {
-      B = item_mask32(w, [](uint32_t x) { return item_eq4(x, 0x5C5C5C5Cu); });
-      H = item_mask32(w, [](uint32_t x) { return x & 0x80808080u; }) & act;
-      if (edge) B &= item_low(end_valid - p0) & ~item_low((int32_t)g.lo_valid - p0);
-      /* is the first byte escaped? An odd run of backslashes ends before it (looked at only where there is one) */
-      uint32_t cin = 0;
-      {
-        int32_t r = p0 - 1;
-        while (r >= (int32_t)g.lo_valid && r < end_valid && win[r] == '\\' && p0 - 1 - r < 4096) --r;
-        cin = (uint32_t)(p0 - 1 - r) & 1u;
-        if (p0 - 1 - r >= 4096) sh.slow = 1;
+      int32_t last = 0x7FFFFFFF;
+      if (x1 != IT_NONE) { stop = x1; done = true; last = (int32_t)x1 + 1; }
+      if (p0 < (int32_t)start || p0 + (int32_t)IT_SPAN > last) {
+#pragma unroll
+        for (uint32_t i = 0; i < IT_SPANW; ++i) {
+          const int32_t p = p0 + (int32_t)(32u * i);
+          const uint32_t act = item_low(last - p) & ~item_low((int32_t)start - p);
+          q[i] &= act; t[i] &= act; c[i] &= act;
+        }
       }
-      q &= ~item_escaped(B, cin);
-      B &= act;
     }
     /* order of the quotes (low half) and separators (high half) */
-    uint32_t at, total;
-    for (uint32_t round = 0;; ++round) {
-      const uint32_t n = (uint32_t)__popc(q) | ((uint32_t)__popc(t) << 16);
+    uint32_t at, total, any = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < IT_SPANW; ++i) any |= t[i];
+    for (;;) {
+      uint32_t n = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < IT_SPANW; ++i) n += (uint32_t)__popc(q[i]) + ((uint32_t)__popc(t[i]) << 16);
       const uint32_t inc = warp_incl_scan(n);
-      uint32_t* ws = sh.wsum[CAREFUL ? 0 : (step & 1u)];
-      if (lane == 31) ws[warp] = inc;
+      if (lane == 31) sh.wsum[warp] = inc;
       __syncthreads();
       at = inc - n; total = 0;
 #pragma unroll
-      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t x = ws[k]; if (k < warp) at += x; total += x; }
-      uint32_t odd = 0;
-      for (uint32_t m = t & ~q; m; m &= m - 1u) { /* separators this thread sees with a string open */
-        const uint32_t low = (m & (0u - m)) - 1u;
-        if ((nq + (at & 0xFFFFu) + (uint32_t)__popc(q & low)) & 1u) { odd = m & (0u - m); break; }
+      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t x = sh.wsum[k]; if (k < warp) at += x; total += x; }
+      uint32_t odd = IT_NONE; /* the first separator this thread sees with a string open */
+      if (any) {
+        uint32_t n0 = nq + (at & 0xFFFFu);
+#pragma unroll
+        for (uint32_t i = 0; i < IT_SPANW; ++i) {
+          for (uint32_t m = t[i] & ~q[i]; m; m &= m - 1u) {
+            const uint32_t low = (m & (0u - m)) - 1u;
+            if (((n0 + (uint32_t)__popc(q[i] & low)) & 1u) && odd == IT_NONE) odd = (uint32_t)(p0 + 32 * (int32_t)i + __ffs((int)m) - 1);
+          }
+          n0 += (uint32_t)__popc(q[i]);
+        }
       }
-      if (!CAREFUL) { if (odd) sh.viol = 1; break; }
-      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, odd != 0);
-      const uint32_t mine = __shfl_sync(0xFFFFFFFFu, (uint32_t)p0 + (uint32_t)__ffs((int)odd), bal ? __ffs((int)bal) - 1 : 0);
-      if (lane == 0) sh.wmin[2][warp] = bal ? mine : IT_NONE;
+      if (!CAREFUL) { if (odd != IT_NONE) sh.viol = 1; break; }
+      const uint32_t mine = __reduce_min_sync(0xFFFFFFFFu, odd);
+      if (lane == 0) sh.wmin[2][warp] = mine;
       __syncthreads();
       uint32_t first = IT_NONE;
 #pragma unroll
       for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t y = sh.wmin[2][k]; first = y < first ? y : first; }
       if (first == IT_NONE) break;
-      if (odd && (uint32_t)p0 + (uint32_t)__ffs((int)odd) == first) q |= odd;
-      __syncthreads();
-    }
-    const uint32_t q0 = nq + (at & 0xFFFFu); /* number of this thread's first quote */
-    /* strings that need a closer look */
-    if ((B | H | ctl) != 0) {
-      const uint32_t instr = item_prefix_xor(q) ^ ((q0 & 1u) ? 0xFFFFFFFFu : 0u);
-      for (uint32_t m = (B | H | ctl) & instr; m; m &= m - 1u) {
-        const uint32_t k = (q0 + (uint32_t)__popc(q & ((m & (0u - m)) - 1u))) >> 1;
-        if (k < IT_MAX_STRS) {
-          const uint32_t bit = 1u << (k & 31u);
-          if (!(atomicOr(&sh.special[k >> 5], bit) & bit)) {
-            const uint32_t i = atomicAdd(&sh.nspecial, 1u);
-            if (i < IT_MAX_SPECIAL) sh.special_list[i] = (uint16_t)k;
-          }
-        }
+      if (odd == first) { /* closed there */
+#pragma unroll
+        for (uint32_t i = 0; i < IT_SPANW; ++i) { const uint32_t d = first - (uint32_t)(p0 + 32 * (int32_t)i); if (d < 32u) q[i] |= 1u << d; }
       }
     }
     {
       const uint32_t n = nq + (total & 0xFFFFu), nl = nline + (total >> 16);
       if (n / 2u + 2u > a.str_words || n / 2u >= IT_MAX_STRS || nl > IT_MAX_LINES || nl > a.row_cap) { fine = false; break; }
-      uint16_t* d = q16 + q0;
-      for (uint32_t m = q; m; m &= m - 1u) *d++ = (uint16_t)((uint32_t)p0 + (uint32_t)__ffs((int)m) - 1u);
-      uint32_t i = nline + (at >> 16) + 1u;
-      for (uint32_t m = t; m; m &= m - 1u, ++i) { /* the line behind every separator */
-        const uint32_t bit = m & (0u - m);
-        sh.line[i] = ((uint32_t)p0 + (uint32_t)__ffs((int)m)) | (((q0 + (uint32_t)__popc(q & (bit | (bit - 1u)))) >> 1) << 16);
+      uint32_t k = nq + (at & 0xFFFFu), ln = nline + (at >> 16) + 1u;
+#pragma unroll
+      for (uint32_t i = 0; i < IT_SPANW; ++i) {
+        const uint32_t p = (uint32_t)(p0 + 32 * (int32_t)i);
+        for (uint32_t m = c[i] & (item_prefix_xor(q[i]) ^ (0u - (k & 1u))); m; m &= m - 1u) { /* strings that need a closer look */
+          const uint32_t z = (k + (uint32_t)__popc(q[i] & ((m & (0u - m)) - 1u))) >> 1;
+          if (z < IT_MAX_STRS) {
+            const uint32_t bit = 1u << (z & 31u);
+            if (!(atomicOr(&sh.special[z >> 5], bit) & bit)) {
+              const uint32_t e = atomicAdd(&sh.nspecial, 1u);
+              if (e < IT_MAX_SPECIAL) sh.special_list[e] = (uint16_t)z;
+            }
+          }
+          /* on behind this string's end */
+          const uint32_t rest = q[i] & ~((m & (0u - m)) - 1u);
+          if (!rest) break;
+          m &= ~((rest & (0u - rest)) - 1u) | (m & (0u - m));
+        }
+        for (uint32_t m = t[i]; m; m &= m - 1u, ++ln) { /* the line behind every separator */
+          const uint32_t bit = m & (0u - m);
+          sh.line[ln] = (p + (uint32_t)__ffs((int)m)) | (((k + (uint32_t)__popc(q[i] & (bit | (bit - 1u)))) >> 1) << 16);
+        }
+        for (uint32_t m = q[i]; m; m &= m - 1u) q16[k++] = (uint16_t)(p + (uint32_t)__ffs((int)m) - 1u);
       }
       nq = n; nline = nl;
     }
@@ -1192,8 +1226,25 @@ __device__ __forceinline__ void item_elem_row(const uint8_t* win, uint32_t* e, u
   e[0] = (uint32_t)(uint64_t)val; e[1] = (uint32_t)((uint64_t)val >> 32);
   e[2] = ((p2 & 0xFFFFu) + 1u) | (((p2 >> 16) - (p2 & 0xFFFFu) - 1u) << 16) | 0xF0000000u;
 }
+/* The elements of the lists of 32 lines (n of a lane's), 32 at a time: f(line's lane, element of the line's list, live). */
+template <class F>
+__device__ __forceinline__ void item_each_element(uint8_t* owner, uint32_t n, F f) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t inc = warp_incl_scan(n), e = inc - n, total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+  const uint32_t some = __ballot_sync(0xFFFFFFFFu, n != 0);
+  if (n) owner[__popc(some & ((1u << lane) - 1u))] = (uint8_t)lane;
+  __syncwarp();
+  for (uint32_t r = 0; r < total; r += 32) {
+    const uint32_t before = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, n != 0 && e < r));
+    const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, n != 0 && e - r < 32u ? 1u << (e - r) : 0u);
+    const uint32_t src = owner[before + (uint32_t)__popc(starts & ((2u << lane) - 1u)) - 1u]; /* lane 31: 2 << 31 wraps to 0, so all ones */
+    const uint32_t se = __shfl_sync(0xFFFFFFFFu, e, (int)src);
+    f(src, r + lane - se, r + lane < total);
+  }
+  __syncwarp();
+}
 template <int SCHEMA>
-__device__ __forceinline__ void item_value(const ItemArgs& a, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t* row, bool live, uint32_t unit) {
+__device__ __forceinline__ void item_value(const ItemArgs& a, uint8_t* owner, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t* row, bool live, uint32_t unit) {
   const uint32_t flags = live ? row[IW_FLAGS] : 0u;
   const bool rec = (flags & IF_RECORD) && !(row[IW_ERR] != IE_NONE && (row[IW_ERR] & 0xFFu) == IE_REFUSED); /* (refused: the exact parser looks at it) */
   const uint32_t type = item_type<SCHEMA>(flags);
@@ -1253,13 +1304,11 @@ __device__ __forceinline__ void item_value(const ItemArgs& a, const uint8_t* win
   } else if constexpr (ItemSlots<SCHEMA>::lists) { /* elements of lists of objects that the walk found */
     const bool mine = rec && type == PJ_TYPE_PET && !(flags & IF_ROWS);
     const uint32_t l = mine ? row[ItWords<OBJ_PET>::n] : 0u, n = l >> 16;
-    uint32_t* e = pairs + (l & 0xFFFFu);
-    if (n <= IT_SHORT) for (uint32_t j = 0; j < n; ++j) item_elem_row(win, e + 3u * j, row);
-    for (uint32_t big = __ballot_sync(0xFFFFFFFFu, n > IT_SHORT); big; big &= big - 1u) {
-      const int src = __ffs((int)big) - 1;
-      const uint32_t bl = __shfl_sync(0xFFFFFFFFu, l, src), r = __shfl_sync(0xFFFFFFFFu, (uint32_t)(row - rows), src);
-      for (uint32_t j = threadIdx.x & 31u; j < bl >> 16; j += 32) item_elem_row(win, pairs + (bl & 0xFFFFu) + 3u * j, rows + r);
-    }
+    const uint32_t at = (uint32_t)(row - rows);
+    item_each_element(owner, n, [&](uint32_t src, uint32_t j, bool has) {
+      const uint32_t k = __shfl_sync(0xFFFFFFFFu, l, (int)src) & 0xFFFFu, r = __shfl_sync(0xFFFFFFFFu, at, (int)src);
+      if (has) item_elem_row(win, pairs + k + 3u * j, rows + r);
+    });
   }
 }
 
@@ -1290,10 +1339,47 @@ __device__ __forceinline__ void item_copy(uint8_t* dst, const uint8_t* win, uint
     if (t > 2) e[2] = (uint8_t)(last >> 16);
   }
 }
+/* The strings of a warp's lanes (n bytes at window offset pos), one behind the other from dst on: put together in shared
+ * memory, so that they leave in whole words side by side. Returns their bytes. rel: bytes of the lanes before. */
+__device__ __forceinline__ void item_emit_run(uint32_t* stage, uint8_t* dst, const uint8_t* win, uint32_t pos, uint32_t n, uint32_t rel, uint32_t total) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t d0 = (uint32_t)reinterpret_cast<uintptr_t>(dst) & 3u, end = d0 + total;
+  if (end > IT_STAGE * 4u) { if (n) item_copy(dst + rel, win, pos, n); return; }
+  const uint32_t nw = (end + 3u) >> 2;
+  for (uint32_t j = lane; j < nw; j += 32) stage[j] = 0;
+  __syncwarp();
+  if (n) {
+    const uint32_t b = d0 + rel, lead = b & 3u, k1 = (lead + n - 1u) >> 2; /* last word */
+    const int32_t from = (int32_t)pos - (int32_t)lead;
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(win) + (from >> 2);
+    const uint32_t sh = ((uint32_t)from & 3u) * 8u;
+    uint32_t* d = stage + (b >> 2);
+    uint32_t x0 = p[0], keep = 0xFFFFFFFFu << (8u * lead);
+    for (uint32_t k = 0; k < k1; ++k) {
+      const uint32_t x1 = p[k + 1];
+      const uint32_t v = __funnelshift_r(x0, x1, sh) & keep;
+      if (k == 0) atomicOr(d, v); else d[k] = v; /* the first word may be shared with the string before */
+      keep = 0xFFFFFFFFu;
+      x0 = x1;
+    }
+    const uint32_t v = __funnelshift_r(x0, p[k1 + 1], sh) & keep & (0xFFFFFFFFu >> (8u * (3u - ((lead + n - 1u) & 3u))));
+    atomicOr(d + k1, v);
+  }
+  __syncwarp();
+  uint32_t* out = reinterpret_cast<uint32_t*>(dst - d0);
+  for (uint32_t j = lane; j < nw; j += 32) {
+    const uint32_t v = stage[j];
+    if ((j > 0 || d0 == 0) && 4u * j + 4u <= end) out[j] = v;
+    else for (uint32_t b = 0; b < 4; ++b) if (4u * j + b >= d0 && 4u * j + b < end) reinterpret_cast<uint8_t*>(out + j)[b] = (uint8_t)(v >> (8u * b));
+  }
+  __syncwarp();
+}
 /* The place of a model root's row among 32 lines and what a lane needs to write it. */
 struct ItemOut {
   const uint8_t* win;
   const uint32_t* row;
+  uint32_t* stage;
+  uint8_t* owner;
   uint32_t flags, chunk;
   bool has_row;
   uint64_t at; /* row of the model's table */
@@ -1327,9 +1413,9 @@ __device__ __forceinline__ void item_emit_strings(const ItemArgs& a, const ItemS
     if constexpr (kind == K_STR) {
       const bool pr = o.has_row && ((o.flags >> (IF_PRESENT + BIT0 + I)) & 1u);
       const uint32_t ref = o.row[word], n = pr ? (ref >> 16) & 0x7FFFu : 0u;
-      const uint32_t at = sh.base[slot] + sh.csum[slot][o.chunk] + warp_incl_scan(n) - n;
-      if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at;
-      if (n) item_copy(colp<uint8_t>(&a.cols, col + 1) + at, o.win, ref & 0xFFFFu, n);
+      const uint32_t at = sh.base[slot] + sh.csum[slot][o.chunk], inc = warp_incl_scan(n);
+      if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at + inc - n;
+      item_emit_run(o.stage, colp<uint8_t>(&a.cols, col + 1) + at, o.win, ref & 0xFFFFu, n, inc - n, __shfl_sync(0xFFFFFFFFu, inc, 31));
     } else if constexpr (kind == K_OBJ) item_emit_strings<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
     item_emit_strings<OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
   }
@@ -1347,73 +1433,39 @@ __device__ __forceinline__ void item_sum_strings(ItemShared& sh, const uint32_t*
     item_sum_strings<OBJ, ROOT, WORD0, BIT0, I + 1>(sh, row, mine, flags, chunk, lane);
   }
 }
-/* one element of a list of strings: number r of the child table, its bytes at `at` */
-__device__ __forceinline__ void item_emit_list_str(const ItemArgs& a, uint32_t col, const uint8_t* win, uint32_t pr, uint64_t r, uint32_t at) {
-  colp<uint32_t>(&a.cols, col + 1)[r] = at;
-  item_copy(colp<uint8_t>(&a.cols, col + 2) + at, win, (pr & 0xFFFFu) + 1u, (pr >> 16) - (pr & 0xFFFFu) - 1u);
-}
-/* one element of a list of objects (three words at e) */
-template <int E, int I = 0>
-__device__ __forceinline__ void item_emit_elem(const ItemArgs& a, const uint8_t* win, const uint32_t* e, uint64_t r, uint32_t at) {
-  if constexpr (I == 0) colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((e[2] >> 28) & 3u);
-  if constexpr (I < CObj<E>::N) {
-    constexpr uint32_t kind = CObj<E>::f[I].kind, col = CObj<E>::f[I].col;
-    const bool pr = (e[2] >> (28 + I)) & 1u;
-    if constexpr (kind == K_STR) {
-      colp<uint32_t>(&a.cols, col)[r] = at;
-      if (pr) item_copy(colp<uint8_t>(&a.cols, col + 1) + at, win, e[2] & 0xFFFFu, (e[2] >> 16) & 0xFFFu);
-    } else colp<int64_t>(&a.cols, col)[r] = pr ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
-    item_emit_elem<E, I + 1>(a, win, e, r, at);
-  }
-}
-/* the lists of 32 lines, a line per lane; long lists by the whole warp */
+/* the lists of 32 lines, an element per lane */
 template <bool OBJS>
 __device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemShared& sh, const ItemOut& o, const uint32_t* pairs, bool mine) {
   constexpr int F = OBJS ? ItModel<OBJ_PET>::ei : ItModel<OBJ_PET>::li;
   constexpr int E = OBJ_TAG;
   constexpr uint32_t col = CObj<OBJ_PET>::f[F].col, slot = CObj<OBJ_PET>::f[F].cnt;
   constexpr uint32_t bslot = OBJS ? CObj<E>::f[it_string_field<E>()].cnt : slot + 1u;
+  static_assert(CObj<E>::f[0].kind == K_I64 && CObj<E>::f[1].kind == K_STR, "list elements: an integer and a string");
+  constexpr uint32_t off_col = OBJS ? CObj<E>::f[1].col : col + 1u;
+  const uint32_t l = mine ? o.row[OBJS ? ItWords<OBJ_PET>::n : (uint32_t)IW_LIST] : 0u, n = l >> 16;
+  const uint64_t r0 = (uint64_t)sh.base[slot] + sh.csum[slot][o.chunk];
+  const uint32_t inc = warp_incl_scan(n);
+  if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = (uint32_t)r0 + inc - n;
+  uint32_t at = sh.base[bslot] + sh.csum[bslot][o.chunk], done = 0;
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t l = mine ? o.row[OBJS ? ItWords<OBJ_PET>::n : (uint32_t)IW_LIST] : 0u, bw = mine ? o.row[ItWords<OBJ_PET>::n + 1u] : 0u;
-  const uint32_t n = l >> 16, bytes = OBJS ? bw >> 16 : bw & 0xFFFFu;
-  const uint32_t inc = warp_incl_scan(n | (bytes << 16)); /* of 32 lines: below 2^16 both */
-  const uint64_t r0 = (uint64_t)sh.base[slot] + sh.csum[slot][o.chunk] + (inc & 0xFFFFu) - n;
-  const uint32_t at0 = sh.base[bslot] + sh.csum[bslot][o.chunk] + (inc >> 16) - bytes;
-  if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = (uint32_t)r0;
-  if (n <= IT_SHORT) {
-    uint32_t at = at0;
-    for (uint32_t j = 0; j < n; ++j) {
-      if constexpr (OBJS) {
-        const uint32_t* e = pairs + (l & 0xFFFFu) + 3u * j;
-        item_emit_elem<E>(a, o.win, e, r0 + j, at);
-        at += (e[2] >> (28 + it_string_field<E>())) & 1u ? (e[2] >> 16) & 0xFFFu : 0u;
-      } else {
-        const uint32_t pr = pairs[(l & 0xFFFFu) + j];
-        item_emit_list_str(a, col, o.win, pr, r0 + j, at);
-        at += (pr >> 16) - (pr & 0xFFFFu) - 1u;
-      }
-    }
-  }
-  for (uint32_t big = __ballot_sync(0xFFFFFFFFu, n > IT_SHORT); big; big &= big - 1u) {
-    const int src = __ffs((int)big) - 1;
-    const uint32_t bl = __shfl_sync(0xFFFFFFFFu, l, src), br = __shfl_sync(0xFFFFFFFFu, (uint32_t)r0, src);
-    uint32_t at = __shfl_sync(0xFFFFFFFFu, at0, src);
-    for (uint32_t j0 = 0; j0 < bl >> 16; j0 += 32) {
-      const uint32_t j = j0 + lane;
-      const bool has = j < bl >> 16;
-      uint32_t x = 0, len = 0;
+  item_each_element(o.owner, n, [&](uint32_t src, uint32_t j, bool has) {
+    const uint32_t k = __shfl_sync(0xFFFFFFFFu, l, (int)src) & 0xFFFFu;
+    const uint64_t r = r0 + done + lane;
+    uint32_t pos = 0, len = 0;
+    if constexpr (OBJS) {
       if (has) {
-        if constexpr (OBJS) { x = pairs[(bl & 0xFFFFu) + 3u * j + 2u]; len = (x >> (28 + it_string_field<E>())) & 1u ? (x >> 16) & 0xFFFu : 0u; }
-        else { x = pairs[(bl & 0xFFFFu) + j]; len = (x >> 16) - (x & 0xFFFFu) - 1u; }
+        const uint32_t* e = pairs + k + 3u * j;
+        const uint32_t x = e[2];
+        colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((x >> 28) & 3u);
+        colp<int64_t>(&a.cols, CObj<E>::f[0].col)[r] = (x >> 28) & 1u ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
+        pos = x & 0xFFFFu; len = (x >> 29) & 1u ? (x >> 16) & 0xFFFu : 0u;
       }
-      const uint32_t sc = warp_incl_scan(len);
-      if (has) {
-        if constexpr (OBJS) item_emit_elem<E>(a, o.win, pairs + (bl & 0xFFFFu) + 3u * j, (uint64_t)br + j, at + sc - len);
-        else item_emit_list_str(a, col, o.win, x, (uint64_t)br + j, at + sc - len);
-      }
-      at += __shfl_sync(0xFFFFFFFFu, sc, 31);
-    }
-  }
+    } else if (has) { const uint32_t pr = pairs[k + j]; pos = (pr & 0xFFFFu) + 1u; len = (pr >> 16) - pos; }
+    const uint32_t sc = warp_incl_scan(len), total = __shfl_sync(0xFFFFFFFFu, sc, 31);
+    if (has) colp<uint32_t>(&a.cols, off_col)[r] = at + sc - len;
+    item_emit_run(o.stage, colp<uint8_t>(&a.cols, off_col + 1u) + at, o.win, pos, len, sc - len, total);
+    at += total; done += 32;
+  });
 }
 
 /* ---- the exact parser -------------------------------------------------------------------------------------------- */
@@ -1422,9 +1474,9 @@ static __constant__ Schema c_schema; /* one copy per translation unit that inclu
 /* A record the fast steps refused, from its first byte at input offset s up to `limit`: kind and offset of its failure in *err,
  * *off, or *err = 0 when it is a valid one after all. */
 template <int SCHEMA>
-__device__ __noinline__ void item_exact(const ItemArgs& a, uint64_t s0, uint64_t limit, uint32_t* err, uint32_t* off) {
+__device__ __noinline__ void item_exact(const ItemArgs& a, const uint8_t* in, uint64_t s0, uint64_t limit, uint32_t* err, uint32_t* off) {
   Rd rd;
-  rd.in = a.in; rd.lf_ws = a.sep ? 1u : 0u; rd.open_end = (a.is_last || a.sep) ? 0u : 1u; rd.limit = limit; rd.opts = a.opts; rd.rec_end = limit;
+  rd.in = in; rd.lf_ws = a.sep ? 1u : 0u; rd.open_end = (a.is_last || a.sep) ? 0u : 1u; rd.limit = limit; rd.opts = a.opts; rd.rec_end = limit;
   PS s;
   s.p = s0; s.err = 0; s.err_pos = 0;
   Out<false> so;
@@ -1575,7 +1627,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
       for (uint32_t c = 0; c < nchunk; ++c, ++u) {
         if ((u & (IT_WARPS - 1u)) != warp) continue;
         const uint32_t i = c * 32u + lane;
-        item_value<SCHEMA>(a, win, pairs, rows, rows + (i < nline ? i : 0u) * STRIDE, i < nline, (uint32_t)v);
+        item_value<SCHEMA>(a, sh.owner[warp], win, pairs, rows, rows + (i < nline ? i : 0u) * STRIDE, i < nline, (uint32_t)v);
       }
     }
   }
@@ -1598,8 +1650,11 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     if (rec && !good) {
       uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
       if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
-        const uint64_t s0 = g.v0 + (row[IW_POS] & 0xFFFFu) - g.mis;
-        item_exact<SCHEMA>(a, s0, ARR ? g.v0 + (sh.line[tid + 1u] & 0xFFFFu) - 1u - g.mis : a.limit, &kind, &off);
+        /* where it lies in shared memory, when that is what the input says and holds the whole record */
+        const uint32_t at = row[IW_POS] & 0xFFFFu, sep = (sh.line[tid + 1u] & 0xFFFFu) - 1u;
+        const uint64_t s0 = g.v0 + at - g.mis;
+        const bool here = sep < g.hi_valid && !((sh.oddline[warp] >> lane) & 1u);
+        item_exact<SCHEMA>(a, here ? win : a.in, here ? at : s0, ARR ? (here ? sep : g.v0 + sep - g.mis) : (here ? sep + 1u : a.limit), &kind, &off);
         if (!kind) sh.slow = 1; /* a valid record of a kind the other steps do not know */
       }
       flags = IF_BAD | IF_RECORD | off;
@@ -1627,15 +1682,16 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
   /* ---- where everything of the tile goes ---- */
   if (warp == 0) {
 #pragma unroll
-    for (uint32_t k0 = 0; k0 < IT_NLB; k0 += 4) { /* four counters a time, eight groups of lines each */
-      if (!((SL::mask >> k0) & 15u)) continue;
-      const uint32_t k = k0 + (lane >> 3), c = lane & 7u;
+    for (uint32_t k0 = 0; k0 < IT_NLB; k0 += 32 / IT_WARPS) { /* as many counters a time as the warp's lanes hold groups of lines */
+      constexpr uint32_t some = (1u << (32 / IT_WARPS)) - 1u;
+      if (!((SL::mask >> k0) & some)) continue;
+      const uint32_t k = k0 + lane / IT_WARPS, c = lane % IT_WARPS;
       const bool used = (SL::mask >> k) & 1u;
       const uint32_t v = used && c < nchunk ? sh.csum[k][c] : 0u;
       uint32_t inc = v;
 #pragma unroll
-      for (int d = 1; d < 8; d <<= 1) { const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, d, 8); if (c >= (uint32_t)d) inc += x; }
-      if (used) { sh.csum[k][c] = inc - v; if (c == 7) sh.tot[k] = inc; }
+      for (uint32_t d = 1; d < IT_WARPS; d <<= 1) { const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, d, IT_WARPS); if (c >= d) inc += x; }
+      if (used) { sh.csum[k][c] = inc - v; if (c == IT_WARPS - 1u) sh.tot[k] = inc; }
     }
     __syncwarp();
     item_resolve<SCHEMA>(a, sh, tile, lane);
@@ -1651,7 +1707,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     const uint32_t what = u / nchunk, c = u - what * nchunk, i = c * 32u + lane;
     const uint32_t* r = rows + (i < nline ? i : 0u) * STRIDE;
     ItemOut o;
-    o.win = win; o.row = r; o.chunk = c;
+    o.win = win; o.row = r; o.chunk = c; o.stage = sh.stage[warp]; o.owner = sh.owner[warp];
     const uint32_t f = i < nline ? r[IW_FLAGS] : 0u;
     const bool rec = (f & IF_RECORD) != 0, good = rec && !(f & IF_BAD);
     const uint32_t lt = (1u << lane) - 1u;
