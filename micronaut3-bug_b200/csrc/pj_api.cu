@@ -109,6 +109,7 @@ struct pj_ctx {
   uint32_t tile_bytes_opt = 0;                /* pj_options.tile_bytes */
   unsigned long long spin_ns = 2000000000ull; /* bound of every device-side wait */
   double avg_rec_bytes[5] = {0, 0, 0, 0, 0};  /* bytes per record seen per schema (sizes the tiles of the next call) */
+  uint32_t max_rec_bytes[5] = {0, 0, 0, 0, 0}; /* bytes of the longest one */
   /* host buffers parsed in pieces: copy streams and one "piece is on the device" event per piece */
   cudaStream_t s_in = nullptr, s_out = nullptr;
   cudaEvent_t ev_in[16] = {};
@@ -274,13 +275,13 @@ uint32_t item_stride(uint32_t schema) {
 }
 TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   static const double dflt[5] = {0, 300, 146, 190, 230};
-  /* dynamic shared memory that lets IT_BLOCKS blocks share an SM (228 KB, 1 KB of which every block costs) */
-  static constexpr uint32_t BUDGET = (228u * 1024u) / IT_BLOCKS - 1024u - (uint32_t)sizeof(ItemShared) - 256u;
   const double avg = c->avg_rec_bytes[schema] > 0 ? c->avg_rec_bytes[schema] : dflt[schema];
   TileShape t;
-  /* room behind the tile for its last records: 13 average records reach the longest ones of a skewed distribution */
-  uint32_t slack = (uint32_t)(avg * 13);
-  slack = (slack < 4096 ? 4096u : (slack > 28672 ? 28672u : slack)) & ~15u;
+  /* room behind the tile for its last record: a quarter more than the longest one of the call before, or 13 average records,
+     which reach the longest ones of a skewed distribution */
+  uint64_t longest = c->max_rec_bytes[schema] ? c->max_rec_bytes[schema] + c->max_rec_bytes[schema] / 4 + 64 : (uint64_t)(avg * 13);
+  const uint64_t shortest = c->max_rec_bytes[schema] ? 1024 : 4096;
+  const uint32_t slack = (longest < shortest ? (uint32_t)shortest : (longest > 28672 ? 28672u : (uint32_t)longest)) & ~15u;
   uint32_t per_word = 9; /* window bytes per word for strings */
   /* what the block indexes in one step, or so that most tiles have fewer than three quarters of the lines they may have */
   uint64_t tile = IT_STEP - (uint64_t)(2 * avg), few = (uint64_t)(avg * (IT_MAX_LINES * 47 / 64));
@@ -289,15 +290,19 @@ TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   /* few tiles: one for every block that can be resident, and room enough */
   if (len / (148 * IT_BLOCKS) < tile) { tile = len / (148 * IT_BLOCKS); if (tile < 4096) tile = 4096; per_word = 2; }
   if (c->tile_bytes_opt) { tile = c->tile_bytes_opt; if (tile < ST_MIN_TILE_BYTES) tile = ST_MIN_TILE_BYTES; if (tile > 32768) tile = 32768; }
-  for (;;) {
+  /* as many resident blocks as leave three quarters of that tile */
+  const uint64_t least = tile - tile / 4;
+  for (uint32_t blocks = IT_BLOCKS;; ) {
     t.tile_bytes = (uint32_t)(tile & ~31ull);
     if (t.tile_bytes < ST_MIN_TILE_BYTES) t.tile_bytes = ST_MIN_TILE_BYTES;
     t.win_bytes = t.tile_bytes + slack;
     t.str_words = t.win_bytes / per_word;
     const double recs = (double)t.tile_bytes / avg * 1.3 + 24;
     t.row_cap = recs > IT_MAX_LINES ? IT_MAX_LINES : (uint32_t)recs;
-    if (per_word == 2 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_words, t.row_cap, item_stride(schema)).total <= BUDGET) return t;
-    tile -= 512;
+    const uint32_t room = (228u * 1024u) / blocks - 1024u - (uint32_t)sizeof(ItemShared) - 256u;
+    if (per_word == 2 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_words, t.row_cap, item_stride(schema)).total <= room) return t;
+    if (tile - 512 >= least || blocks == 2) tile -= 512;
+    else { tile = least + least / 3; --blocks; }
   }
 }
 
@@ -441,6 +446,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   uint64_t total[NSLOT];
   for (uint32_t k = 0; k < NSLOT; ++k) total[k] = 0;
   bool over = false;
+  uint32_t max_rec = 0;
   for (int p = 0; p < np; ++p) {
     PJ_CUDA(c, cudaEventSynchronize(c->ev_done[p]));
     const DevResult& r = c->h_res[p];
@@ -453,6 +459,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     c->stats.lookback_polls += r.lookback_polls; c->stats.lookback_rounds += r.lookback_rounds;
     if (r.timeout) return set_err(c, PJ_ERR_TIMEOUT, "pj_parse: a bounded device-side wait ran out");
     if (r.over) over = true;
+    if (r.max_rec > max_rec) max_rec = r.max_rec;
     const uint64_t rows_new = r.n_records;
     if (host_out && !over) {
       if (pipe) PJ_CUDA(c, cudaStreamWaitEvent(s_out, c->ev_done[p], 0));
@@ -480,7 +487,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   out->doc_err_kind = 0; out->doc_err_off = 0;
   const pj_status st = finish_columns(c, schema, len, pp, rows_done, n_errors, total, over, out);
   if (st) return st;
-  if (rows_done > 1000 && !c->tile_bytes_opt) c->avg_rec_bytes[schema] = (double)len / (double)rows_done;
+  if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; c->max_rec_bytes[schema] = max_rec; }
   if (host_out) PJ_CUDA(c, cudaStreamSynchronize(s_out));
   return PJ_OK;
 }
@@ -567,7 +574,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   if (r.doc_err_off != ~0ull) { out->doc_err_kind = PJ_E_SYNTAX; out->doc_err_off = r.doc_err_off; }
   else if (r.first_opener == ~0ull || r.arr_final_s || r.arr_final_d != 0) { out->doc_err_kind = PJ_E_EOF; out->doc_err_off = len; }
   const pj_status st = finish_columns(c, schema, len, pp, r.n_records, r.n_errors, total, r.over != 0, out);
-  if (!st && r.n_records > 1000 && !c->tile_bytes_opt) c->avg_rec_bytes[schema] = (double)len / (double)r.n_records;
+  if (!st && r.n_records > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)r.n_records; c->max_rec_bytes[schema] = r.max_rec; }
   if (st) return st;
   if (host_out) {
     for (int i = 0; i < pp.nneed; ++i) {
