@@ -280,7 +280,7 @@ TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   /* room behind the tile for its last record: a quarter more than the longest one of the call before, or 13 average records,
      which reach the longest ones of a skewed distribution */
   uint64_t longest = c->max_rec_bytes[schema] ? c->max_rec_bytes[schema] + c->max_rec_bytes[schema] / 4 + 64 : (uint64_t)(avg * 13);
-  const uint64_t shortest = c->max_rec_bytes[schema] ? 1024 : 4096;
+  const uint64_t shortest = 4096;
   const uint32_t slack = (longest < shortest ? (uint32_t)shortest : (longest > 28672 ? 28672u : (uint32_t)longest)) & ~15u;
   uint32_t per_word = 9; /* window bytes per word for strings */
   /* what the block indexes in one step, or so that most tiles have fewer than three quarters of the lines they may have */

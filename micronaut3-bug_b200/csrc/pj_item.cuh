@@ -641,6 +641,7 @@ __device__ __forceinline__ bool item_false(const uint8_t* win, uint32_t pos, uin
 
 __device__ __forceinline__ void item_error(uint32_t* row, uint32_t pos, uint32_t kind) {
   atomicMin(&row[IW_ERR], (pos << 8) | kind);
+  if (kind == IE_REFUSED) atomicOr(&row[IW_FLAGS], IF_BAD); /* whatever else is found: values of refused records are not all looked at */
 }
 /* A scalar token that belongs to no property: only what is cheap to see as valid (integers, literals) passes. */
 static __device__ __noinline__ bool item_plain_scalar(const uint8_t* win, uint32_t s, uint32_t n) {
@@ -1007,7 +1008,7 @@ __device__ __forceinline__ void item_walk_model(ItemWalk& f, uint32_t* row, uint
   else f.ok = f.ok && f.k == f.kend && !f.open && item_only_blanks(f.win, f.p + 1u, f.sep);
 }
 template <int SCHEMA>
-__device__ __noinline__ void item_walk_spaced(ItemWalk& f, uint32_t* row, uint32_t& flags, ItemLists& l, uint32_t type) {
+__device__ __forceinline__ void item_walk_spaced(ItemWalk& f, uint32_t* row, uint32_t& flags, ItemLists& l, uint32_t type) {
   while (f.p < f.sep && item_blank(f.win[f.p])) ++f.p;
   f.ok = f.win[f.p] == '{';
   item_walk_model<SCHEMA, false>(f, row, flags, l, type);
@@ -1161,23 +1162,6 @@ __device__ __forceinline__ uint32_t item_key(const ItemShared& sh, const uint8_t
   const uint32_t f = sh.field[s == IS_ROOT ? 0 : (s == IS_CHILD ? 1 : 2)][slot];
   return (((x0 ^ kt.x) & km.x) | ((x1 ^ kt.y) & km.y) | ((x2 ^ kt.z) & km.z) | ((x3 ^ kt.w) & km.w)) != 0 || len < 2u || len > 15u ? 0u : f;
 }
-/* A key whose gap is none of the texts: does a bracket or brace follow the colon that the property's type rules out? That is
- * PJ_E_TYPE there, whatever the bracket holds (of several models: when the property is every one's). */
-static __device__ __noinline__ uint32_t item_wrong_bracket(const ItemShared& sh, bool mixed, const uint8_t* win, uint32_t open, uint32_t end, uint32_t close, uint32_t sep, uint32_t s, uint32_t* at) {
-  uint32_t p = close + 1u;
-  while (p < sep && item_blank(win[p])) ++p;
-  if (p >= sep || win[p] != ':') return IE_REFUSED;
-  ++p;
-  while (p < sep && item_blank(win[p])) ++p;
-  const uint32_t x = p < sep ? win[p] : 0u;
-  if (x != '[' && x != '{') return IE_REFUSED;
-  const uint32_t f = item_key(sh, win, open + 1u, end - open - 1u, s);
-  const uint32_t kind = ItField::kind(f);
-  if (!f || (mixed && s == IS_ROOT && ItField::models(f) != 7u) || (kind == K_OBJ && x == '{') || ((kind == K_LIST_STR || kind == K_LIST_OBJ) && x == '[')) return IE_REFUSED;
-  *at = p;
-  return (uint32_t)PJ_E_TYPE;
-}
-
 /* Lines [i0, i0 + n), each with a string, by a warp: together at most 32 strings, or one line with more. Returns false when
  * the tile has to take the other road. */
 template <int SCHEMA, bool ARR>
@@ -1283,9 +1267,7 @@ __device__ __noinline__ bool item_pack(const ItemArgs& a, const StreamGeom& g, I
       }
       if (trunc) { item_error(row, close, (uint32_t)PJ_E_EOF); if (!role_ok) item_error(row, open, IE_REFUSED); }
       else if (!ok || !role_ok || !(need == 15u || need == s)) {
-        uint32_t at = close, kind = IE_REFUSED;
-        if (!ok && !isval && s != IS_LIST) kind = item_wrong_bracket(sh, SCHEMA == PJ_SCHEMA_MIXED, win, open, close - freed, close, sep, s, &at);
-        item_error(row, at, kind);
+        item_error(row, close, IE_REFUSED);
         iskey = false;
       }
       if (last) reinterpret_cast<uint16_t*>(&row[IW_POS])[1] = (uint16_t)v.clpos;
@@ -1503,12 +1485,14 @@ __device__ __forceinline__ void item_elem_row(const uint8_t* win, const uint32_t
   uint32_t* e = pairs + k;
   const uint32_t p0 = e[0], p1 = e[1], p2 = e[2];
   uint32_t at = (p0 >> 16) + 1u, end = (p1 & 0xFFFFu) - 1u; /* at the colon and at the comma, but for blanks */
-  while (win[at] != ':') ++at;
-  do ++at; while (item_blank(win[at]));
-  while (win[end] != ',') --end;
-  while (item_blank(win[end - 1u])) --end;
+  const uint32_t from = at, to = end;
+  while (at < to && win[at] != ':') ++at;
+  ++at;
+  while (at < to && item_blank(win[at])) ++at;
+  while (end > from && win[end] != ',') --end;
+  while (end > at && item_blank(win[end - 1u])) --end;
   int64_t val = 0;
-  if (!item_int(win, at, end - at, true, &val)) { const uint32_t x = win[at]; item_error(row, at, (x == 't' || x == 'f') ? (uint32_t)PJ_E_TYPE : IE_REFUSED); }
+  if (end <= at || !item_int(win, at, end - at, true, &val)) { const uint32_t x = win[at]; item_error(row, at, (x == 't' || x == 'f') ? (uint32_t)PJ_E_TYPE : IE_REFUSED); }
   const uint32_t open = p2 & 0xFFFFu, n = (p2 >> 16) - open - 1u - item_freed(win, moved, k + 2u, p2 >> 16);
   e[0] = (uint32_t)(uint64_t)val; e[1] = (uint32_t)((uint64_t)val >> 32);
   e[2] = (open + 1u) | (n << 16) | 0xF0000000u;
@@ -1533,7 +1517,7 @@ __device__ __forceinline__ void item_each_element(uint8_t* owner, uint32_t n, F 
 template <int SCHEMA>
 __device__ __forceinline__ void item_value(const ItemArgs& a, uint8_t* owner, const uint32_t* moved, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t* row, bool live, uint32_t unit) {
   const uint32_t flags = live ? row[IW_FLAGS] : 0u;
-  const bool rec = (flags & IF_RECORD) != 0;
+  const bool rec = (flags & (IF_RECORD | IF_BAD)) == IF_RECORD; /* (refused: the exact parser looks at it) */
   const uint32_t type = item_type<SCHEMA>(flags);
   Win w;
   w.s = win; w.w0 = 0;
@@ -1942,7 +1926,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     const bool good = rec && e == IE_NONE;
     if (rec && !good) {
       uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
-      if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
+      if ((flags & (IF_MOVED | IF_BAD)) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
         /* where it lies in shared memory, when that is what the input says and holds the whole record */
         const uint32_t at = row[IW_POS] & 0xFFFFu, sep = (sh.line[tid + 1u] & 0xFFFFu) - 1u;
         const uint64_t s0 = g.v0 + at - g.mis;
