@@ -906,7 +906,7 @@ __device__ __forceinline__ uint32_t item_dense_flat(ItemWalk& f, uint32_t at, ui
     } else {
       static_assert(I + 1 < CObj<E>::N, "an integer is followed by another property");
       end = (nx & 0xFFFFu) - 1u; /* the comma before the next key */
-      f.ok = f.ok && f.k < f.kend && end > v && end - v < 32u;
+      f.ok = f.ok && f.k < f.kend && end > v && end - v < 32u && f.win[v] > ' ' && f.win[end - 1u] > ' ';
       ref[I] = v | ((end - v) << 16);
     }
     f.ok = f.ok && f.win[f.ok ? end : at] == (I + 1 < CObj<E>::N ? ',' : '}');
@@ -933,7 +933,7 @@ __device__ __forceinline__ void item_dense_members(ItemWalk& f, uint32_t* row, u
       uint32_t end = v; /* behind the value */
       if constexpr (kind == K_I64 || kind == K_I32 || kind == K_BOOL) {
         end = more ? (nx & 0xFFFFu) - 1u : f.sep - 1u;
-        f.ok = end > v && end - v < 32u;
+        f.ok = end > v && end - v < 32u && f.win[v] > ' ' && f.win[end - 1u] > ' ';
         row[word] = v | ((end - v) << 16);
       } else if constexpr (kind == K_STR || kind == K_ENUM || kind == K_DATETIME) {
         end = (nx >> 16) + 1u;
@@ -1007,14 +1007,8 @@ __device__ __forceinline__ void item_walk_model(ItemWalk& f, uint32_t* row, uint
   if constexpr (DENSE) f.ok = f.ok && f.k == f.kend && f.win[f.p] == '}' && f.p + 1u == f.sep;
   else f.ok = f.ok && f.k == f.kend && !f.open && item_only_blanks(f.win, f.p + 1u, f.sep);
 }
-template <int SCHEMA>
-__device__ __forceinline__ void item_walk_spaced(ItemWalk& f, uint32_t* row, uint32_t& flags, ItemLists& l, uint32_t type) {
-  while (f.p < f.sep && item_blank(f.win[f.p])) ++f.p;
-  f.ok = f.win[f.p] == '{';
-  item_walk_model<SCHEMA, false>(f, row, flags, l, type);
-}
 /* One line: its row, or IF_ODD there. */
-template <int SCHEMA, bool ARR>
+template <int SCHEMA, bool ARR, bool DENSE>
 __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t i, uint32_t type) {
   constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
   ItemWalk f = item_walk_open(sh, win, pairs, i);
@@ -1033,16 +1027,14 @@ __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGe
   } else {
     const uint32_t n = f.kend - f.k, bit = 1u << (i & 31u);
     const bool plain = !(sh.movedline[i >> 5] & bit), fit = !cut && !(sh.oddline[i >> 5] & bit);
-    const ItemWalk f0 = f;
     /* A warp waits for its longest line, which takes some 300 cycles a string (1000 with blanks), while item_pack() takes 80 for
        every string of the tile, whoever's it is: few long lines are its. */
-    f.ok = fit && plain && win[start] == '{' && (n <= 32u || n * 4u <= sh.nstr);
-    item_walk_model<SCHEMA, true>(f, row, flags, l, type);
-    if (!f.ok && fit && (n <= 16u || n * 12u <= sh.nstr)) {
-      f = f0; flags = 0;
-      l.k_str = l.n_str = l.k_obj = l.n_obj = l.bytes = 0;
-      item_walk_spaced<SCHEMA>(f, row, flags, l, type);
+    if constexpr (DENSE) f.ok = fit && plain && win[start] == '{' && (n <= 32u || n * 4u <= sh.nstr);
+    else {
+      while (f.p < f.sep && item_blank(win[f.p])) ++f.p;
+      f.ok = fit && win[f.p] == '{' && (n <= 16u || n * 12u <= sh.nstr);
     }
+    item_walk_model<SCHEMA, DENSE>(f, row, flags, l, type);
     if (!plain) flags |= IF_MOVED;
     flags = IF_RECORD | (f.ok ? flags : IF_ODD);
   }
@@ -1082,7 +1074,7 @@ __device__ __forceinline__ void item_sort(ItemShared& sh, uint32_t tid, uint32_t
 /* All lines: one per thread, in order, or, in a stream of several models, sorted by the model the key behind `id` decides,
  * so that a warp walks one model. */
 template <int SCHEMA, bool ARR>
-__device__ __forceinline__ void item_walk(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t tid) {
+__device__ __forceinline__ uint32_t item_walk(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t tid) {
   const uint32_t lane = tid & 31, warp = tid >> 5, nline = sh.nline;
   uint32_t i = tid, type = 0;
   if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
@@ -1104,7 +1096,20 @@ __device__ __forceinline__ void item_walk(const ItemArgs& a, const StreamGeom& g
     type = tid < ends[0] ? (uint32_t)PJ_TYPE_PET : (tid < ends[1] ? (uint32_t)PJ_TYPE_ORDER : (tid < ends[2] ? (uint32_t)PJ_TYPE_USER : (uint32_t)PJ_TYPE_NONE));
     if (tid < nline) i = sh.perm[tid];
   }
-  if (tid < nline) item_walk_line<SCHEMA, ARR>(a, g, sh, win, pairs, rows, i, type);
+  if (tid < nline) item_walk_line<SCHEMA, ARR, true>(a, g, sh, win, pairs, rows, i, type);
+  return i | (type << 16);
+}
+/* The second look at the lines the dense walk left: by the same threads. Out of line, so that the tiles that need none keep
+ * their instructions close together; every thread of the block calls it. */
+template <int SCHEMA, bool ARR>
+__device__ __noinline__ void item_walk_again(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t tid, uint32_t mine) {
+  const uint32_t i = mine & 0xFFFFu, type = mine >> 16;
+  if (tid < sh.nline && ((sh.oddmask[i >> 5] >> (i & 31u)) & 1u)) item_walk_line<SCHEMA, ARR, false>(a, g, sh, win, pairs, rows, i, type);
+  __syncthreads();
+  const bool odd = tid < sh.nline && (rows[tid * ItStride<SCHEMA>::n + IW_FLAGS] & IF_ODD);
+  const uint32_t m = __ballot_sync(0xFFFFFFFFu, odd);
+  if ((tid & 31u) == 0) sh.oddmask[tid >> 5] = m;
+  __syncthreads();
 }
 
 /* ---- 3. strings and gaps ------------------------------------------------------------------------------------------ */
@@ -1872,7 +1877,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     item_specials(a, sh, win, pairs, tid);
     __syncthreads();
   }
-  item_walk<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid);
+  const uint32_t mine = item_walk<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid); /* line, model */
   if (SCHEMA == PJ_SCHEMA_MIXED) __syncthreads(); /* the lines were walked in another order */
   uint32_t* row = rows + (tid < nline ? tid : 0u) * STRIDE; /* from here on a thread has the line of its number */
   {
@@ -1886,7 +1891,12 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
 #pragma unroll
     for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
     if (nodd) {
-      item_packs<SCHEMA, ARR>(a, g, sh, win, pairs, rows, nodd);
+      __syncthreads(); /* oddmask[] is read */
+      item_walk_again<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid, mine);
+      nodd = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
+      if (nodd) item_packs<SCHEMA, ARR>(a, g, sh, win, pairs, rows, nodd);
       if (__syncthreads_or((int)sh.slow)) return false;
     }
   }
