@@ -641,7 +641,6 @@ __device__ __forceinline__ bool item_false(const uint8_t* win, uint32_t pos, uin
 
 __device__ __forceinline__ void item_error(uint32_t* row, uint32_t pos, uint32_t kind) {
   atomicMin(&row[IW_ERR], (pos << 8) | kind);
-  if (kind == IE_REFUSED) atomicOr(&row[IW_FLAGS], IF_BAD); /* whatever else is found: values of refused records are not all looked at */
 }
 /* A scalar token that belongs to no property: only what is cheap to see as valid (integers, literals) passes. */
 static __device__ __noinline__ bool item_plain_scalar(const uint8_t* win, uint32_t s, uint32_t n) {
@@ -1272,7 +1271,20 @@ __device__ __noinline__ bool item_pack(const ItemArgs& a, const StreamGeom& g, I
       }
       if (trunc) { item_error(row, close, (uint32_t)PJ_E_EOF); if (!role_ok) item_error(row, open, IE_REFUSED); }
       else if (!ok || !role_ok || !(need == 15u || need == s)) {
-        item_error(row, close, IE_REFUSED);
+        uint32_t at = close, kind = IE_REFUSED;
+        if (!ok && !isval && s != IS_LIST) { /* does a bracket or brace follow the colon that the property's type rules out? */
+          uint32_t p = close + 1u;
+          while (p < sep && item_blank(win[p])) ++p;
+          if (p < sep && win[p] == ':') {
+            ++p;
+            while (p < sep && item_blank(win[p])) ++p;
+            const uint32_t x = p < sep ? win[p] : 0u;
+            const uint32_t f = item_key(sh, win, open + 1u, close - freed - open - 1u, s), fk = ItField::kind(f);
+            const bool everyones = SCHEMA != PJ_SCHEMA_MIXED || s != IS_ROOT || ItField::models(f) == 7u; /* (another model's property has no type) */
+            if (f && everyones && ((x == '[' && fk != K_LIST_STR && fk != K_LIST_OBJ) || (x == '{' && fk != K_OBJ))) { at = p; kind = (uint32_t)PJ_E_TYPE; }
+          }
+        }
+        item_error(row, at, kind);
         iskey = false;
       }
       if (last) reinterpret_cast<uint16_t*>(&row[IW_POS])[1] = (uint16_t)v.clpos;
@@ -1522,7 +1534,7 @@ __device__ __forceinline__ void item_each_element(uint8_t* owner, uint32_t n, F 
 template <int SCHEMA>
 __device__ __forceinline__ void item_value(const ItemArgs& a, uint8_t* owner, const uint32_t* moved, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t* row, bool live, uint32_t unit) {
   const uint32_t flags = live ? row[IW_FLAGS] : 0u;
-  const bool rec = (flags & (IF_RECORD | IF_BAD)) == IF_RECORD; /* (refused: the exact parser looks at it) */
+  const bool rec = (flags & IF_RECORD) != 0; /* refused ones too: an earlier failure may be found here, and every value present has its reference */
   const uint32_t type = item_type<SCHEMA>(flags);
   Win w;
   w.s = win; w.w0 = 0;
@@ -1936,7 +1948,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     const bool good = rec && e == IE_NONE;
     if (rec && !good) {
       uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
-      if ((flags & (IF_MOVED | IF_BAD)) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
+      if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
         /* where it lies in shared memory, when that is what the input says and holds the whole record */
         const uint32_t at = row[IW_POS] & 0xFFFFu, sep = (sh.line[tid + 1u] & 0xFFFFu) - 1u;
         const uint64_t s0 = g.v0 + at - g.mis;
