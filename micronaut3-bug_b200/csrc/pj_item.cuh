@@ -596,6 +596,8 @@ __device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
   w.s = win; w.w0 = 0;
   return wpeek4(w, p);
 }
+/* first byte of a value that is no number: a literal, an object, a list (as the walk takes whatever is between colon and comma) */
+__device__ __forceinline__ bool item_other_type(uint32_t x) { return x == 't' || x == 'f' || x == '[' || x == '{'; }
 /* -?(0|[1-9][0-9]*) in the n bytes at pos, within int64 / int32. Read from its end, eight digits at a time. */
 /* 8 bytes at p, which may lie up to IT_FRONT bytes before the window */
 __device__ __forceinline__ uint64_t item_back8(const uint8_t* win, int32_t p) {
@@ -1371,7 +1373,7 @@ __device__ __noinline__ bool item_pack(const ItemArgs& a, const StreamGeom& g, I
             const uint32_t at = ref & 0xFFFFu;
             if (!item_int(win, at, n_val, kind == K_I64, &val)) {
               const uint32_t x = win[at];
-              item_error(row, ref >> 31 ? at - 1u : at, (!(ref >> 31) && (x == 't' || x == 'f')) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
+              item_error(row, ref >> 31 ? at - 1u : at, (!(ref >> 31) && item_other_type(x)) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
             }
             if (!slow) { pairs[erow] = (uint32_t)(uint64_t)val; pairs[erow + 1u] = (uint32_t)((uint64_t)val >> 32); }
           }
@@ -1509,7 +1511,7 @@ __device__ __forceinline__ void item_elem_row(const uint8_t* win, const uint32_t
   while (end > from && win[end] != ',') --end;
   while (end > at && item_blank(win[end - 1u])) --end;
   int64_t val = 0;
-  if (end <= at || !item_int(win, at, end - at, true, &val)) { const uint32_t x = win[at]; item_error(row, at, (x == 't' || x == 'f') ? (uint32_t)PJ_E_TYPE : IE_REFUSED); }
+  if (end <= at || !item_int(win, at, end - at, true, &val)) { const uint32_t x = win[at]; item_error(row, at, item_other_type(x) ? (uint32_t)PJ_E_TYPE : IE_REFUSED); }
   const uint32_t open = p2 & 0xFFFFu, n = (p2 >> 16) - open - 1u - item_freed(win, moved, k + 2u, p2 >> 16);
   e[0] = (uint32_t)(uint64_t)val; e[1] = (uint32_t)((uint64_t)val >> 32);
   e[2] = (open + 1u) | (n << 16) | 0xF0000000u;
@@ -1547,7 +1549,7 @@ __device__ __forceinline__ void item_value(const ItemArgs& a, uint8_t* owner, co
       int64_t v = 0;
       if (!item_int(win, pos, (ref >> 16) & 0x7FFFu, is64, &v)) {
         const uint32_t x = win[pos];
-        item_error(row, ref >> 31 ? pos - 1u : pos, (!(ref >> 31) && (x == 't' || x == 'f')) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
+        item_error(row, ref >> 31 ? pos - 1u : pos, (!(ref >> 31) && item_other_type(x)) ? (uint32_t)PJ_E_TYPE : IE_REFUSED);
       }
       row[word] = (uint32_t)(uint64_t)v;
       if (is64) row[word + 1] = (uint32_t)((uint64_t)v >> 32);
