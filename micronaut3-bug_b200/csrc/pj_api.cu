@@ -284,7 +284,7 @@ TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   const uint32_t slack = (longest < shortest ? (uint32_t)shortest : (longest > 28672 ? 28672u : (uint32_t)longest)) & ~15u;
   uint32_t per_word = 9; /* window bytes per word for strings */
   /* what the block indexes in one step, or so that most tiles have fewer than three quarters of the lines they may have */
-  uint64_t tile = IT_STEP - (uint64_t)(2 * avg), few = (uint64_t)(avg * (IT_MAX_LINES * 47 / 64));
+  uint64_t tile = IT_STEP - (uint64_t)(2 * avg), few = (uint64_t)(avg * (c->avg_rec_bytes[schema] > 0 ? IT_MAX_LINES * 47 / 64 : IT_MAX_LINES * 9 / 16)); /* (a first call's records may be shorter) */
   if (avg * 4 > IT_STEP) tile = IT_STEP / 2;
   if (tile > few) tile = few;
   /* few tiles: one for every block that can be resident, and room enough */

@@ -40,10 +40,13 @@
 namespace pj {
 
 #ifndef PJ_IT_BLOCKS
-#define PJ_IT_BLOCKS 5 /* resident blocks per SM the kernel is compiled for */
+#define PJ_IT_BLOCKS 3 /* resident blocks per SM the kernel is compiled for */
 #endif
 static constexpr uint32_t IT_BLOCKS = PJ_IT_BLOCKS;
-static constexpr uint32_t IT_THREADS = 128;
+#ifndef PJ_IT_THREADS
+#define PJ_IT_THREADS 256
+#endif
+static constexpr uint32_t IT_THREADS = PJ_IT_THREADS;
 static constexpr uint32_t IT_WARPS = IT_THREADS / 32;
 static constexpr uint32_t IT_BLK = 9;                /* 16-byte blocks a thread indexes per step: odd, so that a warp's 128-bit loads are free of bank conflicts */
 static constexpr uint32_t IT_SPAN = IT_BLK * 16;
@@ -598,6 +601,7 @@ __device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
 }
 /* first byte of a value that is no number: a literal, an object, a list (as the walk takes whatever is between colon and comma) */
 __device__ __forceinline__ bool item_other_type(uint32_t x) { return x == 't' || x == 'f' || x == '[' || x == '{'; }
+__device__ __forceinline__ bool item_number_start(uint32_t x) { return x - (uint32_t)'0' <= 9u || x == '-'; }
 /* -?(0|[1-9][0-9]*) in the n bytes at pos, within int64 / int32. Read from its end, eight digits at a time. */
 /* 8 bytes at p, which may lie up to IT_FRONT bytes before the window */
 __device__ __forceinline__ uint64_t item_back8(const uint8_t* win, int32_t p) {
@@ -907,7 +911,7 @@ __device__ __forceinline__ uint32_t item_dense_flat(ItemWalk& f, uint32_t at, ui
     } else {
       static_assert(I + 1 < CObj<E>::N, "an integer is followed by another property");
       end = (nx & 0xFFFFu) - 1u; /* the comma before the next key */
-      f.ok = f.ok && f.k < f.kend && end > v && end - v < 32u && f.win[v] > ' ' && f.win[end - 1u] > ' ';
+      f.ok = f.ok && f.k < f.kend && end > v && end - v < 32u && item_number_start(f.win[v]) && f.win[end - 1u] > ' ';
       ref[I] = v | ((end - v) << 16);
     }
     f.ok = f.ok && f.win[f.ok ? end : at] == (I + 1 < CObj<E>::N ? ',' : '}');
@@ -934,7 +938,8 @@ __device__ __forceinline__ void item_dense_members(ItemWalk& f, uint32_t* row, u
       uint32_t end = v; /* behind the value */
       if constexpr (kind == K_I64 || kind == K_I32 || kind == K_BOOL) {
         end = more ? (nx & 0xFFFFu) - 1u : f.sep - 1u;
-        f.ok = end > v && end - v < 32u && f.win[v] > ' ' && f.win[end - 1u] > ' ';
+        const uint32_t x0 = f.win[v];
+        f.ok = end > v && end - v < 32u && (kind == K_BOOL ? x0 == 't' || x0 == 'f' : item_number_start(x0)) && f.win[end - 1u] > ' ';
         row[word] = v | ((end - v) << 16);
       } else if constexpr (kind == K_STR || kind == K_ENUM || kind == K_DATETIME) {
         end = (nx >> 16) + 1u;
