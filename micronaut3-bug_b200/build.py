@@ -53,10 +53,13 @@ def build_library(force: bool = False, verbose_ptxas: bool = False) -> str:
     api_o = os.path.join(CSRC, "pj_api.o")
     jobs = [[nvcc, *NVCC_FLAGS, *extra, "-c", os.path.join(CSRC, "pj_api.cu"), "-o", api_o]]
     tile_objs = []
-    for schema in (1, 2, 3, 4):  # the tile kernel once per model set (Pet, Order, User, mixed), side by side
+    for schema in (1, 2, 3, 4):  # the parse kernels once per model set (Pet, Order, User, mixed), side by side
         obj = os.path.join(CSRC, f"pj_tile_{schema}.o")
         tile_objs.append(obj)
         jobs.append([nvcc, *NVCC_FLAGS, *extra, f"-DPJ_TILE_SCHEMA={schema}", "-c", os.path.join(CSRC, "pj_tile_inst.cu"), "-o", obj])
+        obj = os.path.join(CSRC, f"pj_stream_{schema}.o")
+        tile_objs.append(obj)
+        jobs.append([nvcc, *NVCC_FLAGS, *extra, f"-DPJ_TILE_SCHEMA={schema}", "-c", os.path.join(CSRC, "pj_stream_inst.cu"), "-o", obj])
     with ThreadPoolExecutor(max_workers=len(jobs)) as pool:
         list(pool.map(_run, jobs))
     _run([nvcc, "-shared", "-o", LIB, api_o, *tile_objs, "-ldl", "-lpthread"])

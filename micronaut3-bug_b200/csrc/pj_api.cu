@@ -23,15 +23,20 @@
 #include "pj_kernels.cuh"
 #include "pj_array_kernels.cuh"
 #include "pj_item.cuh"
+#include "pj_stream_kernel.cuh"
 
 using namespace pj;
 
-/* the four instantiations of the parse kernel live in objects of their own (pj_tile_inst.cu) */
+/* the four instantiations of each parse kernel live in objects of their own (pj_tile_inst.cu, pj_stream_inst.cu) */
 namespace pj {
 cudaError_t item_init_1(const Schema*); cudaError_t item_launch_1(const ItemArgs*, cudaStream_t);
+cudaError_t stream_init_1(const Schema*); cudaError_t stream_launch_1(const StreamArgs*, unsigned, cudaStream_t);
 cudaError_t item_init_2(const Schema*); cudaError_t item_launch_2(const ItemArgs*, cudaStream_t);
+cudaError_t stream_init_2(const Schema*); cudaError_t stream_launch_2(const StreamArgs*, unsigned, cudaStream_t);
 cudaError_t item_init_3(const Schema*); cudaError_t item_launch_3(const ItemArgs*, cudaStream_t);
+cudaError_t stream_init_3(const Schema*); cudaError_t stream_launch_3(const StreamArgs*, unsigned, cudaStream_t);
 cudaError_t item_init_4(const Schema*); cudaError_t item_launch_4(const ItemArgs*, cudaStream_t);
+cudaError_t stream_init_4(const Schema*); cudaError_t stream_launch_4(const StreamArgs*, unsigned, cudaStream_t);
 }
 
 namespace {
@@ -110,6 +115,9 @@ struct pj_ctx {
   unsigned long long spin_ns = 2000000000ull; /* bound of every device-side wait */
   double avg_rec_bytes[5] = {0, 0, 0, 0, 0};  /* bytes per record seen per schema (sizes the tiles of the next call) */
   uint32_t max_rec_bytes[5] = {0, 0, 0, 0, 0}; /* bytes of the longest one */
+  /* NDJSON: which kernel the next call takes (use_items()), and how often it changed to k_parse_items */
+  bool items[5] = {false, false, false, false, false};
+  uint8_t to_items[5] = {0, 0, 0, 0, 0};
   /* host buffers parsed in pieces: copy streams and one "piece is on the device" event per piece */
   cudaStream_t s_in = nullptr, s_out = nullptr;
   cudaEvent_t ev_in[16] = {};
@@ -315,7 +323,39 @@ cudaError_t item_launch(uint32_t schema, const ItemArgs* a, cudaStream_t s) {
   }
 }
 
-/* NDJSON: one launch of k_parse_items per piece. Host buffers of a whole stream are parsed in pieces cut after line
+cudaError_t stream_launch(uint32_t schema, const StreamArgs* a, cudaStream_t s) {
+  switch (schema) {
+    case PJ_SCHEMA_PET: return stream_launch_1(a, a->ntiles, s);
+    case PJ_SCHEMA_ORDER: return stream_launch_2(a, a->ntiles, s);
+    case PJ_SCHEMA_USER: return stream_launch_3(a, a->ntiles, s);
+    default: return stream_launch_4(a, a->ntiles, s);
+  }
+}
+uint32_t pick_stream_tile(const pj_ctx* c, uint32_t schema) {
+  static const double dflt[5] = {0, 300, 125, 190, 220};
+  const double avg = c->avg_rec_bytes[schema] > 0 ? c->avg_rec_bytes[schema] : dflt[schema];
+  uint64_t tb = c->tile_bytes_opt ? c->tile_bytes_opt : (uint64_t)(avg * (ST_THREADS * 13 / 16));
+  tb &= ~15ull;
+  if (tb < ST_MIN_TILE_BYTES) tb = ST_MIN_TILE_BYTES;
+  if (tb > ST_MAX_TILE_BYTES) tb = ST_MAX_TILE_BYTES;
+  return (uint32_t)tb;
+}
+/* Which kernel parses the next NDJSON call. A record per thread (k_parse_stream) is the faster one as long as its lockstep pass
+ * takes all records: with 2 % of them outside of it every warp has one that the others wait for. k_parse_items takes over
+ * then, and hands back when its strict walk took all lines and none is long. Text of one producer keeps its spelling, so the
+ * call before says what the next will hold; a stream that changes back and forth stays with k_parse_items, whose time
+ * depends on the spelling by a factor of two at most. The result does not depend on the choice. */
+void note_spelling(pj_ctx* c, uint32_t schema, uint64_t records, uint64_t errors, uint64_t fast, uint64_t dense, uint32_t max_rec) {
+  const uint64_t good = records - errors;
+  if (records < 16) return;
+  if (!c->items[schema]) {
+    if (fast * 100 >= good * 98) return;
+    c->items[schema] = true;
+    if (c->to_items[schema] < 255) ++c->to_items[schema];
+  } else if (c->to_items[schema] < 2 && dense * 100 >= good * 99 && max_rec <= 1024) c->items[schema] = false;
+}
+
+/* NDJSON: one launch of a parse kernel per piece. Host buffers of a whole stream are parsed in pieces cut after line
  * feeds, so that the copy of piece p+1 to the device, the kernel of piece p and the copy of the columns of piece p-1
  * back run at the same time on three streams. Every launch is enqueued before the host waits for anything: a piece
  * starts where the piece before it ended, which it reads from that piece's totals ON THE DEVICE (StreamArgs.prev). */
@@ -384,24 +424,27 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
 
   uint64_t longest = 0;
   for (int p = 0; p < np; ++p) longest = cut[p + 1] - cut[p] > longest ? cut[p + 1] - cut[p] : longest;
+  const bool items = c->items[schema];
   const TileShape shape = pick_tile_shape(c, schema, longest);
+  const uint32_t tile_bytes = items ? shape.tile_bytes : pick_stream_tile(c, schema);
+  const size_t state = items ? sizeof(ItemTile) : sizeof(StreamTile);
   /* look-back states: one buffer per piece, so that no launch waits for the one before it to be read back */
   uint64_t nt[MAX_PIECES], nt_total = 0;
   for (int p = 0; p < np; ++p) {
     const uint8_t* pin = d_in ? d_in + cut[p] : d_in;
     const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(pin) & 15u);
-    nt[p] = stream_tiles(mis, cut[p + 1] - cut[p], 1u, shape.tile_bytes); /* at least one tile: it closes the offset columns */
+    nt[p] = stream_tiles(mis, cut[p + 1] - cut[p], 1u, tile_bytes); /* at least one tile: it closes the offset columns */
     if (nt[p] >= (1ull << 31)) return set_err(c, PJ_ERR_TOO_LARGE, "pj_parse: too many tiles");
     nt_total += nt[p];
   }
-  { pj_status st = ensure(c, &c->tiles, nt_total * sizeof(ItemTile) + (size_t)np * 256 + 256); if (st) return st; }
-  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * sizeof(ItemTile) + (size_t)np * 256, c->stream));
+  { pj_status st = ensure(c, &c->tiles, nt_total * state + (size_t)np * 256 + 256); if (st) return st; }
+  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * state + (size_t)np * 256, c->stream));
   PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult) * np, c->stream));
   if (c->stall_once) { /* test hook: tickets start at 1, tile 0 is never processed, the waits for it run out */
     c->stall_once = false;
     for (int p = 0; p < np; ++p) PJ_CUDA(c, cudaMemsetAsync((uint8_t*)c->tiles.p + (size_t)p * 256, 1, 1, c->stream));
   }
-  c->stats.tile_records = IT_THREADS;
+  c->stats.tile_records = items ? IT_THREADS : ST_THREADS;
   uint64_t tiles_at = 0;
   for (int p = 0; p < np; ++p) {
     ItemArgs sa;
@@ -433,7 +476,18 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     sa.cols = pp.dcols;
     if (pipe) PJ_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_in[p], 0));
     PJ_CUDA(c, cudaEventRecord(c->ev_k0[p], c->stream));
-    PJ_CUDA(c, item_launch(schema, &sa, c->stream));
+    if (items) PJ_CUDA(c, item_launch(schema, &sa, c->stream));
+    else {
+      StreamArgs t;
+      memset(&t, 0, sizeof t);
+      t.in = sa.in; t.len = sa.len; t.limit = sa.limit; t.goff = sa.goff; t.is_first = sa.is_first; t.is_last = sa.is_last;
+      t.tile_bytes = tile_bytes; t.ntiles = sa.ntiles; t.opts = sa.opts; t.spin_limit_ns = sa.spin_limit_ns;
+      t.tiles = (StreamTile*)((uint8_t*)c->tiles.p + (size_t)np * 256) + (tiles_at - nt[p]);
+      t.ticket = sa.ticket; t.res = sa.res; t.prev = sa.prev;
+      memcpy(t.slot_cap, sa.slot_cap, sizeof t.slot_cap);
+      t.rec_cap = sa.rec_cap; t.plan = sa.plan; t.cols = sa.cols;
+      PJ_CUDA(c, stream_launch(schema, &t, c->stream));
+    }
     PJ_CUDA(c, cudaEventRecord(c->ev_k1[p], c->stream));
     PJ_CUDA(c, cudaMemcpyAsync(c->h_res + p, c->d_res + p, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
     PJ_CUDA(c, cudaEventRecord(c->ev_done[p], c->stream));
@@ -447,6 +501,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   for (uint32_t k = 0; k < NSLOT; ++k) total[k] = 0;
   bool over = false;
   uint32_t max_rec = 0;
+  uint64_t n_dense = 0;
   for (int p = 0; p < np; ++p) {
     PJ_CUDA(c, cudaEventSynchronize(c->ev_done[p]));
     const DevResult& r = c->h_res[p];
@@ -460,6 +515,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     if (r.timeout) return set_err(c, PJ_ERR_TIMEOUT, "pj_parse: a bounded device-side wait ran out");
     if (r.over) over = true;
     if (r.max_rec > max_rec) max_rec = r.max_rec;
+    n_dense += r.n_dense;
     const uint64_t rows_new = r.n_records;
     if (host_out && !over) {
       if (pipe) PJ_CUDA(c, cudaStreamWaitEvent(s_out, c->ev_done[p], 0));
@@ -487,7 +543,8 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   out->doc_err_kind = 0; out->doc_err_off = 0;
   const pj_status st = finish_columns(c, schema, len, pp, rows_done, n_errors, total, over, out);
   if (st) return st;
-  if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; c->max_rec_bytes[schema] = max_rec; }
+  if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; if (items) c->max_rec_bytes[schema] = max_rec; }
+  note_spelling(c, schema, rows_done, n_errors, n_fast, n_dense, max_rec);
   if (host_out) PJ_CUDA(c, cudaStreamSynchronize(s_out));
   return PJ_OK;
 }
@@ -683,6 +740,10 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   if (e == cudaSuccess) e = item_init_2(&c->schema);
   if (e == cudaSuccess) e = item_init_3(&c->schema);
   if (e == cudaSuccess) e = item_init_4(&c->schema);
+  if (e == cudaSuccess) e = stream_init_1(&c->schema);
+  if (e == cudaSuccess) e = stream_init_2(&c->schema);
+  if (e == cudaSuccess) e = stream_init_3(&c->schema);
+  if (e == cudaSuccess) e = stream_init_4(&c->schema);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, WTILE_SMEM_BYTES);
 #ifdef PJ_WT_CARVEOUT
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile, cudaFuncAttributePreferredSharedMemoryCarveout, PJ_WT_CARVEOUT);

@@ -35,6 +35,7 @@
 #include "pj_array.cuh"
 #include "pj_item_tables.h"
 #include "pj_result.h"
+#include "pj_schema_const.cuh"
 #include "pj_stream.cuh"
 
 namespace pj {
@@ -142,6 +143,7 @@ struct ItemShared {
   uint32_t nspecial, odd;                  /* odd: some record ends inside a string */
   uint32_t nstr, nline, stop;              /* strings, lines, last separator */
   uint32_t free_word;                      /* first free word behind the strings */
+  uint32_t ndense;                         /* lines the dense walk took */
   uint32_t ok, slow, tile, next;
   unsigned long long mbar;
 };
@@ -1765,7 +1767,6 @@ __device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemSha
 }
 
 /* ---- the exact parser -------------------------------------------------------------------------------------------- */
-static __constant__ Schema c_schema; /* one copy per translation unit that includes this header (each sets its own) */
 
 /* A record the fast steps refused, from its first byte at input offset s up to `limit`: kind and offset of its failure in *err,
  * *off, or *err = 0 when it is a valid one after all. */
@@ -1904,11 +1905,11 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     if (lane == 0) sh.oddmask[warp] = m;
   }
   if (__syncthreads_or((int)sh.slow)) return false;
-  ck[2] = clock64();
   {
     uint32_t nodd = 0;
 #pragma unroll
     for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
+    if (tid == 0) sh.ndense = nline - nodd;
     if (nodd) {
       __syncthreads(); /* oddmask[] is read */
       item_walk_again<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid, mine);
@@ -1919,7 +1920,6 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
       if (__syncthreads_or((int)sh.slow)) return false;
     }
   }
-  ck[7] = clock64();
 
   /* ---- values: fields x groups of 32 lines ---- */
   {
@@ -2092,7 +2092,6 @@ template <int SCHEMA, bool ARR>
 __device__ __forceinline__ bool item_try(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t* rows, uint32_t tile, uint32_t tid, long long* ck) {
   const bool fine = item_index<ARR>(a, g, sh, win, strs, tid, tile);
   if (__syncthreads_or(!fine || sh.slow)) return false; /* (decided together: what a warp that goes on may set there comes too late) */
-  ck[6] = clock64();
   return item_tile<SCHEMA, ARR>(a, g, sh, win, strs, rows, tile, tid, ck);
 }
 
@@ -2110,7 +2109,7 @@ __global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __g
   __syncthreads();
   const uint32_t tile = sh.tile;
   if (tile >= a.ntiles) return;
-  long long ck[8];
+  long long ck[5];
   ck[0] = clock64();
   const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(a.in) & 15u);
   const StreamGeom g = stream_geom(mis, a.len, a.limit, a.tile_bytes, tile, a.win_bytes);
@@ -2151,7 +2150,7 @@ __global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __g
   if (tid == 0) {
     const long long c5 = clock64();
     atomicAdd(&a.res->phase_cycles[0], (unsigned long long)(ck[1] - ck[0]));
-    atomicAdd(&a.res->n_wide, (unsigned long long)(ck[6] - ck[1])); atomicAdd(&a.res->n_wide_fast, (unsigned long long)(ck[2] - ck[6])); atomicAdd(&a.res->wide_cycles[0], (unsigned long long)(ck[7] - ck[2])); atomicAdd(&a.res->wide_cycles[1], (unsigned long long)(ck[3] - ck[7]));
+    if (sh.ndense) atomicAdd(&a.res->n_dense, (unsigned long long)sh.ndense);
     atomicAdd(&a.res->phase_cycles[1], (unsigned long long)(ck[3] - ck[1]));
     atomicAdd(&a.res->phase_cycles[2], (unsigned long long)(ck[4] - ck[3]));
     atomicAdd(&a.res->phase_cycles[3], (unsigned long long)(c5 - ck[4]));
