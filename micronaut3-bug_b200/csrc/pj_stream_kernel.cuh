@@ -2,7 +2,7 @@
  * pj_stream_kernel.cuh — k_parse_stream<SCHEMA>: NDJSON bytes to typed columns in ONE kernel and one pass over HBM, a record
  * per thread. It is the faster one for records all spelled the way a compact serialiser spells them, where the threads of a
  * warp stay together (1M Pets 600 us, k_parse_items 625 us); with blanks or long lists they do not (200k Users with blanks
- * 960 us against 130 us, long lists 44 ms against 4 ms), and pj_api.cu then takes k_parse_items (pj_item.cuh).
+ * 360 us against 130 us, long lists 44 ms against 4 ms), and pj_api.cu then takes k_parse_items (pj_item.cuh).
  *
  * One thread block = one tile of the input (pj_stream.cuh): the tile and what follows it are staged in shared memory
  * by one bulk copy (cp.async.bulk, the untiled TMA form, no multicast), the block builds the line index of the window
@@ -666,10 +666,10 @@ __device__ __forceinline__ void stream_tile_rest(const StreamArgs& a, const Stre
     }
   }
   {
-    uint32_t pk = (r.err ? 1u : 0u) | (r.fast << 16);
+    uint32_t pk = (r.err ? 1u : 0u) | (r.fast << 8) | (r.locked << 16); /* at most 32 of each */
     for (int d = 16; d; d >>= 1) pk += __shfl_down_sync(0xFFFFFFFFu, pk, d);
-    if (lane == 0 && (pk & 0xFFFF)) atomicAdd(&a.res->n_errors, (unsigned long long)(pk & 0xFFFF));
-    if (lane == 0 && (pk >> 16)) atomicAdd(&a.res->n_fast, (unsigned long long)(pk >> 16));
+    if (lane == 0 && (pk & 0xFF)) atomicAdd(&a.res->n_errors, (unsigned long long)(pk & 0xFF));
+    if (lane == 0 && (pk >> 8)) atomicAdd(&a.res->n_fast, (unsigned long long)((pk >> 8) & 0xFF) | ((unsigned long long)(pk >> 16) << 32)); /* high half: those taken in step */
   }
 
   /* ---- positions inside the tile, then the look-back ---- */
