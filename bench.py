@@ -371,7 +371,7 @@ def run_single(args, pj, abi):
                    "l2": "input (295 MB at 1M records) and columns are larger than the 126 MB L2; no flush between steps", "sharding": "single GPU"},
         "gb_per_s": n_rec * args.steps / (ms * 1e-3) * nbytes / R / 1e9,
         "roofline": roofline_block(args, alg_bytes, k_ms, ms / args.steps, R,
-                                   "k_parse_tile over the array index (one launch per step)" if array_wl else
+                                   "k_parse_items over the array index (one launch per step)" if array_wl else
                                    "k_parse_stream (line index, tokenising, validation and emission of one tile per block; one launch per step)"),
         "gpu_launches": launches,
         "tile_kernel": {"threads_per_block": int(last_stats.tile_records), "blocks": int(last_stats.tiles), "fast_records": int(last_stats.fast_records),
