@@ -1,0 +1,157 @@
+"""k_parse_items (csrc/pj_item.cuh) run on the CPU, block by block, against the checker: no GPU needed.
+
+tests/host_emu/pj_block_emu.h gives the kernel's source the threads, warp collectives and barriers of one block and reports lanes
+that part at a collective, threads that part at a barrier and waits that do not end; one test repeats a slice of the others under
+AddressSanitizer and UndefinedBehaviorSanitizer.
+"""
+import ctypes as C
+import os
+import random
+import subprocess
+import sys
+from concurrent.futures import ThreadPoolExecutor
+
+import numpy as np
+import pytest
+
+from pj_testlib import abi, as_u8, nrec_bound, pj, same_result
+from test_host_emulation import blank_mutations
+from test_oracle_crosscheck import mutate
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+NDJSON, ARRAY = abi.PJ_FRAMING_NDJSON, abi.PJ_FRAMING_ARRAY
+PET, ORDER, USER, MIXED = abi.PJ_SCHEMA_PET, abi.PJ_SCHEMA_ORDER, abi.PJ_SCHEMA_USER, abi.PJ_SCHEMA_MIXED
+ALL = abi.PJ_GEN_ESCAPES | abi.PJ_GEN_WHITESPACE | abi.PJ_GEN_MALFORMED | abi.PJ_GEN_SPARSE
+FLAG_SETS = [0, abi.PJ_GEN_ESCAPES, abi.PJ_GEN_WHITESPACE, abi.PJ_GEN_MALFORMED, abi.PJ_GEN_SPARSE, ALL, abi.PJ_GEN_ZIPF_LISTS | ALL]
+
+
+class Opts(C.Structure):
+    _fields_ = [("len", C.c_uint64), ("slack", C.c_uint64), ("goff", C.c_uint64)] + [
+        (k, C.c_uint32) for k in ("array", "is_first", "is_last", "opts", "tile_bytes", "win_bytes", "str_words", "row_cap", "order")] + [("rec_cap", C.c_uint64)]
+
+
+@pytest.fixture(scope="session")
+def emu(native):
+    """The kernel for the host, a library per model set: {schema: CDLL}."""
+    src = os.path.join(HERE, "host_emu", "pj_item_emu.cpp")
+    csrc = os.path.join(ROOT, "micronaut3-bug_b200", "csrc")
+    deps = [src, os.path.join(HERE, "host_emu", "pj_block_emu.h")] + [os.path.join(csrc, f) for f in os.listdir(csrc) if f.endswith((".cuh", ".h", ".inc"))]
+    san = os.environ.get("PJ_EMU_SANITIZE") == "1"
+    flags = ["-O1", "-g", "-fsanitize=address,undefined", "-fno-sanitize-recover=all"] if san else ["-O2"]
+
+    def build(schema):
+        lib = os.path.join(HERE, "host_emu", f"libpj_item_emu{schema}{'_san' if san else ''}.so")
+        if not os.path.exists(lib) or any(os.path.getmtime(d) > os.path.getmtime(lib) for d in deps):
+            subprocess.run(["g++", *flags, "-std=c++17", "-fno-extern-tls-init", "-fPIC", "-shared", "-w", f"-DEMU_SCHEMA={schema}", "-I", os.path.join(ROOT, "include"), "-I", csrc,
+                            "-x", "c++", src, "-o", lib], check=True)
+        cdll = C.CDLL(lib)
+        cdll.emu_item_error.restype = C.c_char_p
+        cdll.emu_item_barriers.restype = C.c_uint64
+        return cdll
+
+    with ThreadPoolExecutor() as pool:
+        return dict(zip((1, 2, 3, 4), pool.map(build, (1, 2, 3, 4))))
+
+
+class Run:
+    """A parse by the emulated kernel: its columns, and what it says about itself."""
+
+    def __init__(self, emu, schema, text, framing=NDJSON, tile=32768, slack=4096, mis=0, opts=0, order=0, str_words=None, row_cap=256, shard_slack=0,
+                 is_first=1, is_last=1, goff=0):
+        buf = as_u8(text)
+        raw = np.full(buf.size + 64, 0xEE, np.uint8)
+        at = (-raw.ctypes.data) % 16 + mis
+        raw[at:at + buf.size] = buf
+        self.cols = abi.HostColumns(schema, abi.default_caps(schema, nrec_bound(buf), buf.size), alloc=lambda nb: np.full(nb, 0xA5, np.uint8))
+        win = min(tile + slack, 65536 - 64)
+        o = Opts(len=buf.size - shard_slack, slack=shard_slack, goff=goff, array=framing == ARRAY, is_first=is_first, is_last=is_last, opts=opts, tile_bytes=tile,
+                 win_bytes=win, str_words=str_words or win // 4, row_cap=row_cap, order=order, rec_cap=nrec_bound(buf))
+        stats = (C.c_uint64 * 4)()
+        lib = emu[schema]
+        self.status = lib.emu_item_parse(C.byref(o), C.c_void_p(raw.ctypes.data + at), C.byref(self.cols.raw), stats)
+        assert self.status >= 0, lib.emu_item_error().decode()
+        self.fast, self.dense, self.longest, self.tiles = stats
+        self.barriers = lib.emu_item_barriers()
+
+
+SHAPES = [dict(), dict(tile=1024, slack=4096, mis=5), dict(tile=4096, slack=1024, mis=15, order=3), dict(tile=16384, slack=28672, str_words=3000, order=6)]
+
+
+@pytest.mark.parametrize("schema", [PET, ORDER, USER, MIXED])
+@pytest.mark.parametrize("flags", FLAG_SETS)
+def test_generated_text(emu, oracle, schema, flags):
+    text = pj.gen_text(schema, 0xE11, 0, 300, flags)
+    want = oracle.parse(schema, text)
+    for shape in SHAPES:
+        got = Run(emu, schema, text, **shape)
+        assert same_result(want, got.cols) == "", shape
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_mutated_text(emu, oracle, seed):
+    rng = random.Random(seed)
+    for it in range(60):
+        schema = rng.choice([1, 1, 2, 3, 4, 4])
+        lines = bytes(pj.gen_text(schema, rng.randrange(1 << 30), rng.randrange(1000), 40, rng.choice(FLAG_SETS))).split(b"\n")[:-1]
+        out = [ln if rng.random() < 0.2 else mutate(rng, ln) for ln in lines]
+        body = as_u8(blank_mutations(rng, b"\n".join(out)))
+        opts = rng.choice([0, 0, 1, 2, 4, 7])
+        got = Run(emu, schema, body, opts=opts, **rng.choice(SHAPES))
+        assert same_result(oracle.parse(schema, body, opts=opts), got.cols) == "", (seed, it, schema, opts)
+
+
+def test_mutated_arrays(emu, oracle):
+    rng = random.Random(9)
+    for it in range(60):
+        schema = rng.choice([1, 2, 3, 4])
+        text = bytes(pj.gen_text(schema, rng.randrange(1 << 30), 0, 40, abi.PJ_GEN_ARRAY | rng.choice(FLAG_SETS[:6])))
+        if it % 3:
+            text = mutate(rng, text)
+        want = oracle.parse(schema, as_u8(text), ARRAY)
+        got = Run(emu, schema, text, ARRAY, **rng.choice(SHAPES))
+        assert same_result(want, got.cols) == "", (it, schema)
+        assert (want.raw.doc_err_kind, want.raw.doc_err_off) == (got.cols.raw.doc_err_kind, got.cols.raw.doc_err_off)
+
+
+def test_shards(emu, oracle):
+    """Cut anywhere, with the bytes behind as slack: every record is parsed by the shard that owns the line feed before it."""
+    rng = random.Random(11)
+    text = as_u8(blank_mutations(rng, pj.gen_text(PET, 3, 0, 300, ALL).tobytes()))
+    want = oracle.parse(PET, text)
+    for parts in (2, 5):
+        cuts = [text.size * k // parts for k in range(parts + 1)]
+        n = 0
+        for k in range(parts):
+            lo, hi = cuts[k], cuts[k + 1]
+            slack = min(65536, text.size - hi)
+            piece = text[lo:hi + slack]
+            kw = dict(is_first=int(k == 0), is_last=int(hi + slack == text.size), goff=lo)
+            got = Run(emu, PET, piece, tile=4096, mis=k, shard_slack=slack, **kw)
+            assert same_result(oracle.parse(PET, piece, slack=slack, **kw), got.cols) == "", (parts, k)
+            n += got.cols.n_records
+        assert n == want.n_records
+
+
+def test_known_answers(emu, oracle):
+    from golden.kat_cases import CASES, OPTION_CASES
+    from pj_testlib import SCHEMA_BY_NAME, records
+
+    for name, schema, framing, data, expected in CASES:
+        sch, fr = SCHEMA_BY_NAME[schema], ARRAY if framing == "array" else NDJSON
+        got = Run(emu, sch, data, fr, tile=1024)
+        assert same_result(oracle.parse(sch, as_u8(data), fr), got.cols) == "", name
+    for name, schema, opts, data, expected in OPTION_CASES:
+        sch = SCHEMA_BY_NAME[schema]
+        assert records(Run(emu, sch, data, opts=opts).cols.as_dict(), sch) == expected, name
+
+
+def test_under_sanitizers():
+    asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
+    if not os.path.isabs(asan) or not os.path.exists(asan):
+        pytest.skip("no libasan beside this gcc")
+    env = dict(os.environ, PJ_EMU_SANITIZE="1", LD_PRELOAD=asan, ASAN_OPTIONS="detect_leaks=0:abort_on_error=0:detect_stack_use_after_return=0", UBSAN_OPTIONS="print_stacktrace=1")
+    r = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "-p", "no:cacheprovider", os.path.abspath(__file__), "-k", "not sanitizers and not (mutated_text and 3)"],
+                       env=env, capture_output=True, text=True, cwd=HERE, timeout=1500)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
+    assert "passed" in r.stdout
