@@ -1173,7 +1173,7 @@ __device__ __forceinline__ uint32_t item_key(const ItemShared& sh, const uint8_t
   const uint32_t slot = it_hash(x0 & 0xFFFFu, len, IT_MUL);
   const uint4 kt = *reinterpret_cast<const uint4*>(&sh.key[slot][0]), km = *reinterpret_cast<const uint4*>(&sh.key[slot][4]);
   const uint32_t f = sh.field[s == IS_ROOT ? 0 : (s == IS_CHILD ? 1 : 2)][slot];
-  return (((x0 ^ kt.x) & km.x) | ((x1 ^ kt.y) & km.y) | ((x2 ^ kt.z) & km.z) | ((x3 ^ kt.w) & km.w)) != 0 || len < 2u || len > 15u ? 0u : f;
+  return (((x0 ^ kt.x) & km.x) | ((x1 ^ kt.y) & km.y) | ((x2 ^ kt.z) & km.z) | ((x3 ^ kt.w) & km.w)) != 0 || len != ItField::len(f) ? 0u : f;
 }
 /* Lines [i0, i0 + n), each with a string, by a warp: together at most 32 strings, or one line with more. Returns false when
  * the tile has to take the other road. */

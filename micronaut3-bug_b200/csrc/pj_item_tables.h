@@ -102,24 +102,26 @@ struct ItStride {
 
 /* A property name in an object. 0: not a property (its value is skipped). */
 struct ItField {
-  static PJ_CX uint32_t make(uint32_t word, uint32_t bit, uint32_t kind, uint32_t models) {
+  static PJ_CX uint32_t make(uint32_t word, uint32_t bit, uint32_t kind, uint32_t models, uint32_t len) {
     uint32_t allowed = 0;
     if (kind == K_I64 || kind == K_I32 || kind == K_BOOL) allowed = 1u << IV_SCALAR;
     else if (kind == K_STR || kind == K_ENUM || kind == K_DATETIME) allowed = 1u << IV_STR;
     else if (kind == K_OBJ) allowed = (1u << IV_OBJ) | (1u << IV_EOBJ);
     else if (kind == K_LIST_STR) allowed = (1u << IV_LIST) | (1u << IV_ELIST);
     else allowed = (1u << IV_ELEM) | (1u << IV_ELIST);
-    return word | (bit << 6) | (kind << 10) | (allowed << 14) | (models << 22) | (1u << 31);
+    return word | (bit << 6) | (kind << 10) | (allowed << 14) | (models << 22) | (len << 25) | (1u << 31);
   }
   static PJ_CX uint32_t word(uint32_t f) { return f & 63u; }
   static PJ_CX uint32_t bit(uint32_t f) { return (f >> 6) & 15u; }
   static PJ_CX uint32_t kind(uint32_t f) { return (f >> 10) & 15u; }
   static PJ_CX uint32_t allowed(uint32_t f) { return (f >> 14) & 255u; }
   static PJ_CX uint32_t models(uint32_t f) { return (f >> 22) & 7u; }
+  static PJ_CX uint32_t len(uint32_t f) { return (f >> 25) & 15u; } /* bytes of the name */
 };
 
 /* Names hash by their first two bytes and their length; the multiplier is searched at compile time so that no two of
- * the names share a slot. An entry is the name and its closing quote (text and byte masks, four words each). */
+ * the names share a slot. An entry is the name (text and byte masks, four words each; its length is in ItField: what follows a key
+ * that was decoded in place is not its quote). */
 static constexpr uint32_t IT_SLOTS = 32;
 struct ItTables {
   uint32_t key[IT_SLOTS][8];
@@ -160,9 +162,7 @@ PJ_CX uint32_t it_find_mul() {
 }
 static constexpr uint32_t IT_MUL = it_find_mul();
 static_assert(IT_MUL != 0, "a hash multiplier without collisions");
-PJ_CX uint32_t it_name_byte(uint64_t lo, uint64_t hi, uint32_t len, uint32_t k) {
-  return k == len ? (uint32_t)'"' : (uint32_t)((k < 8 ? lo >> (8 * k) : hi >> (8 * (k - 8))) & 0xFF);
-}
+PJ_CX uint32_t it_name_byte(uint64_t lo, uint64_t hi, uint32_t k) { return (uint32_t)((k < 8 ? lo >> (8 * k) : hi >> (8 * (k - 8))) & 0xFF); }
 PJ_CX uint32_t it_slot_of(const CF& f) { return it_hash((uint32_t)(f.lo & 0xFFFFu), f.len, IT_MUL); }
 template <int OBJ>
 PJ_CX void it_fill_root(ItTables& t, uint32_t model) {
@@ -171,7 +171,7 @@ PJ_CX void it_fill_root(ItTables& t, uint32_t model) {
     uint32_t& e = t.field[0][it_slot_of(f)];
     uint32_t bit = (uint32_t)i;
     if (e && ItField::bit(e) != bit) bit = IB_SHARED;
-    e = ItField::make(it_root_word<OBJ>(i), bit, f.kind, model | (e ? ItField::models(e) : 0u));
+    e = ItField::make(it_root_word<OBJ>(i), bit, f.kind, model | (e ? ItField::models(e) : 0u), f.len);
   }
 }
 template <int OBJ, int CH>
@@ -179,7 +179,7 @@ PJ_CX void it_fill_flat(ItTables& t, int which, uint32_t word0, uint32_t bit0) {
   if constexpr (CH >= 0) {
     for (int i = 0; i < CObj<CH>::N; ++i) {
       const CF f = CObj<CH>::f[i];
-      t.field[which][it_slot_of(f)] = ItField::make(word0 + (which == 1 ? it_flat_word<CH>(i) : (uint32_t)i), bit0 + (uint32_t)i, f.kind, 7u);
+      t.field[which][it_slot_of(f)] = ItField::make(word0 + (which == 1 ? it_flat_word<CH>(i) : (uint32_t)i), bit0 + (uint32_t)i, f.kind, 7u, f.len);
     }
   }
 }
@@ -194,8 +194,8 @@ PJ_CX ItTables it_tables(int schema) {
   const ItNames s = it_all_names();
   for (uint32_t k = 0; k < s.count; ++k) {
     const uint32_t slot = it_hash((uint32_t)(s.n[k].lo & 0xFFFFu), s.n[k].len, IT_MUL);
-    for (uint32_t b = 0; b <= s.n[k].len && b < 16; ++b) {
-      t.key[slot][b >> 2] |= it_name_byte(s.n[k].lo, s.n[k].hi, s.n[k].len, b) << (8 * (b & 3));
+    for (uint32_t b = 0; b < s.n[k].len; ++b) {
+      t.key[slot][b >> 2] |= it_name_byte(s.n[k].lo, s.n[k].hi, b) << (8 * (b & 3));
       t.key[slot][4 + (b >> 2)] |= 0xFFu << (8 * (b & 3));
     }
   }
