@@ -23,6 +23,7 @@
 #include "pj_kernels.cuh"
 #include "pj_array_kernels.cuh"
 #include "pj_item.cuh"
+#include "pj_item_shape.h"
 #include "pj_stream_kernel.cuh"
 
 using namespace pj;
@@ -98,6 +99,7 @@ struct Buffer {
 enum { PJ_CTX_RESULTS = 16 };
 struct pj_ctx {
   int device = 0;
+  int sms = 148;
   int inclusion = PJ_INCLUDE_NON_EMPTY;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -196,10 +198,8 @@ pj_status ensure_pipe_streams(pj_ctx* c) {
 }
 
 int persistent_grid(pj_ctx* c, uint64_t items, int threads) {
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
   uint64_t want = (items + threads - 1) / threads;
-  uint64_t cap = (uint64_t)sms * 16;
+  uint64_t cap = (uint64_t)c->sms * 16;
   if (want < 1) want = 1;
   return (int)(want < cap ? want : cap);
 }
@@ -276,42 +276,19 @@ pj_status finish_columns(pj_ctx* c, uint32_t schema, uint64_t len, const ParsePl
   return PJ_OK;
 }
 
-/* How a call's input is cut into tiles. The result of a call does not depend on it. */
-struct TileShape { uint32_t tile_bytes, win_bytes, str_words, row_cap; };
 uint32_t item_stride(uint32_t schema) {
   return schema == PJ_SCHEMA_PET ? ItStride<1>::n : (schema == PJ_SCHEMA_ORDER ? ItStride<2>::n : (schema == PJ_SCHEMA_USER ? ItStride<3>::n : ItStride<4>::n));
 }
-TileShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
-  static const double dflt[5] = {0, 300, 146, 190, 230};
-  const double avg = c->avg_rec_bytes[schema] > 0 ? c->avg_rec_bytes[schema] : dflt[schema];
-  TileShape t;
-  /* room behind the tile for its last record: a quarter more than the longest one of the call before, or 13 average records,
-     which reach the longest ones of a skewed distribution */
-  uint64_t longest = c->max_rec_bytes[schema] ? c->max_rec_bytes[schema] + c->max_rec_bytes[schema] / 4 + 64 : (uint64_t)(avg * 13);
-  const uint64_t shortest = 4096;
-  const uint32_t slack = (longest < shortest ? (uint32_t)shortest : (longest > 28672 ? 28672u : (uint32_t)longest)) & ~15u;
-  uint32_t per_word = 9; /* window bytes per word for strings */
-  /* what the block indexes in one step, or so that most tiles have fewer than three quarters of the lines they may have */
-  uint64_t tile = IT_STEP - (uint64_t)(2 * avg), few = (uint64_t)(avg * (c->avg_rec_bytes[schema] > 0 ? IT_MAX_LINES * 47 / 64 : IT_MAX_LINES * 9 / 16)); /* (a first call's records may be shorter) */
-  if (avg * 4 > IT_STEP) tile = IT_STEP / 2;
-  if (tile > few) tile = few;
-  /* few tiles: one for every block that can be resident, and room enough */
-  if (len / (148 * IT_BLOCKS) < tile) { tile = len / (148 * IT_BLOCKS); if (tile < 4096) tile = 4096; per_word = 2; }
-  if (c->tile_bytes_opt) { tile = c->tile_bytes_opt; if (tile < ST_MIN_TILE_BYTES) tile = ST_MIN_TILE_BYTES; if (tile > 32768) tile = 32768; }
-  /* as many resident blocks as leave three quarters of that tile */
-  const uint64_t least = tile - tile / 4;
-  for (uint32_t blocks = IT_BLOCKS;; ) {
-    t.tile_bytes = (uint32_t)(tile & ~31ull);
-    if (t.tile_bytes < ST_MIN_TILE_BYTES) t.tile_bytes = ST_MIN_TILE_BYTES;
-    t.win_bytes = t.tile_bytes + slack;
-    t.str_words = t.win_bytes / per_word;
-    const double recs = (double)t.tile_bytes / avg * 1.3 + 24;
-    t.row_cap = recs > IT_MAX_LINES ? IT_MAX_LINES : (uint32_t)recs;
-    const uint32_t room = (228u * 1024u) / blocks - 1024u - (uint32_t)sizeof(ItemShared) - 256u;
-    if (per_word == 2 || c->tile_bytes_opt || t.tile_bytes <= 4096 || item_layout(t.win_bytes, t.str_words, t.row_cap, item_stride(schema)).total <= room) return t;
-    if (tile - 512 >= least || blocks == 2) tile -= 512;
-    else { tile = least + least / 3; --blocks; }
-  }
+ItemShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
+  static const double guess[5] = {0, 300, 146, 190, 230};
+  ItemShapeIn in;
+  in.len = len;
+  in.avg = c->avg_rec_bytes[schema]; in.guess = guess[schema];
+  in.longest = c->max_rec_bytes[schema];
+  in.tile_opt = c->tile_bytes_opt;
+  in.stride = item_stride(schema);
+  in.sms = (uint32_t)c->sms;
+  return item_shape(in);
 }
 
 cudaError_t item_launch(uint32_t schema, const ItemArgs* a, cudaStream_t s) {
@@ -426,7 +403,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   uint64_t longest = 0;
   for (int p = 0; p < np; ++p) longest = cut[p + 1] - cut[p] > longest ? cut[p + 1] - cut[p] : longest;
   const bool items = c->items[schema];
-  const TileShape shape = pick_tile_shape(c, schema, longest);
+  const ItemShape shape = pick_tile_shape(c, schema, longest);
   const uint32_t tile_bytes = items ? shape.tile_bytes : pick_stream_tile(c, schema);
   const size_t state = items ? sizeof(ItemTile) : sizeof(StreamTile);
   /* look-back states: one buffer per piece, so that no launch waits for the one before it to be read back */
@@ -594,7 +571,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   for (uint32_t k = 0; k < NSLOT; ++k) total[k] = 0;
   ItemArgs sa;
   memset(&sa, 0, sizeof sa);
-  const TileShape shape = pick_tile_shape(c, schema, len);
+  const ItemShape shape = pick_tile_shape(c, schema, len);
   sa.in = d_in; sa.len = len; sa.limit = len;
   sa.is_first = 1; sa.is_last = 1;
   sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_words = shape.str_words; sa.row_cap = shape.row_cap;
@@ -717,6 +694,7 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   c->tile_bytes_opt = opt ? opt->tile_bytes : 0;
   if (opt && opt->spin_limit_us) c->spin_ns = (unsigned long long)opt->spin_limit_us * 1000ull;
   DeviceGuard guard(dev);
+  (void)cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
   auto fail_create = [&](cudaError_t err, const char* what) {
     set_err(nullptr, PJ_ERR_CUDA, "%s: %s", what, cudaGetErrorString(err));
     pj_destroy(c);

@@ -7,6 +7,7 @@
 
 #include "pj_block_emu.h"
 #include "pj_item.cuh"
+#include "pj_item_shape.h"
 
 using namespace pj;
 
@@ -48,8 +49,15 @@ void array_index(const uint8_t* in, uint64_t len, std::vector<uint64_t>& sep, De
 
 extern "C" const char* emu_item_error() { return emu_block::error; }
 extern "C" uint64_t emu_item_barriers() { return emu_block::n_barriers; }
-extern "C" uint32_t emu_item_shared_bytes() { return (uint32_t)sizeof(ItemShared); }
-extern "C" uint32_t emu_item_stride() { return ItStride<EMU_SCHEMA>::n; }
+/* out: tile, window, words for strings, rows, bytes of dynamic shared memory, the most that may be, blocks an SM holds */
+extern "C" void emu_item_shape(uint64_t len, double avg, double guess, uint32_t longest, uint32_t tile_opt, uint32_t* out) {
+  const ItemShape s = item_shape(ItemShapeIn{len, avg, guess, longest, tile_opt, ItStride<EMU_SCHEMA>::n, 148});
+  const uint32_t total = item_layout(s.win_bytes, s.str_words, s.row_cap, ItStride<EMU_SCHEMA>::n).total;
+  uint32_t blocks = IT_BLOCKS;
+  while (blocks > 1 && total > item_room(blocks)) --blocks;
+  const uint32_t v[7] = {s.tile_bytes, s.win_bytes, s.str_words, s.row_cap, total, IT_MAX_DYN_SMEM, blocks};
+  for (int k = 0; k < 7; ++k) out[k] = v[k];
+}
 
 /* in: 16-byte aligned base + the caller's misalignment, readable in whole 16-byte blocks. stats[4]: fast records, lines the strict
  * walk took, longest record, tiles. Returns 0, 1 (some buffer is too small) or -1 (see emu_item_error). */

@@ -163,6 +163,27 @@ def test_keys_spelled_with_escapes(emu, oracle):
             assert want.n_errors == 0 and same_result(want, Run(emu, schema, body).cols) == "", line
 
 
+@pytest.mark.parametrize("schema", [PET, ORDER, USER, MIXED])
+def test_tile_shape_fits_shared_memory(emu, schema):
+    """Every shape a call can get fits the kernel's shared memory and 16-bit window offsets; calls of few tiles get one resident block
+    for each of them. (One record of 23 KB in an earlier call made a later one of 16 MB ask for 211 KB of 200.)"""
+    out = (C.c_uint32 * 7)()
+    guess = [0, 300, 146, 190, 230][schema]
+    lens = [0, 1, 300, 5000, 10**5] + [int(10**5 * 1.21 ** k) for k in range(1, 60)] + list(range(15_000_000, 17_000_000, 40_000))
+    for avg in [0, 1, 9, 40, 146, 200, 230, 250, 300, 700, 2000, 9000, 20_000, 10**6]:
+        for longest in [0, 300, 3277, 9000, 22_000, 22_886, 23_000, 65_000, 1 << 30]:
+            for tile_opt in (0, 1, 4096, 20_000, 32_768, 1 << 20):
+                for n in lens if tile_opt == 0 else lens[:40:8]:
+                    emu[schema].emu_item_shape(C.c_uint64(n), C.c_double(avg), C.c_double(guess), C.c_uint32(longest), C.c_uint32(tile_opt), out)
+                    tile, win, words, rows, total, most, blocks = out
+                    where = (n, avg, longest, tile_opt, list(out))
+                    assert total <= most, where
+                    assert 1024 <= tile <= 36864 and tile % 32 == 0 and tile < win <= 65536 - 64 and win % 16 == 0, where
+                    assert 24 <= rows <= 256 and words * 9 + 9 > win, where
+                    if tile_opt == 0 and longest <= 3277 and avg <= 300:
+                        assert blocks == 3, where
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
