@@ -58,7 +58,7 @@ def test_both_kernels_agree(items_ctx, oracle):
 
 def test_one_long_record_then_a_call_of_few_tiles(oracle):
     """The tile shape of a call of 16 MB whose context has seen a record of 25 KB: it asked for more shared memory than there is."""
-    text = bytes(pj.gen_text(3, 5, 0, 85_000, abi.PJ_GEN_ARRAY))
+    text = bytes(pj.gen_text(3, 5, 0, 83_000, abi.PJ_GEN_ARRAY))
     body = as_u8(text[:-1] + b',{"id":1,"username":"' + b"u" * 25_000 + b'"}]')
     assert 15_400_000 < body.size < 16_200_000
     want = oracle.parse(3, body, ARRAY)
