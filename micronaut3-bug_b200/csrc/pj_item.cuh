@@ -57,7 +57,7 @@ static constexpr uint32_t IT_FRONT = 32;             /* bytes before the window 
 static constexpr uint32_t IT_PAD = IT_SPAN + 16;               /* ... and behind it */
 static constexpr uint32_t IT_MAX_LINES = IT_THREADS; /* lines per tile */
 static constexpr uint32_t IT_MAX_STRS = 4096;        /* strings per tile */
-static constexpr uint32_t IT_MAX_SPECIAL = 512;     /* strings per tile that need a closer look */
+static constexpr uint32_t IT_MAX_SPECIAL = 512;     /* strings per tile that need a closer look and are kept in a list */
 static constexpr uint32_t IT_MAX_WIN = 65536 - 64;   /* window offsets are 16-bit */
 static constexpr uint32_t IT_STAGE = 256;            /* words of a warp to put strings together in */
 static constexpr uint32_t IT_MAX_DYN_SMEM = 200 * 1024; /* dynamic shared memory of a block */
@@ -575,25 +575,31 @@ static __device__ __noinline__ bool item_decode_string(uint8_t* win, uint32_t op
   }
   return true;
 }
-/* The strings item_index() marked, one per thread. */
-__device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh, uint8_t* win, uint32_t* pairs, uint32_t tid) {
-  for (uint32_t i = tid; i < sh.nspecial; i += IT_THREADS) {
-    const uint32_t k = sh.special_list[i], pr = pairs[k];
-    const uint32_t open = pr & 0xFFFFu, close = pr >> 16;
-    uint32_t moved;
-    const bool ok = item_decode_string(win, open, close, a.opts, &moved);
-    if (!ok || !moved) atomicAnd(&sh.special[k >> 5], ~(1u << (k & 31u)));
-    if (ok && !moved) continue; /* plain after all */
-    if (!ok) atomicOr(&sh.broken[k >> 5], 1u << (k & 31u));
-    uint32_t lo = 0, hi = sh.nline; /* its line: the last one that begins at or before it and has a string */
-    while (lo + 1u < hi) { const uint32_t mid = (lo + hi) >> 1; if (sh.line[mid] >> 16 <= k) lo = mid; else hi = mid; }
-    atomicOr(&sh.movedline[lo >> 5], 1u << (lo & 31u));
-    /* a line with a broken string, or with a key in another spelling, is not for the walk */
-    const uint32_t sep = (sh.line[lo + 1u] & 0xFFFFu) - 1u;
-    uint32_t p = close + 1u;
-    while (p < sep && item_blank(win[p])) ++p;
-    if (!ok || win[p] == ':') atomicOr(&sh.oddline[lo >> 5], 1u << (lo & 31u));
+/* One string item_index() marked. */
+__device__ __forceinline__ void item_special(const ItemArgs& a, ItemShared& sh, uint8_t* win, const uint32_t* pairs, uint32_t k) {
+  const uint32_t pr = pairs[k], open = pr & 0xFFFFu, close = pr >> 16;
+  uint32_t moved;
+  const bool ok = item_decode_string(win, open, close, a.opts, &moved);
+  if (!ok || !moved) atomicAnd(&sh.special[k >> 5], ~(1u << (k & 31u)));
+  if (ok && !moved) return; /* plain after all */
+  if (!ok) atomicOr(&sh.broken[k >> 5], 1u << (k & 31u));
+  uint32_t lo = 0, hi = sh.nline; /* its line: the last one that begins at or before it and has a string */
+  while (lo + 1u < hi) { const uint32_t mid = (lo + hi) >> 1; if (sh.line[mid] >> 16 <= k) lo = mid; else hi = mid; }
+  atomicOr(&sh.movedline[lo >> 5], 1u << (lo & 31u));
+  /* a line with a broken string, or with a key in another spelling, is not for the walk */
+  const uint32_t sep = (sh.line[lo + 1u] & 0xFFFFu) - 1u;
+  uint32_t p = close + 1u;
+  while (p < sep && item_blank(win[p])) ++p;
+  if (!ok || win[p] == ':') atomicOr(&sh.oddline[lo >> 5], 1u << (lo & 31u));
+}
+/* All of them: off the list, one per thread, while it holds them; text where more of the strings are of this kind (another script, \/
+ * for every slash) fills the lanes without one: a warp then takes 32 strings that follow each other. */
+__device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh, uint8_t* win, const uint32_t* pairs, uint32_t tid) {
+  if (sh.nspecial <= IT_MAX_SPECIAL) {
+    for (uint32_t i = tid; i < sh.nspecial; i += IT_THREADS) item_special(a, sh, win, pairs, sh.special_list[i]);
+    return;
   }
+  for (uint32_t k = tid; k < sh.nstr; k += IT_THREADS) if ((sh.special[k >> 5] >> (k & 31u)) & 1u) item_special(a, sh, win, pairs, k);
 }
 
 __device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
@@ -1893,7 +1899,6 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
   const uint32_t lane = tid & 31, warp = tid >> 5;
   const uint32_t nline = sh.nline, nchunk = (nline + 31u) >> 5;
   if (sh.nspecial) {
-    if (sh.nspecial > IT_MAX_SPECIAL) return false;
     item_specials(a, sh, win, pairs, tid);
     __syncthreads();
   }

@@ -184,6 +184,19 @@ def test_tile_shape_fits_shared_memory(emu, schema):
                         assert blocks == 3, where
 
 
+@pytest.mark.parametrize("part", [1, 2, 6])
+def test_tiles_full_of_strings_beyond_ascii(emu, oracle, part):
+    """Names in another script, slashes written as \\/: however many strings of a tile take a closer look, no record is left to the exact parser."""
+    words = ["\u0438\u043c\u044f", "\u540d\u524d", "a\\/b\\/c", "\\u00e9t\\u00e9", "na\u00efve", "\\n"]
+    keys = ["username", "firstName", "lastName", "email", "password", "phone"]
+    lines = ['{"id":%d,%s,"userStatus":1}' % (i, ",".join('"%s":"%s%d"' % (k, words[(i + j) % 6] if j < part else "x", i) for j, k in enumerate(keys))) for i in range(400)]
+    body = as_u8("\n".join(lines) + "\n")
+    want = oracle.parse(USER, body)
+    for tile in (32768, 16384):
+        got = Run(emu, USER, body, tile=tile)
+        assert same_result(want, got.cols) == "" and got.fast == want.n_records == 400
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
