@@ -22,9 +22,10 @@
  * The steps detect every deviation from a valid record of the model; the common failures (wrong JSON type, unknown
  * literal, bad date-time, missing property, record ending inside a string) are reported with the exact parser's kind
  * and offset, because the smallest offset of a record's deviations is its first failure. Any other deviation sends the
- * record to the exact parser (pj_core.cuh); should that one accept the record (unknown keys with nested values, repeated
- * keys, ...), or does the tile not fit the shared memory laid out for it (a record longer than the window, many more lines
- * or strings than its bytes suggest), the block walks the tile with the exact parser alone (item_slow_tile).
+ * record to the exact parser (pj_core.cuh); a record that one accepts (unknown keys with nested values, repeated keys, ...) stands apart:
+ * its counts take part in the sums, and it is parsed once more to write its columns (item_emit_apart). Does the tile not fit
+ * the shared memory laid out for it (a record longer than the window, many more lines or strings than its bytes suggest), the
+ * block walks the tile with the exact parser alone (item_slow_tile).
  */
 #ifndef PJ_ITEM_CUH
 #define PJ_ITEM_CUH
@@ -1181,10 +1182,10 @@ __device__ __forceinline__ uint32_t item_key(const ItemShared& sh, const uint8_t
   const uint32_t f = sh.field[s == IS_ROOT ? 0 : (s == IS_CHILD ? 1 : 2)][slot];
   return (((x0 ^ kt.x) & km.x) | ((x1 ^ kt.y) & km.y) | ((x2 ^ kt.z) & km.z) | ((x3 ^ kt.w) & km.w)) != 0 || len != ItField::len(f) ? 0u : f;
 }
-/* Lines [i0, i0 + n), each with a string, by a warp: together at most 32 strings, or one line with more. Returns false when
- * the tile has to take the other road. */
+/* Lines [i0, i0 + n), each with a string, by a warp: together at most 32 strings, or one line with more. What does not fit its words (a
+ * string of 32 KB, more list elements than there is room for) leaves them to the exact parser. */
 template <int SCHEMA, bool ARR>
-__device__ __noinline__ bool item_pack(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t i0, uint32_t n) {
+__device__ __noinline__ void item_pack(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, uint32_t* pairs, uint32_t* rows, uint32_t i0, uint32_t n) {
   constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
   constexpr uint32_t LW = ItWords<OBJ_PET>::n; /* the word of the list of objects, then that of the bytes */
   constexpr int E = OBJ_TAG, ES = it_string_field<E>();
@@ -1402,13 +1403,22 @@ __device__ __noinline__ bool item_pack(const ItemArgs& a, const StreamGeom& g, I
     nT += (uint32_t)__popc(NE);
     st = NI ? __shfl_sync(0xFFFFFFFFu, out, 31 - __clz((int)NI)) : st;
     pk = (PK >> 31) & 1u;
-    if (__any_sync(0xFFFFFFFFu, slow)) return false;
+    if (__any_sync(0xFFFFFFFFu, slow)) {
+      __syncwarp(); /* every lane is through with the rows */
+      if (lane < n) {
+        uint32_t* row = rows + (i0 + lane) * STRIDE;
+        const uint32_t at = sh.line[i0 + lane] & 0xFFFFu;
+        row[IW_FLAGS] = IF_RECORD; row[IW_ERR] = (at << 8) | IE_REFUSED;
+        if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[LW] = 0; row[LW + 1u] = 0; }
+      }
+      __syncwarp();
+      return;
+    }
   }
   if constexpr (ItemSlots<SCHEMA>::lists) {
     if (single && lane == 0) { uint32_t* row = rows + i0 * STRIDE; row[IW_LIST] |= nP << 16; row[LW] |= nT << 16; }
   }
   __syncwarp();
-  return true;
 }
 /* The lines the walk did not recognise: each by a warp when they are few, otherwise runs of them, several to a step. */
 template <int SCHEMA, bool ARR>
@@ -1440,7 +1450,7 @@ __device__ __forceinline__ void item_packs(const ItemArgs& a, const StreamGeom& 
       if (!((sh.oddmask[i >> 5] >> (i & 31u)) & 1u)) { ++i; continue; }
       uint32_t n = 1;
       while (i + n < end && ((sh.oddmask[(i + n) >> 5] >> ((i + n) & 31u)) & 1u) && (sh.line[i + n + 1u] >> 16) - k0 <= 32u && sh.line[i + n + 1u] >> 16 != sh.line[i + n] >> 16) ++n;
-      if (!item_pack<SCHEMA, ARR>(a, g, sh, win, pairs, rows, i, n)) { sh.slow = 1; return; }
+      item_pack<SCHEMA, ARR>(a, g, sh, win, pairs, rows, i, n);
       i += n;
     }
   }
@@ -1685,9 +1695,24 @@ struct ItemOut {
   uint8_t* owner;
   const uint32_t* moved;
   uint32_t flags, chunk;
+  uint32_t apart; /* lanes of this model whose record stands apart */
   bool has_row;
   uint64_t at; /* row of the model's table */
 };
+/* first counter of a model; its row of a record that stands apart holds them in order */
+template <int OBJ> struct ItSlot0 { static constexpr uint32_t n = OBJ == OBJ_USER ? (uint32_t)SLOT_USR_STR0 : (uint32_t)SLOT_PET_CAT_NAME; };
+static constexpr uint32_t IT_APART = 6; /* counters of a model */
+static_assert((uint32_t)SLOT_USR_STR0 - (uint32_t)SLOT_PET_CAT_NAME == IT_APART && NSLOT - (uint32_t)SLOT_USR_STR0 == IT_APART, "as many for Pets as for Users");
+static_assert(ItWords<OBJ_PET>::n >= IW_FIELDS + IT_APART && ItStride<PJ_SCHEMA_USER>::n >= IW_FIELDS + IT_APART, "room for them");
+/* Lanes side by side, without those apart, one run of them after the other: f(first lane, behind the last one). Nearly always one. */
+template <class F>
+__device__ __forceinline__ void item_each_run(uint32_t apart, F f) {
+  for (uint32_t lo = 0; lo < 32;) {
+    const uint32_t rest = apart >> lo, end = rest ? lo + (uint32_t)__ffs((int)rest) - 1u : 32u;
+    if (end > lo) f(lo, end);
+    lo = end + 1u;
+  }
+}
 /* fixed-width columns of root or embedded object OBJ */
 template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
 __device__ __forceinline__ void item_emit_fixed(const ItemArgs& a, const ItemOut& o) {
@@ -1709,19 +1734,23 @@ __device__ __forceinline__ void item_emit_fixed(const ItemArgs& a, const ItemOut
   }
 }
 /* string columns of root or embedded object OBJ (every lane of the warp calls this) */
-template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
+template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
 __device__ __forceinline__ void item_emit_strings(const ItemArgs& a, const ItemShared& sh, const ItemOut& o) {
   if constexpr (I < CObj<OBJ>::N) {
     constexpr uint32_t kind = CObj<OBJ>::f[I].kind, col = CObj<OBJ>::f[I].col, slot = CObj<OBJ>::f[I].cnt;
     constexpr uint32_t word = ROOT ? it_root_word<OBJ>(I) : WORD0 + it_flat_word<OBJ>(I);
     if constexpr (kind == K_STR) {
       const bool pr = o.has_row && ((o.flags >> (IF_PRESENT + BIT0 + I)) & 1u);
-      const uint32_t ref = o.row[word], n = pr ? (ref >> 16) & 0x7FFFu : 0u;
-      const uint32_t at = sh.base[slot] + sh.csum[slot][o.chunk], inc = warp_incl_scan(n);
-      if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at + inc - n;
-      item_emit_run(o.stage, colp<uint8_t>(&a.cols, col + 1) + at, o.win, ref & 0xFFFFu, n, inc - n, __shfl_sync(0xFFFFFFFFu, inc, 31));
-    } else if constexpr (kind == K_OBJ) item_emit_strings<CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
-    item_emit_strings<OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
+      const uint32_t lane = threadIdx.x & 31u, mine = (o.apart >> lane) & 1u;
+      const uint32_t ref = o.row[word], n = pr ? (ref >> 16) & 0x7FFFu : 0u, all = mine ? o.row[IW_FIELDS + slot - ItSlot0<MODEL>::n] : n;
+      const uint32_t at = sh.base[slot] + sh.csum[slot][o.chunk], inc = warp_incl_scan(all);
+      if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at + inc - all;
+      item_each_run(o.apart, [&](uint32_t lo, uint32_t end) {
+        const uint32_t from = __shfl_sync(0xFFFFFFFFu, inc - all, (int)lo), to = __shfl_sync(0xFFFFFFFFu, inc, (int)end - 1);
+        item_emit_run(o.stage, colp<uint8_t>(&a.cols, col + 1) + at + from, o.win, ref & 0xFFFFu, lane >= lo && lane < end ? n : 0u, inc - all - from, to - from);
+      });
+    } else if constexpr (kind == K_OBJ) item_emit_strings<MODEL, CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
+    item_emit_strings<MODEL, OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
   }
 }
 /* bytes of the lines' strings per slot, added up over the warp into csum[slot][chunk] */
@@ -1748,44 +1777,110 @@ __device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemSha
   constexpr uint32_t off_col = OBJS ? CObj<E>::f[1].col : col + 1u;
   const uint32_t l = mine ? o.row[OBJS ? ItWords<OBJ_PET>::n : (uint32_t)IW_LIST] : 0u, n = l >> 16;
   const uint64_t r0 = (uint64_t)sh.base[slot] + sh.csum[slot][o.chunk];
-  const uint32_t inc = warp_incl_scan(n);
-  if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = (uint32_t)r0 + inc - n;
-  uint32_t at = sh.base[bslot] + sh.csum[bslot][o.chunk], done = 0;
   const uint32_t lane = threadIdx.x & 31u;
-  item_each_element(o.owner, n, [&](uint32_t src, uint32_t j, bool has) {
-    const uint32_t k = __shfl_sync(0xFFFFFFFFu, l, (int)src) & 0xFFFFu;
-    const uint64_t r = r0 + done + lane;
-    uint32_t pos = 0, len = 0;
-    if constexpr (OBJS) {
-      if (has) {
-        const uint32_t* e = pairs + k + 3u * j;
-        const uint32_t x = e[2];
-        colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((x >> 28) & 3u);
-        colp<int64_t>(&a.cols, CObj<E>::f[0].col)[r] = (x >> 28) & 1u ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
-        pos = x & 0xFFFFu; len = (x >> 29) & 1u ? (x >> 16) & 0xFFFu : 0u;
-      }
-    } else if (has) { const uint32_t pr = pairs[k + j]; pos = (pr & 0xFFFFu) + 1u; len = (pr >> 16) - pos - item_freed(o.win, o.moved, k + j, pr >> 16); }
-    const uint32_t sc = warp_incl_scan(len), total = __shfl_sync(0xFFFFFFFFu, sc, 31);
-    if (has) colp<uint32_t>(&a.cols, off_col)[r] = at + sc - len;
-    item_emit_run(o.stage, colp<uint8_t>(&a.cols, off_col + 1u) + at, o.win, pos, len, sc - len, total);
-    at += total; done += 32;
+  const bool apart = (o.apart >> lane) & 1u;
+  const uint32_t all = apart ? o.row[IW_FIELDS + slot - ItSlot0<OBJ_PET>::n] : n, inc = warp_incl_scan(all);
+  if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = (uint32_t)r0 + inc - all;
+  const uint32_t at0 = sh.base[bslot] + sh.csum[bslot][o.chunk];
+  uint32_t bytes = 0; /* of the lists of the lanes before: needed from the second run on */
+  if (o.apart) {
+    const uint32_t w = mine ? o.row[ItWords<OBJ_PET>::n + 1u] : 0u, own = apart ? o.row[IW_FIELDS + bslot - ItSlot0<OBJ_PET>::n] : (OBJS ? w >> 16 : w & 0xFFFFu);
+    bytes = warp_incl_scan(own) - own;
+  }
+  item_each_run(o.apart, [&](uint32_t lo, uint32_t end) {
+    uint32_t at = at0 + __shfl_sync(0xFFFFFFFFu, bytes, (int)lo), done = __shfl_sync(0xFFFFFFFFu, inc - all, (int)lo);
+    item_each_element(o.owner, lane >= lo && lane < end ? n : 0u, [&](uint32_t src, uint32_t j, bool has) {
+      const uint32_t k = __shfl_sync(0xFFFFFFFFu, l, (int)src) & 0xFFFFu;
+      const uint64_t r = r0 + done + lane;
+      uint32_t pos = 0, len = 0;
+      if constexpr (OBJS) {
+        if (has) {
+          const uint32_t* e = pairs + k + 3u * j;
+          const uint32_t x = e[2];
+          colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((x >> 28) & 3u);
+          colp<int64_t>(&a.cols, CObj<E>::f[0].col)[r] = (x >> 28) & 1u ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
+          pos = x & 0xFFFFu; len = (x >> 29) & 1u ? (x >> 16) & 0xFFFu : 0u;
+        }
+      } else if (has) { const uint32_t pr = pairs[k + j]; pos = (pr & 0xFFFFu) + 1u; len = (pr >> 16) - pos - item_freed(o.win, o.moved, k + j, pr >> 16); }
+      const uint32_t sc = warp_incl_scan(len), total = __shfl_sync(0xFFFFFFFFu, sc, 31);
+      if (has) colp<uint32_t>(&a.cols, off_col)[r] = at + sc - len;
+      item_emit_run(o.stage, colp<uint8_t>(&a.cols, off_col + 1u) + at, o.win, pos, len, sc - len, total);
+      at += total; done += 32;
+    });
   });
 }
 
 /* ---- the exact parser -------------------------------------------------------------------------------------------- */
 
-/* A record the fast steps refused, from its first byte at input offset s up to `limit`: kind and offset of its failure in *err,
- * *off, or *err = 0 when it is a valid one after all. */
-template <int SCHEMA>
-__device__ __noinline__ void item_exact(const ItemArgs& a, const uint8_t* in, uint64_t s0, uint64_t limit, uint32_t* err, uint32_t* off) {
+__device__ __forceinline__ Rd item_reader(const ItemArgs& a, const uint8_t* in, uint64_t limit) {
   Rd rd;
   rd.in = in; rd.lf_ws = a.sep ? 1u : 0u; rd.open_end = (a.is_last || a.sep) ? 0u : 1u; rd.limit = limit; rd.opts = a.opts; rd.rec_end = limit;
+  return rd;
+}
+/* A record the fast steps refused, from its first byte at input offset s up to `limit`: kind and offset of its failure in *err,
+ * *off. *err = 0: it is a valid one after all, of the model returned, and its row holds what it adds to that model's counters. */
+template <int SCHEMA>
+__device__ __noinline__ uint32_t item_exact(const ItemArgs& a, const uint8_t* in, uint64_t s0, uint64_t limit, uint32_t* err, uint32_t* off, uint32_t* row) {
+  const Rd rd = item_reader(a, in, limit);
   PS s;
   s.p = s0; s.err = 0; s.err_pos = 0;
   Out<false> so;
   so.cols = &a.cols;
-  parse_record<false>(c_schema, rd, s, (uint32_t)SCHEMA, so, 0);
+  const uint32_t type = parse_record<false>(c_schema, rd, s, (uint32_t)SCHEMA, so, 0);
   *err = s.err; *off = (uint32_t)(s.err_pos - s0);
+  if (s.err) return PJ_TYPE_NONE;
+  const uint32_t slot0 = type == PJ_TYPE_USER ? ItSlot0<OBJ_USER>::n : ItSlot0<OBJ_PET>::n;
+  if (type != PJ_TYPE_ORDER) for (uint32_t j = 0; j < IT_APART; ++j) row[IW_FIELDS + j] = so.cnt[slot0 + j];
+  if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[ItWords<OBJ_PET>::n] = 0; row[ItWords<OBJ_PET>::n + 1u] = 0; }
+  return type;
+}
+/* what a record that does not stand apart adds to its model's counters */
+template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
+__device__ __forceinline__ void item_counts(const uint32_t* row, uint32_t flags, uint32_t* cnt) {
+  if constexpr (I < CObj<OBJ>::N) {
+    constexpr uint32_t kind = CObj<OBJ>::f[I].kind, at = CObj<OBJ>::f[I].cnt - ItSlot0<MODEL>::n;
+    constexpr uint32_t word = ROOT ? it_root_word<OBJ>(I) : WORD0 + it_flat_word<OBJ>(I), LW = ItWords<OBJ_PET>::n;
+    if constexpr (kind == K_STR) cnt[at] = (flags >> (IF_PRESENT + BIT0 + I)) & 1u ? (row[word] >> 16) & 0x7FFFu : 0u;
+    else if constexpr (kind == K_OBJ) item_counts<MODEL, CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(row, flags, cnt);
+    else if constexpr (kind == K_LIST_STR) { cnt[at] = row[IW_LIST] >> 16; cnt[at + 1u] = row[LW + 1u] & 0xFFFFu; }
+    else if constexpr (kind == K_LIST_OBJ) {
+      constexpr int E = CObj<OBJ>::f[I].child;
+      cnt[at] = row[LW] >> 16; cnt[CObj<E>::f[it_string_field<E>()].cnt - ItSlot0<MODEL>::n] = row[LW + 1u] >> 16;
+    }
+    item_counts<MODEL, OBJ, ROOT, WORD0, BIT0, I + 1>(row, flags, cnt);
+  }
+}
+/* The columns of the records among 32 lines that stand apart (every lane of the warp calls this): by the exact parser once more, at the
+ * place the records of their model before them leave. n: the lane's record, at: its row in its model's table. */
+template <int SCHEMA>
+__device__ __noinline__ void item_emit_apart(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, const uint32_t* row, uint32_t flags, uint32_t type, uint32_t ln, uint32_t c, uint64_t n, uint64_t at) {
+  const bool apart = (flags & IF_APART) != 0;
+  Out<true> o;
+  o.cols = &a.cols;
+#pragma unroll 1
+  for (uint32_t k = 0; k < NSLOT; ++k) { o.base[k] = (uint32_t)at; o.room[k] = 1; o.cnt[k] = 0; } /* (counters of rows) */
+  auto model = [&](auto obj) {
+    constexpr int OBJ = decltype(obj)::value;
+    const bool mine = type == (OBJ == OBJ_PET ? (uint32_t)PJ_TYPE_PET : (uint32_t)PJ_TYPE_USER);
+    uint32_t cnt[IT_APART];
+#pragma unroll
+    for (uint32_t j = 0; j < IT_APART; ++j) cnt[j] = 0;
+    if (mine && apart) for (uint32_t j = 0; j < IT_APART; ++j) cnt[j] = row[IW_FIELDS + j];
+    else if (mine) item_counts<OBJ, OBJ, true, 0u, 0u>(row, flags, cnt);
+#pragma unroll
+    for (uint32_t j = 0; j < IT_APART; ++j) {
+      const uint32_t slot = ItSlot0<OBJ>::n + j, before = warp_incl_scan(cnt[j]) - cnt[j];
+      o.base[slot] = sh.base[slot] + sh.csum[slot][c] + before; o.room[slot] = cnt[j];
+    }
+  };
+  if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_PET>());
+  if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_USER>());
+  if (apart) {
+    const uint64_t v = g.v0 - g.mis;
+    PS s;
+    s.p = v + (row[IW_POS] & 0xFFFFu); s.err = 0; s.err_pos = 0;
+    parse_record<true>(c_schema, item_reader(a, a.in, a.sep ? v + ((sh.line[ln + 1u] & 0xFFFFu) - 1u) : a.limit), s, (uint32_t)SCHEMA, o, n);
+  }
 }
 
 /* The lines whose preceding separator lies in [lo, hi) of the input, one after the other (head: and before them the one at
@@ -1825,8 +1920,7 @@ __device__ __noinline__ void item_slow_tile(const ItemArgs& a, const StreamGeom&
   for (int pass = 0; pass < 2; ++pass) {
     if (head || lo < hi)
       item_each_line(a, lo, hi, head, [&](uint64_t s0, uint64_t limit, bool blank) {
-        Rd rd;
-        rd.in = a.in; rd.lf_ws = a.sep ? 1u : 0u; rd.open_end = (a.is_last || a.sep) ? 0u : 1u; rd.limit = limit; rd.opts = a.opts; rd.rec_end = limit;
+        const Rd rd = item_reader(a, a.in, limit);
         PS s;
         s.p = s0; s.err = 0; s.err_pos = 0;
         Out<false> so;
@@ -1922,7 +2016,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
 #pragma unroll
       for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
       if (nodd) item_packs<SCHEMA, ARR>(a, g, sh, win, pairs, rows, nodd);
-      if (__syncthreads_or((int)sh.slow)) return false;
+      __syncthreads();
     }
   }
 
@@ -1957,7 +2051,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         if (((flags >> IF_PRESENT) & req) != req) e = ((row[IW_POS] >> 16) << 8) | (uint32_t)PJ_E_REQUIRED;
       }
     }
-    const bool good = rec && e == IE_NONE;
+    bool good = rec && e == IE_NONE;
     if (rec && !good) {
       uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
       if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
@@ -1965,10 +2059,10 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         const uint32_t at = row[IW_POS] & 0xFFFFu, sep = (sh.line[tid + 1u] & 0xFFFFu) - 1u;
         const uint64_t s0 = g.v0 + at - g.mis;
         const bool here = sep < g.hi_valid && !((sh.movedline[warp] >> lane) & 1u);
-        item_exact<SCHEMA>(a, here ? win : a.in, here ? at : s0, ARR ? (here ? sep : g.v0 + sep - g.mis) : (here ? sep + 1u : a.limit), &kind, &off);
-        if (!kind) sh.slow = 1; /* a valid record of a kind the other steps do not know */
+        type = item_exact<SCHEMA>(a, here ? win : a.in, here ? at : s0, ARR ? (here ? sep : g.v0 + sep - g.mis) : (here ? sep + 1u : a.limit), &kind, &off, row);
+        good = !kind; /* a valid record of a kind the other steps do not know */
       }
-      flags = IF_BAD | IF_RECORD | off;
+      flags = good ? IF_APART | IF_RECORD | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD | off;
       row[IW_FLAGS] = flags; row[IW_ERR] = kind;
     }
     if (!good) type = PJ_TYPE_NONE;
@@ -2000,8 +2094,19 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
       if (lane == 0) { sh.csum[PCNT][warp] = n0; sh.csum[TCNT][warp] = n1; sh.csum[PCNT + 1u][warp] = b0; sh.csum[TBYTES][warp] = b1; }
     }
     if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) item_sum_strings<OBJ_USER, true, 0u, 0u>(sh, row, type == PJ_TYPE_USER, flags, warp, lane);
+    if (__any_sync(0xFFFFFFFFu, tid < nline && !(flags & IF_BAD) && (flags & IF_APART))) { /* (an IF_BAD row's other bits are an offset) */
+      const bool apart = tid < nline && !(flags & IF_BAD) && (flags & IF_APART);
+#pragma unroll 1
+      for (uint32_t j = 0; j < 2u * IT_APART; ++j) {
+        const uint32_t slot = (uint32_t)SLOT_PET_CAT_NAME + j;
+        const bool pet = j < IT_APART;
+        if (!((SL::mask >> slot) & 1u)) continue;
+        const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, apart && type == (pet ? (uint32_t)PJ_TYPE_PET : (uint32_t)PJ_TYPE_USER) ? row[IW_FIELDS + (pet ? j : j - IT_APART)] : 0u);
+        if (lane == 0) sh.csum[slot][warp] += s;
+      }
+    }
   }
-  if (__syncthreads_or((int)sh.slow)) return false;
+  __syncthreads();
   ck[3] = clock64();
 
   /* ---- where everything of the tile goes ---- */
@@ -2039,7 +2144,9 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     const uint32_t lt = (1u << lane) - 1u;
     const uint64_t n = (uint64_t)sh.base[IT_REC] + sh.csum[IT_REC][ln >> 5] + (uint32_t)__popc(sh.recs[ln >> 5] & ((1u << (ln & 31u)) - 1u));
     const uint32_t type = good ? item_type<SCHEMA>(f) : (uint32_t)PJ_TYPE_NONE;
-    o.flags = good ? f : 0u;
+    o.flags = good && !(f & IF_APART) ? f : 0u;
+    const bool apart = good && (f & IF_APART);
+    o.apart = __ballot_sync(0xFFFFFFFFu, apart);
     o.at = n;
     uint32_t bp = 0, bo = 0, bu = 0;
     if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
@@ -2052,35 +2159,42 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
       const uint32_t bg = __ballot_sync(0xFFFFFFFFu, good), br = __ballot_sync(0xFFFFFFFFu, rec);
       if (lane == 0) {
         if (br != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(br & ~bg));
-        if (bg) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg));
+        if (bg & ~o.apart) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg & ~o.apart));
       }
+      if (o.apart) item_emit_apart<SCHEMA>(a, g, sh, r, f & ~(good ? 0u : IF_APART), type, ln, c, n, o.at);
       if (rec) {
         colp<uint64_t>(&a.cols, PJ_COL_REC_START)[n] = a.goff + g.v0 + (r[IW_POS] & 0xFFFFu) - g.mis;
         colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[n] = good ? 0 : (uint8_t)r[IW_ERR];
         colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[n] = good ? 0u : f & ~(IF_BAD | IF_RECORD);
+        if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+          colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[n] = (uint8_t)type;
+          colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[n] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : (uint32_t)o.at;
+        }
+      }
+      if (rec && !apart) {
         if constexpr (SCHEMA == PJ_SCHEMA_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
         else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
         else if constexpr (SCHEMA == PJ_SCHEMA_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
         else {
-          colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[n] = (uint8_t)type;
-          colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[n] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : (uint32_t)o.at;
           if (type == PJ_TYPE_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
           else if (type == PJ_TYPE_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
           else if (type == PJ_TYPE_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
         }
       }
     } else if (what == 2u) {
-      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings<OBJ_PET, true, 0u, 0u>(a, sh, o); }
-      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings<OBJ_USER, true, 0u, 0u>(a, sh, o); }
+      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings<OBJ_PET, OBJ_PET, true, 0u, 0u>(a, sh, o); }
+      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings<OBJ_USER, OBJ_USER, true, 0u, 0u>(a, sh, o); }
       else if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
-        o.has_row = type == PJ_TYPE_PET;
-        if (bp) item_emit_strings<OBJ_PET, true, 0u, 0u>(a, sh, o);
-        o.has_row = type == PJ_TYPE_USER;
-        if (bu) item_emit_strings<OBJ_USER, true, 0u, 0u>(a, sh, o);
+        const uint32_t apart_all = o.apart;
+        o.has_row = type == PJ_TYPE_PET; o.apart = apart_all & bp;
+        if (bp) item_emit_strings<OBJ_PET, OBJ_PET, true, 0u, 0u>(a, sh, o);
+        o.has_row = type == PJ_TYPE_USER; o.apart = apart_all & bu;
+        if (bu) item_emit_strings<OBJ_USER, OBJ_USER, true, 0u, 0u>(a, sh, o);
       }
     } else if constexpr (SL::lists) {
       const bool pet = type == PJ_TYPE_PET;
       o.has_row = SCHEMA == PJ_SCHEMA_PET ? rec : pet;
+      if constexpr (SCHEMA == PJ_SCHEMA_MIXED) o.apart &= bp;
       if (SCHEMA == PJ_SCHEMA_PET || bp) { if (what == 0u) item_emit_lists<false>(a, sh, o, pairs, pet); else item_emit_lists<true>(a, sh, o, pairs, pet); }
     }
   }

@@ -197,6 +197,38 @@ def test_tiles_full_of_strings_beyond_ascii(emu, oracle, part):
         assert same_result(want, got.cols) == "" and got.fast == want.n_records == 400
 
 
+UNUSUAL = [b'"price":1.5,', b'"x":{"a":[1,{"b":"c"}],"d":"e"},', b'"x":["y",{"z":[]}],', b'"id":3,', b'"x":1e3,']  # valid, and only the exact parser knows them
+
+
+@pytest.mark.parametrize("schema", [PET, ORDER, USER, MIXED])
+@pytest.mark.parametrize("every", [1, 2, 7, 31, 90])
+def test_unusual_records_stand_apart(emu, oracle, schema, every):
+    """A valid record that only the exact parser knows is written by it alone, between the columns of its neighbours, whatever else its lines hold."""
+    for flags in (0, ALL, abi.PJ_GEN_ZIPF_LISTS | abi.PJ_GEN_ESCAPES):
+        lines = bytes(pj.gen_text(schema, every + flags, 0, 300 if not flags & abi.PJ_GEN_ZIPF_LISTS else 60, flags)).split(b"\n")[:-1]
+        out = [ln[:1 + ln.index(b"{")] + UNUSUAL[(i // every) % len(UNUSUAL)] + ln[1 + ln.index(b"{"):] if i % every == every - 1 and b'":' in ln else ln for i, ln in enumerate(lines)]
+        for framing, body in ((NDJSON, b"\n".join(out) + b"\n"), (ARRAY, b"[" + b",".join(out) + b"]")):
+            body = as_u8(body)
+            want = oracle.parse(schema, body, framing)
+            for kw in (dict(), dict(tile=4096, mis=3, order=5)):
+                got = Run(emu, schema, body, framing, **kw)
+                assert same_result(want, got.cols) == "", (flags, framing, kw)
+                if flags == 0 and framing == NDJSON:
+                    assert got.fast >= want.n_records - want.n_errors - len(out) // every
+
+
+def test_strings_too_long_for_a_reference_stand_apart(emu, oracle):
+    long = '{"id":1,"username":"%s","phone":"5"}' % ("y" * 33000)
+    users = ['{"id":%d,"username":"u%d"}' % (i, i) for i in range(60)]
+    body = as_u8("\n".join(users[:30] + [long] + users[30:]) + "\n")
+    got = Run(emu, USER, body, tile=16384, slack=45000)
+    assert same_result(oracle.parse(USER, body), got.cols) == "" and got.fast >= 59
+    pet = '{"id":1,"name":"n","photoUrls":["a"],"tags":[{"name":"%s"},{"id":2,"name":"t"}]}'
+    body = as_u8("\n".join(pet % ("t" * (5000 if i == 20 else 5)) for i in range(40)) + "\n")
+    got = Run(emu, PET, body, tile=16384, slack=8000)
+    assert same_result(oracle.parse(PET, body), got.cols) == "" and got.fast >= 36  # (four lines are looked at together)
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
