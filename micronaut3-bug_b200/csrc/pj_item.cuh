@@ -1033,11 +1033,18 @@ __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGe
   ItemLists l;
   l.k_str = l.n_str = l.k_obj = l.n_obj = l.bytes = 0;
   const bool cut = f.sep >= g.hi_valid && !a.is_last; /* the readable bytes end here, the stream does not */
-  if (f.k == f.kend) { /* no string */
+  /* array framing: what the separator before the line is. Nothing follows `]`; documents of several arrays are in error at the second one. */
+  const uint32_t before = ARR ? win[start - 1u] : 0u;
+  if (ARR && before == '[') {
+    const uint64_t at = g.v0 + start - 1u - g.mis;
+    if (at > a.res->first_opener) atomicMin(&a.res->doc_err_off, (unsigned long long)at);
+  }
+  if (ARR && before == ']') f.p = start;
+  else if (f.k == f.kend) { /* no string */
     uint32_t p = start;
     while (p < f.sep && item_blank(win[p])) ++p;
     if (p < f.sep || cut) { flags = IF_RECORD; err = (start << 8) | IE_REFUSED; } /* for the exact parser */
-    else if (ARR && !(i + 1u == sh.nline && f.sep >= g.hi_valid)) sh.slow = 1; /* an extent without a value (what follows the closing bracket is none) */
+    else if (ARR && f.sep < g.hi_valid && !(before == '[' && win[f.sep] == ']')) { flags = IF_RECORD; err = (f.sep << 8) | (uint32_t)PJ_E_SYNTAX; } /* an extent without a value */
     f.p = start;
   } else {
     const uint32_t n = f.kend - f.k, bit = 1u << (i & 31u);
@@ -2257,9 +2264,8 @@ __global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __g
   ck[1] = clock64();
 
   bool done = false;
-  if (a.sep) { /* a document that is not one clean array is left to the other road */
-    if (a.res->doc_err_off == ~0ull && a.res->n_openers == 1u && !a.res->arr_final_s && a.res->arr_final_d == 0) done = item_try<SCHEMA, true>(a, g, sh, win, strs, rows, tile, tid, ck);
-  } else done = item_try<SCHEMA, false>(a, g, sh, win, strs, rows, tile, tid, ck);
+  if (a.sep) done = item_try<SCHEMA, true>(a, g, sh, win, strs, rows, tile, tid, ck);
+  else done = item_try<SCHEMA, false>(a, g, sh, win, strs, rows, tile, tid, ck);
   if (!done) {
     __syncthreads();
     item_slow_tile<SCHEMA>(a, g, sh, tile, tid);

@@ -229,6 +229,28 @@ def test_strings_too_long_for_a_reference_stand_apart(emu, oracle):
     assert same_result(oracle.parse(PET, body), got.cols) == "" and got.fast >= 36  # (four lines are looked at together)
 
 
+def test_documents_that_are_not_one_array(emu, oracle):
+    """A text cut off in transfer, something behind the array, several arrays, extents without a value: the records are decoded as those of a
+    clean document."""
+    rng = random.Random(31)
+    for schema in (PET, USER, MIXED):
+        text = bytes(pj.gen_text(schema, 77, 0, 150, abi.PJ_GEN_ARRAY | abi.PJ_GEN_SPARSE))
+        recs = text[1:-1]
+        docs = [text[:cut] for cut in [1, 2, len(text) - 1] + [rng.randrange(len(text)) for _ in range(40)]]
+        docs += [text + t for t in (b"]", b"x", b" \n", b",", b"[]", b'"', b"[" + recs + b"]", b',"a"', b" null ", b"}")]
+        docs += [t + text for t in (b" ", b"x", b"[],", b"{}", b"]", b'"a"')]
+        docs += [b"[" + recs + t + b"]" for t in (b",", b",,", b", ,{}", b"}", b"]", b"},{")] + [b"[ ]", b"[", b"[,]", b"[,,]", b"", b" ", b"[{}] [{}]", b"[{}][ ]", b"{},{}"]
+        docs += [text.replace(b"},{\"id", b"}, \t,{\"id", 5), text.replace(b"},{\"id", b"}]],{\"id", 1), text.replace(b"},{\"id", b'}],"[",[{"id', 2)]
+        for doc in docs:
+            body = as_u8(doc)
+            want = oracle.parse(schema, body, ARRAY)
+            for kw in (dict(), dict(tile=2048, mis=9, order=2)):
+                got = Run(emu, schema, body, ARRAY, **kw)
+                assert same_result(want, got.cols) == "", (schema, doc[-60:], kw)
+                assert (want.raw.doc_err_kind, want.raw.doc_err_off) == (got.cols.raw.doc_err_kind, got.cols.raw.doc_err_off), (schema, doc[-60:])
+                assert got.fast >= (want.n_records - want.n_errors) - 2, (schema, doc[-60:], got.fast, want.n_records)
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
