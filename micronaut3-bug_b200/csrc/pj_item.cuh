@@ -1403,7 +1403,8 @@ __device__ __noinline__ void item_pack(const ItemArgs& a, const StreamGeom& g, I
           const uint32_t nm = SCHEMA == PJ_SCHEMA_MIXED && s == IS_ROOT ? (~ItField::models(f) & 7u) << IF_NOTMODEL : 0u;
           const uint32_t old = atomicOr(&row[IW_FLAGS], bit | nm | (keep ? bit << IF_PRESENT : 0u));
           if (old & bit) item_error(row, close, IE_REFUSED);
-          if (keep && kind <= K_DATETIME) row[word] = ref;
+          /* of a key given twice the first value is judged (a failure there comes before the repetition) */
+          if (keep && kind <= K_DATETIME && !(old & (bit << IF_PRESENT))) row[word] = ref;
         }
       }
     }

@@ -251,6 +251,19 @@ def test_documents_that_are_not_one_array(emu, oracle):
                 assert got.fast >= (want.n_records - want.n_errors) - 2, (schema, doc[-60:], got.fast, want.n_records)
 
 
+def test_the_first_value_of_a_repeated_key_is_judged(emu, oracle):
+    """A failure there comes before everything else of the record, also when the repetition itself is not the first failure."""
+    for first in ("1x2", "1.5", "null", "3", '"a"', "true", "[1]", "1" * 30, ""):
+        for between in ('"category":"c"', '"category":7', '"name":5', '"name":"n"', '"name":"n" "x"'):
+            for second in ("4", "null", "x", '"b"'):
+                for status in ("", ',"status":"gone","status":"sold"', ',"status":null,"status":"gone"'):
+                    line = '{"id":%s,%s,"id":%s%s,"name":"a","photoUrls":[]}' % (first, between, second, status)
+                    body = as_u8(line + "\n")
+                    want = oracle.parse(PET, body)
+                    for order in (0, 1):
+                        assert same_result(want, Run(emu, PET, body, tile=1024, order=order).cols) == "", line
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
