@@ -24,8 +24,8 @@
  * and offset, because the smallest offset of a record's deviations is its first failure. Any other deviation sends the
  * record to the exact parser (pj_core.cuh); a record that one accepts (unknown keys with nested values, repeated keys, ...) stands apart:
  * its counts take part in the sums, and it is parsed once more to write its columns (item_emit_apart). Does the tile not fit
- * the shared memory laid out for it (a record longer than the window, many more lines or strings than its bytes suggest), the
- * block walks the tile with the exact parser alone (item_slow_tile).
+ * the shared memory laid out for it (many more lines or strings than its bytes suggest), the block walks the tile with the
+ * exact parser alone (item_slow_tile). A record that runs out of the window is the exact parser's, where it lies.
  */
 #ifndef PJ_ITEM_CUH
 #define PJ_ITEM_CUH
@@ -142,6 +142,7 @@ struct ItemShared {
   uint32_t recs[IT_WARPS];                 /* lines that are records */
   uint32_t wsum[IT_WARPS], wmin[3][IT_WARPS];
   uint32_t nspecial, odd;                  /* odd: some record ends inside a string */
+  uint32_t open_end;                       /* the last line runs out of the window */
   uint32_t nstr, nline, stop;              /* strings, lines, last separator */
   uint32_t free_word;                      /* first free word behind the strings */
   uint32_t ndense;                         /* lines the dense walk took */
@@ -282,18 +283,19 @@ __device__ __forceinline__ uint32_t item_prefix_xor(uint32_t x) {
   x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8; x ^= x << 16;
   return x;
 }
-/* The strings and lines the tile owns. False (for every thread): the tile does not fit, the block has to take the other road. A record may end
+/* The strings and lines the tile owns. False (for every thread): the tile does not fit, the block has to take the other road. The last line may
+ * run out of the window. A record may end
  * inside a string: its separator then counts as the string's closing quote. */
 template <bool ARR>
 __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint8_t* win, uint32_t* strs, uint32_t tid, uint32_t tile) {
   const uint32_t lane = tid & 31, warp = tid >> 5;
-  bool started = !ARR && tile == 0 && a.is_first && a.limit > 0, done = false, fine = true;
+  bool started = !ARR && tile == 0 && a.is_first && a.limit > 0, done = false, fine = true, open_end = false;
   uint32_t start = g.mis, stop = 0, nq = 0, nline = 0;
   const int32_t end_valid = (int32_t)g.hi_valid + (g.to_limit ? 1 : 0), lo_valid = (int32_t)g.lo_valid; /* the end of the input counts as a separator */
   uint16_t* q16 = reinterpret_cast<uint16_t*>(strs);
   if (tid == 0 && started) sh.line[0] = start;
   for (uint32_t o = 0; !done; o += IT_STEP) {
-    if ((int32_t)o >= end_valid) { fine = !started; break; } /* the last record runs out of the window */
+    if ((int32_t)o >= end_valid) { open_end = started; break; } /* the last record runs out of the window */
     if (!started && o >= g.own_end) break;
     const int32_t p0 = (int32_t)(o + IT_SPAN * tid);
     /* quotes, separators, control characters (later: all that takes a closer look), a bit per byte of the thread's */
@@ -483,9 +485,14 @@ __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& 
       nq = n; nline = nl;
     }
   }
+  if (open_end && (nline >= IT_MAX_LINES || nline >= a.row_cap)) fine = false;
+  if (open_end) __syncthreads(); /* (the line's entry) */
   if (tid == 0) {
-    const bool any = fine && started && done;
-    sh.nstr = any ? nq >> 1 : 0u; sh.nline = any ? nline : 0u; sh.stop = stop;
+    const bool any = fine && started && (done || open_end);
+    /* a line that runs out of the window keeps none of its strings: it is a whole line up to the window's end for those who size lines, and
+       the exact parser's (item_walk_line) */
+    if (open_end) { nq = 2u * (sh.line[nline] >> 16); stop = g.hi_valid; if (any) sh.line[nline + 1u] = (stop + 1u) | ((nq >> 1) << 16); ++nline; }
+    sh.nstr = any ? nq >> 1 : 0u; sh.nline = any ? nline : 0u; sh.stop = stop; sh.open_end = open_end;
     sh.free_word = (any ? nq >> 1 : 0u) + 1u;
     if (any) strs[nq >> 1] = (stop + 1u) | ((stop + 1u) << 16);
   }
@@ -597,7 +604,10 @@ __device__ __forceinline__ void item_special(const ItemArgs& a, ItemShared& sh, 
  * for every slash) fills the lanes without one: a warp then takes 32 strings that follow each other. */
 __device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh, uint8_t* win, const uint32_t* pairs, uint32_t tid) {
   if (sh.nspecial <= IT_MAX_SPECIAL) {
-    for (uint32_t i = tid; i < sh.nspecial; i += IT_THREADS) item_special(a, sh, win, pairs, sh.special_list[i]);
+    for (uint32_t i = tid; i < sh.nspecial; i += IT_THREADS) {
+      const uint32_t k = sh.special_list[i];
+      if (k < sh.nstr) item_special(a, sh, win, pairs, k); /* (a line that runs out of the window has none) */
+    }
     return;
   }
   for (uint32_t k = tid; k < sh.nstr; k += IT_THREADS) if ((sh.special[k >> 5] >> (k & 31u)) & 1u) item_special(a, sh, win, pairs, k);
@@ -1039,8 +1049,17 @@ __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGe
     const uint64_t at = g.v0 + start - 1u - g.mis;
     if (at > a.res->first_opener) atomicMin(&a.res->doc_err_off, (unsigned long long)at);
   }
+  const bool long_line = sh.open_end && i + 1u == sh.nline;
   if (ARR && before == ']') f.p = start;
-  else if (f.k == f.kend) { /* no string */
+  else if (long_line) {
+    const uint64_t s0 = g.v0 + start - g.mis;
+    bool record;
+    if constexpr (ARR) {
+      const ExtentOut x = arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener);
+      record = x.is_record;
+    } else record = nd_is_record(a.in, s0, a.limit, (int)a.is_last);
+    if (record) { flags = IF_RECORD; err = (start << 8) | IE_REFUSED; }
+  } else if (f.k == f.kend) { /* no string */
     uint32_t p = start;
     while (p < f.sep && item_blank(win[p])) ++p;
     if (p < f.sep || cut) { flags = IF_RECORD; err = (start << 8) | IE_REFUSED; } /* for the exact parser */
@@ -1834,13 +1853,23 @@ __device__ __noinline__ uint32_t item_exact(const ItemArgs& a, const uint8_t* in
   s.p = s0; s.err = 0; s.err_pos = 0;
   Out<false> so;
   so.cols = &a.cols;
-  const uint32_t type = parse_record<false>(c_schema, rd, s, (uint32_t)SCHEMA, so, 0);
+  uint32_t type = PJ_TYPE_NONE;
+  uint64_t p = s0;
+  if (a.sep) while (p < limit && (item_blank(in[p]) || in[p] == '\n')) ++p;
+  if (p < limit || !a.sep) type = parse_record<false>(c_schema, rd, s, (uint32_t)SCHEMA, so, 0);
+  else fail(s, PJ_E_SYNTAX, limit); /* an extent without a value */
   *err = s.err; *off = (uint32_t)(s.err_pos - s0);
   if (s.err) return PJ_TYPE_NONE;
   const uint32_t slot0 = type == PJ_TYPE_USER ? ItSlot0<OBJ_USER>::n : ItSlot0<OBJ_PET>::n;
   if (type != PJ_TYPE_ORDER) for (uint32_t j = 0; j < IT_APART; ++j) row[IW_FIELDS + j] = so.cnt[slot0 + j];
   if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[ItWords<OBJ_PET>::n] = 0; row[ItWords<OBJ_PET>::n + 1u] = 0; }
   return type;
+}
+/* where line ln, whose first byte is at input offset s0, ends for the exact parser: NDJSON: it looks for the line feed itself */
+__device__ __forceinline__ uint64_t item_limit(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, uint32_t ln, uint64_t s0) {
+  if (!a.sep) return a.limit;
+  if (sh.open_end && ln + 1u == sh.nline) return arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener).end;
+  return g.v0 + ((sh.line[ln + 1u] & 0xFFFFu) - 1u) - g.mis;
 }
 /* what a record that does not stand apart adds to its model's counters */
 template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
@@ -1884,10 +1913,9 @@ __device__ __noinline__ void item_emit_apart(const ItemArgs& a, const StreamGeom
   if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_PET>());
   if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_USER>());
   if (apart) {
-    const uint64_t v = g.v0 - g.mis;
     PS s;
-    s.p = v + (row[IW_POS] & 0xFFFFu); s.err = 0; s.err_pos = 0;
-    parse_record<true>(c_schema, item_reader(a, a.in, a.sep ? v + ((sh.line[ln + 1u] & 0xFFFFu) - 1u) : a.limit), s, (uint32_t)SCHEMA, o, n);
+    s.p = g.v0 + (row[IW_POS] & 0xFFFFu) - g.mis; s.err = 0; s.err_pos = 0;
+    parse_record<true>(c_schema, item_reader(a, a.in, item_limit(a, g, sh, ln, s.p)), s, (uint32_t)SCHEMA, o, n);
   }
 }
 
@@ -2067,11 +2095,12 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         const uint32_t at = row[IW_POS] & 0xFFFFu, sep = (sh.line[tid + 1u] & 0xFFFFu) - 1u;
         const uint64_t s0 = g.v0 + at - g.mis;
         const bool here = sep < g.hi_valid && !((sh.movedline[warp] >> lane) & 1u);
-        type = item_exact<SCHEMA>(a, here ? win : a.in, here ? at : s0, ARR ? (here ? sep : g.v0 + sep - g.mis) : (here ? sep + 1u : a.limit), &kind, &off, row);
+        type = item_exact<SCHEMA>(a, here ? win : a.in, here ? at : s0, here ? (ARR ? sep : sep + 1u) : item_limit(a, g, sh, tid, s0), &kind, &off, row);
         good = !kind; /* a valid record of a kind the other steps do not know */
       }
-      flags = good ? IF_APART | IF_RECORD | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD | off;
+      flags = good ? IF_APART | IF_RECORD | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD;
       row[IW_FLAGS] = flags; row[IW_ERR] = kind;
+      if (!good) row[IW_LIST] = off;
     }
     if (!good) type = PJ_TYPE_NONE;
     const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, rec ? (sh.line[tid + 1u] & 0xFFFFu) - (row[IW_POS] & 0xFFFFu) : 0u);
@@ -2102,8 +2131,8 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
       if (lane == 0) { sh.csum[PCNT][warp] = n0; sh.csum[TCNT][warp] = n1; sh.csum[PCNT + 1u][warp] = b0; sh.csum[TBYTES][warp] = b1; }
     }
     if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) item_sum_strings<OBJ_USER, true, 0u, 0u>(sh, row, type == PJ_TYPE_USER, flags, warp, lane);
-    if (__any_sync(0xFFFFFFFFu, tid < nline && !(flags & IF_BAD) && (flags & IF_APART))) { /* (an IF_BAD row's other bits are an offset) */
-      const bool apart = tid < nline && !(flags & IF_BAD) && (flags & IF_APART);
+    const bool apart = tid < nline && (flags & IF_APART);
+    if (__any_sync(0xFFFFFFFFu, apart)) {
 #pragma unroll 1
       for (uint32_t j = 0; j < 2u * IT_APART; ++j) {
         const uint32_t slot = (uint32_t)SLOT_PET_CAT_NAME + j;
@@ -2169,11 +2198,11 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         if (br != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(br & ~bg));
         if (bg & ~o.apart) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg & ~o.apart));
       }
-      if (o.apart) item_emit_apart<SCHEMA>(a, g, sh, r, f & ~(good ? 0u : IF_APART), type, ln, c, n, o.at);
+      if (o.apart) item_emit_apart<SCHEMA>(a, g, sh, r, f, type, ln, c, n, o.at);
       if (rec) {
         colp<uint64_t>(&a.cols, PJ_COL_REC_START)[n] = a.goff + g.v0 + (r[IW_POS] & 0xFFFFu) - g.mis;
         colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[n] = good ? 0 : (uint8_t)r[IW_ERR];
-        colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[n] = good ? 0u : f & ~(IF_BAD | IF_RECORD);
+        colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[n] = good ? 0u : r[IW_LIST];
         if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
           colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[n] = (uint8_t)type;
           colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[n] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : (uint32_t)o.at;

@@ -34,7 +34,7 @@ enum { IW_FLAGS = 0, IW_ERR = 1, IW_POS = 2, IW_LIST = 3, IW_FIELDS = 4 };
 /* IW_FLAGS: bits 0-11 keys met, 12-23 values present, 24-26 models the record cannot be (mixed streams), 27: the text of a
  * string was decoded in place (positions in the window are not the input's any more), 28: the line is a record, 29: the walk
  * did not recognise it, 30: the list of objects has rows of its own (else it is read off its strings), 31: the record failed
- * (the rest then is the failure's offset). From the verdicts on bit 29 says that the record is a valid one of a kind only the exact
+ * (IW_LIST then is the failure's offset). From the verdicts on bit 29 says that the record is a valid one of a kind only the exact
  * parser knows: it stands apart, and its row holds, from IW_FIELDS on, what it adds to each of its model's counters. */
 static constexpr uint32_t IF_PRESENT = 12, IF_NOTMODEL = 24, IF_MOVED = 1u << 27, IF_RECORD = 1u << 28, IF_ODD = 1u << 29, IF_APART = IF_ODD, IF_ROWS = 1u << 30, IF_BAD = 1u << 31;
 static constexpr uint32_t IB_CHILD = 8;  /* first bit of the embedded object's properties */

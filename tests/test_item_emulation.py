@@ -264,6 +264,29 @@ def test_the_first_value_of_a_repeated_key_is_judged(emu, oracle):
                         assert same_result(want, Run(emu, PET, body, tile=1024, order=order).cols) == "", line
 
 
+@pytest.mark.parametrize("schema", [PET, USER, MIXED])
+def test_records_longer_than_the_window(emu, oracle, schema):
+    """They are the exact parser's, where they lie; the records beside them in their tile are not."""
+    rng = random.Random(schema)
+    pad = "".join('"%s",' % ("p%d" % i * 3 + ("\\n" if i % 9 == 0 else "") + ("\u00e9" if i % 11 == 0 else "")) for i in range(1500))
+    pet = '{"id":1,"name":"n","photoUrls":[%s"z"],"tags":[{"id":2,"name":"t"}]%s}'
+    user = '{"id":1,"username":"%s","phone":"5"%s}'
+    longs = [pet % (pad, e) if schema != USER else user % ("u" * 9000 + "\\n" * 1500, e) for e in ("", ',"status":"gone"', ',"x":[1.5]', ' } ', '', ',"id":')]
+    longs += [" " * 12000, " " * 9000 + "{}", '{"x":"' + "y" * 9000]
+    for n, where in ((40, "middle"), (3, "first"), (3, "last"), (0, "alone")):
+        for long in longs:
+            lines = bytes(pj.gen_text(schema, 5, 0, n, 0)).decode().split("\n")[:-1]
+            lines.insert({"middle": n // 2, "first": 0}.get(where, len(lines)), long)
+            for framing, text in ((NDJSON, "\n".join(lines) + rng.choice(["", "\n"])), (ARRAY, "[" + ",".join(lines) + "]")):
+                body = as_u8(text)
+                want = oracle.parse(schema, body, framing)
+                for kw in (dict(tile=4096, slack=1024, mis=3), dict(tile=1024, slack=4096, order=7), dict(tile=16384, slack=2048, mis=8, order=3)):
+                    got = Run(emu, schema, body, framing, **kw)
+                    assert same_result(want, got.cols) == "", (where, long[-40:], framing, kw)
+                    assert (want.raw.doc_err_kind, want.raw.doc_err_off) == (got.cols.raw.doc_err_kind, got.cols.raw.doc_err_off)
+                    assert got.fast >= want.n_records - want.n_errors - 1
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
