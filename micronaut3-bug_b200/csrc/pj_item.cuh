@@ -411,12 +411,11 @@ __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& 
         }
       }
     }
-    /* order of the quotes (low half) and separators (high half) */
+    /* order of the quotes (low half) and separators (high half); twice when some record ends inside a string */
     uint32_t at, total, any = 0;
-    bool careful = false;
 #pragma unroll
     for (uint32_t i = 0; i < IT_SPANW; ++i) any |= t[i];
-    for (;;) {
+    for (uint32_t round = 0;; ++round) {
       uint32_t n = 0;
 #pragma unroll
       for (uint32_t i = 0; i < IT_SPANW; ++i) n += (uint32_t)__popc(q[i]) + ((uint32_t)__popc(t[i]) << 16);
@@ -426,33 +425,40 @@ __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& 
       at = inc - n; total = 0;
 #pragma unroll
       for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t x = sh.wsum[k]; if (k < warp) at += x; total += x; }
-      uint32_t odd = IT_NONE; /* the first separator this thread sees with a string open */
+      if (round) break;
+      /* A record that ends inside a string has an odd number of quotes: it changes the parity from separator to separator. */
+      const uint32_t n0 = nq + (at & 0xFFFFu);
+      uint32_t last = 0, odd = 0; /* parity at the thread's last separator; at any of them */
       if (any) {
-        uint32_t n0 = nq + (at & 0xFFFFu);
+        uint32_t m0 = n0;
 #pragma unroll
         for (uint32_t i = 0; i < IT_SPANW; ++i) {
-          for (uint32_t m = t[i] & ~q[i]; m; m &= m - 1u) {
-            const uint32_t low = (m & (0u - m)) - 1u;
-            if (((n0 + (uint32_t)__popc(q[i] & low)) & 1u) && odd == IT_NONE) odd = (uint32_t)(p0 + 32 * (int32_t)i + __ffs((int)m) - 1);
-          }
-          n0 += (uint32_t)__popc(q[i]);
+          for (uint32_t m = t[i]; m; m &= m - 1u) { last = (m0 + (uint32_t)__popc(q[i] & ((m & (0u - m)) - 1u))) & 1u; odd |= last; }
+          m0 += (uint32_t)__popc(q[i]);
         }
       }
-      if (!careful) {
-        if (!__syncthreads_or(odd != IT_NONE)) break;
-        careful = true;
-        if (tid == 0) sh.odd = 1;
-      }
-      const uint32_t mine = __reduce_min_sync(0xFFFFFFFFu, odd);
-      if (lane == 0) sh.wmin[2][warp] = mine;
+      if (!__syncthreads_or((int)odd)) break;
+      if (tid == 0) sh.odd = 1;
+      const uint32_t has = __ballot_sync(0xFFFFFFFFu, any != 0), par = __ballot_sync(0xFFFFFFFFu, last != 0);
+      if (lane == 0) sh.wmin[2][warp] = has ? 2u | ((par >> (31 - __clz((int)has))) & 1u) : 0u;
       __syncthreads();
-      uint32_t first = IT_NONE;
+      uint32_t prev = 0; /* at the separator before the thread's first: even before the step's first one */
 #pragma unroll
-      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t y = sh.wmin[2][k]; first = y < first ? y : first; }
-      if (first == IT_NONE) break;
-      if (odd == first) { /* closed there */
+      for (uint32_t k = 0; k < IT_WARPS; ++k) { const uint32_t x = sh.wmin[2][k]; if (k < warp && x) prev = x & 1u; }
+      const uint32_t below = has & ((1u << lane) - 1u);
+      if (below) prev = (par >> (31 - __clz((int)below))) & 1u;
+      if (any) {
+        uint32_t m0 = n0;
 #pragma unroll
-        for (uint32_t i = 0; i < IT_SPANW; ++i) { const uint32_t d = first - (uint32_t)(p0 + 32 * (int32_t)i); if (d < 32u) q[i] |= 1u << d; }
+        for (uint32_t i = 0; i < IT_SPANW; ++i) {
+          const uint32_t raw = q[i];
+          for (uint32_t m = t[i]; m; m &= m - 1u) {
+            const uint32_t bit = m & (0u - m), here = (m0 + (uint32_t)__popc(raw & (bit - 1u))) & 1u;
+            if (here != prev) q[i] |= bit; /* closed there */
+            prev = here;
+          }
+          m0 += (uint32_t)__popc(raw);
+        }
       }
     }
     {

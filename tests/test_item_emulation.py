@@ -287,6 +287,20 @@ def test_records_longer_than_the_window(emu, oracle, schema):
                     assert got.fast >= want.n_records - want.n_errors - 1
 
 
+def test_lines_that_end_inside_a_string(emu, oracle):
+    """However many they are, the index takes a fixed number of rounds (it closed one of them in each)."""
+    rng = random.Random(4)
+    for line in ('"', '{"id', '{"id":1,"username":"a', '{"id":1,"username":"a","phone":"x\\"', '{"id":"7","username":"a"}"'):
+        for share in (1.0, 0.5, 0.03):
+            text = "\n".join(line if rng.random() < share else '{"id":2,"username":"b"}' for _ in range(3000))
+            body = as_u8(text)
+            want = oracle.parse(USER, body)
+            for kw in (dict(tile=4096), dict(tile=32768, mis=7, order=9)):
+                got = Run(emu, USER, body, **kw)
+                assert same_result(want, got.cols) == "", (line, share, kw)
+                assert got.barriers <= 120 * got.tiles, (line, share, kw, got.barriers, got.tiles)
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
