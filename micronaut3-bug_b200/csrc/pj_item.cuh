@@ -1766,25 +1766,37 @@ __device__ __forceinline__ void item_emit_fixed(const ItemArgs& a, const ItemOut
     item_emit_fixed<OBJ, ROOT, WORD0, BIT0, I + 1>(a, o);
   }
 }
-/* string columns of root or embedded object OBJ (every lane of the warp calls this) */
-template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
+/* (What is called out of line takes its ItemOut by value: the callers' stay in registers.) string columns of root or embedded object OBJ (every lane of the warp calls this). APART: some of the records stand apart; groups without one
+ * do not pay for it (100k Users in an array: 69 us with the loop over runs in every group, 62 us without). */
+template <bool APART, int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
 __device__ __forceinline__ void item_emit_strings(const ItemArgs& a, const ItemShared& sh, const ItemOut& o) {
   if constexpr (I < CObj<OBJ>::N) {
     constexpr uint32_t kind = CObj<OBJ>::f[I].kind, col = CObj<OBJ>::f[I].col, slot = CObj<OBJ>::f[I].cnt;
     constexpr uint32_t word = ROOT ? it_root_word<OBJ>(I) : WORD0 + it_flat_word<OBJ>(I);
     if constexpr (kind == K_STR) {
       const bool pr = o.has_row && ((o.flags >> (IF_PRESENT + BIT0 + I)) & 1u);
-      const uint32_t lane = threadIdx.x & 31u, mine = (o.apart >> lane) & 1u;
-      const uint32_t ref = o.row[word], n = pr ? (ref >> 16) & 0x7FFFu : 0u, all = mine ? o.row[IW_FIELDS + slot - ItSlot0<MODEL>::n] : n;
-      const uint32_t at = sh.base[slot] + sh.csum[slot][o.chunk], inc = warp_incl_scan(all);
-      if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at + inc - all;
-      item_each_run(o.apart, [&](uint32_t lo, uint32_t end) {
-        const uint32_t from = __shfl_sync(0xFFFFFFFFu, inc - all, (int)lo), to = __shfl_sync(0xFFFFFFFFu, inc, (int)end - 1);
-        item_emit_run(o.stage, colp<uint8_t>(&a.cols, col + 1) + at + from, o.win, ref & 0xFFFFu, lane >= lo && lane < end ? n : 0u, inc - all - from, to - from);
-      });
-    } else if constexpr (kind == K_OBJ) item_emit_strings<MODEL, CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
-    item_emit_strings<MODEL, OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
+      const uint32_t ref = o.row[word], n = pr ? (ref >> 16) & 0x7FFFu : 0u, at = sh.base[slot] + sh.csum[slot][o.chunk];
+      if constexpr (!APART) {
+        const uint32_t inc = warp_incl_scan(n);
+        if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at + inc - n;
+        item_emit_run(o.stage, colp<uint8_t>(&a.cols, col + 1) + at, o.win, ref & 0xFFFFu, n, inc - n, __shfl_sync(0xFFFFFFFFu, inc, 31));
+      } else {
+        const uint32_t lane = threadIdx.x & 31u, all = (o.apart >> lane) & 1u ? o.row[IW_FIELDS + slot - ItSlot0<MODEL>::n] : n, inc = warp_incl_scan(all);
+        if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = at + inc - all;
+        item_each_run(o.apart, [&](uint32_t lo, uint32_t end) {
+          const uint32_t from = __shfl_sync(0xFFFFFFFFu, inc - all, (int)lo), to = __shfl_sync(0xFFFFFFFFu, inc, (int)end - 1);
+          item_emit_run(o.stage, colp<uint8_t>(&a.cols, col + 1) + at + from, o.win, ref & 0xFFFFu, lane >= lo && lane < end ? n : 0u, inc - all - from, to - from);
+        });
+      }
+    } else if constexpr (kind == K_OBJ) item_emit_strings<APART, MODEL, CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
+    item_emit_strings<APART, MODEL, OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
   }
+}
+template <int MODEL>
+__device__ __noinline__ void item_emit_strings_apart(const ItemArgs& a, const ItemShared& sh, const ItemOut o) { item_emit_strings<true, MODEL, MODEL, true, 0u, 0u>(a, sh, o); }
+template <int MODEL>
+__device__ __forceinline__ void item_emit_strings_of(const ItemArgs& a, const ItemShared& sh, const ItemOut& o) {
+  if (o.apart) item_emit_strings_apart<MODEL>(a, sh, o); else item_emit_strings<false, MODEL, MODEL, true, 0u, 0u>(a, sh, o);
 }
 /* bytes of the lines' strings per slot, added up over the warp into csum[slot][chunk] */
 template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
@@ -1800,7 +1812,7 @@ __device__ __forceinline__ void item_sum_strings(ItemShared& sh, const uint32_t*
   }
 }
 /* the lists of 32 lines, an element per lane */
-template <bool OBJS>
+template <bool APART, bool OBJS>
 __device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemShared& sh, const ItemOut& o, const uint32_t* pairs, bool mine) {
   constexpr int F = OBJS ? ItModel<OBJ_PET>::ei : ItModel<OBJ_PET>::li;
   constexpr int E = OBJ_TAG;
@@ -1811,36 +1823,44 @@ __device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemSha
   const uint32_t l = mine ? o.row[OBJS ? ItWords<OBJ_PET>::n : (uint32_t)IW_LIST] : 0u, n = l >> 16;
   const uint64_t r0 = (uint64_t)sh.base[slot] + sh.csum[slot][o.chunk];
   const uint32_t lane = threadIdx.x & 31u;
-  const bool apart = (o.apart >> lane) & 1u;
+  const bool apart = APART && ((o.apart >> lane) & 1u);
   const uint32_t all = apart ? o.row[IW_FIELDS + slot - ItSlot0<OBJ_PET>::n] : n, inc = warp_incl_scan(all);
   if (o.has_row) colp<uint32_t>(&a.cols, col)[o.at] = (uint32_t)r0 + inc - all;
   const uint32_t at0 = sh.base[bslot] + sh.csum[bslot][o.chunk];
-  uint32_t bytes = 0; /* of the lists of the lanes before: needed from the second run on */
-  if (o.apart) {
+  uint32_t at = at0, done = 0;
+  auto element = [&](uint32_t src, uint32_t j, bool has) {
+    const uint32_t k = __shfl_sync(0xFFFFFFFFu, l, (int)src) & 0xFFFFu;
+    const uint64_t r = r0 + done + lane;
+    uint32_t pos = 0, len = 0;
+    if constexpr (OBJS) {
+      if (has) {
+        const uint32_t* e = pairs + k + 3u * j;
+        const uint32_t x = e[2];
+        colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((x >> 28) & 3u);
+        colp<int64_t>(&a.cols, CObj<E>::f[0].col)[r] = (x >> 28) & 1u ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
+        pos = x & 0xFFFFu; len = (x >> 29) & 1u ? (x >> 16) & 0xFFFu : 0u;
+      }
+    } else if (has) { const uint32_t pr = pairs[k + j]; pos = (pr & 0xFFFFu) + 1u; len = (pr >> 16) - pos - item_freed(o.win, o.moved, k + j, pr >> 16); }
+    const uint32_t sc = warp_incl_scan(len), total = __shfl_sync(0xFFFFFFFFu, sc, 31);
+    if (has) colp<uint32_t>(&a.cols, off_col)[r] = at + sc - len;
+    item_emit_run(o.stage, colp<uint8_t>(&a.cols, off_col + 1u) + at, o.win, pos, len, sc - len, total);
+    at += total; done += 32;
+  };
+  if constexpr (!APART) item_each_element(o.owner, n, element);
+  else {
     const uint32_t w = mine ? o.row[ItWords<OBJ_PET>::n + 1u] : 0u, own = apart ? o.row[IW_FIELDS + bslot - ItSlot0<OBJ_PET>::n] : (OBJS ? w >> 16 : w & 0xFFFFu);
-    bytes = warp_incl_scan(own) - own;
-  }
-  item_each_run(o.apart, [&](uint32_t lo, uint32_t end) {
-    uint32_t at = at0 + __shfl_sync(0xFFFFFFFFu, bytes, (int)lo), done = __shfl_sync(0xFFFFFFFFu, inc - all, (int)lo);
-    item_each_element(o.owner, lane >= lo && lane < end ? n : 0u, [&](uint32_t src, uint32_t j, bool has) {
-      const uint32_t k = __shfl_sync(0xFFFFFFFFu, l, (int)src) & 0xFFFFu;
-      const uint64_t r = r0 + done + lane;
-      uint32_t pos = 0, len = 0;
-      if constexpr (OBJS) {
-        if (has) {
-          const uint32_t* e = pairs + k + 3u * j;
-          const uint32_t x = e[2];
-          colp<uint8_t>(&a.cols, CObj<E>::present_col)[r] = (uint8_t)((x >> 28) & 3u);
-          colp<int64_t>(&a.cols, CObj<E>::f[0].col)[r] = (x >> 28) & 1u ? (int64_t)((uint64_t)e[0] | ((uint64_t)e[1] << 32)) : 0;
-          pos = x & 0xFFFFu; len = (x >> 29) & 1u ? (x >> 16) & 0xFFFu : 0u;
-        }
-      } else if (has) { const uint32_t pr = pairs[k + j]; pos = (pr & 0xFFFFu) + 1u; len = (pr >> 16) - pos - item_freed(o.win, o.moved, k + j, pr >> 16); }
-      const uint32_t sc = warp_incl_scan(len), total = __shfl_sync(0xFFFFFFFFu, sc, 31);
-      if (has) colp<uint32_t>(&a.cols, off_col)[r] = at + sc - len;
-      item_emit_run(o.stage, colp<uint8_t>(&a.cols, off_col + 1u) + at, o.win, pos, len, sc - len, total);
-      at += total; done += 32;
+    const uint32_t bytes = warp_incl_scan(own) - own; /* of the lists of the lanes before */
+    item_each_run(o.apart, [&](uint32_t lo, uint32_t end) {
+      at = at0 + __shfl_sync(0xFFFFFFFFu, bytes, (int)lo); done = __shfl_sync(0xFFFFFFFFu, inc - all, (int)lo);
+      item_each_element(o.owner, lane >= lo && lane < end ? n : 0u, element);
     });
-  });
+  }
+}
+template <bool OBJS>
+__device__ __noinline__ void item_emit_lists_apart(const ItemArgs& a, const ItemShared& sh, const ItemOut o, const uint32_t* pairs, bool mine) { item_emit_lists<true, OBJS>(a, sh, o, pairs, mine); }
+template <bool OBJS>
+__device__ __forceinline__ void item_emit_lists_of(const ItemArgs& a, const ItemShared& sh, const ItemOut& o, const uint32_t* pairs, bool mine) {
+  if (o.apart) item_emit_lists_apart<OBJS>(a, sh, o, pairs, mine); else item_emit_lists<false, OBJS>(a, sh, o, pairs, mine);
 }
 
 /* ---- the exact parser -------------------------------------------------------------------------------------------- */
@@ -1871,11 +1891,15 @@ __device__ __noinline__ uint32_t item_exact(const ItemArgs& a, const uint8_t* in
   if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[ItWords<OBJ_PET>::n] = 0; row[ItWords<OBJ_PET>::n + 1u] = 0; }
   return type;
 }
-/* where line ln, whose first byte is at input offset s0, ends for the exact parser: NDJSON: it looks for the line feed itself */
-__device__ __forceinline__ uint64_t item_limit(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, uint32_t ln, uint64_t s0) {
-  if (!a.sep) return a.limit;
-  if (sh.open_end && ln + 1u == sh.nline) return arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener).end;
-  return g.v0 + ((sh.line[ln + 1u] & 0xFFFFu) - 1u) - g.mis;
+/* Line ln for the exact parser, in shared memory when what is there is what the input says and the whole line, else where it lies. */
+struct ItemText { const uint8_t* in; uint64_t start, limit; };
+__device__ __forceinline__ ItemText item_text(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, const uint8_t* win, uint32_t ln) {
+  const uint32_t at = sh.line[ln] & 0xFFFFu, sep = (sh.line[ln + 1u] & 0xFFFFu) - 1u;
+  if (sep < g.hi_valid && !((sh.movedline[ln >> 5] >> (ln & 31u)) & 1u)) return ItemText{win, at, a.sep ? sep : sep + 1u};
+  const uint64_t s0 = g.v0 + at - g.mis;
+  if (!a.sep) return ItemText{a.in, s0, a.limit}; /* (it looks for the line feed itself) */
+  if (sh.open_end && ln + 1u == sh.nline) return ItemText{a.in, s0, arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener).end};
+  return ItemText{a.in, s0, g.v0 + sep - g.mis};
 }
 /* what a record that does not stand apart adds to its model's counters */
 template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
@@ -1896,7 +1920,7 @@ __device__ __forceinline__ void item_counts(const uint32_t* row, uint32_t flags,
 /* The columns of the records among 32 lines that stand apart (every lane of the warp calls this): by the exact parser once more, at the
  * place the records of their model before them leave. n: the lane's record, at: its row in its model's table. */
 template <int SCHEMA>
-__device__ __noinline__ void item_emit_apart(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, const uint32_t* row, uint32_t flags, uint32_t type, uint32_t ln, uint32_t c, uint64_t n, uint64_t at) {
+__device__ __noinline__ void item_emit_apart(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, const uint8_t* win, const uint32_t* row, uint32_t flags, uint32_t type, uint32_t ln, uint32_t c, uint64_t n, uint64_t at) {
   const bool apart = (flags & IF_APART) != 0;
   Out<true> o;
   o.cols = &a.cols;
@@ -1919,9 +1943,10 @@ __device__ __noinline__ void item_emit_apart(const ItemArgs& a, const StreamGeom
   if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_PET>());
   if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_USER>());
   if (apart) {
+    const ItemText t = item_text(a, g, sh, win, ln);
     PS s;
-    s.p = g.v0 + (row[IW_POS] & 0xFFFFu) - g.mis; s.err = 0; s.err_pos = 0;
-    parse_record<true>(c_schema, item_reader(a, a.in, item_limit(a, g, sh, ln, s.p)), s, (uint32_t)SCHEMA, o, n);
+    s.p = t.start; s.err = 0; s.err_pos = 0;
+    parse_record<true>(c_schema, item_reader(a, t.in, t.limit), s, (uint32_t)SCHEMA, o, n);
   }
 }
 
@@ -2097,11 +2122,8 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     if (rec && !good) {
       uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
       if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
-        /* where it lies in shared memory, when that is what the input says and holds the whole record */
-        const uint32_t at = row[IW_POS] & 0xFFFFu, sep = (sh.line[tid + 1u] & 0xFFFFu) - 1u;
-        const uint64_t s0 = g.v0 + at - g.mis;
-        const bool here = sep < g.hi_valid && !((sh.movedline[warp] >> lane) & 1u);
-        type = item_exact<SCHEMA>(a, here ? win : a.in, here ? at : s0, here ? (ARR ? sep : sep + 1u) : item_limit(a, g, sh, tid, s0), &kind, &off, row);
+        const ItemText t = item_text(a, g, sh, win, tid);
+        type = item_exact<SCHEMA>(a, t.in, t.start, t.limit, &kind, &off, row);
         good = !kind; /* a valid record of a kind the other steps do not know */
       }
       flags = good ? IF_APART | IF_RECORD | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD;
@@ -2204,7 +2226,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         if (br != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(br & ~bg));
         if (bg & ~o.apart) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg & ~o.apart));
       }
-      if (o.apart) item_emit_apart<SCHEMA>(a, g, sh, r, f, type, ln, c, n, o.at);
+      if (o.apart) item_emit_apart<SCHEMA>(a, g, sh, win, r, f, type, ln, c, n, o.at);
       if (rec) {
         colp<uint64_t>(&a.cols, PJ_COL_REC_START)[n] = a.goff + g.v0 + (r[IW_POS] & 0xFFFFu) - g.mis;
         colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[n] = good ? 0 : (uint8_t)r[IW_ERR];
@@ -2225,20 +2247,20 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         }
       }
     } else if (what == 2u) {
-      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings<OBJ_PET, OBJ_PET, true, 0u, 0u>(a, sh, o); }
-      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings<OBJ_USER, OBJ_USER, true, 0u, 0u>(a, sh, o); }
+      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings_of<OBJ_PET>(a, sh, o); }
+      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings_of<OBJ_USER>(a, sh, o); }
       else if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
         const uint32_t apart_all = o.apart;
         o.has_row = type == PJ_TYPE_PET; o.apart = apart_all & bp;
-        if (bp) item_emit_strings<OBJ_PET, OBJ_PET, true, 0u, 0u>(a, sh, o);
+        if (bp) item_emit_strings_of<OBJ_PET>(a, sh, o);
         o.has_row = type == PJ_TYPE_USER; o.apart = apart_all & bu;
-        if (bu) item_emit_strings<OBJ_USER, OBJ_USER, true, 0u, 0u>(a, sh, o);
+        if (bu) item_emit_strings_of<OBJ_USER>(a, sh, o);
       }
     } else if constexpr (SL::lists) {
       const bool pet = type == PJ_TYPE_PET;
       o.has_row = SCHEMA == PJ_SCHEMA_PET ? rec : pet;
       if constexpr (SCHEMA == PJ_SCHEMA_MIXED) o.apart &= bp;
-      if (SCHEMA == PJ_SCHEMA_PET || bp) { if (what == 0u) item_emit_lists<false>(a, sh, o, pairs, pet); else item_emit_lists<true>(a, sh, o, pairs, pet); }
+      if (SCHEMA == PJ_SCHEMA_PET || bp) { if (what == 0u) item_emit_lists_of<false>(a, sh, o, pairs, pet); else item_emit_lists_of<true>(a, sh, o, pairs, pet); }
     }
   }
   if (tile == a.ntiles - 1) item_close_offsets(a, sh, tid);
