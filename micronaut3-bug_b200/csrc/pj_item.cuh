@@ -24,8 +24,8 @@
  * and offset, because the smallest offset of a record's deviations is its first failure. Any other deviation sends the
  * record to the exact parser (pj_core.cuh); a record that one accepts (unknown keys with nested values, repeated keys, ...) stands apart:
  * its counts take part in the sums, and it is parsed once more to write its columns (item_emit_apart). Does the tile not fit
- * the shared memory laid out for it (many more lines or strings than its bytes suggest), the block walks the tile with the
- * exact parser alone (item_slow_tile). A record that runs out of the window is the exact parser's, where it lies.
+ * the shared memory laid out for it (many more lines or strings than its bytes suggest), every thread of the block walks lines
+ * where they lie (item_slow_tile); a record that runs out of the window is read where it lies as well.
  */
 #ifndef PJ_ITEM_CUH
 #define PJ_ITEM_CUH
@@ -1870,27 +1870,6 @@ __device__ __forceinline__ Rd item_reader(const ItemArgs& a, const uint8_t* in, 
   rd.in = in; rd.lf_ws = a.sep ? 1u : 0u; rd.open_end = (a.is_last || a.sep) ? 0u : 1u; rd.limit = limit; rd.opts = a.opts; rd.rec_end = limit;
   return rd;
 }
-/* A record the fast steps refused, from its first byte at input offset s up to `limit`: kind and offset of its failure in *err,
- * *off. *err = 0: it is a valid one after all, of the model returned, and its row holds what it adds to that model's counters. */
-template <int SCHEMA>
-__device__ __noinline__ uint32_t item_exact(const ItemArgs& a, const uint8_t* in, uint64_t s0, uint64_t limit, uint32_t* err, uint32_t* off, uint32_t* row) {
-  const Rd rd = item_reader(a, in, limit);
-  PS s;
-  s.p = s0; s.err = 0; s.err_pos = 0;
-  Out<false> so;
-  so.cols = &a.cols;
-  uint32_t type = PJ_TYPE_NONE;
-  uint64_t p = s0;
-  if (a.sep) while (p < limit && (item_blank(in[p]) || in[p] == '\n')) ++p;
-  if (p < limit || !a.sep) type = parse_record<false>(c_schema, rd, s, (uint32_t)SCHEMA, so, 0);
-  else fail(s, PJ_E_SYNTAX, limit); /* an extent without a value */
-  *err = s.err; *off = (uint32_t)(s.err_pos - s0);
-  if (s.err) return PJ_TYPE_NONE;
-  const uint32_t slot0 = type == PJ_TYPE_USER ? ItSlot0<OBJ_USER>::n : ItSlot0<OBJ_PET>::n;
-  if (type != PJ_TYPE_ORDER) for (uint32_t j = 0; j < IT_APART; ++j) row[IW_FIELDS + j] = so.cnt[slot0 + j];
-  if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[ItWords<OBJ_PET>::n] = 0; row[ItWords<OBJ_PET>::n + 1u] = 0; }
-  return type;
-}
 /* Line ln for the exact parser, in shared memory when what is there is what the input says and the whole line, else where it lies. */
 struct ItemText { const uint8_t* in; uint64_t start, limit; };
 __device__ __forceinline__ ItemText item_text(const ItemArgs& a, const StreamGeom& g, const ItemShared& sh, const uint8_t* win, uint32_t ln) {
@@ -1900,6 +1879,76 @@ __device__ __forceinline__ ItemText item_text(const ItemArgs& a, const StreamGeo
   if (!a.sep) return ItemText{a.in, s0, a.limit}; /* (it looks for the line feed itself) */
   if (sh.open_end && ln + 1u == sh.nline) return ItemText{a.in, s0, arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener).end};
   return ItemText{a.in, s0, g.v0 + sep - g.mis};
+}
+/* A line where it lies, for the word-at-a-time tokeniser: positions from an aligned word on. It looks ahead, so 32 readable bytes have to
+ * follow the line: in array framing behind its end, in NDJSON behind a limit that no line which uses the tokeniser's answer reaches. */
+struct ItemDirect { Win w; uint32_t start, limit; };
+__device__ __forceinline__ bool item_direct(const ItemArgs& a, const ItemText& t, ItemDirect& d) {
+  if (t.in != a.in || t.limit + (a.sep ? 32u : 0u) > a.limit) return false;
+  const uint64_t end = a.sep ? t.limit : (a.limit < 32u ? 0u : a.limit - 32u);
+  const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(a.in + t.start) & 3u);
+  if (end <= t.start || end - t.start > 0x7FFF0000u) return false;
+  d.w.s = a.in + t.start - mis; d.w.w0 = (int64_t)t.start - mis;
+  d.start = mis; d.limit = (uint32_t)(end - t.start) + mis;
+  return true;
+}
+/* A record's model, what it adds to every counter and whether the word-at-a-time tokeniser took it (else the exact parser did), or
+ * PJ_TYPE_NONE and kind and offset of its failure. */
+struct ItemSize { uint32_t type, err, off, fast, cnt[NSLOT]; };
+template <int SCHEMA>
+__device__ __noinline__ void item_size(const ItemArgs& a, const ItemText t, ItemSize* r) {
+  ItemDirect d;
+  r->type = PJ_TYPE_NONE; r->err = 0; r->off = 0; r->fast = 0;
+  if (item_direct(a, t, d)) {
+    uint32_t tape[TAPE_MIN_CAP], pos = 0;
+    Tape tp;
+    tp.e = tape; tp.stride = 1; tp.cap = TAPE_MIN_CAP; tp.n = 0;
+    uint32_t v = fast_outline<SCHEMA>(d.w, d.start, d.limit, a.sep ? 1u : 0u, a.sep ? 0u : 1u, nullptr, nullptr, 0, tp, r->cnt, &r->type, &r->err, &pos);
+    if (v == FAST_FAILED && ((!a.sep && pos >= d.limit) || ((a.opts & PJ_OPT_ENUM_UNKNOWN_AS_NULL) && r->err == PJ_E_ENUM) || ((a.opts & PJ_OPT_COERCE_SCALARS) && r->err == PJ_E_TYPE))) v = FAST_REFUSED;
+    if (v == FAST_ACCEPTED) { r->err = 0; r->fast = 1; return; }
+    r->type = PJ_TYPE_NONE;
+    if (v == FAST_FAILED) { r->off = pos - d.start; return; }
+    r->err = 0;
+  }
+  PS s;
+  s.p = t.start; s.err = 0; s.err_pos = 0;
+  Out<false> so;
+  so.cols = &a.cols;
+  uint64_t p = t.start;
+  if (a.sep) while (p < t.limit && (item_blank(t.in[p]) || t.in[p] == '\n')) ++p;
+  if (p < t.limit || !a.sep) r->type = parse_record<false>(c_schema, item_reader(a, t.in, t.limit), s, (uint32_t)SCHEMA, so, 0);
+  else fail(s, PJ_E_SYNTAX, t.limit); /* an extent without a value */
+  for (uint32_t k = 0; k < NSLOT; ++k) r->cnt[k] = so.cnt[k];
+  if (s.err) { r->type = PJ_TYPE_NONE; r->err = s.err; r->off = (uint32_t)(s.err_pos - t.start); }
+  else if (t.in == a.in && s.p - t.start > *(volatile uint32_t*)&a.res->max_rec) atomicMax(&a.res->max_rec, (uint32_t)(s.p - t.start < 0x7FFFFFFFu ? s.p - t.start : 0x7FFFFFFFu));
+}
+/* its columns, from the places o gives on; by the parser that sized it */
+template <int SCHEMA>
+__device__ __noinline__ void item_place(const ItemArgs& a, const ItemText t, uint32_t fast, Out<true>& o, uint64_t n) {
+  if (fast) {
+    ItemDirect d;
+    uint32_t tape[TAPE_MIN_CAP], x[3];
+    Tape tp;
+    tp.e = tape; tp.stride = 1; tp.cap = TAPE_MIN_CAP; tp.n = 0;
+    if (item_direct(a, t, d)) fast_outline<SCHEMA>(d.w, d.start, d.limit, a.sep ? 1u : 0u, a.sep ? 0u : 1u, &a.cols, o.base, n, tp, nullptr, &x[0], &x[1], &x[2]);
+    return;
+  }
+  PS s;
+  s.p = t.start; s.err = 0; s.err_pos = 0;
+  parse_record<true>(c_schema, item_reader(a, t.in, t.limit), s, (uint32_t)SCHEMA, o, n);
+}
+/* A record the own steps refused: kind and offset of its failure in *err, *off. *err = 0: it is a valid one after all, of the model returned
+ * (| 256: by the word-at-a-time tokeniser), and its row holds what it adds to that model's counters. */
+template <int SCHEMA>
+__device__ __forceinline__ uint32_t item_judge(const ItemArgs& a, const ItemText& t, uint32_t* err, uint32_t* off, uint32_t* row) {
+  ItemSize r;
+  item_size<SCHEMA>(a, t, &r);
+  *err = r.err; *off = r.off;
+  if (r.err) return PJ_TYPE_NONE;
+  const uint32_t slot0 = r.type == PJ_TYPE_USER ? ItSlot0<OBJ_USER>::n : ItSlot0<OBJ_PET>::n;
+  if (r.type != PJ_TYPE_ORDER) for (uint32_t j = 0; j < IT_APART; ++j) row[IW_FIELDS + j] = r.cnt[slot0 + j];
+  if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[ItWords<OBJ_PET>::n] = 0; row[ItWords<OBJ_PET>::n + 1u] = 0; }
+  return r.type | (r.fast << 8);
 }
 /* what a record that does not stand apart adds to its model's counters */
 template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
@@ -1943,15 +1992,12 @@ __device__ __noinline__ void item_emit_apart(const ItemArgs& a, const StreamGeom
   if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_PET>());
   if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) model(ItInteger<OBJ_USER>());
   if (apart) {
-    const ItemText t = item_text(a, g, sh, win, ln);
-    PS s;
-    s.p = t.start; s.err = 0; s.err_pos = 0;
-    parse_record<true>(c_schema, item_reader(a, t.in, t.limit), s, (uint32_t)SCHEMA, o, n);
+    item_place<SCHEMA>(a, item_text(a, g, sh, win, ln), flags & IF_ROWS, o, n);
   }
 }
 
 /* The lines whose preceding separator lies in [lo, hi) of the input, one after the other (head: and before them the one at
- * byte 0): f(start, limit, blank). */
+ * byte 0): f(start, limit). */
 template <class F>
 __device__ __forceinline__ void item_each_line(const ItemArgs& a, uint64_t lo, uint64_t hi, bool head, F f) {
   if (a.sep) {
@@ -1959,16 +2005,17 @@ __device__ __forceinline__ void item_each_line(const ItemArgs& a, uint64_t lo, u
       if (!((a.sep[p >> 6] >> (p & 63)) & 1u)) continue;
       const ExtentOut x = arr_extent(a.in, a.len, a.sep, p, a.res->first_opener);
       if (x.second_opener) atomicMin(&a.res->doc_err_off, (unsigned long long)p); /* a second document */
-      if (x.is_record) f(x.start, x.end, x.blank != 0);
+      if (x.is_record) f(x.start, x.end);
     }
   } else {
-    if (head && nd_is_record(a.in, 0, a.limit, (int)a.is_last)) f((uint64_t)0, a.limit, false);
+    if (head && nd_is_record(a.in, 0, a.limit, (int)a.is_last)) f((uint64_t)0, a.limit);
     for (uint64_t p = lo; p < hi; ++p)
-      if (a.in[p] == '\n' && nd_is_record(a.in, p + 1, a.limit, (int)a.is_last)) f(p + 1, a.limit, false);
+      if (a.in[p] == '\n' && nd_is_record(a.in, p + 1, a.limit, (int)a.is_last)) f(p + 1, a.limit);
   }
 }
-/* A tile with the exact parser alone, read where it lies: every thread walks the lines that begin in its share of the
- * tile's bytes, once to size them and once to emit them. */
+/* A tile of many more lines or strings than its shared memory has room for, read where it lies: every thread walks the lines that begin in its
+ * share of the tile's bytes, once to size them and once to size and emit them, with the word-at-a-time tokeniser and, for what that one
+ * refuses, the exact parser. */
 template <int SCHEMA>
 __device__ __noinline__ void item_slow_tile(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, uint32_t tile, uint32_t tid) {
   using SL = ItemSlots<SCHEMA>;
@@ -1986,40 +2033,30 @@ __device__ __noinline__ void item_slow_tile(const ItemArgs& a, const StreamGeom&
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     if (head || lo < hi)
-      item_each_line(a, lo, hi, head, [&](uint64_t s0, uint64_t limit, bool blank) {
-        const Rd rd = item_reader(a, a.in, limit);
-        PS s;
-        s.p = s0; s.err = 0; s.err_pos = 0;
-        Out<false> so;
-        so.cols = &a.cols;
-        uint32_t type = PJ_TYPE_NONE;
-        if (blank) fail(s, PJ_E_SYNTAX, limit);
-        else type = parse_record<false>(c_schema, rd, s, (uint32_t)SCHEMA, so, 0);
-        if (s.err) type = PJ_TYPE_NONE;
+      item_each_line(a, lo, hi, head, [&](uint64_t s0, uint64_t limit) {
+        const ItemText t = ItemText{a.in, s0, limit};
+        ItemSize r;
+        item_size<SCHEMA>(a, t, &r);
         if (pass == 0) {
-          const uint64_t n = s.p - s0;
-          if (!s.err && n > *(volatile uint32_t*)&a.res->max_rec) atomicMax(&a.res->max_rec, (uint32_t)(n < 0x7FFFFFFFu ? n : 0x7FFFFFFFu));
           sum[IT_REC]++;
-          nerr += s.err != 0;
-          if (!s.err) for (uint32_t k = SL::lo; k < SL::hi; ++k) sum[k] += so.cnt[k];
+          nerr += r.err != 0;
+          if (!r.err) for (uint32_t k = SL::lo; k < SL::hi; ++k) sum[k] += r.cnt[k];
         } else {
           const uint64_t i = my_base[IT_REC];
           colp<uint64_t>(&a.cols, PJ_COL_REC_START)[i] = a.goff + s0;
-          colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[i] = (uint8_t)s.err;
-          colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[i] = s.err ? (uint32_t)(s.err_pos - s0) : 0u;
+          colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[i] = (uint8_t)r.err;
+          colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[i] = r.off;
           if (SCHEMA == PJ_SCHEMA_MIXED) {
-            colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[i] = (uint8_t)type;
-            colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[i] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : my_base[type - 1];
+            colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[i] = (uint8_t)r.type;
+            colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[i] = r.type == PJ_TYPE_NONE ? 0xFFFFFFFFu : my_base[r.type - 1];
           }
           Out<true> o;
           o.cols = &a.cols;
-          for (uint32_t k = 0; k < NSLOT; ++k) { o.base[k] = my_base[k]; o.room[k] = (k >= SL::lo && k < SL::hi && !s.err) ? so.cnt[k] : 0u; }
-          if (s.err) { if (SCHEMA != PJ_SCHEMA_MIXED) store_absent<true>(c_schema, (uint32_t)SCHEMA, o, i); }
+          for (uint32_t k = 0; k < NSLOT; ++k) { o.base[k] = my_base[k]; o.room[k] = (k >= SL::lo && k < SL::hi && !r.err) ? r.cnt[k] : 0u; }
+          if (r.err) { if (SCHEMA != PJ_SCHEMA_MIXED) store_absent<true>(c_schema, (uint32_t)SCHEMA, o, i); }
           else {
-            PS s2;
-            s2.p = s0; s2.err = 0; s2.err_pos = 0;
-            parse_record<true>(c_schema, rd, s2, (uint32_t)SCHEMA, o, i);
-            for (uint32_t k = SL::lo; k < SL::hi; ++k) my_base[k] += so.cnt[k];
+            item_place<SCHEMA>(a, t, r.fast, o, i);
+            for (uint32_t k = SL::lo; k < SL::hi; ++k) my_base[k] += r.cnt[k];
           }
           my_base[IT_REC]++;
         }
@@ -2120,13 +2157,14 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     }
     bool good = rec && e == IE_NONE;
     if (rec && !good) {
-      uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu);
+      uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu), apart_flags = IF_APART | IF_RECORD;
       if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
-        const ItemText t = item_text(a, g, sh, win, tid);
-        type = item_exact<SCHEMA>(a, t.in, t.start, t.limit, &kind, &off, row);
+        type = item_judge<SCHEMA>(a, item_text(a, g, sh, win, tid), &kind, &off, row);
+        if (type >> 8) apart_flags |= IF_ROWS;
+        type &= 255u;
         good = !kind; /* a valid record of a kind the other steps do not know */
       }
-      flags = good ? IF_APART | IF_RECORD | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD;
+      flags = good ? apart_flags | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD;
       row[IW_FLAGS] = flags; row[IW_ERR] = kind;
       if (!good) row[IW_LIST] = off;
     }

@@ -301,6 +301,27 @@ def test_lines_that_end_inside_a_string(emu, oracle):
                 assert got.barriers <= 120 * got.tiles, (line, share, kw, got.barriers, got.tiles)
 
 
+@pytest.mark.parametrize("schema", [PET, ORDER, USER, MIXED])
+def test_tiles_with_more_lines_or_strings_than_room(emu, oracle, schema):
+    """Their lines are sized and written where they lie, by either parser, up to the last bytes of the input and of a shard's slack."""
+    rng = random.Random(schema)
+    flags = ALL | (abi.PJ_GEN_ZIPF_LISTS if schema in (PET, MIXED) else 0)
+    for it in range(12):
+        lines = bytes(pj.gen_text(schema, it, 0, 60, rng.choice([0, flags]))).split(b"\n")[:-1]
+        lines = [mutate(rng, ln) if rng.random() < 0.2 else ln for ln in lines] + [b'{"id":1}', b'{"x":[1],"id":2}', b"{}", b" "][: it % 5]
+        rng.shuffle(lines)
+        for room in (dict(row_cap=3), dict(str_words=20)):
+            opts = rng.choice([0, 1, 2, 4])
+            for framing, text in ((NDJSON, b"\n".join(lines) + rng.choice([b"", b"\n", b"\n" + b" " * 40])), (ARRAY, b"[" + b",".join(lines) + b"]" + b" " * (it * 5))):
+                body = as_u8(text)
+                got = Run(emu, schema, body, framing, tile=4096, mis=it, opts=opts, **room)
+                assert same_result(oracle.parse(schema, body, framing, opts=opts), got.cols) == "", (it, room, framing)
+            body = as_u8(b"\n".join(lines) + b"\n")
+            cut = body.size // 2
+            got = Run(emu, schema, body, tile=4096, shard_slack=body.size - cut, is_last=0, **room)
+            assert same_result(oracle.parse(schema, body, slack=body.size - cut, is_last=0), got.cols) == "", (it, room)
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
