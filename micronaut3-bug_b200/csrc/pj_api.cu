@@ -117,6 +117,7 @@ struct pj_ctx {
   unsigned long long spin_ns = 2000000000ull; /* bound of every device-side wait */
   double avg_rec_bytes[5] = {0, 0, 0, 0, 0};  /* bytes per record seen per schema (sizes the tiles of the next call) */
   uint32_t max_rec_bytes[5] = {0, 0, 0, 0, 0}; /* bytes of the longest one */
+  uint32_t strs_per_kb[5] = {0, 0, 0, 0, 0};   /* strings per 1024 bytes of the tile with the most */
   /* NDJSON: which kernel the next call takes (use_items()), and how often it changed to k_parse_items */
   bool items[5] = {false, false, false, false, false};
   uint8_t to_items[5] = {0, 0, 0, 0, 0};
@@ -285,6 +286,7 @@ ItemShape pick_tile_shape(const pj_ctx* c, uint32_t schema, uint64_t len) {
   in.len = len;
   in.avg = c->avg_rec_bytes[schema]; in.guess = guess[schema];
   in.longest = c->max_rec_bytes[schema];
+  in.strs_per_kb = c->strs_per_kb[schema];
   in.tile_opt = c->tile_bytes_opt;
   in.stride = item_stride(schema);
   in.sms = (uint32_t)c->sms;
@@ -478,7 +480,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   uint64_t total[NSLOT];
   for (uint32_t k = 0; k < NSLOT; ++k) total[k] = 0;
   bool over = false;
-  uint32_t max_rec = 0;
+  uint32_t max_rec = 0, strs_per_kb = 0;
   uint64_t n_dense = 0;
   for (int p = 0; p < np; ++p) {
     PJ_CUDA(c, cudaEventSynchronize(c->ev_done[p]));
@@ -493,6 +495,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     if (r.timeout) return set_err(c, PJ_ERR_TIMEOUT, "pj_parse: a bounded device-side wait ran out");
     if (r.over) over = true;
     if (r.max_rec > max_rec) max_rec = r.max_rec;
+    if (r.strs_per_kb > strs_per_kb) strs_per_kb = r.strs_per_kb;
     n_dense += items ? r.n_dense : r.n_fast >> 32;
     const uint64_t rows_new = r.n_records;
     if (host_out && !over) {
@@ -521,7 +524,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   out->doc_err_kind = 0; out->doc_err_off = 0;
   const pj_status st = finish_columns(c, schema, len, pp, rows_done, n_errors, total, over, out);
   if (st) return st;
-  if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; if (items) c->max_rec_bytes[schema] = max_rec; }
+  if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; if (items) { c->max_rec_bytes[schema] = max_rec; c->strs_per_kb[schema] = strs_per_kb; } }
   note_spelling(c, schema, rows_done, n_errors, n_fast, n_dense, max_rec);
   if (host_out) PJ_CUDA(c, cudaStreamSynchronize(s_out));
   return PJ_OK;
@@ -609,7 +612,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   if (r.doc_err_off != ~0ull) { out->doc_err_kind = PJ_E_SYNTAX; out->doc_err_off = r.doc_err_off; }
   else if (r.first_opener == ~0ull || r.arr_final_s || r.arr_final_d != 0) { out->doc_err_kind = PJ_E_EOF; out->doc_err_off = len; }
   const pj_status st = finish_columns(c, schema, len, pp, r.n_records, r.n_errors, total, r.over != 0, out);
-  if (!st && r.n_records > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)r.n_records; c->max_rec_bytes[schema] = r.max_rec; }
+  if (!st && r.n_records > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)r.n_records; c->max_rec_bytes[schema] = r.max_rec; c->strs_per_kb[schema] = r.strs_per_kb; }
   if (st) return st;
   if (host_out) {
     for (int i = 0; i < pp.nneed; ++i) {

@@ -283,6 +283,8 @@ __device__ __forceinline__ uint32_t item_prefix_xor(uint32_t x) {
   x ^= x << 1; x ^= x << 2; x ^= x << 4; x ^= x << 8; x ^= x << 16;
   return x;
 }
+/* for the shape of the next call's tiles */
+__device__ __forceinline__ void item_note_strings(const ItemArgs& a, uint32_t n, uint32_t bytes) { if (bytes > 1024u) atomicMax(&a.res->strs_per_kb, n * 1024u / bytes); }
 /* The strings and lines the tile owns. False (for every thread): the tile does not fit, the block has to take the other road. The last line may
  * run out of the window. A record may end
  * inside a string: its separator then counts as the string's closing quote. */
@@ -463,7 +465,11 @@ __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& 
     }
     {
       const uint32_t n = nq + (total & 0xFFFFu), nl = nline + (total >> 16);
-      if (n / 2u + 2u > a.str_words || n / 2u >= IT_MAX_STRS || nl > IT_MAX_LINES || nl > a.row_cap) { fine = false; break; }
+      if (n / 2u + 2u > a.str_words || n / 2u >= IT_MAX_STRS || nl > IT_MAX_LINES || nl > a.row_cap) {
+        if (tid == 0) item_note_strings(a, n / 2u, (int32_t)(o + IT_STEP) < end_valid ? o + IT_STEP - start : (uint32_t)end_valid - start);
+        fine = false;
+        break;
+      }
       uint32_t k = nq + (at & 0xFFFFu), ln = nline + (at >> 16) + 1u;
 #pragma unroll
       for (uint32_t i = 0; i < IT_SPANW; ++i) {
@@ -2372,6 +2378,7 @@ __global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __g
     const long long c5 = clock64();
     atomicAdd(&a.res->phase_cycles[0], (unsigned long long)(ck[1] - ck[0]));
     if (sh.ndense) atomicAdd(&a.res->n_dense, (unsigned long long)sh.ndense);
+    if (sh.nline) item_note_strings(a, sh.nstr, sh.stop - (sh.line[0] & 0xFFFFu));
     atomicAdd(&a.res->phase_cycles[1], (unsigned long long)(ck[3] - ck[1]));
     atomicAdd(&a.res->phase_cycles[2], (unsigned long long)(ck[4] - ck[3]));
     atomicAdd(&a.res->phase_cycles[3], (unsigned long long)(c5 - ck[4]));

@@ -14,6 +14,7 @@ struct ItemShapeIn {
   double avg;         /* bytes per record of the context's last call on the schema; 0: there was none */
   double guess;       /* without one: of records as the workload generator writes them */
   uint32_t longest;   /* bytes of the longest record of that call; 0: not known */
+  uint32_t strs_per_kb; /* strings per 1024 bytes of its tile with the most; 0: not known */
   uint32_t tile_opt;  /* pj_options.tile_bytes; 0: ours to choose */
   uint32_t stride;    /* words per row (ItStride) */
   uint32_t sms;
@@ -36,6 +37,12 @@ inline ItemShape item_shape(const ItemShapeIn& in) {
   const uint64_t most = (uint64_t)(avg * (in.avg > 0 ? IT_MAX_LINES * 47 / 64 : IT_MAX_LINES * 9 / 16));
   uint64_t tile = avg * 4 > IT_STEP ? IT_STEP / 2 : IT_STEP - (uint64_t)(2 * avg);
   if (tile > most) tile = most;
+  /* lists of short strings: 4096 of them are a tile's limit, and each wants its word. (50k Pets of 40 strings of 4 bytes in an array:
+     8.1 ms when their tiles did not fit; records as the generator writes them have 45 to 75 in 1024 bytes.) */
+  if (in.strs_per_kb) {
+    const uint64_t fit = (uint64_t)(IT_MAX_STRS * 7u / 8u) * 1024u / in.strs_per_kb;
+    if (tile + slack > fit) tile = fit > slack + ST_MIN_TILE_BYTES ? fit - slack : ST_MIN_TILE_BYTES;
+  }
   /* few tiles: one for every block that can be resident, and room for many short strings */
   const uint64_t each = in.len / ((uint64_t)in.sms * IT_BLOCKS);
   uint32_t per_word = 9; /* window bytes per word for strings */
@@ -52,6 +59,8 @@ inline ItemShape item_shape(const ItemShapeIn& in) {
     t.row_cap = recs > IT_MAX_LINES ? IT_MAX_LINES : (uint32_t)recs;
     for (uint32_t w = per_word; w <= 9; ++w) {
       t.str_words = t.win_bytes / w;
+      const uint32_t known = (uint32_t)((uint64_t)t.win_bytes * in.strs_per_kb / 819u) + 16u; /* a quarter more, for rows of elements */
+      if (in.strs_per_kb && known > t.str_words) t.str_words = known < 4u * IT_MAX_STRS ? known : 4u * IT_MAX_STRS;
       if (item_layout(t.win_bytes, t.str_words, t.row_cap, in.stride).total <= item_room(blocks)) return t;
     }
     /* (the smallest tile fits two blocks whatever the records are, the largest fits one: tests/test_item_emulation.py) */

@@ -50,8 +50,8 @@ void array_index(const uint8_t* in, uint64_t len, std::vector<uint64_t>& sep, De
 extern "C" const char* emu_item_error() { return emu_block::error; }
 extern "C" uint64_t emu_item_barriers() { return emu_block::n_barriers; }
 /* out: tile, window, words for strings, rows, bytes of dynamic shared memory, the most that may be, blocks an SM holds */
-extern "C" void emu_item_shape(uint64_t len, double avg, double guess, uint32_t longest, uint32_t tile_opt, uint32_t* out) {
-  const ItemShape s = item_shape(ItemShapeIn{len, avg, guess, longest, tile_opt, ItStride<EMU_SCHEMA>::n, 148});
+extern "C" void emu_item_shape(uint64_t len, double avg, double guess, uint32_t longest, uint32_t strs_per_kb, uint32_t tile_opt, uint32_t* out) {
+  const ItemShape s = item_shape(ItemShapeIn{len, avg, guess, longest, strs_per_kb, tile_opt, ItStride<EMU_SCHEMA>::n, 148});
   const uint32_t total = item_layout(s.win_bytes, s.str_words, s.row_cap, ItStride<EMU_SCHEMA>::n).total;
   uint32_t blocks = IT_BLOCKS;
   while (blocks > 1 && total > item_room(blocks)) --blocks;
@@ -59,8 +59,8 @@ extern "C" void emu_item_shape(uint64_t len, double avg, double guess, uint32_t 
   for (int k = 0; k < 7; ++k) out[k] = v[k];
 }
 
-/* in: 16-byte aligned base + the caller's misalignment, readable in whole 16-byte blocks. stats[4]: fast records, lines the strict
- * walk took, longest record, tiles. Returns 0, 1 (some buffer is too small) or -1 (see emu_item_error). */
+/* in: 16-byte aligned base + the caller's misalignment, readable in whole 16-byte blocks. stats[5]: fast records, lines the strict
+ * walk took, longest record, tiles, strings per 1024 bytes. Returns 0, 1 (some buffer is too small) or -1 (see emu_item_error). */
 extern "C" int emu_item_parse(const Opts* o, const uint8_t* in, pj_columns* out, uint64_t* stats) {
   Schema S;
   build_schema(&S);
@@ -97,7 +97,7 @@ extern "C" int emu_item_parse(const Opts* o, const uint8_t* in, pj_columns* out,
   }
   if (fine && res.timeout) { snprintf(emu_block::error, sizeof emu_block::error, "a bounded wait ran out"); fine = false; }
   if (!fine) return -1;
-  stats[0] = res.n_fast; stats[1] = res.n_dense; stats[2] = res.max_rec; stats[3] = a.ntiles;
+  stats[0] = res.n_fast; stats[1] = res.n_dense; stats[2] = res.max_rec; stats[3] = a.ntiles; stats[4] = res.strs_per_kb;
   const uint64_t N = res.n_records;
   for (int c = 0; c < PJ_MAX_COLS; ++c) out->col[c].count = 0;
   out->col[PJ_COL_REC_START].count = out->col[PJ_COL_ERR_KIND].count = out->col[PJ_COL_ERR_OFF].count = N;

@@ -67,11 +67,11 @@ class Run:
         win = min(tile + slack, 65536 - 64)
         o = Opts(len=buf.size - shard_slack, slack=shard_slack, goff=goff, array=framing == ARRAY, is_first=is_first, is_last=is_last, opts=opts, tile_bytes=tile,
                  win_bytes=win, str_words=str_words or win // 4, row_cap=row_cap, order=order, rec_cap=nrec_bound(buf))
-        stats = (C.c_uint64 * 4)()
+        stats = (C.c_uint64 * 5)()
         lib = emu[schema]
         self.status = lib.emu_item_parse(C.byref(o), C.c_void_p(raw.ctypes.data + at), C.byref(self.cols.raw), stats)
         assert self.status >= 0, lib.emu_item_error().decode()
-        self.fast, self.dense, self.longest, self.tiles = stats
+        self.fast, self.dense, self.longest, self.tiles, self.strs_per_kb = stats
         self.barriers = lib.emu_item_barriers()
 
 
@@ -172,15 +172,17 @@ def test_tile_shape_fits_shared_memory(emu, schema):
     lens = [0, 1, 300, 5000, 10**5] + [int(10**5 * 1.21 ** k) for k in range(1, 60)] + list(range(15_000_000, 17_000_000, 40_000))
     for avg in [0, 1, 9, 40, 146, 200, 230, 250, 300, 700, 2000, 9000, 20_000, 10**6]:
         for longest in [0, 300, 3277, 9000, 22_000, 22_886, 23_000, 65_000, 1 << 30]:
-            for tile_opt in (0, 1, 4096, 20_000, 32_768, 1 << 20):
-                for n in lens if tile_opt == 0 else lens[:40:8]:
-                    emu[schema].emu_item_shape(C.c_uint64(n), C.c_double(avg), C.c_double(guess), C.c_uint32(longest), C.c_uint32(tile_opt), out)
+            for tile_opt, strs in ((0, 0), (0, 100), (0, 250), (0, 400), (1, 0), (4096, 0), (20_000, 0), (20_000, 300), (32_768, 0), (1 << 20, 400)):
+                for n in lens if tile_opt == 0 and strs == 0 else lens[:40:8]:
+                    emu[schema].emu_item_shape(C.c_uint64(n), C.c_double(avg), C.c_double(guess), C.c_uint32(longest), C.c_uint32(strs), C.c_uint32(tile_opt), out)
                     tile, win, words, rows, total, most, blocks = out
-                    where = (n, avg, longest, tile_opt, list(out))
+                    where = (n, avg, longest, strs, tile_opt, list(out))
                     assert total <= most, where
                     assert 1024 <= tile <= 36864 and tile % 32 == 0 and tile < win <= 65536 - 64 and win % 16 == 0, where
                     assert 24 <= rows <= 256 and words * 9 + 9 > win, where
-                    if tile_opt == 0 and longest <= 3277 and avg <= 300:
+                    if strs and tile_opt == 0 and longest <= 3277 and avg <= 300:  # a tile's strings have their words and are no more than its limit
+                        assert words >= win * strs // 1024 + 2 and tile * strs // 1024 < 4096, where
+                    if tile_opt == 0 and strs <= 100 and longest <= 3277 and avg <= 300:
                         assert blocks == 3, where
 
 
@@ -320,6 +322,22 @@ def test_tiles_with_more_lines_or_strings_than_room(emu, oracle, schema):
             cut = body.size // 2
             got = Run(emu, schema, body, tile=4096, shard_slack=body.size - cut, is_last=0, **room)
             assert same_result(oracle.parse(schema, body, slack=body.size - cut, is_last=0), got.cols) == "", (it, room)
+
+
+def test_lists_of_short_strings_fit_once_seen(emu, oracle):
+    """More strings than a window's usual room: the kernel says how many there are, and the shape made of that holds them."""
+    lines = ['{"id":%d,"name":"n","photoUrls":[%s]}' % (i, ",".join('"a%d"' % k for k in range(40))) for i in range(500)]
+    body = as_u8("\n".join(lines) + "\n")
+    want = oracle.parse(PET, body)
+    out = (C.c_uint32 * 7)()
+    strs, fast = 0, []
+    for _ in range(3):
+        emu[PET].emu_item_shape(C.c_uint64(10**9), C.c_double(body.size / 500), C.c_double(300), C.c_uint32(280), C.c_uint32(strs), C.c_uint32(0), out)
+        got = Run(emu, PET, body, tile=out[0], slack=out[1] - out[0], str_words=out[2], row_cap=out[3])
+        assert same_result(want, got.cols) == ""
+        strs = got.strs_per_kb
+        fast.append(got.fast)
+    assert fast[0] < 250 and fast[1] == fast[2] == 500, (fast, strs)
 
 
 def test_under_sanitizers():
