@@ -257,6 +257,8 @@ enum {
                                               text as written becomes the string. List elements, enums and date-times are
                                               not coerced                                                                  */
   PJ_OPT_HEX_LOWER = 1u << 3,              /* W3: \u00xx escapes are written with lower-case hex digits                    */
+  PJ_OPT_TEST_RECORDS = 1u << 29, /* test hooks: the context's NDJSON calls all take the parse kernel with a record per thread / the one */
+  PJ_OPT_TEST_ITEMS = 1u << 30,   /* that spreads a tile over strings, instead of the one its earlier calls speak for */
   PJ_OPT_TEST_STALL_ONCE = 1u << 31 /* test hook for the time-out path: in the context's FIRST NDJSON parse call the first
                                        tile is never handed out, so every other tile's bounded wait for it runs out
                                        (after spin_limit_us) and the call answers PJ_ERR_TIMEOUT; later calls are normal */
@@ -300,7 +302,9 @@ typedef struct pj_call_stats {
                                (record count read-back, state reset), [2] the tile kernel; write: [0] state
                                reset and the scan of the string arenas for bytes to escape, [1] the closing
                                kernel, [2] the tile kernel */
-  uint32_t stage_launches[8]; /* kernels launched per stage                                      */
+  uint32_t stage_launches[8]; /* kernels launched per stage; parse: [3] is no stage, but how many of stage 2's
+                                 launches were the kernel that spreads a tile over strings, instead of the
+                                 one with a record per thread                                    */
   uint64_t h2d_bytes;       /* bytes copied host->device by the call                            */
   uint64_t d2h_bytes;       /* bytes copied device->host by the call                            */
   uint64_t algorithmic_bytes; /* input bytes + bytes of every produced column (parse), or column

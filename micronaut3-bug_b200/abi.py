@@ -32,6 +32,8 @@ PJ_GEN_ZIPF_LISTS, PJ_GEN_ESCAPES, PJ_GEN_WHITESPACE, PJ_GEN_MALFORMED, PJ_GEN_A
     1, 2, 4, 8, 16, 32)
 
 PJ_OPT_ENUM_UNKNOWN_AS_NULL, PJ_OPT_LONE_SURROGATE_REPLACE, PJ_OPT_COERCE_SCALARS, PJ_OPT_HEX_LOWER = 1, 2, 4, 8
+PJ_OPT_TEST_RECORDS = 1 << 29
+PJ_OPT_TEST_ITEMS = 1 << 30
 PJ_OPT_TEST_STALL_ONCE = 1 << 31
 
 PJ_MAX_COLS = 64

@@ -24,6 +24,7 @@
 #include "pj_array_kernels.cuh"
 #include "pj_item.cuh"
 #include "pj_item_shape.h"
+#include "pj_choice.h"
 #include "pj_stream_kernel.cuh"
 
 using namespace pj;
@@ -118,9 +119,7 @@ struct pj_ctx {
   double avg_rec_bytes[5] = {0, 0, 0, 0, 0};  /* bytes per record seen per schema (sizes the tiles of the next call) */
   uint32_t max_rec_bytes[5] = {0, 0, 0, 0, 0}; /* bytes of the longest one */
   uint32_t strs_per_kb[5] = {0, 0, 0, 0, 0};   /* strings per 1024 bytes of the tile with the most */
-  /* NDJSON: which kernel the next call takes (use_items()), and how often it changed to k_parse_items */
-  bool items[5] = {false, false, false, false, false};
-  uint8_t to_items[5] = {0, 0, 0, 0, 0};
+  NdChoice choice[5]; /* NDJSON: which kernel the next call takes */
   /* host buffers parsed in pieces: copy streams and one "piece is on the device" event per piece */
   cudaStream_t s_in = nullptr, s_out = nullptr;
   cudaEvent_t ev_in[16] = {};
@@ -319,22 +318,6 @@ uint32_t pick_stream_tile(const pj_ctx* c, uint32_t schema) {
   if (tb > ST_MAX_TILE_BYTES) tb = ST_MAX_TILE_BYTES;
   return (uint32_t)tb;
 }
-/* Which kernel parses the next NDJSON call. A record per thread (k_parse_stream) is the faster one as long as its lockstep pass
- * takes them: with 2 % of the records left to the exact parser every warp has one that the others wait for, and with most of
- * them left to the word-at-a-time tokeniser its threads go separate ways (200k Users with blanks: 360 us, k_parse_items
- * 130 us). k_parse_items takes over then, and hands back when its strict walk took all lines and none is long. Text of one producer keeps its spelling, so the
- * call before says what the next will hold; a stream that changes back and forth stays with k_parse_items, whose time
- * depends on the spelling by a factor of two at most. The result does not depend on the choice. */
-void note_spelling(pj_ctx* c, uint32_t schema, uint64_t records, uint64_t errors, uint64_t fast, uint64_t dense, uint32_t max_rec) {
-  const uint64_t good = records - errors;
-  if (records < 16) return;
-  if (!c->items[schema]) {
-    if (fast * 100 >= good * 98 && dense * 2 >= good) return;
-    c->items[schema] = true;
-    if (c->to_items[schema] < 255) ++c->to_items[schema];
-  } else if (c->to_items[schema] < 2 && dense * 100 >= good * 99 && max_rec <= 1024) c->items[schema] = false;
-}
-
 /* NDJSON: one launch of a parse kernel per piece. Host buffers of a whole stream are parsed in pieces cut after line
  * feeds, so that the copy of piece p+1 to the device, the kernel of piece p and the copy of the columns of piece p-1
  * back run at the same time on three streams. Every launch is enqueued before the host waits for anything: a piece
@@ -404,7 +387,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
 
   uint64_t longest = 0;
   for (int p = 0; p < np; ++p) longest = cut[p + 1] - cut[p] > longest ? cut[p + 1] - cut[p] : longest;
-  const bool items = c->items[schema];
+  const bool items = c->opt_flags & PJ_OPT_TEST_ITEMS ? true : (c->opt_flags & PJ_OPT_TEST_RECORDS ? false : c->choice[schema].items);
   const ItemShape shape = pick_tile_shape(c, schema, longest);
   const uint32_t tile_bytes = items ? shape.tile_bytes : pick_stream_tile(c, schema);
   const size_t state = items ? sizeof(ItemTile) : sizeof(StreamTile);
@@ -472,6 +455,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     PJ_CUDA(c, cudaMemcpyAsync(c->h_res + p, c->d_res + p, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
     PJ_CUDA(c, cudaEventRecord(c->ev_done[p], c->stream));
     count_launch(c, 2);
+    if (items) c->stats.stage_launches[3]++;
     c->stats.tiles += (uint32_t)nt[p];
   }
 
@@ -525,7 +509,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   const pj_status st = finish_columns(c, schema, len, pp, rows_done, n_errors, total, over, out);
   if (st) return st;
   if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; if (items) { c->max_rec_bytes[schema] = max_rec; c->strs_per_kb[schema] = strs_per_kb; } }
-  note_spelling(c, schema, rows_done, n_errors, n_fast, n_dense, max_rec);
+  note_call(c->choice[schema], len, c->stats.stage_ms[2], rows_done, n_errors, n_fast, n_dense, max_rec);
   if (host_out) PJ_CUDA(c, cudaStreamSynchronize(s_out));
   return PJ_OK;
 }
@@ -595,6 +579,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   stage.next(); /* stage 1: set-up */
   PJ_CUDA(c, item_launch(schema, &sa, c->stream));
   count_launch(c, 2);
+  c->stats.stage_launches[3]++;
   stage.next(); /* stage 2: the parse kernel */
   PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));

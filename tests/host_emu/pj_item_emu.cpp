@@ -8,6 +8,7 @@
 #include "pj_block_emu.h"
 #include "pj_item.cuh"
 #include "pj_item_shape.h"
+#include "pj_choice.h"
 
 using namespace pj;
 
@@ -49,6 +50,13 @@ void array_index(const uint8_t* in, uint64_t len, std::vector<uint64_t>& sep, De
 
 extern "C" const char* emu_item_error() { return emu_block::error; }
 extern "C" uint64_t emu_item_barriers() { return emu_block::n_barriers; }
+static NdChoice g_choice;
+extern "C" void emu_choice_reset() { g_choice = NdChoice(); }
+/* the call just made; returns whether the next one takes k_parse_items */
+extern "C" int emu_choice_note(uint64_t len, float ms, uint64_t records, uint64_t errors, uint64_t fast, uint64_t dense, uint32_t max_rec) {
+  note_call(g_choice, len, ms, records, errors, fast, dense, max_rec);
+  return g_choice.items;
+}
 /* out: tile, window, words for strings, rows, bytes of dynamic shared memory, the most that may be, blocks an SM holds */
 extern "C" void emu_item_shape(uint64_t len, double avg, double guess, uint32_t longest, uint32_t strs_per_kb, uint32_t tile_opt, uint32_t* out) {
   const ItemShape s = item_shape(ItemShapeIn{len, avg, guess, longest, strs_per_kb, tile_opt, ItStride<EMU_SCHEMA>::n, 148});

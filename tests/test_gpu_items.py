@@ -4,7 +4,7 @@ import random
 import pytest
 
 from pj_testlib import abi, as_u8, pj, same_result
-from test_gpu_parity import ARRAY, NDJSON, gpu_parse_device
+from test_gpu_parity import ARRAY, NDJSON, gpu_parse_device, gpu_parse_host
 
 pytestmark = pytest.mark.gpu
 
@@ -13,13 +13,16 @@ SPACED = abi.PJ_GEN_WHITESPACE | abi.PJ_GEN_SPARSE
 
 @pytest.fixture(scope="module")
 def items_ctx():
-    """A context whose NDJSON calls have gone over to the kernel for good: its texts changed their spelling twice."""
-    c = pj.Context(device=0)
-    for schema in (1, 2, 3, 4):
-        for flags in (SPACED, 0, SPACED):
-            gpu_parse_device(c, schema, pj.gen_text(schema, 3, 0, 400, flags))
-    yield c
-    c.close()
+    """A context whose NDJSON calls all take the kernel."""
+    with pj.Context(device=0, flags=abi.PJ_OPT_TEST_ITEMS) as c:
+        yield c
+
+
+def parse(ctx, schema, body, framing=NDJSON, offset=0):
+    """gpu_parse_device() by this kernel."""
+    got = gpu_parse_device(ctx, schema, body, framing, offset)
+    assert ctx.stats().stage_launches[3] == ctx.stats().stage_launches[2] > 0
+    return got
 
 
 def corpus(schema, n, kind):
@@ -38,22 +41,67 @@ def corpus(schema, n, kind):
 @pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 2000])
 def test_groups_of_lines(items_ctx, oracle, schema, kind, n):
     body = as_u8(corpus(schema, n, kind))
-    assert same_result(oracle.parse(schema, body, NDJSON), gpu_parse_device(items_ctx, schema, body, NDJSON, n % 16)) == ""
+    assert same_result(oracle.parse(schema, body, NDJSON), parse(items_ctx, schema, body, NDJSON, n % 16)) == ""
 
 
 @pytest.mark.parametrize("n", [1, 32, 257, 3000])
 def test_array_extents(items_ctx, oracle, n):
     body = pj.gen_text(1, 9 + n, 0, n, abi.PJ_GEN_ARRAY | abi.PJ_GEN_ESCAPES)
-    assert same_result(oracle.parse(1, body, ARRAY), gpu_parse_device(items_ctx, 1, body, ARRAY)) == ""
+    assert same_result(oracle.parse(1, body, ARRAY), parse(items_ctx, 1, body, ARRAY)) == ""
 
 
 def test_both_kernels_agree(items_ctx, oracle):
-    """The same text by a new context (a record per thread) and by one that has seen blanks."""
     body = pj.gen_text(4, 21, 0, 5000, 0)
-    fresh = pj.Context(device=0)
     want = oracle.parse(4, body)
-    assert same_result(want, gpu_parse_device(fresh, 4, body)) == "" and same_result(want, gpu_parse_device(items_ctx, 4, body)) == ""
-    fresh.close()
+    with pj.Context(device=0, flags=abi.PJ_OPT_TEST_RECORDS) as records:
+        assert same_result(want, gpu_parse_device(records, 4, body)) == "" and records.stats().stage_launches[3] == 0
+    assert same_result(want, parse(items_ctx, 4, body)) == ""
+
+
+def test_a_new_context_finds_its_kernel(oracle):
+    """The first call takes the kernel with a record per thread; spaced text goes over to the other one, compact text comes back."""
+    took = []
+    with pj.Context(device=0) as c:
+        for flags in (SPACED, SPACED, SPACED, 0, 0, 0):
+            body = pj.gen_text(3, 4, 0, 1000, flags)
+            assert same_result(oracle.parse(3, body), gpu_parse_device(c, 3, body)) == ""
+            took.append(c.stats().stage_launches[3])
+    assert took == [0, 1, 1, 1, 0, 0], took
+
+
+@pytest.mark.parametrize("schema", [1, 2, 3, 4])
+def test_unusual_records(items_ctx, oracle, schema):
+    """Records that stand apart, keys in escapes, strings in another script, lines that end in a string, long records: by the kernel's own steps."""
+    lines = bytes(pj.gen_text(schema, 8, 0, 3000, abi.PJ_GEN_SPARSE)).split(b"\n")[:-1]
+    extra = [b'"x":{"a":[1,2.5]},', b'"\\u0069d":4,', '"y":"\u540d\u524d \\\\",'.encode(), b'"x":1.5,', b'"id":1,', b'"z":"a\\/b",']
+    text = [ln[:1] + extra[i % 6] + ln[1:] if i % 5 == 0 else (ln[: len(ln) // 2] if i % 97 == 0 else ln) for i, ln in enumerate(lines)]
+    text[1500:1500] = [b'{"id":1,"x":"' + b"y" * 90_000 + b'"}', b'{"id":1,"x":["' + b'","'.join([b"u" * 9] * 9000) + b'"]}']
+    for framing, body in ((NDJSON, b"\n".join(text)), (ARRAY, b"[" + b",".join(t for t in text if t.endswith(b"}")) + b"]"), (ARRAY, b"[" + b",".join(lines)), (ARRAY, b"[" + b",".join(lines) + b",] x")):
+        body = as_u8(body)
+        want = oracle.parse(schema, body, framing)
+        for _ in range(2):
+            assert same_result(want, parse(items_ctx, schema, body, framing, 3)) == ""
+
+
+def test_strings_beyond_ascii_and_short_ones_are_the_kernels_own(items_ctx, oracle):
+    keys = ["username", "firstName", "lastName", "email", "password", "phone"]
+    users = "\n".join('{"id":%d,%s}' % (i, ",".join('"%s":"\u0438\u043c\u044f\\n%d"' % (k, i) for k in keys)) for i in range(5000)).encode()
+    pets = "\n".join('{"id":%d,"name":"n","photoUrls":[%s]}' % (i, ",".join('"a%d"' % k for k in range(40))) for i in range(5000)).encode()
+    for schema, body in ((3, as_u8(users)), (1, as_u8(pets))):
+        want = oracle.parse(schema, body)
+        for _ in range(3):
+            assert same_result(want, parse(items_ctx, schema, body)) == ""
+        assert items_ctx.stats().fast_records == want.n_records == 5000  # (from the second call on, where there are more strings than usual)
+
+
+def test_shards_pieces_and_ranges(oracle):
+    """Cut lines, and launches that start from the totals of the one before."""
+    text = as_u8(corpus(4, 4000, "blanks") + b"\n" + corpus(4, 3000, "broken"))
+    want = oracle.parse(4, text)
+    for kw in (dict(host_piece_bytes=50_000), dict(device_piece_bytes=70_001)):
+        with pj.Context(device=0, flags=abi.PJ_OPT_TEST_ITEMS, **kw) as c:
+            got = gpu_parse_host(c, 4, text) if "host_piece_bytes" in kw else gpu_parse_device(c, 4, text)
+            assert same_result(want, got) == "" and c.stats().pieces > 3 and c.stats().stage_launches[3] == c.stats().pieces
 
 
 def test_one_long_record_then_a_call_of_few_tiles(oracle):

@@ -5,12 +5,20 @@ import random
 import numpy as np
 import pytest
 
-from pj_testlib import abi, as_u8, same_result
+from pj_testlib import abi, as_u8, pj, same_result
 from test_gpu_parity import gpu_parse_device, gpu_parse_host
 
 pytestmark = pytest.mark.gpu
 
 PET, MIXED = abi.PJ_SCHEMA_PET, abi.PJ_SCHEMA_MIXED
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    """A context whose calls all take the kernel with a record per thread, which has the warp path: which one another context takes
+    depends on the texts it has seen."""
+    with pj.Context(device=0, flags=abi.PJ_OPT_TEST_RECORDS) as c:
+        yield c
 
 
 def url(rng, n):
@@ -37,6 +45,7 @@ def check(ctx, oracle, schema, lines):
     text = as_u8(("\n".join(lines) + "\n").encode("utf-8", "surrogateescape"))  # \udcXX stands for the raw byte XX
     want = oracle.parse(schema, text)
     assert same_result(want, gpu_parse_device(ctx, schema, text)) == ""
+    assert ctx.stats().wide_records > 0
     assert same_result(want, gpu_parse_host(ctx, schema, text)) == ""
     return want
 

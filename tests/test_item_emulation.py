@@ -340,6 +340,41 @@ def test_lists_of_short_strings_fit_once_seen(emu, oracle):
     assert fast[0] < 250 and fast[1] == fast[2] == 500, (fast, strs)
 
 
+# kinds of text: milliseconds per 19 MB with k_parse_stream / k_parse_items, share of fast and dense records each reports, longest record
+KINDS = {"plain": ((0.050, 1.0, 1.0), (0.062, 1.0, 1.0), 250), "spaced": ((0.195, 1.0, 0.1), (0.089, 1.0, 0.0), 400), "script": ((0.084, 1.0, 0.1), (0.114, 1.0, 1.0), 250),
+         "nested": ((0.340, 0.0, 0.0), (0.740, 0.0, 0.0), 300), "unknown": ((0.344, 0.0, 0.0), (0.130, 1.0, 0.0), 300), "long": ((0.5, 1.0, 0.0), (15.6, 0.0, 0.0), 40000)}
+BEST = {"plain": 0, "spaced": 1, "script": 0, "nested": 0, "unknown": 1, "long": 0}
+
+
+def choose(emu, calls, size=19_000_000):
+    """The kernel each of the calls took: 0 a record per thread, 1 k_parse_items."""
+    lib = emu[PET]
+    lib.emu_choice_reset()
+    took, now = [], 0
+    for kind in calls:
+        took.append(now)
+        (ms, fast, dense), longest = KINDS[kind][now], KINDS[kind][2]
+        n = size // longest
+        now = lib.emu_choice_note(C.c_uint64(size), C.c_float(ms * size / 19e6), C.c_uint64(n), C.c_uint64(0), C.c_uint64(int(n * fast)), C.c_uint64(int(n * dense)), C.c_uint32(longest))
+    return took
+
+
+def test_choice_of_the_kernel(emu):
+    """It settles on the faster kernel for every kind of text, also after other kinds, and text that goes back and forth does not drag it along."""
+    for kind in KINDS:
+        took = choose(emu, [kind] * 500)
+        assert sum(t != BEST[kind] for t in took) <= 10, kind  # of 500
+        assert choose(emu, [kind] * 8)[3:] == [BEST[kind]] * 5, kind
+        for before in KINDS:
+            took = choose(emu, [before] * 6 + [kind] * (12 if (before, kind) != ("nested", "unknown") else 80))  # (those two look the same to k_parse_stream)
+            assert took[-4:] == [BEST[kind]] * 4, (before, kind, took)
+    assert sum(choose(emu, ["long"] * 10)) == 0  # records that fill a window are not even tried
+    took = choose(emu, ["spaced", "plain"] * 200)
+    assert sum(a != b for a, b in zip(took, took[1:])) <= 16
+    assert choose(emu, ["plain", "spaced", "spaced"] + ["plain"] * 100)[-1] == 0  # it does not stay for good
+    assert choose(emu, ["spaced"] * 5, size=20_000) == [0, 1, 1, 1, 1]  # too short to be timed: by the spelling alone
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
