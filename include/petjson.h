@@ -298,8 +298,8 @@ typedef struct pj_call_stats {
   float device_ms;          /* CUDA-event time from first launch to last, on the call's stream  */
   float main_kernel_ms;     /* CUDA-event time of the dominant kernel(s) of the call            */
   float stage_ms[8];        /* CUDA-event time per stage. parse, NDJSON: [2] the parse kernel(s), nothing else
-                               runs; parse, array framing: [0] record index, [1] set-up between the kernels
-                               (record count read-back, state reset), [2] the tile kernel; write: [0] state
+                               runs; parse, array framing: [0] separator index, [1] state reset, [2] the
+                               parse kernel; write: [0] state
                                reset and the scan of the string arenas for bytes to escape, [1] the closing
                                kernel, [2] the tile kernel */
   uint32_t stage_launches[8]; /* kernels launched per stage; parse: [3] is no stage, but how many of stage 2's
@@ -309,7 +309,7 @@ typedef struct pj_call_stats {
   uint64_t d2h_bytes;       /* bytes copied device->host by the call                            */
   uint64_t algorithmic_bytes; /* input bytes + bytes of every produced column (parse), or column
                                  bytes read + JSON bytes written (write)                        */
-  uint64_t fast_records;    /* parse: records decoded by the speculative word-at-a-time pass alone */
+  uint64_t fast_records;    /* parse: records decoded without the exact parser, each by its tile's own steps */
   uint64_t phase_cycles[4]; /* SM cycles summed over the blocks of the tile kernel. parse: staging,
                                tokenising, look-back wait, emission; write: size pass, look-back
                                wait, text into the window, copy-out                              */

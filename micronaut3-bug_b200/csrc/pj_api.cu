@@ -530,8 +530,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   }
   const uint64_t nwords = (len + 63) >> 6;
   const uint64_t atiles = nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1;
-  const size_t off_fn = align_up((atiles + 1) * 4, 256);
-  const size_t off_tin = align_up(off_fn + atiles * sizeof(ArrFn), 256);
+  const size_t off_tin = align_up(atiles * sizeof(ArrFn), 256);
   const size_t off_sep = align_up(off_tin + atiles * sizeof(ArrState), 256);
   const size_t off_end = align_up(off_sep + (nwords + 1) * 8, 256);
   { pj_status st = ensure(c, &c->scratch, off_end + 256); if (st) return st; }
@@ -540,9 +539,9 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   Stage stage(c);
   ArrArgs aa;
   aa.in = d_in; aa.len = len; aa.nwords = nwords;
-  aa.tile_fn = (ArrFn*)((uint8_t*)c->scratch.p + off_fn); aa.tile_in = (ArrState*)((uint8_t*)c->scratch.p + off_tin);
+  aa.tile_fn = (ArrFn*)c->scratch.p; aa.tile_in = (ArrState*)((uint8_t*)c->scratch.p + off_tin);
   aa.sep = (uint64_t*)((uint8_t*)c->scratch.p + off_sep); aa.tile_cnt = nullptr;
-  aa.rec_start = nullptr; aa.rec_end = nullptr; aa.rec_blank = nullptr;
+  aa.rec_start = nullptr;
   aa.cap = 0; aa.goff = 0; aa.ntiles = (uint32_t)atiles; aa.res = c->d_res;
   /* the two running minima start at "none" */
   PJ_CUDA(c, cudaMemsetAsync(&c->d_res->doc_err_off, 0xFF, sizeof(unsigned long long), c->stream));
@@ -835,7 +834,7 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
     aa.in = d_in; aa.len = len; aa.nwords = nwords;
     aa.tile_fn = (ArrFn*)((uint8_t*)c->scratch.p + off_fn); aa.tile_in = (ArrState*)((uint8_t*)c->scratch.p + off_tin);
     aa.sep = (uint64_t*)((uint8_t*)c->scratch.p + off_sep); aa.tile_cnt = d_tile;
-    aa.rec_start = d_rs; aa.rec_end = nullptr; aa.rec_blank = nullptr; /* an index-only call keeps the starts alone */
+    aa.rec_start = d_rs;
     aa.cap = cap; aa.goff = 0; aa.ntiles = (uint32_t)atiles; aa.res = c->d_res;
     PJ_CUDA(c, cudaMemsetAsync(&c->d_res->doc_err_off, 0xFF, sizeof(unsigned long long), c->stream));
     PJ_CUDA(c, cudaMemsetAsync(&c->d_res->first_opener, 0xFF, sizeof(unsigned long long), c->stream));

@@ -7,7 +7,7 @@
  *   k_arr_mark      re-evaluates every word with its exact incoming state (ordered scan inside the block),
  *                   writes the separator bitmap, finds the first opener and the first stray byte
  *   k_arr_records<> one candidate per separator: extent, blank test, keep / drop; count per tile, then
- *                   (after a scan) store rec_start / rec_end / rec_blank
+ *                   (after a scan) store rec_start
  */
 #ifndef PJ_ARRAY_KERNELS_CUH
 #define PJ_ARRAY_KERNELS_CUH
@@ -27,8 +27,6 @@ struct ArrArgs {
   uint64_t* sep;       /* [nwords] separator bitmap */
   uint32_t* tile_cnt;  /* [tiles + 1] */
   uint64_t* rec_start; /* outputs of k_arr_records<true> */
-  uint64_t* rec_end;
-  uint8_t* rec_blank;
   uint64_t cap, goff;
   uint32_t ntiles;
   DevResult* res;
@@ -180,8 +178,6 @@ __global__ void __launch_bounds__(ARR_THREADS) k_arr_records(const __grid_consta
     if (!x.is_record) continue;
     if (at < a.cap) {
       a.rec_start[at] = x.start + a.goff;
-      if (a.rec_end) a.rec_end[at] = x.end;
-      if (a.rec_blank) a.rec_blank[at] = (uint8_t)x.blank;
     }
     at++;
   }

@@ -5,7 +5,7 @@
  * One thread block = one tile of the input, staged in shared memory by one bulk copy. A tile owns the lines (in array
  * framing: the extents) whose preceding separator lies in it and follows its last one to its end. The steps:
  *
- *  1. item_index: 32 bytes per thread. Byte-parallel masks of quotes and control characters give the positions of all
+ *  1. item_index: 144 bytes per thread. Byte-parallel masks of quotes and control characters give the positions of all
  *     quotes of the tile in order: string k = (open, close); and the lines: first byte and first string. Backslashes, bytes
  *     beyond ASCII and control characters take extra work only where they are; strings with escapes are decoded in place.
  *  2. item_walk: one line per thread. A record as a serialiser writes it is walked property by property; every string's end

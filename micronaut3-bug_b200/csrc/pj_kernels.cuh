@@ -1,7 +1,8 @@
 /*
  * pj_kernels.cuh — sm_100a kernels of the record index, the writer and the checksums.
  *
- * JSON is parsed by k_parse_items (pj_item.cuh), which builds its own line index. This header holds
+ * JSON is parsed by k_parse_stream (pj_stream_kernel.cuh) and k_parse_items (pj_item.cuh), which build their own line index. This
+ * header holds
  *   - the NDJSON record index on its own (k_nd_index<false> / k_scan_single / k_nd_index<true>: pj_index_records and
  *     its allocation-free variant);
  *   - the writer: columns --k_arena_flags--> "any byte to escape?" --k_write_tile--> text --k_write_close--> brackets, total.

@@ -1,8 +1,9 @@
 /*
  * pj_stream_kernel.cuh — k_parse_stream<SCHEMA>: NDJSON bytes to typed columns in ONE kernel and one pass over HBM, a record
  * per thread. It is the faster one for records all spelled the way a compact serialiser spells them, where the threads of a
- * warp stay together (1M Pets 600 us, k_parse_items 625 us); with blanks or long lists they do not (200k Users with blanks
- * 360 us against 130 us, long lists 44 ms against 4 ms), and pj_api.cu then takes k_parse_items (pj_item.cuh).
+ * warp stay together (1M Pets 600 us, k_parse_items 625 us); with blanks or long lists they do not (100k Users with blanks
+ * 195 us against 89 us, 20k Pets with long lists 7.9 ms against 0.87 ms), and note_call() (pj_choice.h) then tries k_parse_items
+ * (pj_item.cuh).
  *
  * One thread block = one tile of the input (pj_stream.cuh): the tile and what follows it are staged in shared memory
  * by one bulk copy (cp.async.bulk, the untiled TMA form, no multicast), the block builds the line index of the window

@@ -98,7 +98,7 @@ def test_shards_pieces_and_ranges(oracle):
     """Cut lines, and launches that start from the totals of the one before."""
     text = as_u8(corpus(4, 4000, "blanks") + b"\n" + corpus(4, 3000, "broken"))
     want = oracle.parse(4, text)
-    for kw in (dict(host_piece_bytes=50_000), dict(device_piece_bytes=70_001)):
+    for kw in (dict(host_piece_bytes=50_000), dict(device_piece_bytes=150_001)):
         with pj.Context(device=0, flags=abi.PJ_OPT_TEST_ITEMS, **kw) as c:
             got = gpu_parse_host(c, 4, text) if "host_piece_bytes" in kw else gpu_parse_device(c, 4, text)
             assert same_result(want, got) == "" and c.stats().pieces > 3 and c.stats().stage_launches[3] == c.stats().pieces
