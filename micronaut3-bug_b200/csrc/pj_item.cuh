@@ -146,7 +146,7 @@ struct ItemShared {
   uint32_t nstr, nline, stop;              /* strings, lines, last separator */
   uint32_t free_word;                      /* first free word behind the strings */
   uint32_t ndense;                         /* lines the dense walk took */
-  uint32_t ok, slow, tile, next;
+  uint32_t ok, slow, tile, next, apart;    /* apart: a record of the tile stands apart */
   unsigned long long mbar;
 };
 
@@ -1044,6 +1044,10 @@ __device__ __forceinline__ void item_walk_model(ItemWalk& f, uint32_t* row, uint
   if constexpr (DENSE) f.ok = f.ok && f.k == f.kend && f.win[f.p] == '}' && f.p + 1u == f.sep;
   else f.ok = f.ok && f.k == f.kend && !f.open && item_only_blanks(f.win, f.p + 1u, f.sep);
 }
+/* is the line at input offset s0, which runs out of the window, a record? */
+static __device__ __noinline__ bool item_long_is_record(const ItemArgs& a, uint64_t s0) {
+  return a.sep ? arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener).is_record != 0 : nd_is_record(a.in, s0, a.limit, (int)a.is_last);
+}
 /* One line: its row, or IF_ODD there. */
 template <int SCHEMA, bool ARR, bool DENSE>
 __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, uint32_t* rows, uint32_t i, uint32_t type) {
@@ -1064,13 +1068,7 @@ __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGe
   const bool long_line = sh.open_end && i + 1u == sh.nline;
   if (ARR && before == ']') f.p = start;
   else if (long_line) {
-    const uint64_t s0 = g.v0 + start - g.mis;
-    bool record;
-    if constexpr (ARR) {
-      const ExtentOut x = arr_extent(a.in, a.len, a.sep, s0 - 1u, a.res->first_opener);
-      record = x.is_record;
-    } else record = nd_is_record(a.in, s0, a.limit, (int)a.is_last);
-    if (record) { flags = IF_RECORD; err = (start << 8) | IE_REFUSED; }
+    if (item_long_is_record(a, g.v0 + start - g.mis)) { flags = IF_RECORD; err = (start << 8) | IE_REFUSED; }
   } else if (f.k == f.kend) { /* no string */
     uint32_t p = start;
     while (p < f.sep && item_blank(win[p])) ++p;
@@ -1772,8 +1770,7 @@ __device__ __forceinline__ void item_emit_fixed(const ItemArgs& a, const ItemOut
     item_emit_fixed<OBJ, ROOT, WORD0, BIT0, I + 1>(a, o);
   }
 }
-/* (What is called out of line takes its ItemOut by value: the callers' stay in registers.) string columns of root or embedded object OBJ (every lane of the warp calls this). APART: some of the records stand apart; groups without one
- * do not pay for it (100k Users in an array: 69 us with the loop over runs in every group, 62 us without). */
+/* string columns of root or embedded object OBJ (every lane of the warp calls this). APART: some of the tile's records stand apart */
 template <bool APART, int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
 __device__ __forceinline__ void item_emit_strings(const ItemArgs& a, const ItemShared& sh, const ItemOut& o) {
   if constexpr (I < CObj<OBJ>::N) {
@@ -1797,12 +1794,6 @@ __device__ __forceinline__ void item_emit_strings(const ItemArgs& a, const ItemS
     } else if constexpr (kind == K_OBJ) item_emit_strings<APART, MODEL, CObj<OBJ>::f[I].child, false, ItModel<OBJ>::child_word, IB_CHILD>(a, sh, o);
     item_emit_strings<APART, MODEL, OBJ, ROOT, WORD0, BIT0, I + 1>(a, sh, o);
   }
-}
-template <int MODEL>
-__device__ __noinline__ void item_emit_strings_apart(const ItemArgs& a, const ItemShared& sh, const ItemOut o) { item_emit_strings<true, MODEL, MODEL, true, 0u, 0u>(a, sh, o); }
-template <int MODEL>
-__device__ __forceinline__ void item_emit_strings_of(const ItemArgs& a, const ItemShared& sh, const ItemOut& o) {
-  if (o.apart) item_emit_strings_apart<MODEL>(a, sh, o); else item_emit_strings<false, MODEL, MODEL, true, 0u, 0u>(a, sh, o);
 }
 /* bytes of the lines' strings per slot, added up over the warp into csum[slot][chunk] */
 template <int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
@@ -1862,13 +1853,6 @@ __device__ __forceinline__ void item_emit_lists(const ItemArgs& a, const ItemSha
     });
   }
 }
-template <bool OBJS>
-__device__ __noinline__ void item_emit_lists_apart(const ItemArgs& a, const ItemShared& sh, const ItemOut o, const uint32_t* pairs, bool mine) { item_emit_lists<true, OBJS>(a, sh, o, pairs, mine); }
-template <bool OBJS>
-__device__ __forceinline__ void item_emit_lists_of(const ItemArgs& a, const ItemShared& sh, const ItemOut& o, const uint32_t* pairs, bool mine) {
-  if (o.apart) item_emit_lists_apart<OBJS>(a, sh, o, pairs, mine); else item_emit_lists<false, OBJS>(a, sh, o, pairs, mine);
-}
-
 /* ---- the exact parser -------------------------------------------------------------------------------------------- */
 
 __device__ __forceinline__ Rd item_reader(const ItemArgs& a, const uint8_t* in, uint64_t limit) {
@@ -1943,18 +1927,31 @@ __device__ __noinline__ void item_place(const ItemArgs& a, const ItemText t, uin
   s.p = t.start; s.err = 0; s.err_pos = 0;
   parse_record<true>(c_schema, item_reader(a, t.in, t.limit), s, (uint32_t)SCHEMA, o, n);
 }
-/* A record the own steps refused: kind and offset of its failure in *err, *off. *err = 0: it is a valid one after all, of the model returned
- * (| 256: by the word-at-a-time tokeniser), and its row holds what it adds to that model's counters. */
+/* Line ln, a record the own steps refused: its row says how it failed or, if it is a valid one after all, that it stands apart (IF_ROWS: by the
+ * word-at-a-time tokeniser), and what it adds to its model's counters. */
 template <int SCHEMA>
-__device__ __forceinline__ uint32_t item_judge(const ItemArgs& a, const ItemText& t, uint32_t* err, uint32_t* off, uint32_t* row) {
+__device__ __noinline__ void item_judge(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, uint32_t* row, uint32_t ln) {
   ItemSize r;
-  item_size<SCHEMA>(a, t, &r);
-  *err = r.err; *off = r.off;
-  if (r.err) return PJ_TYPE_NONE;
+  item_size<SCHEMA>(a, item_text(a, g, sh, win, ln), &r);
+  row[IW_ERR] = r.err;
+  if (r.err) { row[IW_FLAGS] = IF_BAD | IF_RECORD; row[IW_LIST] = r.off; return; }
   const uint32_t slot0 = r.type == PJ_TYPE_USER ? ItSlot0<OBJ_USER>::n : ItSlot0<OBJ_PET>::n;
   if (r.type != PJ_TYPE_ORDER) for (uint32_t j = 0; j < IT_APART; ++j) row[IW_FIELDS + j] = r.cnt[slot0 + j];
   if constexpr (ItemSlots<SCHEMA>::lists) { row[IW_LIST] = 0; row[ItWords<OBJ_PET>::n] = 0; row[ItWords<OBJ_PET>::n + 1u] = 0; }
-  return r.type | (r.fast << 8);
+  row[IW_FLAGS] = IF_APART | IF_RECORD | (r.fast ? IF_ROWS : 0u) | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (r.type - 1u)) & 7u) << IF_NOTMODEL : 0u);
+  sh.apart = 1;
+}
+/* what the records of a warp's lines that stand apart add to the sums of its group */
+template <int SCHEMA>
+__device__ __noinline__ void item_sum_apart(ItemShared& sh, const uint32_t* row, bool apart, uint32_t type) {
+#pragma unroll 1
+  for (uint32_t j = 0; j < 2u * IT_APART; ++j) {
+    const uint32_t slot = (uint32_t)SLOT_PET_CAT_NAME + j;
+    const bool pet = j < IT_APART;
+    if (!((ItemSlots<SCHEMA>::mask >> slot) & 1u)) continue;
+    const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, apart && type == (pet ? (uint32_t)PJ_TYPE_PET : (uint32_t)PJ_TYPE_USER) ? row[IW_FIELDS + (pet ? j : j - IT_APART)] : 0u);
+    if ((threadIdx.x & 31u) == 0) sh.csum[slot][threadIdx.x >> 5] += s;
+  }
 }
 /* what a record that does not stand apart adds to its model's counters */
 template <int MODEL, int OBJ, bool ROOT, uint32_t WORD0, uint32_t BIT0, int I = 0>
@@ -2089,6 +2086,86 @@ __device__ __noinline__ void item_slow_tile(const ItemArgs& a, const StreamGeom&
   if (tile == a.ntiles - 1) item_close_offsets(a, sh, tid);
 }
 
+/* The columns of a tile that knows its place: four kinds of them x groups of 32 lines. APART: records stand apart; a version of its own, out of
+ * line, because tiles without one paid for it: with one version for both the kernel spilled 1140 bytes per thread instead of 120 and 200k Users
+ * with blanks took 140 us instead of 129, 100k Users in an array 70 instead of 61. */
+template <int SCHEMA, bool APART>
+__device__ __forceinline__ void item_emit_tile(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, const uint32_t* rows) {
+  using SL = ItemSlots<SCHEMA>;
+  constexpr uint32_t STRIDE = ItStride<SCHEMA>::n;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nline = sh.nline, nchunk = (nline + 31u) >> 5;
+  for (uint32_t u = warp; u < 4u * nchunk; u += IT_WARPS) {
+    /* groups differ in cost (mixed streams: by model) as well as kinds: a warp gets another group of each kind */
+    const uint32_t what = u / nchunk, c = (u + what) % nchunk, i = c * 32u + lane;
+    const uint32_t ln = i < nline ? (SCHEMA == PJ_SCHEMA_MIXED ? (uint32_t)sh.perm[i] : i) : 0u;
+    const uint32_t* r = rows + ln * STRIDE;
+    ItemOut o;
+    o.win = win; o.row = r; o.chunk = c; o.stage = sh.stage[warp]; o.owner = sh.owner[warp]; o.moved = sh.nspecial ? sh.special : nullptr;
+    const uint32_t f = i < nline ? r[IW_FLAGS] : 0u;
+    const bool rec = (f & IF_RECORD) != 0, good = rec && !(f & IF_BAD);
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint64_t n = (uint64_t)sh.base[IT_REC] + sh.csum[IT_REC][ln >> 5] + (uint32_t)__popc(sh.recs[ln >> 5] & ((1u << (ln & 31u)) - 1u));
+    const uint32_t type = good ? item_type<SCHEMA>(f) : (uint32_t)PJ_TYPE_NONE;
+    const bool apart = APART && good && (f & IF_APART);
+    o.flags = good && !apart ? f : 0u;
+    o.apart = APART ? __ballot_sync(0xFFFFFFFFu, apart) : 0u;
+    o.at = n;
+    uint32_t bp = 0, bo = 0, bu = 0;
+    if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+      bp = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_PET); bo = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_ORDER); bu = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_USER);
+      const uint32_t mine = type == PJ_TYPE_PET ? bp : (type == PJ_TYPE_ORDER ? bo : bu);
+      const uint32_t slot = type == PJ_TYPE_PET ? SLOT_ROWS_PET : (type == PJ_TYPE_ORDER ? SLOT_ROWS_ORD : SLOT_ROWS_USR);
+      o.at = sh.base[slot] + sh.csum[slot][c] + (uint32_t)__popc(mine & lt);
+    }
+    if (what == 3u) {
+      const uint32_t bg = __ballot_sync(0xFFFFFFFFu, good), br = __ballot_sync(0xFFFFFFFFu, rec);
+      if (lane == 0) {
+        if (br != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(br & ~bg));
+        if (bg & ~o.apart) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg & ~o.apart));
+      }
+      if (APART && o.apart) item_emit_apart<SCHEMA>(a, g, sh, win, r, f, type, ln, c, n, o.at);
+      if (rec) {
+        colp<uint64_t>(&a.cols, PJ_COL_REC_START)[n] = a.goff + g.v0 + (r[IW_POS] & 0xFFFFu) - g.mis;
+        colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[n] = good ? 0 : (uint8_t)r[IW_ERR];
+        colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[n] = good ? 0u : r[IW_LIST];
+        if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+          colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[n] = (uint8_t)type;
+          colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[n] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : (uint32_t)o.at;
+        }
+      }
+      if (rec && !apart) {
+        if constexpr (SCHEMA == PJ_SCHEMA_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
+        else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
+        else if constexpr (SCHEMA == PJ_SCHEMA_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
+        else {
+          if (type == PJ_TYPE_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
+          else if (type == PJ_TYPE_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
+          else if (type == PJ_TYPE_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
+        }
+      }
+    } else if (what == 2u) {
+      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings<APART, OBJ_PET, OBJ_PET, true, 0u, 0u>(a, sh, o); }
+      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings<APART, OBJ_USER, OBJ_USER, true, 0u, 0u>(a, sh, o); }
+      else if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+        const uint32_t apart_all = o.apart;
+        o.has_row = type == PJ_TYPE_PET; o.apart = apart_all & bp;
+        if (bp) item_emit_strings<APART, OBJ_PET, OBJ_PET, true, 0u, 0u>(a, sh, o);
+        o.has_row = type == PJ_TYPE_USER; o.apart = apart_all & bu;
+        if (bu) item_emit_strings<APART, OBJ_USER, OBJ_USER, true, 0u, 0u>(a, sh, o);
+      }
+    } else if constexpr (SL::lists) {
+      const bool pet = type == PJ_TYPE_PET;
+      o.has_row = SCHEMA == PJ_SCHEMA_PET ? rec : pet;
+      if constexpr (SCHEMA == PJ_SCHEMA_MIXED) o.apart &= bp;
+      if (SCHEMA == PJ_SCHEMA_PET || bp) { if (what == 0u) item_emit_lists<APART, false>(a, sh, o, pairs, pet); else item_emit_lists<APART, true>(a, sh, o, pairs, pet); }
+    }
+  }
+}
+template <int SCHEMA>
+__device__ __noinline__ void item_emit_tile_apart(const ItemArgs& a, const StreamGeom& g, ItemShared& sh, const uint8_t* win, const uint32_t* pairs, const uint32_t* rows) {
+  item_emit_tile<SCHEMA, true>(a, g, sh, win, pairs, rows);
+}
+
 /* ---- a tile ------------------------------------------------------------------------------------------------------ */
 /* Steps 2 to 5 of a tile whose index stands. False (for every thread): the other road; nothing was published. */
 template <int SCHEMA, bool ARR>
@@ -2161,20 +2238,13 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
         if (((flags >> IF_PRESENT) & req) != req) e = ((row[IW_POS] >> 16) << 8) | (uint32_t)PJ_E_REQUIRED;
       }
     }
-    bool good = rec && e == IE_NONE;
-    if (rec && !good) {
-      uint32_t kind = e & 0xFFu, off = (e >> 8) - (row[IW_POS] & 0xFFFFu), apart_flags = IF_APART | IF_RECORD;
-      if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) {
-        type = item_judge<SCHEMA>(a, item_text(a, g, sh, win, tid), &kind, &off, row);
-        if (type >> 8) apart_flags |= IF_ROWS;
-        type &= 255u;
-        good = !kind; /* a valid record of a kind the other steps do not know */
-      }
-      flags = good ? apart_flags | (SCHEMA == PJ_SCHEMA_MIXED ? (~(1u << (type - 1u)) & 7u) << IF_NOTMODEL : 0u) : IF_BAD | IF_RECORD;
-      row[IW_FLAGS] = flags; row[IW_ERR] = kind;
-      if (!good) row[IW_LIST] = off;
-    }
-    if (!good) type = PJ_TYPE_NONE;
+    if (rec && e != IE_NONE) {
+      const uint32_t kind = e & 0xFFu;
+      if ((flags & IF_MOVED) || kind == IE_REFUSED || ((a.opts & PJ_OPT_COERCE_SCALARS) && kind == PJ_E_TYPE)) item_judge<SCHEMA>(a, g, sh, win, row, tid);
+      else { row[IW_FLAGS] = IF_BAD | IF_RECORD; row[IW_ERR] = kind; row[IW_LIST] = (e >> 8) - (row[IW_POS] & 0xFFFFu); }
+      flags = row[IW_FLAGS];
+      type = flags & IF_BAD ? (uint32_t)PJ_TYPE_NONE : item_type<SCHEMA>(flags);
+    } else if (!rec) type = PJ_TYPE_NONE;
     const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, rec ? (sh.line[tid + 1u] & 0xFFFFu) - (row[IW_POS] & 0xFFFFu) : 0u);
     if (lane == 0 && most > *(volatile uint32_t*)&a.res->max_rec) atomicMax(&a.res->max_rec, most); /* (seldom more than a few times) */
     const uint32_t br = __ballot_sync(0xFFFFFFFFu, rec);
@@ -2204,16 +2274,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
     }
     if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) item_sum_strings<OBJ_USER, true, 0u, 0u>(sh, row, type == PJ_TYPE_USER, flags, warp, lane);
     const bool apart = tid < nline && (flags & IF_APART);
-    if (__any_sync(0xFFFFFFFFu, apart)) {
-#pragma unroll 1
-      for (uint32_t j = 0; j < 2u * IT_APART; ++j) {
-        const uint32_t slot = (uint32_t)SLOT_PET_CAT_NAME + j;
-        const bool pet = j < IT_APART;
-        if (!((SL::mask >> slot) & 1u)) continue;
-        const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, apart && type == (pet ? (uint32_t)PJ_TYPE_PET : (uint32_t)PJ_TYPE_USER) ? row[IW_FIELDS + (pet ? j : j - IT_APART)] : 0u);
-        if (lane == 0) sh.csum[slot][warp] += s;
-      }
-    }
+    if (__any_sync(0xFFFFFFFFu, apart)) item_sum_apart<SCHEMA>(sh, row, apart, type);
   }
   __syncthreads();
   ck[3] = clock64();
@@ -2241,72 +2302,7 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
   if (!sh.ok) return true;
 
   /* ---- emission: four kinds of columns x groups of 32 lines ---- */
-  for (uint32_t u = warp; u < 4u * nchunk; u += IT_WARPS) {
-    /* groups differ in cost (mixed streams: by model) as well as kinds: a warp gets another group of each kind */
-    const uint32_t what = u / nchunk, c = (u + what) % nchunk, i = c * 32u + lane;
-    const uint32_t ln = i < nline ? (SCHEMA == PJ_SCHEMA_MIXED ? (uint32_t)sh.perm[i] : i) : 0u;
-    const uint32_t* r = rows + ln * STRIDE;
-    ItemOut o;
-    o.win = win; o.row = r; o.chunk = c; o.stage = sh.stage[warp]; o.owner = sh.owner[warp]; o.moved = sh.nspecial ? sh.special : nullptr;
-    const uint32_t f = i < nline ? r[IW_FLAGS] : 0u;
-    const bool rec = (f & IF_RECORD) != 0, good = rec && !(f & IF_BAD);
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint64_t n = (uint64_t)sh.base[IT_REC] + sh.csum[IT_REC][ln >> 5] + (uint32_t)__popc(sh.recs[ln >> 5] & ((1u << (ln & 31u)) - 1u));
-    const uint32_t type = good ? item_type<SCHEMA>(f) : (uint32_t)PJ_TYPE_NONE;
-    o.flags = good && !(f & IF_APART) ? f : 0u;
-    const bool apart = good && (f & IF_APART);
-    o.apart = __ballot_sync(0xFFFFFFFFu, apart);
-    o.at = n;
-    uint32_t bp = 0, bo = 0, bu = 0;
-    if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
-      bp = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_PET); bo = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_ORDER); bu = __ballot_sync(0xFFFFFFFFu, type == PJ_TYPE_USER);
-      const uint32_t mine = type == PJ_TYPE_PET ? bp : (type == PJ_TYPE_ORDER ? bo : bu);
-      const uint32_t slot = type == PJ_TYPE_PET ? SLOT_ROWS_PET : (type == PJ_TYPE_ORDER ? SLOT_ROWS_ORD : SLOT_ROWS_USR);
-      o.at = sh.base[slot] + sh.csum[slot][c] + (uint32_t)__popc(mine & lt);
-    }
-    if (what == 3u) {
-      const uint32_t bg = __ballot_sync(0xFFFFFFFFu, good), br = __ballot_sync(0xFFFFFFFFu, rec);
-      if (lane == 0) {
-        if (br != bg) atomicAdd(&a.res->n_errors, (unsigned long long)__popc(br & ~bg));
-        if (bg & ~o.apart) atomicAdd(&a.res->n_fast, (unsigned long long)__popc(bg & ~o.apart));
-      }
-      if (o.apart) item_emit_apart<SCHEMA>(a, g, sh, win, r, f, type, ln, c, n, o.at);
-      if (rec) {
-        colp<uint64_t>(&a.cols, PJ_COL_REC_START)[n] = a.goff + g.v0 + (r[IW_POS] & 0xFFFFu) - g.mis;
-        colp<uint8_t>(&a.cols, PJ_COL_ERR_KIND)[n] = good ? 0 : (uint8_t)r[IW_ERR];
-        colp<uint32_t>(&a.cols, PJ_COL_ERR_OFF)[n] = good ? 0u : r[IW_LIST];
-        if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
-          colp<uint8_t>(&a.cols, PJ_COL_REC_TYPE)[n] = (uint8_t)type;
-          colp<uint32_t>(&a.cols, PJ_COL_REC_ROW)[n] = type == PJ_TYPE_NONE ? 0xFFFFFFFFu : (uint32_t)o.at;
-        }
-      }
-      if (rec && !apart) {
-        if constexpr (SCHEMA == PJ_SCHEMA_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
-        else if constexpr (SCHEMA == PJ_SCHEMA_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
-        else if constexpr (SCHEMA == PJ_SCHEMA_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
-        else {
-          if (type == PJ_TYPE_PET) item_emit_fixed<OBJ_PET, true, 0u, 0u>(a, o);
-          else if (type == PJ_TYPE_ORDER) item_emit_fixed<OBJ_ORDER, true, 0u, 0u>(a, o);
-          else if (type == PJ_TYPE_USER) item_emit_fixed<OBJ_USER, true, 0u, 0u>(a, o);
-        }
-      }
-    } else if (what == 2u) {
-      if constexpr (SCHEMA == PJ_SCHEMA_PET) { o.has_row = rec; item_emit_strings_of<OBJ_PET>(a, sh, o); }
-      else if constexpr (SCHEMA == PJ_SCHEMA_USER) { o.has_row = rec; item_emit_strings_of<OBJ_USER>(a, sh, o); }
-      else if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
-        const uint32_t apart_all = o.apart;
-        o.has_row = type == PJ_TYPE_PET; o.apart = apart_all & bp;
-        if (bp) item_emit_strings_of<OBJ_PET>(a, sh, o);
-        o.has_row = type == PJ_TYPE_USER; o.apart = apart_all & bu;
-        if (bu) item_emit_strings_of<OBJ_USER>(a, sh, o);
-      }
-    } else if constexpr (SL::lists) {
-      const bool pet = type == PJ_TYPE_PET;
-      o.has_row = SCHEMA == PJ_SCHEMA_PET ? rec : pet;
-      if constexpr (SCHEMA == PJ_SCHEMA_MIXED) o.apart &= bp;
-      if (SCHEMA == PJ_SCHEMA_PET || bp) { if (what == 0u) item_emit_lists_of<false>(a, sh, o, pairs, pet); else item_emit_lists_of<true>(a, sh, o, pairs, pet); }
-    }
-  }
+  if (sh.apart) item_emit_tile_apart<SCHEMA>(a, g, sh, win, pairs, rows); else item_emit_tile<SCHEMA, false>(a, g, sh, win, pairs, rows);
   if (tile == a.ntiles - 1) item_close_offsets(a, sh, tid);
   return true;
 }
@@ -2333,7 +2329,7 @@ __global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __g
   uint32_t* strs = reinterpret_cast<uint32_t*>(smem + lay.strs);
   uint32_t* rows = reinterpret_cast<uint32_t*>(smem + lay.rows);
 
-  if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); mbar_init(&sh.mbar, 1); sh.slow = 0; sh.next = 0; sh.odd = 0; sh.nspecial = 0; }
+  if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); mbar_init(&sh.mbar, 1); sh.slow = 0; sh.next = 0; sh.odd = 0; sh.nspecial = 0; sh.apart = 0; }
   __syncthreads();
   const uint32_t tile = sh.tile;
   if (tile >= a.ntiles) return;
