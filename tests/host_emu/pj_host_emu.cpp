@@ -1,8 +1,8 @@
 /*
  * pj_host_emu.cpp — TEST INFRASTRUCTURE. Compiles the per-record device code of the library
  * (pj_core.cuh, pj_fast.cuh, pj_write_core.cuh, pj_write_fast.cuh, pj_array.cuh: every function in them is
- * host + device) for the host and runs it one "thread" after another, with the tile kernel's bookkeeping
- * (windows, tapes, tile-local scans) restated sequentially. tests/test_host_emulation.py fuzzes it against
+ * host + device) for the host and runs it one "thread" after another, with a tile's bookkeeping
+ * (windows, tapes, tile-local scans) restated sequentially. (Whole blocks of k_parse_items run in pj_item_emu.cpp.) tests/test_host_emulation.py fuzzes it against
  * the CPU checker, so the exactness of the device-side parsers and writers is tested without a GPU.
  * Nothing in the product links or loads this file.
  */

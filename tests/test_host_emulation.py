@@ -55,7 +55,7 @@ def extents(oracle, buf):
 
 
 def emu_parse_tiles(emu, oracle, schema, buf, framing=NDJSON, tile=128, win=45056, tape=20, lock=False, opts=0):
-    """The tile kernel's per-record work on the host: windows of `win` bytes, tapes of `tape` words, `tile` records a tile.
+    """The per-record work of the record-per-thread kernel (and, read where they lie, of k_parse_items' lines) on the host: windows of `win` bytes, tapes of `tape` words, `tile` records a tile.
     lock: the lockstep tokeniser (pj_lock.cuh) gets the first try at every staged NDJSON record, as in the stream kernel."""
     emu.emu_use_lock(1 if lock else 0)
     emu.emu_set_options(u32(opts))
