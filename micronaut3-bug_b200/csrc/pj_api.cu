@@ -25,6 +25,7 @@
 #include "pj_item.cuh"
 #include "pj_item_shape.h"
 #include "pj_choice.h"
+#include "pj_write_shape.h"
 #include "pj_stream_kernel.cuh"
 
 using namespace pj;
@@ -710,10 +711,10 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   if (e == cudaSuccess) e = stream_init_2(&c->schema);
   if (e == cudaSuccess) e = stream_init_3(&c->schema);
   if (e == cudaSuccess) e = stream_init_4(&c->schema);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, WTILE_SMEM_BYTES);
-#ifdef PJ_WT_CARVEOUT
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile, cudaFuncAttributePreferredSharedMemoryCarveout, PJ_WT_CARVEOUT);
-#endif
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_PET>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_USER>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
   if (e != cudaSuccess) return fail_create(e, "cudaFuncSetAttribute");
   *out = c;
   return PJ_OK;
@@ -961,58 +962,61 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
     if (st) return st;
     d_out = (uint8_t*)c->out_stage.p;
   }
-  DevResult init;
-  memset(&init, 0, sizeof init);
-  init.n_records = n;
-  init.ok = 1;
-  *c->h_res = init;
-  PJ_CUDA(c, cudaMemcpyAsync(c->d_res, c->h_res, sizeof(DevResult), cudaMemcpyHostToDevice, c->stream));
   WriteArgs wa;
   wa.n = n; wa.schema = schema; wa.array = framing == PJ_FRAMING_ARRAY; wa.inclusion = c->inclusion;
   wa.hexa = (c->opt_flags & PJ_OPT_HEX_LOWER) ? 'a' : 'A';
   wa.out = d_out; wa.cap = cap; wa.res = c->d_res; wa.cols = dcols;
-  {
-    /* the single-pass tile writer; stages: [0] state reset and the look at the string arenas, [1] the closing kernel, [2] the tile kernel */
-    const uint64_t ntiles = n ? (n + WT_THREADS - 1) / WT_THREADS : 1;
-    { pj_status st = ensure(c, &c->tiles, 256 + ntiles * 16 + 256); if (st) return st; }
-    WTileArgs ta;
-    ta.w = wa;
-    ta.ticket = (uint32_t*)c->tiles.p;
-    ta.agg = (unsigned long long*)((uint8_t*)c->tiles.p + 256);
-    ta.inc = ta.agg + ntiles;
-    ta.ntiles = (uint32_t)ntiles;
-    ta.spin_limit_ns = c->spin_ns;
-    /* the string arenas of the schema */
-    ArenaArgs aa;
-    memset(&aa, 0, sizeof aa);
-    aa.res = c->d_res;
-    auto add_arenas = [&](const ObjDesc& O, auto&& self) -> void {
-      for (int i = 0; i < (int)O.nfields; ++i) {
-        const FieldDesc& F = O.f[i];
-        int col = -1;
-        if (F.kind == K_STR) col = F.col + 1;
-        else if (F.kind == K_LIST_STR) col = F.col + 2;
-        else if (F.kind == K_OBJ || F.kind == K_LIST_OBJ) self(c->schema.obj[F.child], self);
-        if (col >= 0 && cols->col[col].count && aa.count < 12) { aa.p[aa.count] = (const uint8_t*)dcols.ptr[col]; aa.n[aa.count] = cols->col[col].count; aa.count++; }
-      }
-    };
-    if (schema == PJ_SCHEMA_PET || mixed) add_arenas(c->schema.obj[OBJ_PET], add_arenas);
-    if (schema == PJ_SCHEMA_ORDER || mixed) add_arenas(c->schema.obj[OBJ_ORDER], add_arenas);
-    if (schema == PJ_SCHEMA_USER || mixed) add_arenas(c->schema.obj[OBJ_USER], add_arenas);
-    Stage stage(c);
-    PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, 256 + ntiles * 16, c->stream));
-    if (aa.count) { k_arena_flags<<<persistent_grid(c, col_bytes / 16 + 1, 256), 256, 0, c->stream>>>(aa); count_launch(c, 0); }
-    stage.next();
-    cudaEvent_t ev_tile0 = c->ev[8], ev_tile1 = c->ev[9];
-    PJ_CUDA(c, cudaEventRecord(ev_tile0, c->stream));
-    k_write_tile<<<(unsigned)ntiles, WT_THREADS, WTILE_SMEM_BYTES, c->stream>>>(ta);
-    PJ_CUDA(c, cudaEventRecord(ev_tile1, c->stream));
-    k_write_close<<<1, 32, 0, c->stream>>>(wa);
-    count_launch(c, 2); count_launch(c, 1);
-    PJ_CUDA(c, cudaGetLastError());
-    stage.next();
-    stage.next();
+  /* tiles as large as the columns' sizes suggest */
+  WriteShapeIn si;
+  memset(&si, 0, sizeof si);
+  si.n = n; si.sms = (uint32_t)c->sms;
+  auto add_arenas = [&](const ObjDesc& O, auto&& self) -> void {
+    for (int i = 0; i < (int)O.nfields; ++i) {
+      const FieldDesc& F = O.f[i];
+      if (F.kind == K_STR) si.arena_bytes += cols->col[F.col + 1].count;
+      else if (F.kind == K_LIST_STR) { const uint64_t k = cols->col[F.col + 1].count; si.strs += k ? k - 1 : 0; si.arena_bytes += cols->col[F.col + 2].count; }
+      else if (F.kind == K_LIST_OBJ) { si.objs += cols->col[c->schema.obj[F.child].present_col].count; self(c->schema.obj[F.child], self); }
+      else if (F.kind == K_OBJ) self(c->schema.obj[F.child], self);
+    }
+  };
+  const uint32_t roots[3] = {OBJ_PET, OBJ_ORDER, OBJ_USER};
+  for (uint32_t m = 0; m < 3; ++m)
+    if (mixed || schema == m + 1) { si.rows[m] = mixed ? cols->col[c->schema.obj[roots[m]].present_col].count : n; add_arenas(c->schema.obj[roots[m]], add_arenas); }
+  const WriteShape shape = write_shape(si, WT_MAX_RECS, WT_MAX_SMEM);
+  const uint64_t ntiles = n ? (n + shape.recs - 1) / shape.recs : 1;
+  if (ntiles >= (1ull << 31)) return set_err(c, PJ_ERR_TOO_LARGE, "pj_write: too many tiles");
+  { pj_status st = ensure(c, &c->tiles, 256 + ntiles * 16 + 256); if (st) return st; }
+  /* stages: [0] state reset, [1] the closing kernel, [2] the tile kernel */
+  WTileArgs ta;
+  memset(&ta, 0, sizeof ta);
+  ta.w = wa;
+  wt_columns(c->schema, schema, dcols, &ta);
+  ta.ticket = (uint32_t*)c->tiles.p;
+  ta.agg = (unsigned long long*)((uint8_t*)c->tiles.p + 256);
+  ta.inc = ta.agg + ntiles;
+  ta.ntiles = (uint32_t)ntiles;
+  ta.recs = shape.recs; ta.smem = shape.smem;
+  ta.spin_limit_ns = c->spin_ns;
+  WriteResetArgs ra;
+  ra.state = (unsigned long long*)c->tiles.p; ra.words = 32 + 2 * ntiles; ra.res = c->d_res;
+  Stage stage(c);
+  k_write_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
+  count_launch(c, 0);
+  stage.next();
+  cudaEvent_t ev_tile0 = c->ev[8], ev_tile1 = c->ev[9];
+  PJ_CUDA(c, cudaEventRecord(ev_tile0, c->stream));
+  switch (schema) {
+    case PJ_SCHEMA_PET: k_write_tile<PJ_SCHEMA_PET><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
+    case PJ_SCHEMA_ORDER: k_write_tile<PJ_SCHEMA_ORDER><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
+    case PJ_SCHEMA_USER: k_write_tile<PJ_SCHEMA_USER><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
+    default: k_write_tile<PJ_SCHEMA_MIXED><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
   }
+  PJ_CUDA(c, cudaEventRecord(ev_tile1, c->stream));
+  k_write_close<<<1, 32, 0, c->stream>>>(wa);
+  count_launch(c, 2); count_launch(c, 1);
+  PJ_CUDA(c, cudaGetLastError());
+  stage.next();
+  stage.next();
   PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   PJ_CUDA(c, cudaGetLastError());
@@ -1024,7 +1028,7 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
     c->stats.main_kernel_ms = c->stats.stage_ms[2];
   }
   for (int k = 0; k < 4; ++k) c->stats.phase_cycles[k] = c->h_res->phase_cycles[k];
-  c->stats.tiles = (uint32_t)(n ? (n + WT_THREADS - 1) / WT_THREADS : 1);
+  c->stats.tiles = (uint32_t)ntiles;
   if (c->h_res->timeout) return set_err(c, PJ_ERR_TIMEOUT, "pj_write: a bounded device-side wait ran out");
   *out_len = c->h_res->out_bytes;
   c->stats.algorithmic_bytes = col_bytes + *out_len;
