@@ -515,7 +515,40 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   return PJ_OK;
 }
 
-/* Array framing: the separator bitmap of pj_array_kernels.cuh, then the parse kernel with it in the place of the line
+/* The separators of an array: its state lies behind `before` bytes of c->tiles, its bitmap behind `scratch` bytes of c->scratch. */
+struct ArrIndex { ArrIndexArgs a; ResetArgs reset; uint32_t words; };
+pj_status array_index_plan(pj_ctx* c, const uint8_t* in, uint64_t len, size_t before, size_t scratch, ArrIndex* ix) {
+  memset(ix, 0, sizeof *ix);
+  const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(in) & 15u);
+  /* large tiles look back less and scan less per byte; small inputs are spread over the SMs */
+  ix->words = len >= (uint64_t)c->sms * 2u * 64u * 1024u ? 4u : 1u;
+  ArrIndexArgs& a = ix->a;
+  a.in = in; a.len = len;
+  a.ntiles = arr_tiles(mis, len, ix->words);
+  const uint64_t nwords = (len + 63) >> 6;
+  const size_t state = 256 + 3 * (size_t)a.ntiles * 8;
+  { pj_status st = ensure(c, &c->scratch, scratch + (nwords + 1) * 8 + 256); if (st) return st; }
+  { pj_status st = ensure(c, &c->tiles, before + state + 256); if (st) return st; }
+  a.sep = (uint64_t*)((uint8_t*)c->scratch.p + scratch);
+  a.ticket = (uint32_t*)((uint8_t*)c->tiles.p + before);
+  a.fn0 = (unsigned long long*)((uint8_t*)c->tiles.p + before + 256);
+  a.fn1 = a.fn0 + a.ntiles; a.inc = a.fn1 + a.ntiles;
+  a.spin_limit_ns = c->spin_ns;
+  a.res = c->d_res;
+  ix->reset.state = (unsigned long long*)c->tiles.p; ix->reset.words = (before + state) / 8;
+  ix->reset.more = (unsigned long long*)a.sep; ix->reset.more_words = mis ? nwords + 1 : 0;
+  ix->reset.res = c->d_res;
+  return PJ_OK;
+}
+cudaError_t array_index_launch(pj_ctx* c, const ArrIndex& ix) {
+  k_reset<<<persistent_grid(c, ix.reset.words + ix.reset.more_words, 256), 256, 0, c->stream>>>(ix.reset);
+  if (ix.words == 4u) k_arr_index<4><<<ix.a.ntiles, AI_THREADS, 0, c->stream>>>(ix.a);
+  else k_arr_index<1><<<ix.a.ntiles, AI_THREADS, 0, c->stream>>>(ix.a);
+  count_launch(c, 0, 2);
+  return cudaGetLastError();
+}
+
+/* Array framing: the separator bitmap of pj_array_index.cuh, then the parse kernel with it in the place of the line
  * feeds. */
 pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t len, uint32_t in_kind, pj_columns* out) {
   ParsePlan pp;
@@ -529,45 +562,27 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
     PJ_CUDA(c, cudaMemcpyAsync(c->in_stage.p, in, len, cudaMemcpyHostToDevice, c->stream));
     c->stats.h2d_bytes += len;
   }
-  const uint64_t nwords = (len + 63) >> 6;
-  const uint64_t atiles = nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1;
-  const size_t off_tin = align_up(atiles * sizeof(ArrFn), 256);
-  const size_t off_sep = align_up(off_tin + atiles * sizeof(ArrState), 256);
-  const size_t off_end = align_up(off_sep + (nwords + 1) * 8, 256);
-  { pj_status st = ensure(c, &c->scratch, off_end + 256); if (st) return st; }
-
-  PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult), c->stream));
+  const ItemShape shape = pick_tile_shape(c, schema, len);
+  const uint64_t nt = stream_tiles((uint32_t)(reinterpret_cast<uintptr_t>(d_in) & 15u), len, 1u, shape.tile_bytes);
+  const size_t item_state = align_up(256 + nt * sizeof(ItemTile), 256);
+  ArrIndex ix;
+  { pj_status st = array_index_plan(c, d_in, len, item_state, 0, &ix); if (st) return st; }
   Stage stage(c);
-  ArrArgs aa;
-  aa.in = d_in; aa.len = len; aa.nwords = nwords;
-  aa.tile_fn = (ArrFn*)c->scratch.p; aa.tile_in = (ArrState*)((uint8_t*)c->scratch.p + off_tin);
-  aa.sep = (uint64_t*)((uint8_t*)c->scratch.p + off_sep); aa.tile_cnt = nullptr;
-  aa.rec_start = nullptr;
-  aa.cap = 0; aa.goff = 0; aa.ntiles = (uint32_t)atiles; aa.res = c->d_res;
-  /* the two running minima start at "none" */
-  PJ_CUDA(c, cudaMemsetAsync(&c->d_res->doc_err_off, 0xFF, sizeof(unsigned long long), c->stream));
-  PJ_CUDA(c, cudaMemsetAsync(&c->d_res->first_opener, 0xFF, sizeof(unsigned long long), c->stream));
-  k_arr_summary<<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-  k_arr_scan_tiles<<<1, 32, 0, c->stream>>>(aa);
-  k_arr_mark<<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-  count_launch(c, 0, 3);
-  PJ_CUDA(c, cudaGetLastError());
+  PJ_CUDA(c, array_index_launch(c, ix));
   stage.next();
 
   uint64_t total[NSLOT];
   for (uint32_t k = 0; k < NSLOT; ++k) total[k] = 0;
   ItemArgs sa;
   memset(&sa, 0, sizeof sa);
-  const ItemShape shape = pick_tile_shape(c, schema, len);
   sa.in = d_in; sa.len = len; sa.limit = len;
   sa.is_first = 1; sa.is_last = 1;
   sa.tile_bytes = shape.tile_bytes; sa.win_bytes = shape.win_bytes; sa.str_words = shape.str_words; sa.row_cap = shape.row_cap;
-  sa.ntiles = (uint32_t)stream_tiles((uint32_t)(reinterpret_cast<uintptr_t>(d_in) & 15u), len, 1u, shape.tile_bytes);
+  sa.ntiles = (uint32_t)nt;
   sa.spin_limit_ns = c->spin_ns;
   sa.opts = c->opt_flags;
-  sa.sep = aa.sep;
+  sa.sep = ix.a.sep;
   c->stats.tile_records = IT_THREADS; c->stats.tiles += sa.ntiles;
-  { pj_status st = ensure(c, &c->tiles, sa.ntiles * sizeof(ItemTile) + 512); if (st) return st; }
   sa.ticket = (uint32_t*)c->tiles.p;
   sa.tiles = (ItemTile*)((uint8_t*)c->tiles.p + 256);
   sa.res = c->d_res;
@@ -575,8 +590,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   sa.rec_cap = pp.rec_cap;
   sa.plan = pp.plan;
   sa.cols = pp.dcols;
-  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, sa.ntiles * sizeof(ItemTile) + 256, c->stream));
-  stage.next(); /* stage 1: set-up */
+  stage.next(); /* stage 1: nothing */
   PJ_CUDA(c, item_launch(schema, &sa, c->stream));
   count_launch(c, 2);
   c->stats.stage_launches[3]++;
@@ -804,10 +818,8 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   const uint64_t ntiles = (len + 15 + INDEX_TILE) / INDEX_TILE;
   const uint64_t nwords = (len + 63) >> 6;
   const uint64_t atiles = nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1;
-  size_t off_fn = align_up(((ntiles > atiles ? ntiles : atiles) + 1) * 4, 256);
-  size_t off_tin = align_up(off_fn + (array ? atiles * sizeof(ArrFn) : 0), 256);
-  size_t off_sep = align_up(off_tin + (array ? atiles * sizeof(ArrState) : 0), 256);
-  size_t off_rs = align_up(off_sep + (array ? (nwords + 1) * 8 : 0), 256);
+  const size_t off_sep = align_up(((ntiles > atiles ? ntiles : atiles) + 1) * 4, 256);
+  const size_t off_rs = align_up(off_sep + (array ? (nwords + 1) * 8 : 0), 256);
   { pj_status st = ensure(c, &c->scratch, off_rs + (kind == PJ_MEM_HOST ? cap * 8 : 0) + 256); if (st) return st; }
   if (kind == PJ_MEM_HOST) {
     if (len) {
@@ -820,7 +832,9 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
     d_rs = (uint64_t*)((uint8_t*)c->scratch.p + off_rs);
   }
   uint32_t* d_tile = (uint32_t*)c->scratch.p;
-  PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult), c->stream));
+  ArrIndex ix;
+  if (array) { pj_status st = array_index_plan(c, d_in, len, 0, off_sep, &ix); if (st) return st; }
+  else PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult), c->stream));
   Stage stage(c);
   if (!array) {
     IndexArgs ia;
@@ -831,21 +845,16 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
     k_nd_index<true><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia);
     count_launch(c, 0, 3);
   } else {
+    PJ_CUDA(c, array_index_launch(c, ix));
     ArrArgs aa;
     aa.in = d_in; aa.len = len; aa.nwords = nwords;
-    aa.tile_fn = (ArrFn*)((uint8_t*)c->scratch.p + off_fn); aa.tile_in = (ArrState*)((uint8_t*)c->scratch.p + off_tin);
-    aa.sep = (uint64_t*)((uint8_t*)c->scratch.p + off_sep); aa.tile_cnt = d_tile;
+    aa.sep = ix.a.sep; aa.tile_cnt = d_tile;
     aa.rec_start = d_rs;
-    aa.cap = cap; aa.goff = 0; aa.ntiles = (uint32_t)atiles; aa.res = c->d_res;
-    PJ_CUDA(c, cudaMemsetAsync(&c->d_res->doc_err_off, 0xFF, sizeof(unsigned long long), c->stream));
-    PJ_CUDA(c, cudaMemsetAsync(&c->d_res->first_opener, 0xFF, sizeof(unsigned long long), c->stream));
-    k_arr_summary<<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-    k_arr_scan_tiles<<<1, 32, 0, c->stream>>>(aa);
-    k_arr_mark<<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
+    aa.cap = cap; aa.goff = 0; aa.res = c->d_res;
     k_arr_records<false><<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
     k_scan_single<uint32_t><<<1, 1024, 0, c->stream>>>(d_tile, atiles, &c->d_res->n_records);
     k_arr_records<true><<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-    count_launch(c, 0, 6);
+    count_launch(c, 0, 3);
   }
   PJ_CUDA(c, cudaGetLastError());
   stage.next();
@@ -853,6 +862,7 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   collect_times(c, 1);
   c->stats.main_kernel_ms = c->stats.stage_ms[0];
+  if (c->h_res->timeout) return set_err(c, PJ_ERR_TIMEOUT, "pj_index_records: a bounded device-side wait ran out");
   *n = c->h_res->n_records;
   uint64_t got = *n < cap ? *n : cap;
   c->stats.algorithmic_bytes = len + got * 8;
@@ -997,10 +1007,10 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
   ta.ntiles = (uint32_t)ntiles;
   ta.recs = shape.recs; ta.smem = shape.smem;
   ta.spin_limit_ns = c->spin_ns;
-  WriteResetArgs ra;
-  ra.state = (unsigned long long*)c->tiles.p; ra.words = 32 + 2 * ntiles; ra.res = c->d_res;
+  ResetArgs ra;
+  ra.state = (unsigned long long*)c->tiles.p; ra.words = 32 + 2 * ntiles; ra.more = nullptr; ra.more_words = 0; ra.res = c->d_res;
   Stage stage(c);
-  k_write_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
+  k_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
   count_launch(c, 0);
   stage.next();
   cudaEvent_t ev_tile0 = c->ev[8], ev_tile1 = c->ev[9];

@@ -5,7 +5,7 @@
  * header holds
  *   - the NDJSON record index on its own (k_nd_index<false> / k_scan_single / k_nd_index<true>: pj_index_records and
  *     its allocation-free variant);
- *   - what runs before and behind the writer's tiles (k_write_tile: pj_write_tile.cuh): k_write_reset and k_write_close.
+ *   - what runs before and behind the writer's tiles (k_write_tile: pj_write_tile.cuh): k_reset and k_write_close.
  *
  * Kernels that wait on other blocks (the look-backs) take their tile from an atomic ticket, so every block they
  * wait for is running or done, and every wait is bounded (the spin limit of the kernel's arguments ->
@@ -124,18 +124,24 @@ __global__ void __launch_bounds__(1024) k_scan_single(T* data, uint64_t n, unsig
   if (threadIdx.x == 0) { data[n] = carry; if (total_out) *total_out = (unsigned long long)carry; }
 }
 
-/* ---- before and behind the writer's tiles --------------------------------------------------------------------------- */
-struct WriteResetArgs {
-  unsigned long long* state; /* ticket and look-back words */
-  uint64_t words;
+/* ---- the state of a call --------------------------------------------------------------------------------------------- */
+struct ResetArgs {
+  unsigned long long *state, *more; /* tickets, look-back words; a bitmap that is or-ed into (or null) */
+  uint64_t words, more_words;
   DevResult* res;
 };
-/* the state of a call: no ticket taken, no tile's bytes known, nothing counted */
-static __global__ void __launch_bounds__(256) k_write_reset(const __grid_constant__ WriteResetArgs a) {
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.words; k += (uint64_t)gridDim.x * blockDim.x) a.state[k] = 0;
+/* no ticket taken, no tile's totals known, nothing counted */
+static __global__ void __launch_bounds__(256) k_reset(const __grid_constant__ ResetArgs a) {
+  const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t k = first; k < a.words; k += step) a.state[k] = 0;
+  for (uint64_t k = first; k < a.more_words; k += step) a.more[k] = 0;
   if (blockIdx.x == 0) {
     uint32_t* r = reinterpret_cast<uint32_t*>(a.res);
-    for (uint32_t k = threadIdx.x; k < sizeof(DevResult) / 4; k += blockDim.x) r[k] = k == offsetof(DevResult, ok) / 4 ? 1u : 0u;
+    for (uint32_t k = threadIdx.x; k < sizeof(DevResult) / 4; k += blockDim.x) {
+      const uint32_t at = 4u * k;
+      const bool none = at - (uint32_t)offsetof(DevResult, doc_err_off) < 8u || at - (uint32_t)offsetof(DevResult, first_opener) < 8u; /* running minima */
+      r[k] = none ? 0xFFFFFFFFu : (at == offsetof(DevResult, ok) ? 1u : 0u);
+    }
   }
 }
 /* closes the text: brackets of array framing, the total, the verdict */
