@@ -522,6 +522,11 @@ __device__ __forceinline__ uint32_t item_freed(const uint8_t* win, const uint32_
   const uint32_t n = win[close - 1u];
   return n < 255u ? n : (uint32_t)win[close - 3u] | ((uint32_t)win[close - 2u] << 8);
 }
+__device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
+  Win w;
+  w.s = win; w.w0 = 0;
+  return wpeek4(w, p);
+}
 /* One string that holds a backslash, a control character or a byte beyond ASCII: decoded in place (the decoded text is
  * never longer); what is left over up to the old closing quote becomes blanks. False: not a valid string. */
 static __device__ __noinline__ bool item_decode_string(uint8_t* win, uint32_t open, uint32_t close, uint32_t opts, uint32_t* moved) {
@@ -529,6 +534,14 @@ static __device__ __noinline__ bool item_decode_string(uint8_t* win, uint32_t op
   *moved = 0;
   if (win[close] != '"') return false; /* the record ends inside it */
   while (p < close) {
+    if (p + 4u <= close) { /* four characters that stay as they are */
+      const uint32_t x4 = item_peek4(win, p), b4 = x4 ^ 0x5C5C5C5Cu;
+      if (!((x4 | ((x4 - 0x20202020u) & ~x4) | ((b4 - 0x01010101u) & ~b4)) & 0x80808080u)) {
+        if (d != p) { win[d] = (uint8_t)x4; win[d + 1u] = (uint8_t)(x4 >> 8); win[d + 2u] = (uint8_t)(x4 >> 16); win[d + 3u] = (uint8_t)(x4 >> 24); }
+        d += 4u; p += 4u;
+        continue;
+      }
+    }
     const uint32_t x = win[p];
     if (x < 0x20) return false;
     if (x == '\\') {
@@ -612,11 +625,12 @@ __device__ __forceinline__ void item_special(const ItemArgs& a, ItemShared& sh, 
   while (p < sep && item_blank(win[p])) ++p;
   if (!ok || win[p] == ':') atomicOr(&sh.oddline[lo >> 5], 1u << (lo & 31u));
 }
-/* All of them: off the list, one per thread, while it holds them; text where more of the strings are of this kind (another script, \/
- * for every slash) fills the lanes without one: a warp then takes 32 strings that follow each other. */
+/* All of them: off the list, one per thread, while it holds them, and as many for every warp: its lanes part in them (31 strings of a tile of Pets
+ * in the lanes of one warp took 55 000 cycles, four for each warp take 30 000, a warp per string with a byte per lane 27 000). Text where more of
+ * the strings are of this kind (another script, \/ for every slash) fills the lanes without one: a warp then takes 32 strings that follow each other. */
 __device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh, uint8_t* win, const uint32_t* pairs, uint32_t tid) {
   if (sh.nspecial <= IT_MAX_SPECIAL) {
-    for (uint32_t i = tid; i < sh.nspecial; i += IT_THREADS) {
+    for (uint32_t i = (tid & 31u) * IT_WARPS + (tid >> 5); i < sh.nspecial; i += IT_THREADS) {
       const uint32_t k = sh.special_list[i];
       if (k < sh.nstr) item_special(a, sh, win, pairs, k); /* (a line that runs out of the window has none) */
     }
@@ -625,11 +639,6 @@ __device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh,
   for (uint32_t k = tid; k < sh.nstr; k += IT_THREADS) if ((sh.special[k >> 5] >> (k & 31u)) & 1u) item_special(a, sh, win, pairs, k);
 }
 
-__device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
-  Win w;
-  w.s = win; w.w0 = 0;
-  return wpeek4(w, p);
-}
 /* first byte of a value that is no number: a literal, an object, a list (as the walk takes whatever is between colon and comma) */
 __device__ __forceinline__ bool item_other_type(uint32_t x) { return x == 't' || x == 'f' || x == '[' || x == '{'; }
 __device__ __forceinline__ bool item_number_start(uint32_t x) { return x - (uint32_t)'0' <= 9u || x == '-'; }
@@ -892,8 +901,8 @@ __device__ __forceinline__ void item_walk_members(ItemWalk& f, uint32_t* row, ui
     item_walk_members<OBJ, I + 1, ROOT, WORD0, BIT0>(f, row, flags, l);
   }
 }
-/* The same for records without a blank and without null, and with embedded objects whole: no byte is looked at twice. It is
- * tried first, because most producers write this way (1M Pets: 617 us against 790 us with the walk above alone). */
+/* The same for records without a blank and without null, and with embedded objects whole: no byte is looked at twice. (Strings that were
+ * decoded are shorter than their quotes tell.) It is tried first, because most producers write this way (1M Pets: 617 us against 790 us with the walk above alone). */
 /* is `"name":` of property I at p? */
 template <int OBJ, int I>
 __device__ __forceinline__ bool item_at_key_colon(const uint8_t* win, uint32_t p) {
@@ -936,8 +945,8 @@ __device__ __forceinline__ uint32_t item_dense_flat(ItemWalk& f, uint32_t at, ui
     if constexpr (kind == K_STR) {
       f.ok = f.ok && f.k < f.kend && (nx & 0xFFFFu) == v;
       end = (nx >> 16) + 1u;
-      ref[I] = (v + 1u) | ((end - v - 2u) << 16);
       f.ok = f.ok && end - v < 0x1000u; /* a length that fits its row */
+      ref[I] = (v + 1u) | ((end - v - 2u - (f.ok ? item_freed(f.win, f.moved, f.k, nx >> 16) : 0u)) << 16);
       f.k++;
     } else {
       static_assert(I + 1 < CObj<E>::N, "an integer is followed by another property");
@@ -975,8 +984,8 @@ __device__ __forceinline__ void item_dense_members(ItemWalk& f, uint32_t* row, u
       } else if constexpr (kind == K_STR || kind == K_ENUM || kind == K_DATETIME) {
         end = (nx >> 16) + 1u;
         f.ok = more && (nx & 0xFFFFu) == v && end - v <= 0x8000u;
+        row[word] = (v + 1u) | ((end - v - 2u - (f.ok ? item_freed(f.win, f.moved, f.k, nx >> 16) : 0u)) << 16);
         f.k++;
-        row[word] = (v + 1u) | ((end - v - 2u) << 16);
       } else if constexpr (kind == K_OBJ) {
         constexpr int CH = CObj<OBJ>::f[I].child;
         uint32_t ref[8];
@@ -993,10 +1002,10 @@ __device__ __forceinline__ void item_dense_members(ItemWalk& f, uint32_t* row, u
           uint32_t behind;
           if constexpr (kind == K_LIST_STR) {
             const uint32_t pr = f.pairs[f.k < f.kend ? f.k : f.kend];
-            f.k++;
             behind = (pr >> 16) + 1u;
-            f.ok = f.k <= f.kend && (pr & 0xFFFFu) == end && behind - end < 0x8000u;
-            l.bytes += behind - end - 2u;
+            f.ok = f.k < f.kend && (pr & 0xFFFFu) == end && behind - end < 0x8000u;
+            l.bytes += behind - end - 2u - (f.ok ? item_freed(f.win, f.moved, f.k, pr >> 16) : 0u);
+            f.k++;
           } else {
             uint32_t ref[8];
             behind = item_dense_flat<CObj<OBJ>::f[I].child>(f, end, ref);
@@ -1078,12 +1087,13 @@ __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGe
   } else {
     const uint32_t n = f.kend - f.k, bit = 1u << (i & 31u);
     const bool plain = !(sh.movedline[i >> 5] & bit), fit = !cut && !(sh.oddline[i >> 5] & bit);
-    /* A warp waits for its longest line, which takes some 300 cycles a string (1000 with blanks), while item_pack() takes 80 for
-       every string of the tile, whoever's it is: few long lines are its. */
-    if constexpr (DENSE) f.ok = fit && plain && win[start] == '{' && (n <= 32u || n * 4u <= sh.nstr);
+    /* A warp waits for its longest line, which takes some 300 cycles a string (1000 with blanks), while the warps together take 10 (25) in
+       item_pack() for every string of the tile, whoever's it is: lines much longer than the others are its. (50 k Pets with long lists 610 -> 575 us,
+       with blanks 1620 -> 1270, the line for both at a quarter and a twelfth of the tile's strings before.) */
+    if constexpr (DENSE) f.ok = fit && win[start] == '{' && (n <= 32u || n * 30u <= sh.nstr);
     else {
       while (f.p < f.sep && item_blank(win[f.p])) ++f.p;
-      f.ok = fit && win[f.p] == '{' && (n <= 16u || n * 12u <= sh.nstr);
+      f.ok = fit && win[f.p] == '{' && (n <= 16u || n * 40u <= sh.nstr);
     }
     item_walk_model<SCHEMA, DENSE>(f, row, flags, l, type);
     if (!plain) flags |= IF_MOVED;
@@ -2192,16 +2202,20 @@ __device__ __forceinline__ bool item_tile(const ItemArgs& a, const StreamGeom& g
   }
   if (__syncthreads_or((int)sh.slow)) return false;
   {
-    uint32_t nodd = 0;
+    uint32_t nodd = 0, nmoved = 0;
 #pragma unroll
-    for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
-    if (tid == 0) sh.ndense = nline - nodd;
+    for (uint32_t k = 0; k < IT_WARPS; ++k) { nodd += (uint32_t)__popc(sh.oddmask[k]); nmoved += (uint32_t)__popc(sh.movedline[k] & ~sh.oddmask[k]); }
+    if (tid == 0) sh.ndense = nline - nodd - nmoved; /* in one spelling, nothing decoded */
     if (nodd) {
-      __syncthreads(); /* oddmask[] is read */
-      item_walk_again<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid, mine);
-      nodd = 0;
+      /* the second walk takes 1000 cycles a string, however few lines are left; a line or two per warp go to the packs at once (300 k mixed
+         records, 1 % malformed: 328 -> 278 us) */
+      if (nodd > 2u * IT_WARPS) {
+        __syncthreads(); /* oddmask[] is read */
+        item_walk_again<SCHEMA, ARR>(a, g, sh, win, pairs, rows, tid, mine);
+        nodd = 0;
 #pragma unroll
-      for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
+        for (uint32_t k = 0; k < IT_WARPS; ++k) nodd += (uint32_t)__popc(sh.oddmask[k]);
+      }
       if (nodd) item_packs<SCHEMA, ARR>(a, g, sh, win, pairs, rows, nodd);
       __syncthreads();
     }
