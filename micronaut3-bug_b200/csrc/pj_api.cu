@@ -716,6 +716,7 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   for (auto& ev : c->ev_k0) { e = cudaEventCreate(&ev); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
   for (auto& ev : c->ev_k1) { e = cudaEventCreate(&ev); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
   for (auto& ev : c->ev_done) { e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
+  c->choice[PJ_SCHEMA_MIXED].several = c->choice[PJ_SCHEMA_MIXED].items = true;
   build_schema(&c->schema);
   e = item_init_1(&c->schema);
   if (e == cudaSuccess) e = item_init_2(&c->schema);
