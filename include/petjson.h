@@ -302,7 +302,8 @@ typedef struct pj_call_stats {
                                parse kernel; write: [0] state
                                reset and the scan of the string arenas for bytes to escape, [1] the closing
                                kernel, [2] the tile kernel */
-  uint32_t stage_launches[8]; /* kernels launched per stage; parse: [3] is no stage, but how many of stage 2's
+  uint32_t stage_launches[8]; /* kernels launched per stage; [4]: small calls, the kernel that brings the result to host memory
+                                 (no stage: it is not timed); parse: [3] is no stage, but how many of stage 2's
                                  launches were the kernel that spreads a tile over strings, instead of the
                                  one with a record per thread                                    */
   uint64_t h2d_bytes;       /* bytes copied host->device by the call                            */

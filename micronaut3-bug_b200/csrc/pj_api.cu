@@ -112,6 +112,7 @@ struct pj_ctx {
   Buffer tiles;     /* look-back state of the tile kernel + its ticket */
   DevResult* d_res = nullptr; /* [PJ_CTX_RESULTS]: one per piece of a call; [0] serves every other call */
   DevResult* h_res = nullptr; /* pinned, same shape */
+  uint8_t *h_in = nullptr, *h_out = nullptr; /* pinned, FETCH_ROOM each (behind h_res): columns of small calls on their way there and back */
   cudaEvent_t ev[10] = {};
   cudaEvent_t ev_k0[16] = {}, ev_k1[16] = {}; /* around the kernel of every piece */
   cudaEvent_t ev_done[16] = {};               /* the totals of a piece have reached the host */
@@ -319,6 +320,41 @@ uint32_t pick_stream_tile(const pj_ctx* c, uint32_t schema) {
   if (tb > ST_MAX_TILE_BYTES) tb = ST_MAX_TILE_BYTES;
   return (uint32_t)tb;
 }
+/* Calls up to here are told their result by a kernel (k_fetch) and reset by one (k_reset): a copy engine and a memset each cost a small call 4 - 6 us
+ * of its 40. Above, a kernel's time does not matter, and an NDJSON call stays one launch. */
+static constexpr uint64_t SMALL_CALL = 1u << 20;
+/* Columns of a small call that go to host memory with the result: none when `out` lies on the device or the input suggests more than there is room for. */
+void fetch_columns(const ParsePlan& pp, const pj_columns* out, uint64_t len, FetchArgs* fa) {
+  if (out->mem_kind != PJ_MEM_HOST || len > FETCH_ROOM * 3 / 4) return;
+  auto add = [&](int col, uint32_t slot, uint32_t plus) {
+    FetchCol& f = fa->col[fa->n++];
+    f.p = (const uint8_t*)pp.dcols.ptr[col]; f.slot = (uint8_t)slot; f.plus = (uint8_t)plus;
+    f.shift = (uint8_t)(col_info(col)->elem == 8 ? 3 : (col_info(col)->elem == 4 ? 2 : 0));
+  };
+  for (int i = 0; i < pp.nrc; ++i) add(pp.rcols[i], FETCH_RECORDS, 0);
+  for (uint32_t k = 0; k < pp.plan.n; ++k) { const FinalizeItem& it = pp.plan.item[k]; add(it.col, it.rows_slot == 0xFF ? FETCH_RECORDS : it.rows_slot, it.sentinel_slot != 0xFF); }
+}
+cudaError_t launch_fetch(pj_ctx* c, FetchArgs& fa) {
+  fa.res = c->d_res; fa.host_res = c->h_res; fa.host = c->h_out;
+  k_fetch<<<fa.n ? 24 : 1, 256, 0, c->stream>>>(fa);
+  count_launch(c, 4);
+  return cudaGetLastError();
+}
+/* The columns k_fetch brought along, to where the caller wants them; false when they did not fit. */
+bool take_columns(pj_ctx* c, const ParsePlan& pp, const FetchArgs& fa, pj_columns* out) {
+  uint64_t at = 0;
+  for (uint32_t k = 0; k < fa.n && at <= FETCH_ROOM; ++k) at = fetch_place(at, fetch_bytes(fa.col[k], *c->h_res));
+  if (!fa.n || at > FETCH_ROOM) return false;
+  at = 0;
+  for (uint32_t k = 0; k < fa.n; ++k) {
+    const int col = k < (uint32_t)pp.nrc ? pp.rcols[k] : (int)pp.plan.item[k - (uint32_t)pp.nrc].col;
+    const uint64_t nb = fetch_bytes(fa.col[k], *c->h_res);
+    if (nb) memcpy(out->col[col].ptr, c->h_out + at, nb);
+    c->stats.d2h_bytes += nb;
+    at = fetch_place(at, nb);
+  }
+  return true;
+}
 /* NDJSON: one launch of a parse kernel per piece. Host buffers of a whole stream are parsed in pieces cut after line
  * feeds, so that the copy of piece p+1 to the device, the kernel of piece p and the copy of the columns of piece p-1
  * back run at the same time on three streams. Every launch is enqueued before the host waits for anything: a piece
@@ -402,8 +438,19 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     nt_total += nt[p];
   }
   { pj_status st = ensure(c, &c->tiles, nt_total * state + (size_t)np * 256 + 256); if (st) return st; }
-  PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * state + (size_t)np * 256, c->stream));
-  PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult) * np, c->stream));
+  const bool small = np == 1 && limit <= SMALL_CALL;
+  FetchArgs fa;
+  fa.n = 0;
+  if (small) {
+    fetch_columns(pp, out, limit, &fa);
+    ResetArgs ra;
+    ra.state = (unsigned long long*)c->tiles.p; ra.words = (nt_total * state + 256) / 8; ra.more = nullptr; ra.more_words = 0; ra.res = c->d_res;
+    k_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
+    count_launch(c, 0);
+  } else {
+    PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * state + (size_t)np * 256, c->stream));
+    PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult) * np, c->stream));
+  }
   if (c->stall_once) { /* test hook: tickets start at 1, tile 0 is never processed, the waits for it run out */
     c->stall_once = false;
     for (int p = 0; p < np; ++p) PJ_CUDA(c, cudaMemsetAsync((uint8_t*)c->tiles.p + (size_t)p * 256, 1, 1, c->stream));
@@ -453,7 +500,8 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
       PJ_CUDA(c, stream_launch(schema, &t, c->stream));
     }
     PJ_CUDA(c, cudaEventRecord(c->ev_k1[p], c->stream));
-    PJ_CUDA(c, cudaMemcpyAsync(c->h_res + p, c->d_res + p, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
+    if (small) PJ_CUDA(c, launch_fetch(c, fa));
+    else PJ_CUDA(c, cudaMemcpyAsync(c->h_res + p, c->d_res + p, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
     PJ_CUDA(c, cudaEventRecord(c->ev_done[p], c->stream));
     count_launch(c, 2);
     if (items) c->stats.stage_launches[3]++;
@@ -483,7 +531,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     if (r.strs_per_kb > strs_per_kb) strs_per_kb = r.strs_per_kb;
     n_dense += items ? r.n_dense : r.n_fast >> 32;
     const uint64_t rows_new = r.n_records;
-    if (host_out && !over) {
+    if (host_out && !over && !take_columns(c, pp, fa, out)) {
       if (pipe) PJ_CUDA(c, cudaStreamWaitEvent(s_out, c->ev_done[p], 0));
       auto copy_back = [&](int col, uint64_t from, uint64_t to) -> cudaError_t {
         const size_t e = col_info(col)->elem;
@@ -595,7 +643,10 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   count_launch(c, 2);
   c->stats.stage_launches[3]++;
   stage.next(); /* stage 2: the parse kernel */
-  PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
+  FetchArgs fa;
+  fa.n = 0;
+  if (len <= SMALL_CALL) { fetch_columns(pp, out, len, &fa); PJ_CUDA(c, launch_fetch(c, fa)); }
+  else PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   PJ_CUDA(c, cudaGetLastError());
   collect_times(c, 3);
@@ -613,7 +664,7 @@ pj_status parse_array(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t le
   const pj_status st = finish_columns(c, schema, len, pp, r.n_records, r.n_errors, total, r.over != 0, out);
   if (!st && r.n_records > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)r.n_records; c->max_rec_bytes[schema] = r.max_rec; c->strs_per_kb[schema] = r.strs_per_kb; }
   if (st) return st;
-  if (host_out) {
+  if (host_out && !take_columns(c, pp, fa, out)) {
     for (int i = 0; i < pp.nneed; ++i) {
       const int col = pp.need[i];
       const size_t nb = (size_t)out->col[col].count * col_info(col)->elem;
@@ -710,8 +761,11 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   }
   e = cudaMalloc(&c->d_res, sizeof(DevResult) * PJ_CTX_RESULTS);
   if (e != cudaSuccess) return fail_create(e, "cudaMalloc");
-  e = cudaMallocHost(&c->h_res, sizeof(DevResult) * PJ_CTX_RESULTS);
+  const size_t res_bytes = align_up(sizeof(DevResult) * PJ_CTX_RESULTS, 4096);
+  e = cudaMallocHost(&c->h_res, res_bytes + 2 * FETCH_ROOM);
   if (e != cudaSuccess) return fail_create(e, "cudaMallocHost");
+  c->h_in = (uint8_t*)c->h_res + res_bytes;
+  c->h_out = c->h_in + FETCH_ROOM;
   for (auto& ev : c->ev) { e = cudaEventCreate(&ev); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
   for (auto& ev : c->ev_k0) { e = cudaEventCreate(&ev); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
   for (auto& ev : c->ev_k1) { e = cudaEventCreate(&ev); if (e != cudaSuccess) return fail_create(e, "cudaEventCreate"); }
@@ -859,7 +913,10 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   }
   PJ_CUDA(c, cudaGetLastError());
   stage.next();
-  PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
+  FetchArgs fa;
+  fa.n = 0;
+  if (len <= SMALL_CALL) PJ_CUDA(c, launch_fetch(c, fa));
+  else PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   collect_times(c, 1);
   c->stats.main_kernel_ms = c->stats.stage_ms[0];
@@ -957,13 +1014,16 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
     pj_status st = ensure(c, &c->col_stage, tot + 256);
     if (st) return st;
     size_t at = 0;
+    const bool together = tot <= FETCH_ROOM; /* one copy of small columns (20 Pets: 14 of them, 5 us each) */
     for (int i = 0; i < nneed; ++i) {
       size_t nb = (size_t)cols->col[need[i]].count * col_info(need[i])->elem;
       dcols.ptr[need[i]] = (uint8_t*)c->col_stage.p + at;
-      if (nb) PJ_CUDA(c, cudaMemcpyAsync(dcols.ptr[need[i]], cols->col[need[i]].ptr, nb, cudaMemcpyHostToDevice, c->stream));
+      if (nb && together) memcpy(c->h_in + at, cols->col[need[i]].ptr, nb);
+      else if (nb) PJ_CUDA(c, cudaMemcpyAsync(dcols.ptr[need[i]], cols->col[need[i]].ptr, nb, cudaMemcpyHostToDevice, c->stream));
       c->stats.h2d_bytes += nb;
       at += align_up(nb, 256);
     }
+    if (together && tot) PJ_CUDA(c, cudaMemcpyAsync(c->col_stage.p, c->h_in, tot, cudaMemcpyHostToDevice, c->stream));
   } else {
     for (int i = 0; i < nneed; ++i) dcols.ptr[need[i]] = cols->col[need[i]].ptr;
   }
@@ -1023,12 +1083,18 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
     default: k_write_tile<PJ_SCHEMA_MIXED><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
   }
   PJ_CUDA(c, cudaEventRecord(ev_tile1, c->stream));
-  k_write_close<<<1, 32, 0, c->stream>>>(wa);
+  k_write_close<<<1, 32, 0, c->stream>>>(wa, c->h_res);
   count_launch(c, 2); count_launch(c, 1);
   PJ_CUDA(c, cudaGetLastError());
   stage.next();
   stage.next();
-  PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
+  FetchArgs fa; /* a small text comes along with the result */
+  fa.n = 0;
+  if (out_kind == PJ_MEM_HOST && col_bytes <= FETCH_ROOM / 2) {
+    fa.n = 1;
+    fa.col[0].p = d_out; fa.col[0].slot = FETCH_TEXT; fa.col[0].plus = 0; fa.col[0].shift = 0;
+    PJ_CUDA(c, launch_fetch(c, fa));
+  }
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   PJ_CUDA(c, cudaGetLastError());
   collect_times(c, 3);
@@ -1044,7 +1110,8 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
   *out_len = c->h_res->out_bytes;
   c->stats.algorithmic_bytes = col_bytes + *out_len;
   if (!c->h_res->ok) return set_err(c, PJ_ERR_CAPACITY, "pj_write: %llu bytes needed, room for %llu", (unsigned long long)*out_len, (unsigned long long)cap);
-  if (out_kind == PJ_MEM_HOST && *out_len) {
+  if (fa.n && *out_len <= FETCH_ROOM) { memcpy(out, c->h_out, *out_len); c->stats.d2h_bytes += *out_len; }
+  else if (out_kind == PJ_MEM_HOST && *out_len) {
     PJ_CUDA(c, cudaMemcpyAsync(out, d_out, *out_len, cudaMemcpyDeviceToHost, c->stream));
     PJ_CUDA(c, cudaStreamSynchronize(c->stream));
     c->stats.d2h_bytes += *out_len;
