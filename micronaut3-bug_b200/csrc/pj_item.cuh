@@ -511,21 +511,49 @@ __device__ __forceinline__ bool item_index(const ItemArgs& a, const StreamGeom& 
   return fine;
 }
 
-__device__ __forceinline__ bool item_blank(uint32_t x) { return x <= ' ' && ((0x100002600ull >> x) & 1u); } /* (a line feed is none in a line, and then no line holds one) */
-__device__ __forceinline__ bool item_only_blanks(const uint8_t* win, uint32_t p, uint32_t end) {
-  while (p < end && item_blank(win[p])) ++p;
-  return p == end;
+/* 8 bytes at p, which may lie up to IT_FRONT bytes before the window */
+__device__ __forceinline__ uint64_t item_back8(const uint8_t* win, int32_t p) {
+  const uint32_t* a = reinterpret_cast<const uint32_t*>(win) + (p >> 2);
+  const uint32_t sh = ((uint32_t)p & 3u) * 8u, x0 = a[0], x1 = a[1], x2 = a[2];
+  return (uint64_t)__funnelshift_r(x0, x1, sh) | ((uint64_t)__funnelshift_r(x1, x2, sh) << 32);
 }
+__device__ __forceinline__ bool item_blank(uint32_t x) { return x <= ' ' && ((0x100002600ull >> x) & 1u); } /* (a line feed is none in a line, and then no line holds one) */
+__device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
+  Win w;
+  w.s = win; w.w0 = 0;
+  return wpeek4(w, p);
+}
+/* 0x80 in every byte of x that is a blank */
+__device__ __forceinline__ uint32_t item_blank4(uint32_t x) { return item_eq4(x, 0x20202020u) | item_eq4(x, 0x09090909u) | item_eq4(x, 0x0A0A0A0Au) | item_eq4(x, 0x0D0D0D0Du); }
+/* from p over blanks, up to end; four bytes a step, because the lanes of a warp wait for the one with the most blanks, and a byte's load takes as
+ * long as a word's */
+__device__ __forceinline__ uint32_t item_skip(const uint8_t* win, uint32_t p, uint32_t end) {
+  if (p >= end) return p;
+  for (;;) {
+    const uint32_t no = ~item_blank4(item_peek4(win, p)) & 0x80808080u;
+    if (no) { p += ((uint32_t)__ffs((int)no) - 1u) >> 3; break; }
+    p += 4u;
+    if (p >= end) break;
+  }
+  return p < end ? p : end;
+}
+/* from p back over blanks, down to `from`: the first position behind them, where p - 1 is none */
+__device__ __forceinline__ uint32_t item_skip_back(const uint8_t* win, uint32_t from, uint32_t p) {
+  if (p <= from) return p;
+  for (;;) {
+    const uint32_t no = ~item_blank4((uint32_t)(item_back8(win, (int32_t)p - 8) >> 32)) & 0x80808080u;
+    if (no) { p -= (uint32_t)__clz((int)no) >> 3; break; }
+    p = p < from + 4u ? from : p - 4u;
+    if (p <= from) break;
+  }
+  return p > from ? p : from;
+}
+__device__ __forceinline__ bool item_only_blanks(const uint8_t* win, uint32_t p, uint32_t end) { return item_skip(win, p, end) == end; }
 /* bytes that string k, which ends at close, lost when it was decoded; moved: bit per string, null when there is none */
 __device__ __forceinline__ uint32_t item_freed(const uint8_t* win, const uint32_t* moved, uint32_t k, uint32_t close) {
   if (!moved || !((moved[k >> 5] >> (k & 31u)) & 1u)) return 0;
   const uint32_t n = win[close - 1u];
   return n < 255u ? n : (uint32_t)win[close - 3u] | ((uint32_t)win[close - 2u] << 8);
-}
-__device__ __forceinline__ uint32_t item_peek4(const uint8_t* win, uint32_t p) {
-  Win w;
-  w.s = win; w.w0 = 0;
-  return wpeek4(w, p);
 }
 /* One string that holds a backslash, a control character or a byte beyond ASCII: decoded in place (the decoded text is
  * never longer); what is left over up to the old closing quote becomes blanks. False: not a valid string. */
@@ -643,12 +671,6 @@ __device__ __forceinline__ void item_specials(const ItemArgs& a, ItemShared& sh,
 __device__ __forceinline__ bool item_other_type(uint32_t x) { return x == 't' || x == 'f' || x == '[' || x == '{'; }
 __device__ __forceinline__ bool item_number_start(uint32_t x) { return x - (uint32_t)'0' <= 9u || x == '-'; }
 /* -?(0|[1-9][0-9]*) in the n bytes at pos, within int64 / int32. Read from its end, eight digits at a time. */
-/* 8 bytes at p, which may lie up to IT_FRONT bytes before the window */
-__device__ __forceinline__ uint64_t item_back8(const uint8_t* win, int32_t p) {
-  const uint32_t* a = reinterpret_cast<const uint32_t*>(win) + (p >> 2);
-  const uint32_t sh = ((uint32_t)p & 3u) * 8u, x0 = a[0], x1 = a[1], x2 = a[2];
-  return (uint64_t)__funnelshift_r(x0, x1, sh) | ((uint64_t)__funnelshift_r(x1, x2, sh) << 32);
-}
 __device__ __forceinline__ bool item_int(const uint8_t* win, uint32_t pos, uint32_t n, bool is64, int64_t* out) {
   const bool neg = n && win[pos] == '-';
   pos += neg; n -= neg;
@@ -746,14 +768,11 @@ __device__ __forceinline__ bool item_at_key(const uint8_t* win, uint32_t p) {
 }
 /* from p over blanks to c and over the blanks behind it; the position there */
 __device__ __forceinline__ uint32_t item_over(ItemWalk& f, uint32_t p, uint32_t c) {
-  uint32_t x = f.win[p];
-  if (x != c) {
-    while (p < f.sep && item_blank(x)) x = f.win[++p];
-    f.ok = f.ok && x == c;
+  if (f.win[p] != c) {
+    p = item_skip(f.win, p, f.sep);
+    f.ok = f.ok && f.win[p] == c;
   }
-  ++p;
-  while (item_blank(f.win[p]) && p < f.sep) ++p;
-  return p;
+  return item_skip(f.win, p + 1u, f.sep);
 }
 /* back from q over blanks to a comma (or closing brace: last) and over the blanks before it; where the comma is, and in *end
  * the end of what is before it */
@@ -761,12 +780,10 @@ __device__ __forceinline__ uint32_t item_back(ItemWalk& f, uint32_t from, uint32
   const uint32_t c = last ? '}' : ',';
   uint32_t r = q - 1u;
   if (f.win[r] != c) {
-    while (r > from && item_blank(f.win[r])) --r;
+    r = item_skip_back(f.win, from + 1u, q) - 1u;
     f.ok = f.ok && f.win[r] == c;
   }
-  uint32_t e = r;
-  while (e > from && item_blank(f.win[e - 1u])) --e;
-  *end = e;
+  *end = item_skip_back(f.win, from, r);
   return r;
 }
 /* the flat object E whose brace is behind the blanks from at on, all of its properties there: bytes of its string in *bytes,
@@ -792,8 +809,7 @@ __device__ __forceinline__ uint32_t item_walk_flat(ItemWalk& f, uint32_t at, uin
     f.ok = f.ok && open == v && close - open < 0x1000u; /* a length that fits its row */
     *bytes = close - open - 1u - item_freed(f.win, f.moved, f.k + 1u, close);
     f.k += 2u;
-    uint32_t p = close + 1u;
-    while (p < f.sep && item_blank(f.win[p])) ++p;
+    const uint32_t p = item_skip(f.win, close + 1u, f.sep);
     f.ok = f.ok && f.win[p] == '}';
     return p + 1u;
   }
@@ -807,7 +823,7 @@ __device__ __forceinline__ uint32_t item_walk_list(ItemWalk& f, uint32_t v, Item
   f.ok = f.ok && f.win[v] == '[';
   uint32_t n = 0, p = v + 1u;
   const uint32_t k0 = f.k;
-  while (p < f.sep && item_blank(f.win[p])) ++p;
+  p = item_skip(f.win, p, f.sep);
   bool go = f.ok && f.win[p] != ']';
   p += go ? 0u : 1u;
   while (go) {
@@ -823,13 +839,12 @@ __device__ __forceinline__ uint32_t item_walk_list(ItemWalk& f, uint32_t v, Item
       l.bytes += bytes << 16;
     }
     ++n;
-    p = f.ok ? p : v;
-    uint32_t x = f.win[p];
-    while (p < f.sep && item_blank(x)) x = f.win[++p];
+    p = item_skip(f.win, f.ok ? p : v, f.sep);
+    const uint32_t x = f.win[p];
     go = f.ok && x == ',';
     f.ok = f.ok && (x == ',' || x == ']');
     ++p;
-    if (go) while (p < f.sep && item_blank(f.win[p])) ++p;
+    if (go) p = item_skip(f.win, p, f.sep);
   }
   if constexpr (kind == K_LIST_STR) { l.k_str = k0; l.n_str = n; } else { l.k_obj = k0; l.n_obj = n; }
   return p;
@@ -861,7 +876,7 @@ __device__ __forceinline__ void item_walk_members(ItemWalk& f, uint32_t* row, ui
             end = item_back(f, v, more ? nx & 0xFFFFu : f.sep, !more, &e);
             if (!ROOT && f.win[e - 1u] == '}') { /* the embedded object ends here, and the comma is its root's */
               end = --e;
-              while (e > v && item_blank(f.win[e - 1u])) --e;
+              e = item_skip_back(f.win, v, e);
             }
           } else {
             e = v;
@@ -890,8 +905,8 @@ __device__ __forceinline__ void item_walk_members(ItemWalk& f, uint32_t* row, ui
           end = f.p + 1u;
         } else end = item_walk_list<OBJ, I>(f, v, l);
         end = f.ok ? end : f.p;
-        uint32_t x = f.win[end];
-        if (to_delimiter) while (end < f.sep && item_blank(x)) x = f.win[++end];
+        if (to_delimiter) end = item_skip(f.win, end, f.sep);
+        const uint32_t x = f.win[end];
         f.open = x == ',';
         f.ok = f.ok && (x == ',' || x == '}');
         flags |= bit;
@@ -1092,7 +1107,7 @@ __device__ __forceinline__ void item_walk_line(const ItemArgs& a, const StreamGe
        with blanks 1620 -> 1270, the line for both at a quarter and a twelfth of the tile's strings before.) */
     if constexpr (DENSE) f.ok = fit && win[start] == '{' && (n <= 32u || n * 30u <= sh.nstr);
     else {
-      while (f.p < f.sep && item_blank(win[f.p])) ++f.p;
+      f.p = item_skip(win, f.p, f.sep);
       f.ok = fit && win[f.p] == '{' && (n <= 16u || n * 40u <= sh.nstr);
     }
     item_walk_model<SCHEMA, DENSE>(f, row, flags, l, type);
@@ -1193,7 +1208,7 @@ __device__ __forceinline__ void item_gap_spaced(const ItemShared& sh, const uint
   v.vpos = b; v.vend = 0; v.clpos = b;
   while (p < b && n <= 8u) {
     uint32_t c = win[p];
-    if (item_blank(c)) { ++p; continue; }
+    if (item_blank(c)) { p = item_skip(win, p + 1u, b); continue; }
     if (n == 1u) v.vpos = p;
     if (c - (uint32_t)'0' <= 9u || c == '-' || (c | 0x20u) - (uint32_t)'a' <= 25u) {
       ++p;
