@@ -870,11 +870,10 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   c->stats = pj_call_stats{};
   const uint8_t* d_in = in;
   uint64_t* d_rs = rec_start;
-  const uint64_t ntiles = (len + 15 + INDEX_TILE) / INDEX_TILE;
   const uint64_t nwords = (len + 63) >> 6;
-  const uint64_t atiles = nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1;
-  const size_t off_sep = align_up(((ntiles > atiles ? ntiles : atiles) + 1) * 4, 256);
-  const size_t off_rs = align_up(off_sep + (array ? (nwords + 1) * 8 : 0), 256);
+  const uint32_t words = !array && len >= (uint64_t)c->sms * 2u * 64u * 1024u ? 4u : 1u; /* of 64 bytes per thread, as in array_index_plan() */
+  const uint64_t ntiles = array ? (nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1) : (len + 15 + (uint64_t)INDEX_TILE * words) / ((uint64_t)INDEX_TILE * words);
+  const size_t off_rs = align_up(array ? (nwords + 1) * 8 : 0, 256);
   { pj_status st = ensure(c, &c->scratch, off_rs + (kind == PJ_MEM_HOST ? cap * 8 : 0) + 256); if (st) return st; }
   if (kind == PJ_MEM_HOST) {
     if (len) {
@@ -886,30 +885,36 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
     }
     d_rs = (uint64_t*)((uint8_t*)c->scratch.p + off_rs);
   }
-  uint32_t* d_tile = (uint32_t*)c->scratch.p;
+  RecordTiles rt;
+  const size_t state = align_up(256 + ntiles * 16, 256);
   ArrIndex ix;
-  if (array) { pj_status st = array_index_plan(c, d_in, len, 0, off_sep, &ix); if (st) return st; }
-  else PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult), c->stream));
+  if (array) { pj_status st = array_index_plan(c, d_in, len, state, 0, &ix); if (st) return st; }
+  else {
+    pj_status st = ensure(c, &c->tiles, state); if (st) return st;
+    memset(&ix, 0, sizeof ix);
+    ix.reset.state = (unsigned long long*)c->tiles.p; ix.reset.words = state / 8; ix.reset.res = c->d_res;
+  }
+  rt.ticket = (uint32_t*)c->tiles.p;
+  rt.agg = (unsigned long long*)((uint8_t*)c->tiles.p + 256); rt.inc = rt.agg + ntiles;
+  rt.ntiles = (uint32_t)ntiles; rt.spin_limit_ns = c->spin_ns; rt.res = c->d_res;
   Stage stage(c);
   if (!array) {
+    k_reset<<<persistent_grid(c, ix.reset.words, 256), 256, 0, c->stream>>>(ix.reset);
     IndexArgs ia;
     ia.in = d_in; ia.len = len; ia.limit = len; ia.is_first = 1; ia.is_last = 1;
-    ia.tile = d_tile; ia.rec_start = d_rs; ia.cap = cap; ia.goff = 0;
-    k_nd_index<false><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia);
-    k_scan_single<uint32_t><<<1, 1024, 0, c->stream>>>(d_tile, ntiles, &c->d_res->n_records);
-    k_nd_index<true><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia);
-    count_launch(c, 0, 3);
+    ia.tile = nullptr; ia.rec_start = d_rs; ia.cap = cap; ia.goff = 0;
+    if (words == 4u) k_nd_records<4><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia, rt);
+    else k_nd_records<1><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia, rt);
+    count_launch(c, 0, 2);
   } else {
     PJ_CUDA(c, array_index_launch(c, ix));
     ArrArgs aa;
     aa.in = d_in; aa.len = len; aa.nwords = nwords;
-    aa.sep = ix.a.sep; aa.tile_cnt = d_tile;
+    aa.sep = ix.a.sep;
     aa.rec_start = d_rs;
     aa.cap = cap; aa.goff = 0; aa.res = c->d_res;
-    k_arr_records<false><<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-    k_scan_single<uint32_t><<<1, 1024, 0, c->stream>>>(d_tile, atiles, &c->d_res->n_records);
-    k_arr_records<true><<<(unsigned)atiles, ARR_THREADS, 0, c->stream>>>(aa);
-    count_launch(c, 0, 3);
+    k_arr_records<<<(unsigned)ntiles, ARR_THREADS, 0, c->stream>>>(aa, rt);
+    count_launch(c, 0, 1);
   }
   PJ_CUDA(c, cudaGetLastError());
   stage.next();

@@ -7,8 +7,9 @@
  * functions of the earlier tiles (two 64-bit words each, and one for a state that is known). With the state known each word's separators are
  * the brackets at depth 0 and 1 and the commas between them; a word that stays deeper has none and is done.
  *
- * Bound by the instructions of the masks, about 9 per byte, and the look-back. 300 k Pets (88 MB): 480 us in three launches and two passes
- * before, 157 us now; 100 k: 175 -> 60.
+ * Bound by the instructions of the masks, about 9 per byte, and the look-back. 300 k Pets with escapes (91 MB): 480 us in three launches and two passes
+ * before, 123 now; 1 M (295 MB): 1600 -> 337, of which 100 are the look-back's. Four blocks per SM (64 registers): with three, five, six
+ * of them 355, 370, 375 us; read through shared memory 421 against 415 before that.
  * The bitmap's bits are input bytes; the words are those of the 16-byte aligned addresses, so that any alignment is read alike. Where the two differ the
  * bitmap is zeroed before and words are or-ed into it.
  */
@@ -191,8 +192,26 @@ __device__ __forceinline__ uint64_t arr_mark(const uint8_t* p, const ArrWord& m,
   return sep;
 }
 
+/* The same for a word that starts at depth 2 or more, as far as it does not come below depth 1 (false: arr_mark() has to look): only the closers
+ * that come down to depth 1 matter, and the bytes up to the opener behind them. (1 M Pets: 446 us event by event, 415 so.) */
+__device__ __forceinline__ bool arr_mark_deep(const uint8_t* p, const ArrWord& m, uint64_t quotes, uint64_t in, int32_t d, int32_t hi, uint64_t* sep_out) {
+  const uint64_t outside = ~in & ~quotes & (hi >= 64 ? ~0ull : (1ull << hi) - 1u);
+  const uint64_t O = m.O & outside, C = m.C & outside;
+  uint64_t sep = 0;
+  for (uint64_t c = C; c; c &= c - 1u) {
+    const uint64_t upto = c ^ (c - 1u); /* the closer and the bytes before it */
+    if (d + (int32_t)popc64(O & upto) - (int32_t)popc64(C & upto) > 1) continue;
+    const uint64_t next = (O | C) & ~upto, first = next & (0ull - next);
+    if (first & C) return false; /* down to depth 0 */
+    for (uint64_t t = outside & ~upto & (first - 1u); t; t &= t - 1u) if (p[ctz64a(t)] == ',') sep |= t & (0ull - t);
+    if (!first) break; /* depth 1 up to the word's end (first - 1 above: all ones) */
+  }
+  *sep_out = sep;
+  return true;
+}
+
 template <int W>
-__global__ void __launch_bounds__(AI_THREADS) k_arr_index(const __grid_constant__ ArrIndexArgs a) {
+__global__ void __launch_bounds__(AI_THREADS, 4) k_arr_index(const __grid_constant__ ArrIndexArgs a) {
   __shared__ ArrFn sh_fn[AI_WARPS];
   __shared__ ArrState sh_in[AI_WARPS];
   __shared__ uint32_t sh_tile, sh_ok;
@@ -264,7 +283,8 @@ __global__ void __launch_bounds__(AI_THREADS) k_arr_index(const __grid_constant_
     sep[k] = 0;
     if (v < end && d - (int32_t)down <= 1) { /* (deeper all through: no separator) */
       uint32_t bad = 64u, opener = 64u, openers = 0;
-      sep[k] = arr_mark(base + v, m[k], q[k], in, d, v ? 0 : (int32_t)mis, end - v >= 64u ? 64 : (int32_t)(end - v), &bad, &opener, &openers);
+      const int32_t hi = end - v >= 64u ? 64 : (int32_t)(end - v);
+      if (d < 2 || !arr_mark_deep(base + v, m[k], q[k], in, d, hi, &sep[k])) sep[k] = arr_mark(base + v, m[k], q[k], in, d, v ? 0 : (int32_t)mis, hi, &bad, &opener, &openers);
       if (ok && bad < 64u) atomicMin(&a.res->doc_err_off, (unsigned long long)(v + bad - mis));
       if (ok && opener < 64u) { atomicMin(&a.res->first_opener, (unsigned long long)(v + opener - mis)); atomicAdd(&a.res->n_openers, openers); }
     }
