@@ -1082,10 +1082,10 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
   cudaEvent_t ev_tile0 = c->ev[8], ev_tile1 = c->ev[9];
   PJ_CUDA(c, cudaEventRecord(ev_tile0, c->stream));
   switch (schema) {
-    case PJ_SCHEMA_PET: k_write_tile<PJ_SCHEMA_PET><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
-    case PJ_SCHEMA_ORDER: k_write_tile<PJ_SCHEMA_ORDER><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
-    case PJ_SCHEMA_USER: k_write_tile<PJ_SCHEMA_USER><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
-    default: k_write_tile<PJ_SCHEMA_MIXED><<<(unsigned)ntiles, WT_THREADS, shape.smem, c->stream>>>(ta); break;
+    case PJ_SCHEMA_PET: k_write_tile<PJ_SCHEMA_PET><<<(unsigned)ntiles, WtT<PJ_SCHEMA_PET>::threads, shape.smem, c->stream>>>(ta); break;
+    case PJ_SCHEMA_ORDER: k_write_tile<PJ_SCHEMA_ORDER><<<(unsigned)ntiles, WtT<PJ_SCHEMA_ORDER>::threads, shape.smem, c->stream>>>(ta); break;
+    case PJ_SCHEMA_USER: k_write_tile<PJ_SCHEMA_USER><<<(unsigned)ntiles, WtT<PJ_SCHEMA_USER>::threads, shape.smem, c->stream>>>(ta); break;
+    default: k_write_tile<PJ_SCHEMA_MIXED><<<(unsigned)ntiles, WtT<PJ_SCHEMA_MIXED>::threads, shape.smem, c->stream>>>(ta); break;
   }
   PJ_CUDA(c, cudaEventRecord(ev_tile1, c->stream));
   k_write_close<<<1, 32, 0, c->stream>>>(wa, c->h_res);

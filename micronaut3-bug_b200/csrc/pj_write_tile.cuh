@@ -20,12 +20,12 @@
  * not fit shared memory, take the general road: a record per thread (pj_write_fast.cuh).
  *
  * What bounds it: instruction issue and waiting for one another. 300 k Pets: 180 instructions of a warp per record, a third of the issue slots
- * used; 8 warps of a block wait for the first one's offsets and look-back, and three blocks per SM (shared memory) cover half of that.
+ * used; the warps of a block wait for the first one's offsets and look-back, and two or three blocks per SM (shared memory) cover half of that.
  * Integers and strings are written by functions that are called, not expanded: the instruction cache does not hold the text of three
  * models otherwise (400 k mixed records 449 -> 336 us, Pets the same).
  *
- * Measured (kernel, against a record per thread with byte stores and a pass over the arenas before it): 1 M Pets 401 + 45 -> 420 us, 400 k Users
- * 130 -> 95, Orders 81 -> 62, Pets with escapes 487 -> 250, mixed records with escapes 617 -> 337, 66 k Pets with long lists 1 090 -> 330.
+ * Measured (kernel, against a record per thread with byte stores and a pass over the arenas before it; us): 600 k Pets 268 -> 221, Users
+ * 205 -> 135, Orders 123 -> 87, Pets with escapes 735 -> 340, mixed records with escapes 925 -> 367, 100 k Pets with long lists 1 670 -> 450.
  */
 #ifndef PJ_WRITE_TILE_CUH
 #define PJ_WRITE_TILE_CUH
@@ -44,16 +44,17 @@ namespace pj {
 #define PJ_CX constexpr
 #endif
 #endif
-#ifndef PJ_WT_BLOCKS
-#define PJ_WT_BLOCKS 3 /* resident blocks per SM the kernel is compiled for */
-#endif
-#ifndef PJ_WT_THREADS
-#define PJ_WT_THREADS 256
-#endif
-static constexpr uint32_t WT_THREADS = PJ_WT_THREADS;
-static constexpr uint32_t WT_WARPS = WT_THREADS / 32;
-static constexpr uint32_t WT_MAX_RECS = 256;        /* records per tile */
-static constexpr uint32_t WT_PER = (WT_MAX_RECS + WT_THREADS - 1) / WT_THREADS; /* ... and thread */
+static constexpr uint32_t WT_MAX_RECS = 256; /* records per tile */
+/* Threads of a block, and blocks per SM. 600 k records, us of the kernel: mixed 256 threads / three blocks 520, 512 / two 373 (three models' records
+ * fill twice as many groups of 32); Pets, of which 256 share a block that writes them in two windows, 240 and 224; Users 133 and 152, Orders 86
+ * and 117: their tiles are short, and more blocks wait in turn. */
+template <int SCHEMA> struct WtT {
+  static constexpr uint32_t threads = SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED ? 512u : 256u, blocks = threads == 512u ? 2u : 3u;
+  static constexpr uint32_t warps = threads / 32u;
+};
+static_assert(WT_MAX_RECS <= 256, "a record per thread");
+inline uint32_t wt_threads(uint32_t schema) { return schema == PJ_SCHEMA_PET ? WtT<1>::threads : (schema == PJ_SCHEMA_ORDER ? WtT<2>::threads : (schema == PJ_SCHEMA_USER ? WtT<3>::threads : WtT<4>::threads)); }
+static constexpr uint32_t WT_MOST_WARPS = 16;
 static constexpr uint32_t WT_MAX_SMEM = 128 * 1024;
 static constexpr uint32_t WT_MIN_WINDOW = 2048;
 static constexpr uint32_t WT_ESC = 160;             /* strings with escapes a round keeps for later */
@@ -170,7 +171,7 @@ struct WtShared {
   uint32_t nhit;                                   /* 16-byte blocks with a byte to escape */
   uint16_t hit[WT_HITS];
   uint32_t odd, ok, tile, nesc;                    /* odd: the tile takes the general road */
-  uint32_t wsum[WT_WARPS * WT_PER], cls[3][WT_WARPS * WT_PER];
+  uint32_t wsum[WT_MOST_WARPS], cls[3][WT_MOST_WARPS];
   uint32_t pos[WT_MAX_RECS + 1];                   /* a record's bytes, then where it starts in the tile's text */
   uint32_t mid[WT_MAX_RECS];                       /* where its second half starts | no property before it << 31 */
   uint32_t list[2][WT_MAX_RECS];                   /* where its lists' elements start, from its first byte; WT_NONE: none are written */
@@ -835,49 +836,32 @@ __device__ __forceinline__ void wt_count_block(const WTileArgs& a, WtShared& sh,
 /* Mixed streams: the tile's records by model, in order; odd when the rows of a model do not follow each other. */
 __device__ __forceinline__ void wt_sort(const WTileArgs& a, WtShared& sh, uint64_t rec0, uint32_t nrec, uint32_t tid) {
   const uint32_t lane = tid & 31u, warp = tid >> 5;
-  uint32_t m[WT_PER], rank[WT_PER];
-  uint64_t row[WT_PER];
-#pragma unroll
-  for (uint32_t p = 0; p < WT_PER; ++p) {
-    const uint32_t t = tid + p * WT_THREADS;
-    m[p] = 3; row[p] = 0;
-    if (t < nrec) {
-      uint32_t type;
-      if (write_locate(PJ_SCHEMA_MIXED, &a.w.cols, rec0 + t, &type, &row[p])) m[p] = type == PJ_TYPE_PET ? 0u : (type == PJ_TYPE_ORDER ? 1u : 2u);
-      sh.pos[t] = 0;
-    }
+  uint32_t m = 3, rank = 0;
+  uint64_t row = 0;
+  if (tid < nrec) {
+    uint32_t type;
+    if (write_locate(PJ_SCHEMA_MIXED, &a.w.cols, rec0 + tid, &type, &row)) m = type == PJ_TYPE_PET ? 0u : (type == PJ_TYPE_ORDER ? 1u : 2u);
+    sh.pos[tid] = 0;
   }
 #pragma unroll
-  for (uint32_t p = 0; p < WT_PER; ++p) {
-    rank[p] = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < 3; ++k) {
-      const uint32_t b = __ballot_sync(0xFFFFFFFFu, m[p] == k);
-      if (lane == 0) sh.cls[k][warp + p * WT_WARPS] = (uint32_t)__popc(b);
-      if (m[p] == k) rank[p] = (uint32_t)__popc(b & ((1u << lane) - 1u));
-    }
+  for (uint32_t k = 0; k < 3; ++k) {
+    const uint32_t b = __ballot_sync(0xFFFFFFFFu, m == k);
+    if (lane == 0) sh.cls[k][warp] = (uint32_t)__popc(b);
+    if (m == k) rank = (uint32_t)__popc(b & ((1u << lane) - 1u));
   }
   __syncthreads();
   uint32_t cnt[3] = {0, 0, 0};
 #pragma unroll
   for (uint32_t k = 0; k < 3; ++k)
 #pragma unroll
-    for (uint32_t w = 0; w < WT_WARPS * WT_PER; ++w) {
-      const uint32_t v = sh.cls[k][w];
-#pragma unroll
-      for (uint32_t p = 0; p < WT_PER; ++p) if (m[p] == k && w < warp + p * WT_WARPS) rank[p] += v;
-      cnt[k] += v;
-    }
-#pragma unroll
-  for (uint32_t p = 0; p < WT_PER; ++p)
-    if (m[p] < 3u) {
-      sh.perm[(m[p] == 0 ? 0u : (m[p] == 1 ? cnt[0] : cnt[0] + cnt[1])) + rank[p]] = (uint8_t)(tid + p * WT_THREADS);
-      if (rank[p] == 0) sh.row0[m[p]] = row[p];
-    }
+    for (uint32_t w = 0; w < WtT<PJ_SCHEMA_MIXED>::warps; ++w) { const uint32_t v = sh.cls[k][w]; if (m == k && w < warp) rank += v; cnt[k] += v; }
+  if (m < 3u) {
+    sh.perm[(m == 0 ? 0u : (m == 1 ? cnt[0] : cnt[0] + cnt[1])) + rank] = (uint8_t)tid;
+    if (rank == 0) sh.row0[m] = row;
+  }
   if (tid < 3u) { sh.cnt[tid] = tid == 0 ? cnt[0] : (tid == 1 ? cnt[1] : cnt[2]); sh.pre[tid] = tid == 0 ? 0u : (tid == 1 ? cnt[0] : cnt[0] + cnt[1]); }
   __syncthreads();
-#pragma unroll
-  for (uint32_t p = 0; p < WT_PER; ++p) if (m[p] < 3u && row[p] != sh.row0[m[p]] + rank[p]) sh.odd = 1;
+  if (m < 3u && row != sh.row0[m] + rank) sh.odd = 1;
 }
 template <int SCHEMA>
 __device__ __forceinline__ uint32_t wt_groups(const WtShared& sh) {
@@ -902,6 +886,7 @@ __device__ __forceinline__ void wt_zero(uint8_t* w8, uint32_t from, uint32_t to,
 }
 /* the window's n bytes from `pad` on to gbase[pad..]: the 16-byte multiples in the middle leave with one bulk copy, the odd bytes at both
  * ends with plain stores. All threads, behind a barrier; thread 0 waits until the window has been read. */
+template <uint32_t THREADS>
 __device__ __forceinline__ void wt_copy_out(uint8_t* gbase, const uint8_t* win, uint32_t pad, uint32_t n, uint32_t tid) {
   const uint32_t end = pad + n, lo16 = (pad + 15u) & ~15u, hi16 = end & ~15u;
   if (hi16 > lo16) {
@@ -909,12 +894,13 @@ __device__ __forceinline__ void wt_copy_out(uint8_t* gbase, const uint8_t* win, 
     if (tid >= 32 && tid < 32 + (lo16 - pad)) gbase[pad + tid - 32] = win[pad + tid - 32];
     if (tid >= 64 && tid < 64 + (end - hi16)) gbase[hi16 + tid - 64] = win[hi16 + tid - 64];
   } else {
-    for (uint32_t b = pad + tid; b < end; b += WT_THREADS) gbase[b] = win[b];
+    for (uint32_t b = pad + tid; b < end; b += THREADS) gbase[b] = win[b];
   }
 }
 
 template <int SCHEMA>
-__global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const __grid_constant__ WTileArgs a) {
+__global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_write_tile(const __grid_constant__ WTileArgs a) {
+  constexpr uint32_t THREADS = WtT<SCHEMA>::threads, WARPS = WtT<SCHEMA>::warps;
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) WtShared sh;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -949,7 +935,7 @@ __global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const _
   if (!odd) {
     const uint32_t b0 = sh.text >> 4, b1 = sh.stage >> 4;
     uint32_t any = 0;
-    for (uint32_t b = b0 + tid; b < b1; b += WT_THREADS) {
+    for (uint32_t b = b0 + tid; b < b1; b += THREADS) {
       const uint4 v = *reinterpret_cast<const uint4*>(smem + 16u * b);
       if (word_needs_escape(v.x) | word_needs_escape(v.y) | word_needs_escape(v.z) | word_needs_escape(v.w)) {
         const uint32_t k = atomicAdd(&sh.nhit, 1u);
@@ -961,22 +947,22 @@ __global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const _
       x.dirty = true;
       uint32_t* ex = wt_extras(sh, smem); /* (the window begins behind them) */
       if (tid == 0) sh.win = (sh.extra + 4u * sh.nstr + 15u) & ~15u;
-      for (uint32_t k = tid; k < sh.nstr; k += WT_THREADS) ex[k] = 0;
+      for (uint32_t k = tid; k < sh.nstr; k += THREADS) ex[k] = 0;
       __syncthreads();
       const bool all = sh.nhit > WT_HITS; /* (more than the list holds: every block) */
-      for (uint32_t k = warp; k < (all ? b1 - b0 : sh.nhit); k += WT_WARPS) wt_count_block(a, sh, smem, all ? b0 + k : sh.hit[k], lane);
+      for (uint32_t k = warp; k < (all ? b1 - b0 : sh.nhit); k += WARPS) wt_count_block(a, sh, smem, all ? b0 + k : sh.hit[k], lane);
       __syncthreads();
     }
     bool bad = false;
     if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) {
       const uint32_t npet = (sh.cnt[0] + 31u) / 32u;
-      for (uint32_t u = warp; u < 2u * npet; u += WT_WARPS) {
+      for (uint32_t u = warp; u < 2u * npet; u += WARPS) {
         const WtGroup g = wt_group<SCHEMA>(sh, u >> 1);
         if (u & 1u) wt_sum_items<SCHEMA, 1>(x, sh, smem, g, lane, bad); else wt_sum_items<SCHEMA, 0>(x, sh, smem, g, lane, bad);
       }
       __syncthreads();
     }
-    for (uint32_t u = warp; u < ngroups; u += WT_WARPS) {
+    for (uint32_t u = warp; u < ngroups; u += WARPS) {
       const WtGroup g = wt_group<SCHEMA>(sh, u);
       if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 0) wt_size_records<SCHEMA, OBJ_PET>(x, sh, smem, g, lane, bad);
       if constexpr (SCHEMA == PJ_SCHEMA_ORDER || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 1) wt_size_records<SCHEMA, OBJ_ORDER>(x, sh, smem, g, lane, bad);
@@ -985,27 +971,17 @@ __global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const _
     odd = __syncthreads_or((int)bad) != 0;
   }
   /* where the records start */
-  uint32_t len[WT_PER], at[WT_PER];
-#pragma unroll
-  for (uint32_t p = 0; p < WT_PER; ++p) {
-    const uint32_t t = tid + p * WT_THREADS;
-    len[p] = t < nrec ? (odd ? wt_general<SCHEMA, false>(&a.w.cols, rec0 + t, x.incl, x.hexa, nullptr, 0) : sh.pos[t]) : 0u;
-    at[p] = warp_incl_scan(len[p]);
-    if (lane == 31) sh.wsum[warp + p * WT_WARPS] = at[p];
-    at[p] -= len[p];
-  }
+  uint32_t len = 0;
+  if (tid < nrec) len = odd ? wt_general<SCHEMA, false>(&a.w.cols, rec0 + tid, x.incl, x.hexa, nullptr, 0) : sh.pos[tid];
+  uint32_t at = warp_incl_scan(len);
+  if (lane == 31) sh.wsum[warp] = at;
+  at -= len;
   __syncthreads();
   const long long c1 = clock64();
   uint32_t total = 0;
 #pragma unroll
-  for (uint32_t q = 0; q < WT_WARPS * WT_PER; ++q) {
-    const uint32_t v = sh.wsum[q];
-#pragma unroll
-    for (uint32_t p = 0; p < WT_PER; ++p) if (q < warp + p * WT_WARPS) at[p] += v;
-    total += v;
-  }
-#pragma unroll
-  for (uint32_t p = 0; p < WT_PER; ++p) { const uint32_t t = tid + p * WT_THREADS; if (t < nrec) sh.pos[t] = at[p]; }
+  for (uint32_t q = 0; q < WARPS; ++q) { const uint32_t v = sh.wsum[q]; if (q < warp) at += v; total += v; }
+  if (tid < nrec) sh.pos[tid] = at;
   if (tid == 0) sh.pos[nrec] = total;
   const uint64_t lead = a.w.array ? 1 : 0; /* the opening bracket */
   const uint32_t win = odd ? 0u : sh.win, room = a.smem - win - 48u; /* (the last word and the output's alignment) */
@@ -1024,7 +1000,7 @@ __global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const _
       sh.base = excl;
       sh.ok = ok && fits;
     }
-  } else if (!odd) wt_zero(smem, win, win + 32u + (total < room ? total : room), tid - 32u, WT_THREADS - 32u);
+  } else if (!odd) wt_zero(smem, win, win + 32u + (total < room ? total : room), tid - 32u, THREADS - 32u);
   __syncthreads();
   const long long c2 = clock64();
   if (!sh.ok) return;
@@ -1043,21 +1019,21 @@ __global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const _
     uint8_t* const dst0 = out0 + start;
     if (rb == ra || (odd && rb != nrec)) { /* no window for it: straight to global memory */
       rb = odd ? nrec : ra + 1u;
-      for (uint32_t t = ra + tid; t < rb; t += WT_THREADS) wt_general<SCHEMA, true>(&a.w.cols, rec0 + t, x.incl, x.hexa, out0 + sh.pos[t], after);
+      for (uint32_t t = ra + tid; t < rb; t += THREADS) wt_general<SCHEMA, true>(&a.w.cols, rec0 + t, x.incl, x.hexa, out0 + sh.pos[t], after);
       ra = rb;
       continue;
     }
     const uint32_t pad = (uint32_t)(reinterpret_cast<uintptr_t>(dst0) & 15u), bytes = sh.pos[rb] - start;
     /* the window mirrors the output's alignment: window byte k goes to (dst0 - pad)[k] */
-    if (odd) { for (uint32_t t = tid; t < nrec; t += WT_THREADS) wt_general<SCHEMA, true>(&a.w.cols, rec0 + t, x.incl, x.hexa, smem + pad + sh.pos[t], after); }
+    if (odd) { for (uint32_t t = tid; t < nrec; t += THREADS) wt_general<SCHEMA, true>(&a.w.cols, rec0 + t, x.incl, x.hexa, smem + pad + sh.pos[t], after); }
     else {
-      if (ra) { wt_zero(smem, win, win + 32u + bytes, tid, WT_THREADS); if (tid == 0) sh.nesc = 0; __syncthreads(); }
+      if (ra) { wt_zero(smem, win, win + 32u + bytes, tid, THREADS); if (tid == 0) sh.nesc = 0; __syncthreads(); }
       const uint32_t at0 = win + pad - start;
       /* the units of all groups, the long ones first: a unit's number turns with its group, so that a warp's are not all of one kind */
       constexpr uint32_t KINDS = SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED ? 4u : 2u;
       const bool single = KINDS == 4u && ngroups == 1u; /* a tile of long lists: their elements are spread over the warps */
-      constexpr uint32_t PARTS = (WT_WARPS - 2u) / 2u;
-      for (uint32_t u = warp; u < (single ? 2u + 2u * PARTS : KINDS * ngroups); u += WT_WARPS) {
+      constexpr uint32_t PARTS = (WARPS - 2u) / 2u;
+      for (uint32_t u = warp; u < (single ? 2u + 2u * PARTS : KINDS * ngroups); u += WARPS) {
         const WtGroup g = wt_group<SCHEMA>(sh, single ? 0u : u / KINDS);
         const uint32_t k = single ? (u < 2u ? u : 2u + (u & 1u)) : (u + u / KINDS) % KINDS, part = single && u >= 2u ? (u - 2u) / 2u : 0u, parts = single ? PARTS : 1u;
         if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 0) wt_unit<SCHEMA, OBJ_PET>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
@@ -1067,13 +1043,13 @@ __global__ void __launch_bounds__(WT_THREADS, PJ_WT_BLOCKS) k_write_tile(const _
       if (x.dirty) {
         __syncthreads();
         const uint32_t n = sh.nesc < WT_ESC ? sh.nesc : WT_ESC;
-        for (uint32_t k = warp; k < n; k += WT_WARPS) wt_escape(smem, sh.esc[k].at, sh.esc[k].n, sh.esc[k].dst, x.hexa, lane);
+        for (uint32_t k = warp; k < n; k += WARPS) wt_escape(smem, sh.esc[k].at, sh.esc[k].n, sh.esc[k].dst, x.hexa, lane);
       }
     }
     fence_async_smem();
     __syncthreads();
     c3 = clock64();
-    wt_copy_out(dst0 - pad, smem + win, pad, bytes, tid);
+    wt_copy_out<THREADS>(dst0 - pad, smem + win, pad, bytes, tid);
     ra = rb;
     if (ra < nrec) __syncthreads();
   }

@@ -66,7 +66,7 @@ extern "C" int emu_write_tiles(uint32_t schema, uint32_t array, int inclusion, u
   for (uint32_t t = 0; t < a.ntiles && fine; ++t) {
     memset(smem, 0xC3, shared);
     EMU_POISON(smem + shared, sizeof smem - shared);
-    fine = emu_block::run(WT_THREADS, one_thread, nullptr, order + t);
+    fine = emu_block::run(wt_threads(schema), one_thread, nullptr, order + t);
     EMU_UNPOISON(smem + shared, sizeof smem - shared);
   }
   if (fine && res.timeout) { snprintf(emu_block::error, sizeof emu_block::error, "a bounded wait ran out"); fine = false; }
