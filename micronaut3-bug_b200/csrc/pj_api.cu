@@ -320,9 +320,9 @@ uint32_t pick_stream_tile(const pj_ctx* c, uint32_t schema) {
   if (tb > ST_MAX_TILE_BYTES) tb = ST_MAX_TILE_BYTES;
   return (uint32_t)tb;
 }
-/* Calls up to here are told their result by a kernel (k_fetch) and reset by one (k_reset): a copy engine and a memset each cost a small call 4 - 6 us
- * of its 40. Above, a kernel's time does not matter, and an NDJSON call stays one launch. */
-static constexpr uint64_t SMALL_CALL = 1u << 20;
+/* Calls of up to so many bytes are told their result by a kernel (k_fetch) and reset by one (k_reset): a copy engine and a memset each cost 4 - 6 us, of
+ * the 40 that a small call takes. Above, that does not matter, and an NDJSON call stays one launch. */
+static constexpr uint64_t SMALL_CALL = 16u << 20;
 /* Columns of a small call that go to host memory with the result: none when `out` lies on the device or the input suggests more than there is room for. */
 void fetch_columns(const ParsePlan& pp, const pj_columns* out, uint64_t len, FetchArgs* fa) {
   if (out->mem_kind != PJ_MEM_HOST || len > FETCH_ROOM * 3 / 4) return;

@@ -26,7 +26,8 @@ struct NdChoice {
  * them 340 / 740), so it is tried, and of two calls of like size one with each kernel the time per byte decides. It hands back what its
  * strict walk took at 99 %, at once the first time, after twice as many such calls each time the text turned out to change its spelling.
  * Streams of several models start with k_parse_items and stay with it: it sorts a tile's lines by model, where a warp of the other one runs the
- * three models' code one after the other (300k records, us: compact 312 / 250, 1 % malformed 371 / 283).
+ * three models' code one after the other (300k records, us: compact 312 / 250, 1 % malformed 371 / 283); only text that leaves its records to
+ * the exact parser has the other one tried, and then the time decides.
  * Records of 16 KB leave its blocks too little to do side by side: they are not tried (300 Pets of 40 KB: 0.5 / 15.6 ms). The
  * result does not depend on the choice. */
 inline void note_call(NdChoice& k, uint64_t len, float ms, uint64_t records, uint64_t errors, uint64_t fast, uint64_t dense, uint32_t max_rec) {
@@ -49,7 +50,7 @@ inline void note_call(NdChoice& k, uint64_t len, float ms, uint64_t records, uin
   } else if (lost) {
     k.tried = k.ns[0];
     k.items = k.handed_back = false;
-  } else if (k.several && len / (records ? records : 1) >= 16384) {
+  } else if (k.several && (len / (records ? records : 1) >= 16384 || (timed && !alike && fast * 100 < good * 98))) {
     k.items = false; k.handed_back = true;
   } else if (!k.several && dense * 100 >= good * 99 && max_rec <= 1024) {
     if (++k.clean >= k.wait) { k.items = false; k.handed_back = true; }
