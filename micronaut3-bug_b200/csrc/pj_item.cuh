@@ -1729,12 +1729,21 @@ __device__ __forceinline__ void item_emit_run(uint32_t* stage, uint8_t* dst, con
     const uint32_t* p = reinterpret_cast<const uint32_t*>(win) + (from >> 2);
     const uint32_t sh = ((uint32_t)from & 3u) * 8u;
     uint32_t* d = stage + (b >> 2);
-    uint32_t x0 = p[0], keep = 0xFFFFFFFFu << (8u * lead);
-    for (uint32_t k = 0; k < k1; ++k) {
-      const uint32_t x1 = p[k + 1];
-      const uint32_t v = __funnelshift_r(x0, x1, sh) & keep;
-      if (k == 0) atomicOr(d, v); else d[k] = v; /* the first word may be shared with the string before */
+    uint32_t x0 = p[0], keep = 0xFFFFFFFFu << (8u * lead), k = 0;
+    if (k1) { /* the first word may be shared with the string before */
+      const uint32_t x1 = p[1];
+      atomicOr(d, __funnelshift_r(x0, x1, sh) & keep);
       keep = 0xFFFFFFFFu;
+      x0 = x1; k = 1;
+    }
+    for (; k + 4u <= k1; k += 4u) { /* four loads on their way at a time: 2 M mixed records 2.02 -> 1.97 ms */
+      const uint32_t x1 = p[k + 1], x2 = p[k + 2], x3 = p[k + 3], x4 = p[k + 4];
+      d[k] = __funnelshift_r(x0, x1, sh); d[k + 1] = __funnelshift_r(x1, x2, sh); d[k + 2] = __funnelshift_r(x2, x3, sh); d[k + 3] = __funnelshift_r(x3, x4, sh);
+      x0 = x4;
+    }
+    for (; k < k1; ++k) {
+      const uint32_t x1 = p[k + 1];
+      d[k] = __funnelshift_r(x0, x1, sh);
       x0 = x1;
     }
     const uint32_t v = __funnelshift_r(x0, p[k1 + 1], sh) & keep & (0xFFFFFFFFu >> (8u * (3u - ((lead + n - 1u) & 3u))));

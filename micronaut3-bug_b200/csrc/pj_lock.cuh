@@ -396,7 +396,13 @@ PJ_HD void lk_copy(uint8_t* dst, const Win& w, uint32_t pos, uint32_t n) {
   const uint32_t sh = (pos & 3u) * 8u, nw = n >> 2;
   uint32_t x0 = a[0];
   uint32_t* d4 = reinterpret_cast<uint32_t*>(dst);
-  for (uint32_t i = 0; i < nw; ++i) {
+  uint32_t i = 0;
+  for (; i + 4u <= nw; i += 4u) { /* four loads on their way at a time: 600 k Pets 0.357 -> 0.351 ms */
+    const uint32_t x1 = a[i + 1], x2 = a[i + 2], x3 = a[i + 3], x4 = a[i + 4];
+    d4[i] = lk_funnel(x0, x1, sh); d4[i + 1] = lk_funnel(x1, x2, sh); d4[i + 2] = lk_funnel(x2, x3, sh); d4[i + 3] = lk_funnel(x3, x4, sh);
+    x0 = x4;
+  }
+  for (; i < nw; ++i) {
     const uint32_t x1 = a[i + 1];
     d4[i] = lk_funnel(x0, x1, sh);
     x0 = x1;
