@@ -299,8 +299,7 @@ typedef struct pj_call_stats {
   float main_kernel_ms;     /* CUDA-event time of the dominant kernel(s) of the call            */
   float stage_ms[8];        /* CUDA-event time per stage. parse, NDJSON: [2] the parse kernel(s), nothing else
                                runs; parse, array framing: [0] separator index, [1] state reset, [2] the
-                               parse kernel; write: [0] state
-                               reset and the scan of the string arenas for bytes to escape, [1] the closing
+                               parse kernel; write: [0] state reset, [1] the closing
                                kernel, [2] the tile kernel */
   uint32_t stage_launches[8]; /* kernels launched per stage; [4]: small calls, the kernel that brings the result to host memory
                                  (no stage: it is not timed); parse: [3] is no stage, but how many of stage 2's
