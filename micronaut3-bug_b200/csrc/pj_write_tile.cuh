@@ -16,8 +16,8 @@
  *     Strings with a byte to escape are left out and written afterwards, a warp per string.
  *  5. The window leaves with one bulk copy. Text longer than the window goes in several rounds of 4 and 5.
  *
- * Tables whose rows a tile does not find in order (a record map of the caller's own making, offsets that fall), or whose strings do
- * not fit shared memory, take the general road: a record per thread (pj_write_fast.cuh).
+ * Tables whose rows a tile does not find in order (a record map of the caller's own making, offsets of written strings that fall, or of any
+ * where there is a byte to escape), or whose strings do not fit shared memory, take the general road: a record per thread (pj_write_fast.cuh).
  *
  * What bounds it: instruction issue and waiting for one another. 300 k Pets: 180 instructions of a warp per record, a third of the issue slots
  * used; the warps of a block wait for the first one's offsets and look-back, and two or three blocks per SM (shared memory) cover half of that.
@@ -237,6 +237,17 @@ __device__ __forceinline__ void wt_load(const WtShared& sh, const uint8_t* w8, u
   wt_snap<OBJ, LO, HI>(sh, w8, row, r);
   constexpr int E = wt_child<OBJ, LO, HI>();
   if constexpr (E >= 0) { rc.present = *wt_at<uint8_t>(sh, w8, CObj<E>::present_col, row); wt_snap<E, 0, CObj<E>::N>(sh, w8, row, rc); }
+}
+/* does a string of properties [I, N), present or not, end before it begins? wt_count_block() finds a byte's string by offsets that never fall. */
+template <int OBJ, int I = 0>
+__device__ __forceinline__ bool wt_falls(const RowSnap& r, const RowSnap& rc) {
+  if constexpr (I >= CObj<OBJ>::N) return false;
+  else {
+    bool f = false;
+    if constexpr (FK<OBJ, I>::kind == K_STR) f = r.a[I] > r.b[I];
+    else if constexpr (FK<OBJ, I>::kind == K_OBJ) f = wt_falls<FK<OBJ, I>::child>(rc, rc);
+    return f || wt_falls<OBJ, I + 1>(r, rc);
+  }
 }
 PJ_HD uint32_t wt_frac_digits(uint32_t u) { /* of 1..999999999, without the zeros at the end */
   uint32_t nd = 9;
@@ -622,6 +633,7 @@ __device__ __forceinline__ void wt_sum_items(const WtRead& x, WtShared& sh, uint
         RowSnap r;
         r.present = *wt_at<uint8_t>(sh, w8, CObj<E>::present_col, k);
         wt_snap<E, 0, CObj<E>::N>(sh, w8, k, r);
+        if (x.dirty && wt_falls<E>(r, r)) bad = true;
         bool first = true;
         n = wt_size<SCHEMA, E, 0, CObj<E>::N>(x, sh, w8, k - base, r, r, nullptr, nullptr, 0, first, bad) + 2u + first;
       }
@@ -644,6 +656,7 @@ __device__ __forceinline__ void wt_size_records(const WtRead& x, WtShared& sh, c
     lists[0] = wt_list<0>(sh, w8, r.a[WT_LIST_STR], r.b[WT_LIST_STR], *wt_at<uint32_t>(sh, w8, FK<OBJ, WT_LIST_STR>::col, row - lane), bad);
     lists[1] = wt_list<1>(sh, w8, r.a[WT_LIST_OBJ], r.b[WT_LIST_OBJ], *wt_at<uint32_t>(sh, w8, FK<OBJ, WT_LIST_OBJ>::col, row - lane), bad);
   }
+  if (x.dirty && wt_falls<OBJ>(r, rc)) bad = true;
   bool first = true;
   uint32_t list_at[2] = {WT_NONE, WT_NONE};
   const uint32_t n0 = wt_size<SCHEMA, OBJ, 0, WtMid<OBJ>::v>(x, sh, w8, index, r, rc, lists, list_at, 0, first, bad);

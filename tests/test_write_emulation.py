@@ -146,6 +146,56 @@ def test_literals_out_of_range_and_present_bits(writer, oracle):
     write(writer, ORDER, cols, oracle.write(ORDER, cols, NDJSON, abi.PJ_INCLUDE_NON_NULL))
 
 
+def fall(off, row, by):
+    """The range of string `row` goes back by `by` bytes: the string behind it shares them."""
+    off[row + 1] = off[row] - by
+
+
+@pytest.mark.parametrize("recs", [3, 32, 128])
+def test_offsets_that_fall_where_no_string_is(writer, oracle, recs):
+    """A string that is absent, or not written, may have any offsets: what two rows then share is escaped in both."""
+    rng = random.Random(recs)
+    esc = [b'\\"', b"\\n", b"\\u0001", b"x"]
+    word = lambda k: b"".join(rng.choice(esc) for _ in range(k))
+    # a table of Users: every string column falls at rows of its own
+    n = 96
+    keys = [b"username", b"firstName", b"lastName", b"email", b"password", b"phone"]
+    cols = oracle.parse(USER, as_u8(b"\n".join(b'{"id":%d,%s}' % (i, b",".join(b'"%s":"%s"' % (k, word(12)) for k in keys)) for i in range(n))))
+    present = cols.arrays[COL["usr_present"]]
+    for f, name in enumerate(["username", "firstname", "lastname", "email", "password", "phone"]):
+        off = cols.arrays[COL[f"usr_{name}_off"]].view(np.uint32)
+        for row in range(1 + f, n - 1, 7):
+            present[row] &= ~(2 << f) & 0xFF
+            fall(off, row, 9)
+    for inclusion in INCLUSIONS:
+        write(writer, USER, cols, oracle.write(USER, cols, NDJSON, inclusion), inclusion=inclusion, recs=recs)
+    # Pets: a category that is not there, a category's name, an element's name
+    n = 64
+    pet = b'{"id":%d,"category":{"id":1,"name":"%s"},"name":"%s","photoUrls":["%s"],"tags":[{"id":2,"name":"%s"},{"id":3,"name":"%s"}]}'
+    for where in ("category", "category name", "name", "tag name", "photo"):
+        cols = oracle.parse(PET, as_u8(b"\n".join(pet % ((i,) + tuple(word(12) for _ in range(5))) for i in range(n))))
+        assert cols.n_errors == 0
+        a = {k: cols.arrays[v] for k, v in COL.items() if k.startswith("pet_")}
+        for row in range(1, n - 1, 5):
+            if where == "category":
+                a["pet_present"][row] &= ~2 & 0xFF
+                fall(a["pet_cat_name_off"].view(np.uint32), row, 7)
+            elif where == "category name":
+                a["pet_cat_present"][row] &= ~2 & 0xFF
+                fall(a["pet_cat_name_off"].view(np.uint32), row, 7)
+            elif where == "name":
+                a["pet_present"][row] &= ~4 & 0xFF
+                fall(a["pet_name_off"].view(np.uint32), row, 7)
+            elif where == "tag name":
+                a["pet_tag_present"][2 * row] &= ~2 & 0xFF
+                fall(a["pet_tag_name_off"].view(np.uint32), 2 * row, 7)
+            else:
+                a["pet_present"][row] &= ~8 & 0xFF
+                fall(a["pet_photo_str_off"].view(np.uint32), row, 7)
+        for inclusion in INCLUSIONS:
+            write(writer, PET, cols, oracle.write(PET, cols, NDJSON, inclusion), inclusion=inclusion, recs=recs)
+
+
 def test_no_records(writer, oracle):
     cols = abi.HostColumns(PET, abi.default_caps(PET, 1, 16))
     n = C.c_uint64()
