@@ -111,6 +111,7 @@ struct pj_ctx {
   Buffer out_stage; /* device copy of a host output (writer) */
   Buffer tiles;     /* look-back state of the tile kernel + its ticket */
   DevResult* d_res = nullptr; /* [PJ_CTX_RESULTS]: one per piece of a call; [0] serves every other call */
+  uint32_t* d_looks = nullptr; /* [ND_LOOKS], behind them */
   DevResult* h_res = nullptr; /* pinned, same shape */
   uint8_t *h_in = nullptr, *h_out = nullptr; /* pinned, FETCH_ROOM each (behind h_res): columns of small calls on their way there and back */
   cudaEvent_t ev[10] = {};
@@ -355,12 +356,22 @@ bool take_columns(pj_ctx* c, const ParsePlan& pp, const FetchArgs& fa, pj_column
   }
   return true;
 }
+/* the same look as the device's, for input that is in host memory and on its way in pieces */
+bool nd_host_looks_long(const uint8_t* in, uint64_t len) {
+  uint32_t n = 0;
+  for (uint32_t k = 0; k < ND_LOOKS; ++k) {
+    const uint8_t *p = in + nd_look_at(len, k), *end = p + ND_LOOK_BYTES;
+    while ((p = (const uint8_t*)memchr(p, '\n', (size_t)(end - p))) != nullptr) { ++n; ++p; }
+  }
+  return nd_looks_long(n);
+}
 /* NDJSON: one launch of a parse kernel per piece. Host buffers of a whole stream are parsed in pieces cut after line
  * feeds, so that the copy of piece p+1 to the device, the kernel of piece p and the copy of the columns of piece p-1
  * back run at the same time on three streams. Every launch is enqueued before the host waits for anything: a piece
- * starts where the piece before it ended, which it reads from that piece's totals ON THE DEVICE (StreamArgs.prev). */
+ * starts where the piece before it ended, which it reads from that piece's totals ON THE DEVICE (StreamArgs.prev).
+ * again: k_parse_items put the call aside, whose input is on the device by now. */
 pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t len, uint64_t slack, int is_first, int is_last,
-                       uint64_t goff, uint32_t in_kind, pj_columns* out) {
+                       uint64_t goff, uint32_t in_kind, pj_columns* out, bool again = false) {
   const uint64_t limit = len + slack;
   ParsePlan pp;
   { pj_status st = plan_columns(c, schema, out, limit, false, &pp); if (st) return st; }
@@ -414,7 +425,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     if (st) return st;
     d_in = (const uint8_t*)c->in_stage.p;
     if (pipe) { PJ_CUDA(c, cudaEventRecord(c->ev_in[0], c->stream)); PJ_CUDA(c, cudaStreamWaitEvent(s_in, c->ev_in[0], 0)); }
-    for (int p = 0; p < np; ++p) {
+    for (int p = 0; p < np && !again; ++p) {
       const uint64_t nb = cut[p + 1] - cut[p] + (p == np - 1 ? slack : 0);
       if (nb) PJ_CUDA(c, cudaMemcpyAsync((uint8_t*)c->in_stage.p + cut[p], in + cut[p], nb, cudaMemcpyHostToDevice, s_in));
       if (pipe) PJ_CUDA(c, cudaEventRecord(c->ev_in[p], s_in));
@@ -424,7 +435,11 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
 
   uint64_t longest = 0;
   for (int p = 0; p < np; ++p) longest = cut[p + 1] - cut[p] > longest ? cut[p + 1] - cut[p] : longest;
-  const bool items = c->opt_flags & PJ_OPT_TEST_ITEMS ? true : (c->opt_flags & PJ_OPT_TEST_RECORDS ? false : c->choice[schema].items);
+  bool items = c->opt_flags & PJ_OPT_TEST_ITEMS ? true : (c->opt_flags & PJ_OPT_TEST_RECORDS ? false : c->choice[schema].items && !again);
+  /* streams of several models: long records are not for k_parse_items; it finds out, the host does where the input comes piece by piece */
+  bool look = items && c->choice[schema].several && !(c->opt_flags & PJ_OPT_TEST_ITEMS) && len >= ND_LONG;
+  bool aside = again;
+  if (look && pipe) { aside = nd_host_looks_long(in, len); items = !aside; look = false; }
   const ItemShape shape = pick_tile_shape(c, schema, longest);
   const uint32_t tile_bytes = items ? shape.tile_bytes : pick_stream_tile(c, schema);
   const size_t state = items ? sizeof(ItemTile) : sizeof(StreamTile);
@@ -441,15 +456,23 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   const bool small = np == 1 && limit <= SMALL_CALL;
   FetchArgs fa;
   fa.n = 0;
-  if (small) {
-    fetch_columns(pp, out, limit, &fa);
-    ResetArgs ra;
-    ra.state = (unsigned long long*)c->tiles.p; ra.words = (nt_total * state + 256) / 8; ra.more = nullptr; ra.more_words = 0; ra.res = c->d_res;
-    k_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
+  ResetArgs ra;
+  memset(&ra, 0, sizeof ra);
+  if (small) fetch_columns(pp, out, limit, &fa);
+  if (small || (look && np == 1)) {
+    ra.state = (unsigned long long*)c->tiles.p; ra.words = (nt_total * state + 256) / 8; ra.res = c->d_res;
+    if (look) { ra.in = d_in; ra.len = len; ra.looks = c->d_looks; }
+    const int grid = persistent_grid(c, ra.words, 256);
+    k_reset<<<look && grid < (int)ND_LOOKS ? (int)ND_LOOKS : grid, 256, 0, c->stream>>>(ra);
     count_launch(c, 0);
   } else {
     PJ_CUDA(c, cudaMemsetAsync(c->tiles.p, 0, nt_total * state + (size_t)np * 256, c->stream));
     PJ_CUDA(c, cudaMemsetAsync(c->d_res, 0, sizeof(DevResult) * np, c->stream));
+    if (look) {
+      ra.res = c->d_res; ra.in = d_in; ra.len = len; ra.looks = c->d_looks;
+      k_reset<<<ND_LOOKS, 256, 0, c->stream>>>(ra);
+      count_launch(c, 0);
+    }
   }
   if (c->stall_once) { /* test hook: tickets start at 1, tile 0 is never processed, the waits for it run out */
     c->stall_once = false;
@@ -481,6 +504,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
     tiles_at += nt[p];
     sa.res = c->d_res + p;
     sa.prev = p ? c->d_res + p - 1 : nullptr;
+    sa.looks = look ? c->d_looks : nullptr;
     for (uint32_t k = 0; k < NSLOT; ++k) sa.slot_cap[k] = pp.slot_cap[k];
     sa.rec_cap = pp.rec_cap;
     sa.plan = pp.plan;
@@ -518,6 +542,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   for (int p = 0; p < np; ++p) {
     PJ_CUDA(c, cudaEventSynchronize(c->ev_done[p]));
     const DevResult& r = c->h_res[p];
+    if (r.aside) return parse_stream(c, schema, in, len, slack, is_first, is_last, goff, in_kind, out, true); /* (then of every piece) */
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, c->ev_k0[p], c->ev_k1[p]) == cudaSuccess) { c->stats.stage_ms[2] += ms; c->stats.device_ms += ms; }
     n_fast += items ? r.n_fast : r.n_fast & 0xFFFFFFFFull; n_errors += r.n_errors;
@@ -558,7 +583,8 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
   const pj_status st = finish_columns(c, schema, len, pp, rows_done, n_errors, total, over, out);
   if (st) return st;
   if (rows_done > 1000 && !c->tile_bytes_opt) { c->avg_rec_bytes[schema] = (double)len / (double)rows_done; if (items) { c->max_rec_bytes[schema] = max_rec; c->strs_per_kb[schema] = strs_per_kb; } }
-  note_call(c->choice[schema], len, c->stats.stage_ms[2], rows_done, n_errors, n_fast, n_dense, max_rec);
+  if (aside) note_aside(c->choice[schema]);
+  else note_call(c->choice[schema], len, c->stats.stage_ms[2], rows_done, n_errors, n_fast, n_dense, max_rec);
   if (host_out) PJ_CUDA(c, cudaStreamSynchronize(s_out));
   return PJ_OK;
 }
@@ -759,8 +785,9 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
     if (e != cudaSuccess) return fail_create(e, "cudaStreamCreate");
     c->own_stream = true;
   }
-  e = cudaMalloc(&c->d_res, sizeof(DevResult) * PJ_CTX_RESULTS);
+  e = cudaMalloc(&c->d_res, sizeof(DevResult) * PJ_CTX_RESULTS + sizeof(uint32_t) * ND_LOOKS);
   if (e != cudaSuccess) return fail_create(e, "cudaMalloc");
+  c->d_looks = (uint32_t*)(c->d_res + PJ_CTX_RESULTS);
   const size_t res_bytes = align_up(sizeof(DevResult) * PJ_CTX_RESULTS, 4096);
   e = cudaMallocHost(&c->h_res, res_bytes + 2 * FETCH_ROOM);
   if (e != cudaSuccess) return fail_create(e, "cudaMallocHost");
@@ -1074,7 +1101,8 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
   ta.recs = shape.recs; ta.smem = shape.smem;
   ta.spin_limit_ns = c->spin_ns;
   ResetArgs ra;
-  ra.state = (unsigned long long*)c->tiles.p; ra.words = 32 + 2 * ntiles; ra.more = nullptr; ra.more_words = 0; ra.res = c->d_res;
+  memset(&ra, 0, sizeof ra);
+  ra.state = (unsigned long long*)c->tiles.p; ra.words = 32 + 2 * ntiles; ra.res = c->d_res;
   Stage stage(c);
   k_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
   count_launch(c, 0);

@@ -8,6 +8,8 @@
 
 namespace pj {
 
+static constexpr uint64_t ND_LONG = 16384; /* bytes per record */
+
 /* Which kernel a schema's next call takes, and what note_call() remembers of the calls before. */
 struct NdChoice {
   bool items = false;           /* k_parse_items, else k_parse_stream */
@@ -15,7 +17,9 @@ struct NdChoice {
   bool handed_back = false;     /* the last change was back, because the text was all in one compact spelling */
   uint32_t clean = 0, wait = 1; /* such calls in a row, and how many it takes */
   double ns[2] = {0, 0};        /* per input byte, of the last timed call with k_parse_stream / k_parse_items, */
-  uint64_t len[2] = {0, 0};     /* and that call's bytes */
+  uint64_t len[2] = {0, 0};     /* that call's bytes */
+  uint64_t per[2] = {0, 0};     /* and its records' */
+  uint32_t aside = 0;           /* several: calls in a row that k_parse_items put aside because of their long records */
   double tried = 0;             /* what k_parse_stream takes for the text that k_parse_items was last slower on, */
   uint32_t spared = 0;          /* and calls on such text since */
 };
@@ -28,19 +32,26 @@ struct NdChoice {
  * Streams of several models start with k_parse_items and stay with it: it sorts a tile's lines by model, where a warp of the other one runs the
  * three models' code one after the other (300k records, us: compact 312 / 250, 1 % malformed 371 / 283); only text that leaves its records to
  * the exact parser has the other one tried, and then the time decides.
- * Records of 16 KB leave its blocks too little to do side by side: they are not tried (300 Pets of 40 KB: 0.5 / 15.6 ms). The
- * result does not depend on the choice. */
+ * Records of 16 KB leave its blocks too little to do side by side: they are not tried (300 Pets of 40 KB: 0.5 / 15.6 ms), and such calls on
+ * streams of several models are put aside when a look at some of their bytes shows them (pj_index.cuh). Times are only compared between calls
+ * of like bytes and like record length. The result does not depend on the choice. */
 inline void note_call(NdChoice& k, uint64_t len, float ms, uint64_t records, uint64_t errors, uint64_t fast, uint64_t dense, uint32_t max_rec) {
   if (records < 16 && len < (1u << 16)) return;
+  const uint64_t per = len / (records ? records : 1);
+  if (k.several && per >= ND_LONG) { /* says nothing of usual records, which have k_parse_items again */
+    k.items = false;
+    return;
+  }
+  k.aside = 0;
   const bool timed = len >= (1u << 18); /* below, a call's time is not its text's */
   const int now = k.items ? 1 : 0, other = 1 - now;
-  if (timed) { k.ns[now] = ms * 1e6 / (double)len; k.len[now] = len; }
-  const bool alike = timed && k.len[other] && k.len[other] / 2 <= len && len / 2 <= k.len[other]; /* the two can be compared */
+  if (timed) { k.ns[now] = ms * 1e6 / (double)len; k.len[now] = len; k.per[now] = per; }
+  const bool alike = timed && k.len[other] && k.len[other] / 2 <= len && len / 2 <= k.len[other] && k.per[other] / 2 <= per && per / 2 <= k.per[other]; /* the two can be compared */
   const bool lost = alike && k.ns[other] < k.ns[now];
   const uint64_t good = records - errors;
   if (!k.items) {
     if (!k.several && fast * 100 >= good * 98 && dense * 2 >= good) return;
-    if (len / (records ? records : 1) >= 16384) return;
+    if (per >= ND_LONG) return;
     if (k.handed_back && alike && !lost) k.tried = k.ns[0];
     /* text as that which k_parse_items was slower on; every 64th such call tries all the same */
     if (timed && k.ns[0] < k.tried * 1.15 && k.ns[0] > k.tried * 0.87 && ++k.spared < 64) return;
@@ -50,11 +61,15 @@ inline void note_call(NdChoice& k, uint64_t len, float ms, uint64_t records, uin
   } else if (lost) {
     k.tried = k.ns[0];
     k.items = k.handed_back = false;
-  } else if (k.several && (len / (records ? records : 1) >= 16384 || (timed && !alike && fast * 100 < good * 98))) {
+  } else if (k.several && timed && !alike && fast * 100 < good * 98) {
     k.items = false; k.handed_back = true;
   } else if (!k.several && dense * 100 >= good * 99 && max_rec <= 1024) {
     if (++k.clean >= k.wait) { k.items = false; k.handed_back = true; }
   } else k.clean = 0;
+}
+/* ... and when a call was put aside: the second in a row takes the next one to k_parse_stream at once. */
+inline void note_aside(NdChoice& k) {
+  if (++k.aside >= 2) k.items = false;
 }
 
 }  // namespace pj

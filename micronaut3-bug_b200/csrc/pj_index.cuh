@@ -6,9 +6,17 @@
 #ifndef PJ_INDEX_CUH
 #define PJ_INDEX_CUH
 
+#include "pj_choice.h"
 #include "pj_core.cuh"
 
 namespace pj {
+
+/* NDJSON of several models: how long its records are is looked up in ND_LOOKS pieces of ND_LOOK_BYTES, spread over an input of ND_LONG bytes or
+ * more, by counting line feeds; k_parse_items then leaves long records to k_parse_stream before any of its blocks has begun (pj_choice.h). */
+static constexpr uint32_t ND_LOOKS = 64, ND_LOOK_BYTES = 4096;
+static_assert(ND_LONG > ND_LOOK_BYTES, "an input that is looked at holds a piece");
+PJ_HD uint64_t nd_look_at(uint64_t len, uint32_t k) { return (len - ND_LOOK_BYTES) / (ND_LOOKS - 1u) * k; }
+PJ_HD bool nd_looks_long(uint32_t line_feeds) { return line_feeds * ND_LONG <= (uint64_t)ND_LOOKS * ND_LOOK_BYTES; }
 
 /* NDJSON: p is the first byte of a line (byte 0 of the stream or the byte after an LF). The line is
  * a record unless it holds only space / tab / CR. A line that runs into the end of the readable

@@ -90,6 +90,7 @@ struct ItemArgs {
   uint32_t* ticket;
   DevResult* res;
   const DevResult* prev;    /* totals of the pieces of the same call parsed by earlier launches (null: none) */
+  const uint32_t* looks;    /* several models: [ND_LOOKS] line feeds in pieces of the input (null: whatever it is) */
   uint64_t slot_cap[NSLOT]; /* largest total per slot the caller's buffers can take */
   uint64_t rec_cap;         /* records the per-record and row-indexed buffers can take */
   FinalizePlan plan;
@@ -147,6 +148,7 @@ struct ItemShared {
   uint32_t free_word;                      /* first free word behind the strings */
   uint32_t ndense;                         /* lines the dense walk took */
   uint32_t ok, slow, tile, next, apart;    /* apart: a record of the tile stands apart */
+  uint32_t aside;                          /* the input is left to k_parse_stream */
   unsigned long long mbar;
 };
 
@@ -2368,9 +2370,19 @@ __global__ void __launch_bounds__(IT_THREADS, IT_BLOCKS) k_parse_items(const __g
   uint32_t* rows = reinterpret_cast<uint32_t*>(smem + lay.rows);
 
   if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); mbar_init(&sh.mbar, 1); sh.slow = 0; sh.next = 0; sh.odd = 0; sh.nspecial = 0; sh.apart = 0; }
+  if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+    if (a.looks && (tid >> 5) == 1u) { /* (beside the ticket's way to memory and back) */
+      static_assert(ND_LOOKS == 64, "two each");
+      const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, a.looks[tid & 31u] + a.looks[tid]);
+      if (tid == 32u) sh.aside = nd_looks_long(n);
+    } else if (tid == 32u) sh.aside = 0;
+  }
   __syncthreads();
   const uint32_t tile = sh.tile;
   if (tile >= a.ntiles) return;
+  if constexpr (SCHEMA == PJ_SCHEMA_MIXED) {
+    if (sh.aside) { if (tile == 0 && tid == 0) a.res->aside = 1u; return; }
+  }
   long long ck[5];
   ck[0] = clock64();
   const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(a.in) & 15u);

@@ -201,7 +201,21 @@ struct ResetArgs {
   unsigned long long *state, *more; /* tickets, look-back words; a bitmap that is or-ed into (or null) */
   uint64_t words, more_words;
   DevResult* res;
+  const uint8_t* in; /* the input and where the line feeds in pieces of it go (or null), see nd_look_at() */
+  uint64_t len;
+  uint32_t* looks;
 };
+/* line feeds of piece k; a block of ND_LOOK_BYTES / 16 threads */
+__device__ __forceinline__ uint32_t nd_look(const uint8_t* in, uint64_t len, uint32_t k, uint32_t* sh) {
+  const uint8_t* p = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(in + nd_look_at(len, k)) & ~(uintptr_t)15) + 16u * threadIdx.x;
+  uint32_t n = 0;
+  if (p >= in && p + 16 <= in + len) n = (uint32_t)__popcll(lf_mask64(p, 16));
+  if (threadIdx.x == 0) *sh = 0;
+  __syncthreads();
+  if (n) atomicAdd(sh, n);
+  __syncthreads();
+  return *sh;
+}
 /* no ticket taken, no tile's totals known, nothing counted */
 static __global__ void __launch_bounds__(256) k_reset(const __grid_constant__ ResetArgs a) {
   const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
@@ -215,7 +229,13 @@ static __global__ void __launch_bounds__(256) k_reset(const __grid_constant__ Re
       r[k] = none ? 0xFFFFFFFFu : (at == offsetof(DevResult, ok) ? 1u : 0u);
     }
   }
+  if (a.looks && blockIdx.x < ND_LOOKS) {
+    __shared__ uint32_t sh;
+    const uint32_t n = nd_look(a.in, a.len, blockIdx.x, &sh);
+    if (threadIdx.x == 0) a.looks[blockIdx.x] = n;
+  }
 }
+static_assert(ND_LOOK_BYTES == 16 * 256, "16 bytes a thread");
 /* closes the text: brackets of array framing, the total, the verdict; the result goes to host memory (one warp) */
 static __global__ void k_write_close(const __grid_constant__ WriteArgs a, DevResult* host) {
   if (threadIdx.x == 0) {

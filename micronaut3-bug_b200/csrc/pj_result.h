@@ -19,6 +19,7 @@ struct DevResult {
   uint32_t ok;      /* every output fits its buffer */
   uint32_t over;    /* stream kernel: some output does not fit its buffer */
   uint32_t timeout; /* a bounded wait ran out */
+  uint32_t aside;   /* k_parse_items: left to k_parse_stream, nothing done */
   unsigned long long n_fast;  /* records decoded by the speculative pass alone; k_parse_stream: low half, in the high half those its warps took in step */
   unsigned long long phase_cycles[4]; /* tile kernel, summed over blocks: staging, tokenising, look-back, emit */
   unsigned long long lookback_polls, lookback_rounds;

@@ -113,3 +113,42 @@ def test_one_long_record_then_a_call_of_few_tiles(oracle):
     with pj.Context(device=0) as c:
         for _ in range(3):
             assert same_result(want, gpu_parse_device(c, 3, body, ARRAY)) == ""
+
+
+def long_pets(n, name):
+    return b"\n".join(b'{"id":%d,"name":"%s","photoUrls":["u%d"]}' % (i, b"n" * (name + i % 7), i) for i in range(n))
+
+
+@pytest.mark.parametrize("offset", [0, 5])
+@pytest.mark.parametrize("name", [16_400, 40_000])
+def test_long_records_of_several_models_are_put_aside(oracle, name, offset):
+    """A fresh context's first call on them does not wait for the kernel it starts with; the third in a row does not ask any more; usual records have it again."""
+    long_ = as_u8(long_pets(40, name))
+    usual = pj.gen_text(4, 11, 0, 20_000, abi.PJ_GEN_MALFORMED)
+    took = []
+    with pj.Context(device=0) as c:
+        for body in (long_, long_, long_, usual, usual):
+            assert same_result(oracle.parse(4, body), gpu_parse_device(c, 4, body, NDJSON, offset)) == ""
+            s = c.stats()
+            took.append((s.stage_launches[2], s.stage_launches[3]))
+    assert took == [(2, 1), (2, 1), (1, 0), (1, 0), (1, 1)], took
+
+
+@pytest.mark.parametrize("kw", [dict(host_piece_bytes=1 << 18), dict(device_piece_bytes=300_001)])
+def test_long_records_in_pieces(oracle, kw):
+    body = as_u8(long_pets(60, 30_000) + b"\n" + bytes(pj.gen_text(4, 5, 0, 4, 0)))
+    with pj.Context(device=0, **kw) as c:
+        for _ in range(2):
+            got = gpu_parse_host(c, 4, body) if "host_piece_bytes" in kw else gpu_parse_device(c, 4, body, NDJSON, 3)
+            assert same_result(oracle.parse(4, body), got) == ""
+            s = c.stats()
+            assert s.pieces > 1 and s.stage_launches[3] == (0 if "host_piece_bytes" in kw else s.pieces)
+
+
+def test_few_bytes_of_several_models(items_ctx, oracle):
+    """Around the input size that is looked at; one line, and line feeds only."""
+    with pj.Context(device=0) as c:
+        for body in (b"\n" * 16_383, b"\n" * 16_384, b" " * 16_384, long_pets(1, 16_384), long_pets(1, 16_300), long_pets(1, 300_000)):
+            for off in (0, 1, 15):
+                assert same_result(oracle.parse(4, as_u8(body)), gpu_parse_device(c, 4, body, NDJSON, off)) == ""
+            assert same_result(oracle.parse(4, as_u8(body)), gpu_parse_host(c, 4, body)) == ""

@@ -48,3 +48,16 @@ def test_records_of_16_kb(note):
     assert note(1.0, records=100, per=40_000) is False
     assert note(0.1, records=100, per=40_000) is False
     assert note(0.1) is True  # records of a usual size: back again
+
+
+def test_long_records_between_usual_ones(note):
+    """Calls of both kinds and of like size in turn: long records say nothing of what the kernels take for usual ones."""
+    note.reset()
+    items, seen = True, []
+    for k in range(60):
+        seen.append(items)
+        if k % 3 == 0:  # 300 records of 40 KB
+            items = note(15.6 if items else 0.5, records=300, per=40_000)
+        else:           # 20 MB of usual ones
+            items = note(0.25 if items else 0.31)
+    assert all(seen[k] for k in range(60) if k % 3 == 2), seen
