@@ -33,8 +33,9 @@ struct NdChoice {
  * three models' code one after the other (300k records, us: compact 312 / 250, 1 % malformed 371 / 283); only text that leaves its records to
  * the exact parser has the other one tried, and then the time decides.
  * Records of 16 KB leave its blocks too little to do side by side: they are not tried (300 Pets of 40 KB: 0.5 / 15.6 ms), and such calls on
- * streams of several models are put aside when a look at some of their bytes shows them (pj_index.cuh). Times are only compared between calls
- * of like bytes and like record length. The result does not depend on the choice. */
+ * streams of several models are put aside when a look at some of their bytes shows them (pj_index.cuh). Their times are only compared between
+ * calls of like record length; one model's are by bytes alone, so that a call on longer records finds its way back (it is not put aside). The
+ * result does not depend on the choice. */
 inline void note_call(NdChoice& k, uint64_t len, float ms, uint64_t records, uint64_t errors, uint64_t fast, uint64_t dense, uint32_t max_rec) {
   if (records < 16 && len < (1u << 16)) return;
   const uint64_t per = len / (records ? records : 1);
@@ -46,7 +47,7 @@ inline void note_call(NdChoice& k, uint64_t len, float ms, uint64_t records, uin
   const bool timed = len >= (1u << 18); /* below, a call's time is not its text's */
   const int now = k.items ? 1 : 0, other = 1 - now;
   if (timed) { k.ns[now] = ms * 1e6 / (double)len; k.len[now] = len; k.per[now] = per; }
-  const bool alike = timed && k.len[other] && k.len[other] / 2 <= len && len / 2 <= k.len[other] && k.per[other] / 2 <= per && per / 2 <= k.per[other]; /* the two can be compared */
+  const bool alike = timed && k.len[other] && k.len[other] / 2 <= len && len / 2 <= k.len[other] && (!k.several || (k.per[other] / 2 <= per && per / 2 <= k.per[other])); /* the two can be compared */
   const bool lost = alike && k.ns[other] < k.ns[now];
   const uint64_t good = records - errors;
   if (!k.items) {
