@@ -13,6 +13,7 @@ struct WOut {
   uint8_t* dst;
   uint32_t hexa = 'A'; /* first letter of the hex digits of \u00xx escapes: 'A', or 'a' with PJ_OPT_HEX_LOWER */
   uint64_t n;
+  uint32_t escapes = 0; /* measured: not 0 when a byte has to be escaped */
 };
 template <bool WR>
 PJ_HD void wput(WOut& w, uint32_t b) {
@@ -42,23 +43,38 @@ template <bool WR>
 PJ_HD void wput_2d(WOut& w, uint32_t v) { wput<WR>(w, '0' + v / 10); wput<WR>(w, '0' + v % 10); }
 
 /* bytes the escapes of W3 add to the n bytes at s: 1 for the two-character escapes, 5 for \u00XX.
- * Reads aligned 4-byte words where it can and looks closer only at words that hold a byte to escape. */
+ * Reads the aligned 4-byte words that hold them and looks closer only at words that hold a byte to escape. */
 PJ_HD uint32_t escape_extra_byte(uint32_t c) {
   if (c >= 0x20) return (c == '"' || c == '\\') ? 1u : 0u;
   return (c == 8 || c == 9 || c == 10 || c == 12 || c == 13) ? 1u : 5u;
 }
-PJ_HD uint32_t str_escape_extra(const uint8_t* s, uint32_t n) {
-  uint32_t extra = 0, i = 0;
-  while (i < n && ((uintptr_t)(s + i) & 3u)) extra += escape_extra_byte(ld_byte(s + i++));
-  for (; i + 4 <= n; i += 4) {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(s + i);
-    const uint32_t xq = w ^ 0x22222222u, xb = w ^ 0x5C5C5C5Cu;
-    const uint32_t m = ((w - 0x20202020u) & ~w) | ((xq - 0x01010101u) & ~xq) | ((xb - 0x01010101u) & ~xb);
-    if (m & 0x80808080u)
-      for (uint32_t k = 0; k < 4; ++k) extra += escape_extra_byte((w >> (8 * k)) & 0xFFu);
-  }
-  for (; i < n; ++i) extra += escape_extra_byte(ld_byte(s + i));
+/* not 0 when a byte of x has to be escaped */
+PJ_HD uint32_t word_needs_escape(uint32_t x) {
+  const uint32_t xq = x ^ 0x22222222u, xb = x ^ 0x5C5C5C5Cu;
+  return (((x - 0x20202020u) & ~x) | ((xq - 0x01010101u) & ~xq) | ((xb - 0x01010101u) & ~xb)) & 0x80808080u;
+}
+PJ_HD uint32_t word_escape_extra(uint32_t x) {
+  uint32_t extra = 0;
+  for (uint32_t k = 0; k < 4; ++k) extra += escape_extra_byte((x >> (8 * k)) & 0xFFu);
   return extra;
+}
+PJ_HD uint32_t str_escape_extra(const uint8_t* s, uint32_t n) {
+  if (!n) return 0;
+  const uint32_t lead = (uint32_t)((uintptr_t)s & 3u), last = (lead + n - 1u) >> 2, end = (lead + n) & 3u;
+  const uint32_t* p = reinterpret_cast<const uint32_t*>((uintptr_t)s & ~(uintptr_t)3);
+  const uint32_t letters = 0x61616161u, tail = end ? letters << (8 * end) : 0u, keep = end ? ~(0xFFFFFFFFu << (8 * end)) : 0xFFFFFFFFu; /* bytes that are not the string's count as letters */
+  uint32_t extra = 0, k = 0;
+  uint32_t x = p[0];
+  if (lead) x = (x & (0xFFFFFFFFu << (8 * lead))) | letters >> (32 - 8 * lead);
+  for (; k < last; x = p[++k]) {
+    if (word_needs_escape(x)) extra += word_escape_extra(x);
+    for (; k + 4 < last; k += 4) { /* four words on their way at a time */
+      const uint32_t a = p[k + 1], b = p[k + 2], c = p[k + 3], d = p[k + 4];
+      if (word_needs_escape(a) | word_needs_escape(b) | word_needs_escape(c) | word_needs_escape(d)) extra += word_escape_extra(a) + word_escape_extra(b) + word_escape_extra(c) + word_escape_extra(d);
+    }
+  }
+  x = (x & keep) | tail;
+  return extra + (word_needs_escape(x) ? word_escape_extra(x) : 0u);
 }
 
 /* W3 */

@@ -4,7 +4,7 @@
  * what differs is how it gets there: property names, kinds and columns are template constants, so a
  * record is a straight line of loads and stores; `"name":` is stored from immediates; integers are
  * converted in 8-digit groups with 32-bit arithmetic; strings without a byte to escape are copied
- * four bytes per load.
+ * four bytes per load. The writer's general road (pj_write_tile.cuh) takes it, a record per thread.
  */
 #ifndef PJ_WRITE_FAST_CUH
 #define PJ_WRITE_FAST_CUH
@@ -108,7 +108,7 @@ PJ_HD void copy_bytes_fast(uint8_t* d, const uint8_t* s, uint32_t n) {
 }
 
 /* W3 with the common case first: the string has no byte to escape. PLAIN: the caller knows that no string
- * of the column set has a byte to escape, so lengths need no look at the bytes and the copy needs no checks. */
+ * of the record has a byte to escape, so the copy needs no checks. */
 template <bool WR, bool PLAIN>
 PJ_HD void fput_str(WOut& w, const uint8_t* s, uint32_t n) {
   if (PLAIN) {
@@ -116,57 +116,29 @@ PJ_HD void fput_str(WOut& w, const uint8_t* s, uint32_t n) {
     w.n += 2 + (uint64_t)n;
     return;
   }
-  if (!WR) { w.n += 2 + (uint64_t)n + str_escape_extra(s, n); return; }
+  if (!WR) { const uint32_t extra = str_escape_extra(s, n); w.n += 2 + (uint64_t)n + extra; w.escapes |= extra; return; }
+  /* four bytes per load, one at a time where there is one to escape (one loop for both, so that a warp's lanes stay together) */
   uint8_t* d = w.dst + w.n;
   *d++ = '"';
-  uint32_t i = 0;
-  bool plain = true;
-  while (i < n && ((uintptr_t)(s + i) & 3u)) {
-    const uint32_t c = ld_byte(s + i);
-    if (escape_extra_byte(c)) { plain = false; break; }
-    *d++ = (uint8_t)c; ++i;
-  }
-  if (plain) {
-    for (; i + 4 <= n; i += 4) {
-      const uint32_t x = *reinterpret_cast<const uint32_t*>(s + i);
-      const uint32_t xq = x ^ 0x22222222u, xb = x ^ 0x5C5C5C5Cu;
-      const uint32_t m = ((x - 0x20202020u) & ~x) | ((xq - 0x01010101u) & ~xq) | ((xb - 0x01010101u) & ~xb);
-      if (m & 0x80808080u) { plain = false; break; }
+  for (uint32_t i = 0; i < n;) {
+    const bool whole = i + 4 <= n && !((uintptr_t)(s + i) & 3u);
+    const uint32_t x = whole ? *reinterpret_cast<const uint32_t*>(s + i) : ld_byte(s + i);
+    if (whole && !word_needs_escape(x)) {
       d[0] = (uint8_t)x; d[1] = (uint8_t)(x >> 8); d[2] = (uint8_t)(x >> 16); d[3] = (uint8_t)(x >> 24);
-      d += 4;
+      d += 4; i += 4;
+      continue;
+    }
+    for (uint32_t k = 0; k < (whole ? 4u : 1u); ++k, ++i) {
+      const uint32_t c = (x >> (8 * k)) & 0xFFu, more = escape_extra_byte(c);
+      if (!more) { *d++ = (uint8_t)c; continue; }
+      d[0] = '\\';
+      d[1] = (uint8_t)(more > 1u ? 'u' : (c == 8 ? 'b' : (c == 9 ? 't' : (c == 10 ? 'n' : (c == 12 ? 'f' : (c == 13 ? 'r' : c))))));
+      if (more > 1u) { d[2] = '0'; d[3] = '0'; d[4] = (uint8_t)('0' + (c >> 4)); d[5] = (uint8_t)((c & 15) < 10 ? '0' + (c & 15) : w.hexa + (c & 15) - 10); }
+      d += 1u + more;
     }
   }
-  if (plain) {
-    for (; i < n; ++i) {
-      const uint32_t c = ld_byte(s + i);
-      if (escape_extra_byte(c)) { plain = false; break; }
-      *d++ = (uint8_t)c;
-    }
-  }
+  *d++ = '"';
   w.n = (uint64_t)(d - w.dst);
-  if (!plain) {
-    /* the rest byte by byte, with the escapes of W3 */
-    for (; i < n; ++i) {
-      const uint32_t c = ld_byte(s + i);
-      if (c >= 0x20 && c != '"' && c != '\\') { wput<WR>(w, c); continue; }
-      wput<WR>(w, '\\');
-      switch (c) {
-        case '"': wput<WR>(w, '"'); break;
-        case '\\': wput<WR>(w, '\\'); break;
-        case 8: wput<WR>(w, 'b'); break;
-        case 9: wput<WR>(w, 't'); break;
-        case 10: wput<WR>(w, 'n'); break;
-        case 12: wput<WR>(w, 'f'); break;
-        case 13: wput<WR>(w, 'r'); break;
-        default:
-          wput<WR>(w, 'u'); wput<WR>(w, '0'); wput<WR>(w, '0');
-          wput<WR>(w, '0' + (c >> 4));
-          wput<WR>(w, (c & 15) < 10 ? '0' + (c & 15) : w.hexa + (c & 15) - 10);
-          break;
-      }
-    }
-  }
-  wput<WR>(w, '"');
 }
 
 template <bool WR, int E, int I = 0>
@@ -177,29 +149,12 @@ PJ_HD void fput_enum(WOut& w, uint32_t e) {
   }
 }
 
-template <bool WR, bool PLAIN, int OBJ, int LEVEL>
-PJ_HD void fwrite_object(const DevCols* c, uint64_t row, int incl, WOut& w);
+/* Values that the caller of a record leaves for later (long strings and lists, which several threads then measure and write): put() takes the one
+ * of `kind` at [a, b) of column col, and the record goes on behind its text. This one leaves none. */
+struct WriteAll { static constexpr bool on = false; };
 
-/* a hint to start fetching the line at p (nothing on the host) */
-PJ_HD void wr_prefetch(const void* p) {
-#if defined(__CUDA_ARCH__)
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-#else
-  (void)p;
-#endif
-}
-/* the scalar columns of flat object E (a list element) at `row` */
-template <int E, int I = 0>
-PJ_HD void wr_prefetch_row(const DevCols* c, uint64_t row) {
-  if constexpr (I == 0) wr_prefetch(colp<uint8_t>(c, CObj<E>::present_col) + row);
-  if constexpr (I < CObj<E>::N) {
-    constexpr uint32_t kind = FK<E, I>::kind, col = FK<E, I>::col;
-    if constexpr (kind == K_I64) wr_prefetch(colp<int64_t>(c, col) + row);
-    else if constexpr (kind == K_I32 || kind == K_STR) wr_prefetch(colp<uint32_t>(c, col) + row);
-    else if constexpr (kind == K_BOOL || kind == K_ENUM) wr_prefetch(colp<uint8_t>(c, col) + row);
-    wr_prefetch_row<E, I + 1>(c, row);
-  }
-}
+template <bool WR, bool PLAIN, int OBJ, int LEVEL, class LATER>
+PJ_HD void fwrite_object(const DevCols* c, uint64_t row, int incl, LATER& later, WOut& w);
 
 /* Every row-indexed value of one object, loaded before any of them is used: the loads are issued back to back and
  * their latencies overlap, instead of one load per property each waiting behind the stores of the one before.
@@ -228,26 +183,14 @@ PJ_HD void snap_row(const DevCols* c, uint64_t row, RowSnap& r) {
 }
 
 /* property I of OBJ and, by recursion, the ones after it */
-template <bool WR, bool PLAIN, int OBJ, int LEVEL, int I = 0>
-PJ_HD void fwrite_fields(const DevCols* c, uint64_t row, int incl, const RowSnap& r, bool& first, WOut& w) {
+template <bool WR, bool PLAIN, int OBJ, int LEVEL, class LATER, int I = 0>
+PJ_HD void fwrite_fields(const DevCols* c, uint64_t row, int incl, const RowSnap& r, bool& first, LATER& later, WOut& w) {
   if constexpr (I < CObj<OBJ>::N) {
     constexpr uint32_t kind = FK<OBJ, I>::kind, col = FK<OBJ, I>::col;
     const bool pr = (r.present >> I) & 1;
     bool empty = false;
     uint32_t a = 0, b = 0;
-    if constexpr (kind == K_STR || kind == K_LIST_STR || kind == K_LIST_OBJ) {
-      a = r.a[I]; b = r.b[I];
-      empty = a == b;
-      if constexpr (!WR && PLAIN) {
-        /* the measuring pass does not look at string bytes or child rows here: ask for them now, the writing pass
-           that follows finds them on their way */
-        if (a < b) {
-          if constexpr (kind == K_STR) wr_prefetch(colp<uint8_t>(c, col + 1) + a);
-          else if constexpr (kind == K_LIST_STR) wr_prefetch(colp<uint8_t>(c, col + 2) + colp<uint32_t>(c, col + 1)[a]);
-          else if constexpr (LEVEL == 0) wr_prefetch_row<FK<OBJ, I>::child>(c, a);
-        }
-      }
-    }
+    if constexpr (kind == K_STR || kind == K_LIST_STR || kind == K_LIST_OBJ) { a = r.a[I]; b = r.b[I]; empty = a == b; }
     if (included(incl, pr, empty)) {
       if (!first) wput<WR>(w, ',');
       first = false;
@@ -262,52 +205,60 @@ PJ_HD void fwrite_fields(const DevCols* c, uint64_t row, int incl, const RowSnap
       } else if constexpr (kind == K_DATETIME) {
         wput_datetime<WR>(w, r.v[I], (int32_t)r.a[I], (int32_t)r.b[I]);
       } else if constexpr (kind == K_STR) {
-        fput_str<WR, PLAIN>(w, colp<uint8_t>(c, col + 1) + a, b - a);
+        bool done = false;
+        if constexpr (LATER::on) done = later.template put<WR>(kind, col + 1, a, b, w);
+        if (!done) fput_str<WR, PLAIN>(w, colp<uint8_t>(c, col + 1) + a, b - a);
       } else if constexpr (kind == K_OBJ) {
-        if constexpr (LEVEL == 0) fwrite_object<WR, PLAIN, FK<OBJ, I>::child, 1>(c, row, incl, w);
+        if constexpr (LEVEL == 0) fwrite_object<WR, PLAIN, FK<OBJ, I>::child, 1>(c, row, incl, later, w);
       } else if constexpr (kind == K_LIST_STR) {
-        const uint32_t* so = colp<uint32_t>(c, col + 1);
-        const uint8_t* data = colp<uint8_t>(c, col + 2);
-        if constexpr (!WR && PLAIN) {
-          /* brackets, and per string two quotes and (but for the first) a comma */
-          w.n += 2 + (a < b ? (uint64_t)(so[b] - so[a]) + 3ull * (b - a) - 1 : 0);
-        } else {
-        wput<WR>(w, '[');
-        uint32_t s0 = a < b ? so[a] : 0;
-        for (uint32_t k = a; k < b; ++k) {
-          if (k > a) wput<WR>(w, ',');
-          const uint32_t s1 = so[k + 1];
-          fput_str<WR, PLAIN>(w, data + s0, s1 - s0);
-          s0 = s1;
-        }
-        wput<WR>(w, ']');
+        bool done = false;
+        if constexpr (LATER::on) done = later.template put<WR>(kind, col + 2, a, b, w);
+        if (!done) {
+          const uint32_t* so = colp<uint32_t>(c, col + 1);
+          const uint8_t* data = colp<uint8_t>(c, col + 2);
+          wput<WR>(w, '[');
+          uint32_t s0 = a < b ? so[a] : 0;
+          for (uint32_t k = a; k < b; ++k) {
+            if (k > a) wput<WR>(w, ',');
+            const uint32_t s1 = so[k + 1];
+            bool one = false;
+            if constexpr (LATER::on) one = later.template put<WR>(K_STR, col + 2, s0, s1, w);
+            if (!one) fput_str<WR, PLAIN>(w, data + s0, s1 - s0);
+            s0 = s1;
+          }
+          wput<WR>(w, ']');
         }
       } else if constexpr (kind == K_LIST_OBJ) {
-        wput<WR>(w, '[');
-        if constexpr (LEVEL == 0)
-          for (uint32_t k = a; k < b; ++k) { if (k > a) wput<WR>(w, ','); fwrite_object<WR, PLAIN, FK<OBJ, I>::child, 1>(c, k, incl, w); }
-        wput<WR>(w, ']');
+        bool done = false;
+        if constexpr (LATER::on) done = later.template put<WR>(kind, 0, a, b, w);
+        if (!done) {
+          wput<WR>(w, '[');
+          if constexpr (LEVEL == 0)
+            for (uint32_t k = a; k < b; ++k) { if (k > a) wput<WR>(w, ','); fwrite_object<WR, PLAIN, FK<OBJ, I>::child, 1>(c, k, incl, later, w); }
+          wput<WR>(w, ']');
+        }
       }
     }
-    fwrite_fields<WR, PLAIN, OBJ, LEVEL, I + 1>(c, row, incl, r, first, w);
+    fwrite_fields<WR, PLAIN, OBJ, LEVEL, LATER, I + 1>(c, row, incl, r, first, later, w);
   }
 }
 /* LEVEL 0: model root; LEVEL 1: Category / Tag */
-template <bool WR, bool PLAIN, int OBJ, int LEVEL>
-PJ_HD void fwrite_object(const DevCols* c, uint64_t row, int incl, WOut& w) {
+template <bool WR, bool PLAIN, int OBJ, int LEVEL, class LATER>
+PJ_HD void fwrite_object(const DevCols* c, uint64_t row, int incl, LATER& later, WOut& w) {
   RowSnap r;
   snap_row<OBJ>(c, row, r);
   bool first = true;
   wput<WR>(w, '{');
-  fwrite_fields<WR, PLAIN, OBJ, LEVEL>(c, row, incl, r, first, w);
+  fwrite_fields<WR, PLAIN, OBJ, LEVEL, LATER>(c, row, incl, r, first, later, w);
   wput<WR>(w, '}');
 }
 
 template <bool WR, bool PLAIN>
 PJ_HD void fwrite_record(const DevCols* c, uint32_t type, uint64_t row, int incl, WOut& w) {
-  if (type == PJ_TYPE_PET) fwrite_object<WR, PLAIN, OBJ_PET, 0>(c, row, incl, w);
-  else if (type == PJ_TYPE_ORDER) fwrite_object<WR, PLAIN, OBJ_ORDER, 0>(c, row, incl, w);
-  else fwrite_object<WR, PLAIN, OBJ_USER, 0>(c, row, incl, w);
+  WriteAll all;
+  if (type == PJ_TYPE_PET) fwrite_object<WR, PLAIN, OBJ_PET, 0>(c, row, incl, all, w);
+  else if (type == PJ_TYPE_ORDER) fwrite_object<WR, PLAIN, OBJ_ORDER, 0>(c, row, incl, all, w);
+  else fwrite_object<WR, PLAIN, OBJ_USER, 0>(c, row, incl, all, w);
 }
 
 }  // namespace pj

@@ -13,11 +13,13 @@
  *  4. Text: the first half of a record's properties, the second half, the strings of its list and the objects of its list are units
  *     of their own, each a lane's, so that the lanes of a warp do the same and long lists are spread over lanes. A lane puts its text
  *     together in a register and stores whole words into a window in shared memory; words that two units share are or-ed.
- *     Strings with a byte to escape are left out and written afterwards, a warp per string.
+ *     Strings with a byte to escape and strings of 512 bytes and more are left out and written afterwards, a warp per string or per 2 KB of it (by the
+ *     lane that meets them, 300 MB of Users: strings of 300 bytes 780 us with it, 940 without; of 1000 bytes 666 and 440).
  *  5. The window leaves with one bulk copy. Text longer than the window goes in several rounds of 4 and 5.
  *
  * Tables whose rows a tile does not find in order (a record map of the caller's own making, offsets of written strings that fall, or of any
- * where there is a byte to escape), or whose strings do not fit shared memory, take the general road: a record per thread (pj_write_fast.cuh).
+ * where there is a byte to escape), or whose strings do not fit shared memory, take the general road: a record per thread (pj_write_fast.cuh), its
+ * long strings and lists by whole warps. So does a record whose text outgrows the window.
  *
  * What bounds it: instruction issue and waiting for one another. 300 k Pets: 180 instructions of a warp per record, a third of the issue slots
  * used; the warps of a block wait for the first one's offsets and look-back, and two or three blocks per SM (shared memory) cover half of that.
@@ -57,7 +59,10 @@ inline uint32_t wt_threads(uint32_t schema) { return schema == PJ_SCHEMA_PET ? W
 static constexpr uint32_t WT_MOST_WARPS = 16;
 static constexpr uint32_t WT_MAX_SMEM = 128 * 1024;
 static constexpr uint32_t WT_MIN_WINDOW = 2048;
-static constexpr uint32_t WT_ESC = 160;             /* strings with escapes a round keeps for later */
+static constexpr uint32_t WT_ESC = 160;             /* strings with escapes, and long ones, a round keeps for later */
+static constexpr uint32_t WT_LONG = 512;            /* bytes of a string that a warp copies */
+static constexpr uint32_t WT_LONG_LIST = 8;         /* elements of a list that a warp writes on the general road */
+static constexpr uint32_t WT_PART = 2048;           /* bytes of a long string a warp takes at a time */
 static constexpr uint32_t WT_HITS = 192;            /* 16-byte blocks with a byte to escape that are kept in a list */
 static constexpr uint32_t WT_BACK = 4;              /* tiles a lane looks back at per round */
 static constexpr uint32_t WT_COLS = 48;             /* columns of a schema */
@@ -157,7 +162,17 @@ static_assert(wt_list_field<OBJ_ORDER>(K_LIST_STR) < 0 && wt_list_field<OBJ_ORDE
 template <int OBJ> struct WtMid { static constexpr int v = CObj<OBJ>::N / 2; };
 static_assert(WT_LIST_STR >= WtMid<OBJ_PET>::v && WT_LIST_OBJ >= WtMid<OBJ_PET>::v, "the lists' places come from one unit");
 
-struct WtEsc { uint32_t at, n, dst; };
+struct WtEsc { uint32_t at, n, dst; }; /* n: bytes | to be escaped << 31 */
+/* General road: a long string or list of a record, measured and written by whole warps. */
+struct WtLater {
+  uint8_t* dst;    /* where its text goes */
+  unsigned long long size; /* bytes of it */
+  uint32_t a, b;   /* bytes of the arena, or elements */
+  uint16_t rec, link; /* the record of the tile; the record's next one */
+  uint8_t kind, col;  /* of the data */
+};
+static constexpr uint32_t WT_LATERS = 192; /* a tile's */
+static constexpr uint16_t WT_LAST = 0xFFFF;
 struct WtShared {
   unsigned long long mbar[3], base;                /* copies of: columns with an element per row; those of list elements; arenas */
   unsigned long long row0[3];                      /* per model: the tile's first row */
@@ -171,18 +186,21 @@ struct WtShared {
   uint32_t nhit;                                   /* 16-byte blocks with a byte to escape */
   uint16_t hit[WT_HITS];
   uint32_t odd, ok, tile, nesc;                    /* odd: the tile takes the general road */
-  uint32_t wsum[WT_MOST_WARPS], cls[3][WT_MOST_WARPS];
+  uint32_t longs, nlater;                          /* some string of the tile is long; how many WtLater */
+  uint16_t ar0[32], ar1[32];                       /* arenas: their first 16-byte block, and one more than the last */
+  uint8_t arcol[32], arlevel[32], armodel[32];
+  union { uint32_t wsum[WT_MOST_WARPS]; unsigned long long wsum8[WT_MOST_WARPS]; };
+  uint32_t cls[3][WT_MOST_WARPS];
   uint32_t pos[WT_MAX_RECS + 1];                   /* a record's bytes, then where it starts in the tile's text */
   uint32_t mid[WT_MAX_RECS];                       /* where its second half starts | no property before it << 31 */
-  uint32_t list[2][WT_MAX_RECS];                   /* where its lists' elements start, from its first byte; WT_NONE: none are written */
+  union {
+    uint32_t list[2][WT_MAX_RECS];                 /* where its lists' elements start, from its first byte; WT_NONE: none are written */
+    unsigned long long bytes[WT_MAX_RECS];         /* general road: a record's bytes, then where it starts */
+  };
   uint8_t perm[WT_MAX_RECS];                       /* mixed: the tile's records by model */
   WtEsc esc[WT_ESC];
 };
 
-__device__ __forceinline__ uint32_t word_needs_escape(uint32_t x) {
-  const uint32_t xq = x ^ 0x22222222u, xb = x ^ 0x5C5C5C5Cu;
-  return (((x - 0x20202020u) & ~x) | ((xq - 0x01010101u) & ~xq) | ((xb - 0x01010101u) & ~xb)) & 0x80808080u;
-}
 /* element `row` of column COL, staged */
 template <class T>
 __device__ __forceinline__ const T* wt_at(const WtShared& sh, const uint8_t* w8, uint32_t col, uint32_t row) { return reinterpret_cast<const T*>(w8 + (uint32_t)(sh.at[col] + row * (uint32_t)sizeof(T))); }
@@ -196,15 +214,17 @@ __device__ __forceinline__ uint32_t wt_extra(const WtShared& sh, const uint8_t* 
 struct WtRead { /* what the units of a tile read */
   int incl;
   bool dirty; /* some string of the tile has to be escaped */
+  bool later; /* ... or is long: not all are written where they are met */
   uint32_t hexa;
 };
 /* length of string [x, y) of arena COL, quotes and escapes included; index: its number among the tile's strings of the arena. Sets bad when it
  * does not lie in what is staged. */
-__device__ __forceinline__ uint32_t wt_str_size(const WtRead& r, const WtShared& sh, const uint8_t* w8, uint32_t col, uint32_t index, uint32_t x, uint32_t y, bool& bad) {
+__device__ __forceinline__ uint32_t wt_str_size(const WtRead& r, WtShared& sh, const uint8_t* w8, uint32_t col, uint32_t index, uint32_t x, uint32_t y, bool& bad) {
   const uint32_t lo = sh.lo[col];
   const uint32_t u = x - lo, v = y - lo;
   if (u > v || v > sh.span[col]) { bad = true; return 2; }
   uint32_t n = y - x + 2u;
+  if (n >= WT_LONG + 2u) sh.longs = 1u;
   if (r.dirty) n += wt_extra(sh, w8, col, index);
   return n;
 }
@@ -257,7 +277,7 @@ PJ_HD uint32_t wt_frac_digits(uint32_t u) { /* of 1..999999999, without the zero
 struct WtList { uint32_t a, b, bytes; }; /* elements [a, b) of a list, and their text with a comma or bracket behind each */
 /* bytes of properties [I, HI) of an object: a separator and the name before every value. bad: not for this road. */
 template <int SCHEMA, int OBJ, int I, int HI>
-__device__ __forceinline__ uint32_t wt_size(const WtRead& x, const WtShared& sh, const uint8_t* w8, uint32_t index, const RowSnap& r, const RowSnap& rc, const WtList* lists, uint32_t* list_at, uint32_t at, bool& first, bool& bad) {
+__device__ __forceinline__ uint32_t wt_size(const WtRead& x, WtShared& sh, const uint8_t* w8, uint32_t index, const RowSnap& r, const RowSnap& rc, const WtList* lists, uint32_t* list_at, uint32_t at, bool& first, bool& bad) {
   if constexpr (I >= HI) return 0;
   else {
     constexpr uint32_t kind = FK<OBJ, I>::kind, col = FK<OBJ, I>::col;
@@ -471,29 +491,71 @@ static __device__ __noinline__ WtOut wt_put_escaped(WtOut e, uint32_t s, uint32_
   }
   return e;
 }
-/* the same by a warp, a byte per lane; dst: where it goes */
-__device__ __forceinline__ void wt_escape(uint8_t* w8, uint32_t s, uint32_t n, uint32_t dst, uint32_t hexa, uint32_t lane) {
-  for (uint32_t i0 = 0; i0 < n; i0 += 32u) {
-    const bool have = i0 + lane < n;
-    const uint32_t c = have ? w8[s + i0 + lane] : 0u, extra = have ? escape_extra_byte(c) : 0u, len = have ? 1u + extra : 0u;
-    const uint32_t end = warp_incl_scan(len), p = dst + end - len;
-    if (have) {
-      const uint32_t y = c == 8 ? 'b' : (c == 9 ? 't' : (c == 10 ? 'n' : (c == 12 ? 'f' : (c == 13 ? 'r' : c))));
-      uint64_t v = c;
-      if (extra == 1u) v = '\\' | (y << 8);
-      else if (extra) v = 0x3030755Cull | (uint64_t)(('0' + (c >> 4)) | (((c & 15) < 10 ? '0' + (c & 15) : hexa + (c & 15) - 10) << 8)) << 32;
-      const uint32_t sh = (p & 3u) * 8u, at = p & ~3u;
-      wt_or(w8, at, (uint32_t)(v << sh));
-      if ((p & 3u) + len > 4u) wt_or(w8, at + 4u, (uint32_t)((v << sh) >> 32));
-      if ((p & 3u) + len > 8u) wt_or(w8, at + 8u, (uint32_t)(v >> (64u - sh)));
-    }
-    dst += __shfl_sync(0xFFFFFFFFu, end, 31);
-  }
-}
 __device__ __forceinline__ uint32_t wt_peek4(const uint8_t* w8, uint32_t s) {
   return __funnelshift_r(wt_ld(w8, s & ~3u), wt_ld(w8, (s & ~3u) + 4u), (s & 3u) * 8u);
 }
 __device__ __forceinline__ uint32_t wt_low(uint32_t v, uint32_t n) { return n >= 4u ? v : v & ((1u << (8u * n)) - 1u); }
+/* byte c as W3 writes it: bytes from the lowest on, and how many */
+__device__ __forceinline__ uint64_t wt_escaped(uint32_t c, uint32_t hexa, uint32_t* len) {
+  const uint32_t extra = escape_extra_byte(c);
+  *len = 1u + extra;
+  if (extra == 0u) return c;
+  if (extra == 1u) return '\\' | ((c == 8 ? 'b' : (c == 9 ? 't' : (c == 10 ? 'n' : (c == 12 ? 'f' : (c == 13 ? 'r' : c))))) << 8);
+  return 0x3030755Cull | (uint64_t)(('0' + (c >> 4)) | (((c & 15) < 10 ? '0' + (c & 15) : hexa + (c & 15) - 10) << 8)) << 32;
+}
+/* bytes that the escapes of the `have` lowest bytes of x add */
+__device__ __forceinline__ uint32_t wt_word_extra(uint32_t x, uint32_t have) {
+  if (have < 4u) x |= 0x61616161u << (8u * have); /* (letters) */
+  return word_needs_escape(x) ? word_escape_extra(x) : 0u;
+}
+/* the len (1 .. 6) bytes of v to byte p of the window */
+__device__ __forceinline__ void wt_or_bytes(uint8_t* w8, uint32_t p, uint64_t v, uint32_t len) {
+  const uint32_t sh = (p & 3u) * 8u, at = p & ~3u;
+  wt_or(w8, at, (uint32_t)(v << sh));
+  if ((p & 3u) + len > 4u) wt_or(w8, at + 4u, (uint32_t)((v << sh) >> 32));
+  if ((p & 3u) + len > 8u) wt_or(w8, at + 8u, (uint32_t)(v >> (64u - sh)));
+}
+/* n staged bytes at byte s, escaped, by a warp: a byte per lane, four of a string of more than 256 bytes (Pets whose name has 43 KB 22.9 -> 14.2 ms;
+ * short strings take longer so); dst: where it goes */
+__device__ __forceinline__ void wt_escape(uint8_t* w8, uint32_t s, uint32_t n, uint32_t dst, uint32_t hexa, uint32_t lane) {
+  if (n <= 256u) {
+    for (uint32_t i0 = 0; i0 < n; i0 += 32u) {
+      uint32_t len = 0;
+      const uint64_t v = i0 + lane < n ? wt_escaped(w8[s + i0 + lane], hexa, &len) : 0ull;
+      const uint32_t end = warp_incl_scan(len);
+      if (len) wt_or_bytes(w8, dst + end - len, v, len);
+      dst += __shfl_sync(0xFFFFFFFFu, end, 31);
+    }
+    return;
+  }
+  for (uint32_t i0 = 0; i0 < n; i0 += 128u) {
+    const uint32_t i = i0 + 4u * lane, have = i >= n ? 0u : (n - i < 4u ? n - i : 4u);
+    const uint32_t x = have ? wt_low(wt_peek4(w8, s + i), have) : 0u;
+    const uint32_t extra = wt_word_extra(x, have), end = warp_incl_scan(have + extra);
+    uint32_t p = dst + end - have - extra;
+    if (extra == 0u) { if (have) wt_or_bytes(w8, p, x, have); }
+    else
+      for (uint32_t k = 0; k < have; ++k) {
+        uint32_t len;
+        const uint64_t v = wt_escaped((x >> (8u * k)) & 0xFFu, hexa, &len);
+        wt_or_bytes(w8, p, v, len);
+        p += len;
+      }
+    dst += __shfl_sync(0xFFFFFFFFu, end, 31);
+  }
+}
+/* n staged bytes at byte s that stay as they are, by a warp, a word of the window per lane */
+__device__ __forceinline__ void wt_copy(uint8_t* w8, uint32_t s, uint32_t n, uint32_t dst, uint32_t lane) {
+  const uint32_t lead = dst & 3u, end = lead + n; /* (bytes from the word that holds the first on) */
+  s -= lead; dst -= lead;
+  for (uint32_t k = 4u * lane; k < end; k += 128u) {
+    uint32_t v = wt_peek4(w8, s + k);
+    if (k >= lead && k + 4u <= end) { wt_st(w8, dst + k, v); continue; }
+    if (k < lead) v &= 0xFFFFFFFFu << (8u * (lead - k));
+    if (k + 4u > end) v &= 0xFFFFFFFFu >> (8u * (k + 4u - end));
+    wt_or(w8, dst + k, v); /* shared with the text beside it */
+  }
+}
 /* n bytes at byte s and a closing quote: up to the next word of the window, then whole words, then the rest */
 static __device__ __noinline__ WtOut wt_put_plain(WtOut e, uint32_t s, uint32_t n) {
   const uint32_t room = 4u - (e.fill >> 3), h = n < room ? n : room;
@@ -520,18 +582,19 @@ static __device__ __noinline__ WtOut wt_put_plain(WtOut e, uint32_t s, uint32_t 
 }
 /* the n staged bytes at byte s, string `index` of the tile's in arena col, and the closing quote, behind the opening one */
 __device__ __forceinline__ void wt_put_str(const WtRead& r, WtShared& sh, WtOut& e, uint32_t col, uint32_t index, uint32_t s, uint32_t n) {
-  if (r.dirty) {
-    const uint32_t extra = wt_extra(sh, e.w8, col, index);
-    if (extra) {
+  if (r.later) {
+    const uint32_t extra = r.dirty ? wt_extra(sh, e.w8, col, index) : 0u;
+    if (extra || n >= WT_LONG) {
       const uint32_t k = atomicAdd(&sh.nesc, 1u);
       if (k < WT_ESC) { /* later, by a warp */
         const uint32_t pos = wt_pos(e);
-        sh.esc[k].at = s; sh.esc[k].n = n; sh.esc[k].dst = pos;
+        sh.esc[k].at = s; sh.esc[k].n = n | (extra ? 0x80000000u : 0u); sh.esc[k].dst = pos;
         wt_end(e);
         wt_begin(e, pos + n + extra);
-      } else e = wt_put_escaped(e, s, n, r.hexa);
-      wt_put(e, '"', 8);
-      return;
+        wt_put(e, '"', 8);
+        return;
+      }
+      if (extra) { e = wt_put_escaped(e, s, n, r.hexa); wt_put(e, '"', 8); return; }
     }
   }
   e = wt_put_plain(e, s, n);
@@ -820,6 +883,11 @@ __device__ __forceinline__ void wt_stage(const WTileArgs& a, WtShared& sh, uint8
     at = wt_place(sh, w8, at, c, have && !c.off && n, x, y, a.smem, 1u, lane, bad);
     if (lane == 0) sh.text = at;
     if (!bad) at = wt_place(sh, w8, at, c, have && c.off, x, y, a.smem, 2u, lane, bad);
+    /* whose text a block is: a column starts in a block of its own */
+    const bool text = !bad && have && c.off && y > x;
+    const uint32_t first = text ? sh.at[c.col] + (uint32_t)x : 0u;
+    sh.ar0[lane] = (uint16_t)(first >> 4); sh.ar1[lane] = (uint16_t)(text ? (first + (uint32_t)(y - x) + 15u) >> 4 : 0u);
+    sh.arcol[lane] = c.col; sh.arlevel[lane] = c.level; sh.armodel[lane] = c.model;
   }
   else if (lane == 0) sh.text = at;
   const uint32_t sums = at + 16u, extra = (sums + 4u * (n0 + n1) + 15u) & ~15u;
@@ -827,22 +895,15 @@ __device__ __forceinline__ void wt_stage(const WTileArgs& a, WtShared& sh, uint8
   if (lane == 0) { sh.stage = at; sh.sums = sums; sh.extra = sh.win = extra; sh.nstr = strs; if (bad) sh.odd = 1; }
 }
 /* a 16-byte block with a byte to escape: counted for the strings it lies in, by a warp */
-__device__ __forceinline__ void wt_count_block(const WTileArgs& a, WtShared& sh, uint8_t* w8, uint32_t block, uint32_t lane) {
-  /* whose it is: a column starts in a block of its own */
-  const bool have = lane < a.ncol - a.nrow && a.col[a.nrow + lane].off;
-  const uint32_t mine = have ? a.col[a.nrow + lane].col : 0u;
-  uint32_t lead = 0; /* of the arena's first byte in its block */
-  if (have) lead = (sh.at[mine] + sh.lo[mine]) & 15u;
-  const uint32_t x0 = 16u * block - (have ? sh.at[mine] + sh.lo[mine] - lead : 0u);
-  const uint32_t who = __ballot_sync(0xFFFFFFFFu, have && sh.span[mine] && x0 < lead + sh.span[mine]);
+__device__ __forceinline__ void wt_count_block(WtShared& sh, uint8_t* w8, uint32_t block, uint32_t lane) {
+  const uint32_t who = __ballot_sync(0xFFFFFFFFu, block - sh.ar0[lane] < (uint32_t)sh.ar1[lane] - sh.ar0[lane]);
   if (!who) return;
-  const WtCol& c = a.col[a.nrow + (uint32_t)__ffs((int)who) - 1u];
-  const uint32_t col = c.col, p = 16u * block + lane, x = p - sh.at[col];
+  const uint32_t c = (uint32_t)__ffs((int)who) - 1u, col = sh.arcol[c], level = sh.arlevel[c], model = sh.armodel[c], p = 16u * block + lane, x = p - sh.at[col];
   const uint32_t extra = lane < 16u && x - sh.lo[col] < sh.span[col] ? escape_extra_byte(w8[p]) : 0u;
   if (!extra) return;
-  const uint32_t first = c.level == 0 ? (uint32_t)sh.row0[c.model] : sh.item0[c.level - 1u];
+  const uint32_t first = level == 0 ? (uint32_t)sh.row0[model] : sh.item0[level - 1u];
   const uint32_t* o = wt_at<uint32_t>(sh, w8, col - 1u, first); /* (an arena's column follows its offsets') */
-  uint32_t lo = 0, hi = c.level == 0 ? sh.cnt[c.model] : sh.itemn[c.level - 1u]; /* the last string that begins at or before it */
+  uint32_t lo = 0, hi = level == 0 ? sh.cnt[model] : sh.itemn[level - 1u]; /* the last string that begins at or before it */
   while (lo + 1u < hi) { const uint32_t mid = (lo + hi) >> 1; if (o[mid] <= x) lo = mid; else hi = mid; }
   atomicAdd(wt_extras(sh, w8) + sh.str0[col] + lo, extra);
 }
@@ -881,18 +942,184 @@ __device__ __forceinline__ uint32_t wt_groups(const WtShared& sh) {
   if constexpr (SCHEMA != PJ_SCHEMA_MIXED) return (sh.cnt[SCHEMA - 1] + 31u) / 32u;
   else return (sh.cnt[0] + 31u) / 32u + (sh.cnt[1] + 31u) / 32u + (sh.cnt[2] + 31u) / 32u;
 }
-/* A record of a tile on the general road. */
-template <int SCHEMA, bool WR>
-__device__ __noinline__ uint32_t wt_general(const DevCols* c, uint64_t i, int incl, uint32_t hexa, uint8_t* dst, uint32_t after) {
-  uint32_t type;
-  uint64_t row;
-  if (!write_locate(SCHEMA, c, i, &type, &row)) return 0;
-  if (SCHEMA != PJ_SCHEMA_MIXED) type = SCHEMA;
+/* ---- the general road: a record per thread, its long strings and lists by whole warps ------------------------------------ */
+/* What a record's thread leaves (see WriteAll of pj_write_fast.cuh): noted while it is measured, found again in the same order while it is written. */
+struct WtLeave {
+  static constexpr bool on = true;
+  WtShared* sh;
+  WtLater* e;
+  uint32_t cap, rec, last;
+  template <bool WR>
+  __device__ __forceinline__ bool put(uint32_t kind, uint32_t col, uint32_t a, uint32_t b, WOut& w) {
+    if (kind == K_STR ? b - a < WT_LONG : b - a < WT_LONG_LIST || b < a) return false;
+    if (WR) {
+      const uint32_t k = last == WT_NONE ? sh->mid[rec] : (uint32_t)e[last].link;
+      if (k == WT_LAST || e[k].kind != kind || e[k].col != col || e[k].a != a || e[k].b != b) return false;
+      e[k].dst = w.dst + w.n;
+      w.n += e[k].size;
+      last = k;
+      return true;
+    }
+    const uint32_t k = atomicAdd(&sh->nlater, 1u);
+    if (k >= cap) return false;
+    e[k].dst = nullptr; e[k].size = 0; e[k].a = a; e[k].b = b; e[k].rec = (uint16_t)rec; e[k].link = WT_LAST; e[k].kind = (uint8_t)kind; e[k].col = (uint8_t)col;
+    if (last == WT_NONE) sh->mid[rec] = k; else e[last].link = (uint16_t)k;
+    last = k;
+    return true;
+  }
+};
+template <int SCHEMA>
+__device__ __forceinline__ uint64_t wt_row(const DevCols& c, uint64_t i) { return SCHEMA == PJ_SCHEMA_MIXED ? (uint64_t)colp<uint32_t>(&c, PJ_COL_REC_ROW)[i] : i; }
+/* Record `rec` of the tile, row `row` of model OBJ: bytes of its text and of what follows it, without what is left to the warps (top bit: a byte has
+ * to be escaped), or the text itself. PLAIN: no byte has to. */
+template <int OBJ, bool WR, bool PLAIN>
+__device__ __noinline__ unsigned long long wt_general(const DevCols* c, uint64_t row, int incl, uint32_t hexa, uint8_t* dst, uint32_t after, WtShared* sh, WtLater* e, uint32_t cap, uint32_t rec) {
   WOut w;
   w.dst = dst; w.n = 0; w.hexa = hexa;
-  fwrite_record<WR, false>(c, type, row, incl, w);
+  WtLeave l;
+  l.sh = sh; l.e = e; l.cap = cap; l.rec = rec; l.last = WT_NONE;
+  if (!WR) sh->mid[rec] = WT_LAST;
+  fwrite_object<WR, PLAIN, OBJ, 0>(c, row, incl, l, w);
   if (WR) dst[w.n] = (uint8_t)after;
-  return (uint32_t)w.n + 1u;
+  return (w.n + 1u) | (!WR && w.escapes ? TS_VALID : 0ull);
+}
+template <int SCHEMA, bool WR>
+__device__ __forceinline__ unsigned long long wt_general_any(const DevCols* c, uint32_t model, uint64_t row, int incl, uint32_t hexa, uint8_t* dst, uint32_t after, WtShared* sh, WtLater* e, uint32_t cap, uint32_t rec, bool plain) {
+  if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED)
+    if (model == 0) return WR && plain ? wt_general<OBJ_PET, WR, WR>(c, row, incl, hexa, dst, after, sh, e, cap, rec) : wt_general<OBJ_PET, WR, false>(c, row, incl, hexa, dst, after, sh, e, cap, rec);
+  if constexpr (SCHEMA == PJ_SCHEMA_ORDER || SCHEMA == PJ_SCHEMA_MIXED)
+    if (model == 1) return wt_general<OBJ_ORDER, WR, false>(c, row, incl, hexa, dst, after, sh, e, cap, rec);
+  if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED)
+    if (model == 2) return WR && plain ? wt_general<OBJ_USER, WR, WR>(c, row, incl, hexa, dst, after, sh, e, cap, rec) : wt_general<OBJ_USER, WR, false>(c, row, incl, hexa, dst, after, sh, e, cap, rec);
+  return 0;
+}
+/* bytes the escapes of the n bytes at s add, all lanes of a warp: 16-byte blocks, looked at again where there is one */
+__device__ __forceinline__ uint32_t wt_warp_extra(const uint8_t* s, uint32_t n, uint32_t lane) {
+  const uintptr_t from = reinterpret_cast<uintptr_t>(s), to = from + n;
+  uint32_t extra = 0;
+  for (uintptr_t p = (from & ~(uintptr_t)15) + 16u * lane; p < to; p += 512u) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+    if (word_needs_escape(x[0]) | word_needs_escape(x[1]) | word_needs_escape(x[2]) | word_needs_escape(x[3]))
+      for (uint32_t k = 0; k < 16u; ++k) if (p + k >= from && p + k < to) extra += escape_extra_byte((x[k >> 2] >> (8u * (k & 3u))) & 0xFFu);
+  }
+  return __reduce_add_sync(0xFFFFFFFFu, extra);
+}
+/* the n bytes at s to d, as they are, all lanes of a warp: 16-byte blocks of d */
+__device__ __forceinline__ void wt_warp_copy(uint8_t* d, const uint8_t* s, uint32_t n, uint32_t lane) {
+  const uint32_t head = (0u - (uint32_t)reinterpret_cast<uintptr_t>(d)) & 15u, lead = head < n ? head : n;
+  if (lane < lead) d[lane] = s[lane];
+  d += lead; s += lead; n -= lead;
+  const uint32_t shift = ((uint32_t)reinterpret_cast<uintptr_t>(s) & 3u) * 8u, whole = n & ~15u;
+  for (uint32_t k = 16u * lane; k < whole; k += 512u) {
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(s + k) & ~(uintptr_t)3);
+    const uint32_t x0 = p[0], x1 = p[1], x2 = p[2], x3 = p[3], x4 = shift ? p[4] : 0u; /* (never a word that holds none of the n bytes) */
+    uint4 v;
+    v.x = __funnelshift_r(x0, x1, shift); v.y = __funnelshift_r(x1, x2, shift); v.z = __funnelshift_r(x2, x3, shift); v.w = __funnelshift_r(x3, x4, shift);
+    *reinterpret_cast<uint4*>(d + k) = v;
+  }
+  if (lane < n - whole) d[whole + lane] = s[whole + lane];
+}
+/* ... escaped, four bytes per lane */
+__device__ __forceinline__ void wt_warp_escape(uint8_t* d, const uint8_t* s, uint32_t n, uint32_t hexa, uint32_t lane) {
+  const uint32_t shift = ((uint32_t)reinterpret_cast<uintptr_t>(s) & 3u) * 8u;
+  for (uint32_t i0 = 0; i0 < n; i0 += 128u) {
+    const uint32_t i = i0 + 4u * lane, have = i >= n ? 0u : (n - i < 4u ? n - i : 4u);
+    uint32_t x = 0;
+    if (have) { /* (never a word that holds none of the n bytes) */
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(s + i) & ~(uintptr_t)3);
+      x = wt_low(__funnelshift_r(p[0], shift + 8u * have > 32u ? p[1] : 0u, shift), have);
+    }
+    const uint32_t extra = wt_word_extra(x, have), end = warp_incl_scan(have + extra);
+    uint8_t* p = d + (end - have - extra);
+    for (uint32_t k = 0; k < have; ++k) {
+      uint32_t len = 1;
+      uint64_t v = (x >> (8u * k)) & 0xFFu;
+      if (extra) v = wt_escaped((uint32_t)v, hexa, &len);
+      for (uint32_t b = 0; b < len; ++b) p[b] = (uint8_t)(v >> (8u * b));
+      p += len;
+    }
+    d += __shfl_sync(0xFFFFFFFFu, end, 31);
+  }
+}
+/* Element k of a list: its text, measured or written, by one lane. PLAIN: it has no byte to escape. */
+template <bool WR, bool PLAIN>
+__device__ __forceinline__ void wt_element(const DevCols* c, const WtLater& e, uint32_t k, int incl, WOut& w) {
+  if (e.kind == K_LIST_STR) {
+    const uint32_t* so = colp<uint32_t>(c, FK<OBJ_PET, WT_LIST_STR>::col + 1);
+    fput_str<WR, PLAIN>(w, colp<uint8_t>(c, FK<OBJ_PET, WT_LIST_STR>::col + 2) + so[k], so[k + 1] - so[k]);
+  } else {
+    WriteAll all;
+    fwrite_object<WR, PLAIN, FK<OBJ_PET, WT_LIST_OBJ>::child, 1>(c, k, incl, all, w);
+  }
+}
+/* Measures what the records' threads have left, n of them: a string in parts of WT_PART bytes that go round the warps, a list by one warp, an element
+ * per lane. bytes: whether the records' totals are wanted. */
+static __device__ __noinline__ void wt_measure_later(const DevCols* c, WtShared& sh, WtLater* e, uint32_t n, int incl, bool bytes, uint32_t warp, uint32_t warps, uint32_t lane) {
+  for (uint32_t j = 0; j < n; ++j) {
+    WtLater& l = e[j];
+    const uint32_t first = (warp + warps - j % warps) % warps; /* the first part that is the warp's */
+    unsigned long long size = 0;
+    if (l.kind == K_STR) {
+      const uint8_t* s = colp<uint8_t>(c, l.col) + l.a;
+      const uint32_t len = l.b - l.a;
+      for (uint32_t from = first * WT_PART; from < len; from += WT_PART * warps) {
+        size += wt_warp_extra(s + from, len - from < WT_PART ? len - from : WT_PART, lane);
+        if (len - from <= WT_PART * warps) break; /* (a sum could pass 2^32) */
+      }
+      if (first == 0) size += 2ull + len;
+    } else if (first == 0) {
+      unsigned long long sum = 0;
+      for (uint32_t k = l.a + lane; k < l.b; k += 32u) {
+        WOut w;
+        w.dst = nullptr; w.n = 0;
+        wt_element<false, false>(c, l, k, incl, w);
+        sum += w.n + 1u;
+        if (l.b - k <= 32u) break;
+      }
+      for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+      size = sum + 1u;
+    }
+    if (size && lane == 0) { atomicAdd(&l.size, size); if (bytes) atomicAdd(&sh.bytes[l.rec], size); }
+    __syncwarp();
+  }
+}
+/* ... and writes them. */
+static __device__ __noinline__ void wt_write_later(const DevCols* c, WtLater* e, uint32_t n, int incl, uint32_t hexa, uint32_t warp, uint32_t warps, uint32_t lane) {
+  for (uint32_t j = 0; j < n; ++j) {
+    const WtLater& l = e[j];
+    const uint32_t first = (warp + warps - j % warps) % warps;
+    if (l.kind == K_STR) {
+      const uint8_t* s = colp<uint8_t>(c, l.col) + l.a;
+      const uint32_t len = l.b - l.a;
+      if (first == 0 && lane == 0) { l.dst[0] = '"'; l.dst[l.size - 1u] = '"'; }
+      if (l.size != 2ull + len) { if (first == 0) wt_warp_escape(l.dst + 1, s, len, hexa, lane); continue; }
+      for (uint32_t from = first * WT_PART; from < len; from += WT_PART * warps) {
+        wt_warp_copy(l.dst + 1 + from, s + from, len - from < WT_PART ? len - from : WT_PART, lane);
+        if (len - from <= WT_PART * warps) break;
+      }
+    } else if (first == 0) {
+      uint8_t* d = l.dst;
+      if (lane == 0) *d = '[';
+      ++d;
+      for (uint32_t k0 = l.a; k0 < l.b; k0 += 32u) {
+        const uint32_t k = k0 + lane;
+        const bool have = k0 <= k && k < l.b;
+        WOut w;
+        w.dst = nullptr; w.n = 0; w.hexa = hexa;
+        if (have) { wt_element<false, false>(c, l, k, incl, w); w.n++; }
+        const unsigned long long end = warp_incl_scan((unsigned long long)w.n);
+        if (have) {
+          const bool plain = w.escapes == 0;
+          w.dst = d + (end - w.n); w.n = 0;
+          if (plain) wt_element<true, true>(c, l, k, incl, w); else wt_element<true, false>(c, l, k, incl, w);
+          wput<true>(w, k + 1u < l.b ? ',' : ']');
+        }
+        d += __shfl_sync(0xFFFFFFFFu, end, 31);
+        if (l.b - k0 <= 32u) break;
+      }
+    }
+  }
 }
 __device__ __forceinline__ void wt_zero(uint8_t* w8, uint32_t from, uint32_t to, uint32_t t, uint32_t nt) {
   for (uint32_t k = from + 16u * t; k < to; k += 16u * nt) *reinterpret_cast<uint4*>(w8 + k) = uint4{0, 0, 0, 0};
@@ -911,13 +1138,117 @@ __device__ __forceinline__ void wt_copy_out(uint8_t* gbase, const uint8_t* win, 
   }
 }
 
+/* The tile's text has `total` bytes: where it goes (sh.base), and whether it fits (sh.ok). Warp 0. */
+__device__ __forceinline__ void wt_find_place(const WTileArgs& a, WtShared& sh, uint32_t tile, unsigned long long total, uint32_t lane) {
+  if (lane == 0) {
+    st_relaxed_u64(&a.agg[tile], TS_VALID | total);
+    if (tile == 0) st_relaxed_u64(&a.inc[tile], TS_VALID | total);
+  }
+  unsigned long long excl = 0;
+  const bool ok = lookback_u64(a.agg, a.inc, &a.w.res->timeout, a.spin_limit_ns, tile, lane, &excl);
+  if (lane == 0) {
+    if (tile != 0 && ok) st_relaxed_u64(&a.inc[tile], TS_VALID | (excl + total));
+    const bool fits = (a.w.array ? 1u : 0u) + excl + total <= a.w.cap; /* (the opening bracket) */
+    if (ok && !fits) a.w.res->ok = 0;
+    if (tile == a.ntiles - 1) a.w.res->out_bytes = excl + total; /* text bytes of all records */
+    sh.base = excl;
+    sh.ok = ok && fits;
+  }
+}
+/* cycles per phase: sizes, look-back, text into the window, copy-out */
+__device__ __forceinline__ void wt_note_cycles(DevResult* res, long long c0, long long c1, long long c2, long long c3) {
+  const long long c4 = clock64();
+  atomicAdd(&res->phase_cycles[0], (unsigned long long)(c1 - c0));
+  atomicAdd(&res->phase_cycles[1], (unsigned long long)(c2 - c1));
+  atomicAdd(&res->phase_cycles[2], (unsigned long long)(c3 - c2));
+  atomicAdd(&res->phase_cycles[3], (unsigned long long)(c4 - c3));
+}
+/* A tile on the general road: a record per thread, those of one model side by side; the warps measure and write what the threads leave. The text goes
+ * through a window behind the list of that, if it fits, else straight to global memory. Out of line, like the next one: few tiles come here.
+ * 300 MB against a record per thread with all of its strings (kernel, us): Users of 72 KB 30 200 -> 430, of 1.2 MB 67 600 -> 425, Pets of 3000 short
+ * strings 31 700 -> 1 230; 100 k Users of which one in a thousand has 96 KB 6 270 -> 117; 300 k records of three models in the caller's own order 490 -> 260, with escapes 590 -> 355 (and 240 and 435 in tiles of 128
+ * records of 128 threads, five to an SM, whose strings were looked over for escapes by a kernel of their own, 40 us more). */
+template <int SCHEMA>
+__device__ __noinline__ void wt_general_tile(const WTileArgs& a, WtShared& sh, uint8_t* smem, uint64_t rec0, uint32_t nrec, uint32_t tile, long long c0) {
+  constexpr uint32_t THREADS = WtT<SCHEMA>::threads, WARPS = WtT<SCHEMA>::warps;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, ngroups = wt_groups<SCHEMA>(sh);
+  WtLater* const e = reinterpret_cast<WtLater*>(smem);
+  if (tid < nrec) sh.bytes[tid] = 0;
+  __syncthreads();
+  bool esc = false; /* a byte has to be escaped, but for what is left to the warps */
+  for (uint32_t u = warp; u < ngroups; u += WARPS) {
+    const WtGroup g = wt_group<SCHEMA>(sh, u);
+    const uint32_t rec = wt_record<SCHEMA>(sh, g, lane);
+    if (rec == WT_NONE) continue;
+    const unsigned long long n = wt_general_any<SCHEMA, false>(&a.w.cols, g.model, wt_row<SCHEMA>(a.w.cols, rec0 + rec), a.w.inclusion, a.w.hexa, nullptr, 0, &sh, e, WT_LATERS, rec, false);
+    sh.bytes[rec] = n & ~TS_VALID;
+    esc = esc || n >> 63;
+  }
+  const bool plain = !__syncthreads_or((int)esc);
+  const uint32_t nlater = sh.nlater < WT_LATERS ? sh.nlater : WT_LATERS;
+  wt_measure_later(&a.w.cols, sh, e, nlater, a.w.inclusion, true, warp, WARPS, lane);
+  __syncthreads();
+  const unsigned long long len = tid < nrec ? sh.bytes[tid] : 0ull;
+  unsigned long long at = warp_incl_scan(len), total = 0;
+  if (lane == 31) sh.wsum8[warp] = at;
+  at -= len;
+  __syncthreads();
+  const long long c1 = clock64();
+  for (uint32_t q = 0; q < WARPS; ++q) { const unsigned long long v = sh.wsum8[q]; if (q < warp) at += v; total += v; }
+  if (tid < nrec) sh.bytes[tid] = at; /* where it starts */
+  if (warp == 0) wt_find_place(a, sh, tile, total, lane);
+  __syncthreads();
+  const long long c2 = clock64();
+  if (!sh.ok) return;
+  uint8_t* const out0 = a.w.out + (a.w.array ? 1 : 0) + sh.base;
+  constexpr uint32_t win = WT_LATERS * (uint32_t)sizeof(WtLater);
+  static_assert(win % 16u == 0 && win + WT_MIN_WINDOW <= 8192u, "the smallest tile has a window");
+  const bool inside = total + 48u <= a.smem - win;
+  const uint32_t pad = (uint32_t)(reinterpret_cast<uintptr_t>(out0) & 15u);
+  for (uint32_t u = warp; u < ngroups; u += WARPS) {
+    const WtGroup g = wt_group<SCHEMA>(sh, u);
+    const uint32_t rec = wt_record<SCHEMA>(sh, g, lane);
+    if (rec != WT_NONE) (void)wt_general_any<SCHEMA, true>(&a.w.cols, g.model, wt_row<SCHEMA>(a.w.cols, rec0 + rec), a.w.inclusion, a.w.hexa, (inside ? smem + win + pad : out0) + sh.bytes[rec], a.w.array ? ',' : '\n', &sh, e, WT_LATERS, rec, plain);
+  }
+  __syncthreads();
+  wt_write_later(&a.w.cols, e, nlater, a.w.inclusion, a.w.hexa, warp, WARPS, lane);
+  fence_async_smem();
+  __syncthreads();
+  const long long c3 = clock64();
+  if (inside) wt_copy_out<THREADS>(out0 - pad, smem + win, pad, (uint32_t)total, tid);
+  __syncthreads();
+  if (tid == 0) wt_note_cycles(a.w.res, c0, c1, c2, c3);
+}
+/* One record of a staged tile whose text has no window: the same steps, straight to dst. w8: `bytes` of shared memory that are free. */
+template <int SCHEMA>
+__device__ __noinline__ void wt_general_one(const WTileArgs& a, WtShared& sh, uint8_t* w8, uint32_t bytes, uint64_t i, uint32_t rec, uint8_t* dst) {
+  constexpr uint32_t WARPS = WtT<SCHEMA>::warps;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, most = bytes / (uint32_t)sizeof(WtLater), cap = most < WT_LATERS ? most : WT_LATERS;
+  WtLater* const e = reinterpret_cast<WtLater*>(w8);
+  uint32_t model = SCHEMA - 1u; /* thread 0's */
+  bool plain = true;
+  if (tid == 0) {
+    if constexpr (SCHEMA == PJ_SCHEMA_MIXED) { const uint32_t type = colp<uint8_t>(&a.w.cols, PJ_COL_REC_TYPE)[i]; model = type == PJ_TYPE_PET ? 0u : (type == PJ_TYPE_ORDER ? 1u : 2u); }
+    sh.nlater = 0;
+    plain = !(wt_general_any<SCHEMA, false>(&a.w.cols, model, wt_row<SCHEMA>(a.w.cols, i), a.w.inclusion, a.w.hexa, nullptr, 0, &sh, e, cap, rec, false) >> 63);
+  }
+  __syncthreads();
+  const uint32_t nlater = sh.nlater < cap ? sh.nlater : cap;
+  wt_measure_later(&a.w.cols, sh, e, nlater, a.w.inclusion, false, warp, WARPS, lane);
+  __syncthreads();
+  if (tid == 0) (void)wt_general_any<SCHEMA, true>(&a.w.cols, model, wt_row<SCHEMA>(a.w.cols, i), a.w.inclusion, a.w.hexa, dst, a.w.array ? ',' : '\n', &sh, e, cap, rec, plain);
+  __syncthreads();
+  wt_write_later(&a.w.cols, e, nlater, a.w.inclusion, a.w.hexa, warp, WARPS, lane);
+  __syncthreads();
+}
+
 template <int SCHEMA>
 __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_write_tile(const __grid_constant__ WTileArgs a) {
   constexpr uint32_t THREADS = WtT<SCHEMA>::threads, WARPS = WtT<SCHEMA>::warps;
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) WtShared sh;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); for (uint32_t k = 0; k < 3u; ++k) mbar_init(&sh.mbar[k], 1u); sh.odd = 0; sh.nesc = 0; sh.ok = 0; sh.nhit = 0; sh.flight = 0; }
+  if (tid == 0) { sh.tile = atomicAdd(a.ticket, 1u); for (uint32_t k = 0; k < 3u; ++k) mbar_init(&sh.mbar[k], 1u); sh.odd = 0; sh.nesc = 0; sh.ok = 0; sh.nhit = 0; sh.flight = 0; sh.longs = 0; sh.nlater = 0; }
   __syncthreads();
   const uint32_t tile = sh.tile;
   if (tile >= a.ntiles) return;
@@ -930,7 +1261,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
   if (warp == 0) wt_stage<SCHEMA>(a, sh, smem, lane);
   __syncthreads();
   WtRead x;
-  x.incl = a.w.inclusion; x.hexa = a.w.hexa; x.dirty = false;
+  x.incl = a.w.inclusion; x.hexa = a.w.hexa; x.dirty = x.later = false;
   bool odd = sh.odd != 0;
   const uint32_t ngroups = wt_groups<SCHEMA>(sh);
   if (sh.flight) {
@@ -963,7 +1294,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
       for (uint32_t k = tid; k < sh.nstr; k += THREADS) ex[k] = 0;
       __syncthreads();
       const bool all = sh.nhit > WT_HITS; /* (more than the list holds: every block) */
-      for (uint32_t k = warp; k < (all ? b1 - b0 : sh.nhit); k += WARPS) wt_count_block(a, sh, smem, all ? b0 + k : sh.hit[k], lane);
+      for (uint32_t k = warp; k < (all ? b1 - b0 : sh.nhit); k += WARPS) wt_count_block(sh, smem, all ? b0 + k : sh.hit[k], lane);
       __syncthreads();
     }
     bool bad = false;
@@ -982,10 +1313,11 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
       if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 2) wt_size_records<SCHEMA, OBJ_USER>(x, sh, smem, g, lane, bad);
     }
     odd = __syncthreads_or((int)bad) != 0;
+    x.later = x.dirty || sh.longs;
   }
+  if (odd) { wt_general_tile<SCHEMA>(a, sh, smem, rec0, nrec, tile, c0); return; }
   /* where the records start */
-  uint32_t len = 0;
-  if (tid < nrec) len = odd ? wt_general<SCHEMA, false>(&a.w.cols, rec0 + tid, x.incl, x.hexa, nullptr, 0) : sh.pos[tid];
+  const uint32_t len = tid < nrec ? sh.pos[tid] : 0u;
   uint32_t at = warp_incl_scan(len);
   if (lane == 31) sh.wsum[warp] = at;
   at -= len;
@@ -996,28 +1328,13 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
   for (uint32_t q = 0; q < WARPS; ++q) { const uint32_t v = sh.wsum[q]; if (q < warp) at += v; total += v; }
   if (tid < nrec) sh.pos[tid] = at;
   if (tid == 0) sh.pos[nrec] = total;
-  const uint64_t lead = a.w.array ? 1 : 0; /* the opening bracket */
-  const uint32_t win = odd ? 0u : sh.win, room = a.smem - win - 48u; /* (the last word and the output's alignment) */
-  if (warp == 0) {
-    if (lane == 0) {
-      st_relaxed_u64(&a.agg[tile], TS_VALID | total);
-      if (tile == 0) st_relaxed_u64(&a.inc[tile], TS_VALID | total);
-    }
-    unsigned long long excl = 0;
-    const bool ok = lookback_u64(a.agg, a.inc, &a.w.res->timeout, a.spin_limit_ns, tile, lane, &excl);
-    if (lane == 0) {
-      if (tile != 0 && ok) st_relaxed_u64(&a.inc[tile], TS_VALID | (excl + total));
-      const bool fits = lead + excl + total <= a.w.cap;
-      if (ok && !fits) a.w.res->ok = 0;
-      if (tile == a.ntiles - 1) a.w.res->out_bytes = excl + total; /* text bytes of all records */
-      sh.base = excl;
-      sh.ok = ok && fits;
-    }
-  } else if (!odd) wt_zero(smem, win, win + 32u + (total < room ? total : room), tid - 32u, THREADS - 32u);
+  const uint32_t win = sh.win, room = a.smem - win - 48u; /* (the last word and the output's alignment) */
+  if (warp == 0) wt_find_place(a, sh, tile, total, lane);
+  else wt_zero(smem, win, win + 32u + (total < room ? total : room), tid - 32u, THREADS - 32u);
   __syncthreads();
   const long long c2 = clock64();
   if (!sh.ok) return;
-  uint8_t* const out0 = a.w.out + lead + sh.base; /* where the tile's text starts */
+  uint8_t* const out0 = a.w.out + (a.w.array ? 1 : 0) + sh.base; /* where the tile's text starts */
   const uint32_t after = a.w.array ? (uint32_t)',' : (uint32_t)'\n';
   long long c3 = c2;
   uint32_t ra = 0;
@@ -1030,34 +1347,32 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
       rb = lo - ra > 32u ? lo - (lo - ra) % 32u : lo; /* whole groups */
     }
     uint8_t* const dst0 = out0 + start;
-    if (rb == ra || (odd && rb != nrec)) { /* no window for it: straight to global memory */
-      rb = odd ? nrec : ra + 1u;
-      for (uint32_t t = ra + tid; t < rb; t += THREADS) wt_general<SCHEMA, true>(&a.w.cols, rec0 + t, x.incl, x.hexa, out0 + sh.pos[t], after);
-      ra = rb;
-      continue;
-    }
+    if (rb == ra) { wt_general_one<SCHEMA>(a, sh, smem + win, room + 48u, rec0 + ra, ra, dst0); ++ra; continue; } /* no window for this one */
     const uint32_t pad = (uint32_t)(reinterpret_cast<uintptr_t>(dst0) & 15u), bytes = sh.pos[rb] - start;
     /* the window mirrors the output's alignment: window byte k goes to (dst0 - pad)[k] */
-    if (odd) { for (uint32_t t = tid; t < nrec; t += THREADS) wt_general<SCHEMA, true>(&a.w.cols, rec0 + t, x.incl, x.hexa, smem + pad + sh.pos[t], after); }
-    else {
-      if (ra) { wt_zero(smem, win, win + 32u + bytes, tid, THREADS); if (tid == 0) sh.nesc = 0; __syncthreads(); }
-      const uint32_t at0 = win + pad - start;
-      /* the units of all groups, the long ones first: a unit's number turns with its group, so that a warp's are not all of one kind */
-      constexpr uint32_t KINDS = SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED ? 4u : 2u;
-      const bool single = KINDS == 4u && ngroups == 1u; /* a tile of long lists: their elements are spread over the warps */
-      constexpr uint32_t PARTS = (WARPS - 2u) / 2u;
-      for (uint32_t u = warp; u < (single ? 2u + 2u * PARTS : KINDS * ngroups); u += WARPS) {
-        const WtGroup g = wt_group<SCHEMA>(sh, single ? 0u : u / KINDS);
-        const uint32_t k = single ? (u < 2u ? u : 2u + (u & 1u)) : (u + u / KINDS) % KINDS, part = single && u >= 2u ? (u - 2u) / 2u : 0u, parts = single ? PARTS : 1u;
-        if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 0) wt_unit<SCHEMA, OBJ_PET>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
-        if constexpr (SCHEMA == PJ_SCHEMA_ORDER || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 1) wt_unit<SCHEMA, OBJ_ORDER>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
-        if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 2) wt_unit<SCHEMA, OBJ_USER>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
-      }
-      if (x.dirty) {
-        __syncthreads();
-        const uint32_t n = sh.nesc < WT_ESC ? sh.nesc : WT_ESC;
-        for (uint32_t k = warp; k < n; k += WARPS) wt_escape(smem, sh.esc[k].at, sh.esc[k].n, sh.esc[k].dst, x.hexa, lane);
-      }
+    if (ra) { wt_zero(smem, win, win + 32u + bytes, tid, THREADS); if (tid == 0) sh.nesc = 0; __syncthreads(); }
+    const uint32_t at0 = win + pad - start;
+    /* the units of all groups, the long ones first: a unit's number turns with its group, so that a warp's are not all of one kind */
+    constexpr uint32_t KINDS = SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED ? 4u : 2u;
+    const bool single = KINDS == 4u && ngroups == 1u; /* a tile of long lists: their elements are spread over the warps */
+    constexpr uint32_t PARTS = (WARPS - 2u) / 2u;
+    for (uint32_t u = warp; u < (single ? 2u + 2u * PARTS : KINDS * ngroups); u += WARPS) {
+      const WtGroup g = wt_group<SCHEMA>(sh, single ? 0u : u / KINDS);
+      const uint32_t k = single ? (u < 2u ? u : 2u + (u & 1u)) : (u + u / KINDS) % KINDS, part = single && u >= 2u ? (u - 2u) / 2u : 0u, parts = single ? PARTS : 1u;
+      if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 0) wt_unit<SCHEMA, OBJ_PET>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
+      if constexpr (SCHEMA == PJ_SCHEMA_ORDER || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 1) wt_unit<SCHEMA, OBJ_ORDER>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
+      if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED) if (g.model == 2) wt_unit<SCHEMA, OBJ_USER>(x, sh, smem, g, k, part, parts, lane, ra, rb, at0, after);
+    }
+    if (x.later) {
+      __syncthreads();
+      const uint32_t n = sh.nesc < WT_ESC ? sh.nesc : WT_ESC;
+      for (uint32_t k = warp; k < n; k += WARPS) if (sh.esc[k].n >> 31) wt_escape(smem, sh.esc[k].at, sh.esc[k].n & 0x7FFFFFFFu, sh.esc[k].dst, x.hexa, lane);
+      if (sh.longs)
+        for (uint32_t k = 0; k < n; ++k) {
+          const WtEsc l = sh.esc[k];
+          if (l.n >> 31 || (l.n <= WT_PART && k % WARPS != warp)) continue;
+          for (uint32_t from = (warp + WARPS - k % WARPS) % WARPS * WT_PART; from < l.n; from += WT_PART * WARPS) wt_copy(smem, l.at + from, l.n - from < WT_PART ? l.n - from : WT_PART, l.dst + from, lane);
+        }
     }
     fence_async_smem();
     __syncthreads();
@@ -1067,13 +1382,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
     if (ra < nrec) __syncthreads();
   }
   __syncthreads();
-  if (tid == 0) { /* cycles per phase: sizes, look-back, text into the window, copy-out */
-    const long long c4 = clock64();
-    atomicAdd(&a.w.res->phase_cycles[0], (unsigned long long)(c1 - c0));
-    atomicAdd(&a.w.res->phase_cycles[1], (unsigned long long)(c2 - c1));
-    atomicAdd(&a.w.res->phase_cycles[2], (unsigned long long)(c3 - c2));
-    atomicAdd(&a.w.res->phase_cycles[3], (unsigned long long)(c4 - c3));
-  }
+  if (tid == 0) wt_note_cycles(a.w.res, c0, c1, c2, c3);
 }
 
 /* ---- host: the schema's columns as the tiles stage them ---------------------------------------------------------------- */

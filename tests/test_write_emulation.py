@@ -146,6 +146,49 @@ def test_literals_out_of_range_and_present_bits(writer, oracle):
     write(writer, ORDER, cols, oracle.write(ORDER, cols, NDJSON, abi.PJ_INCLUDE_NON_NULL))
 
 
+SIZES = [0, 1, 17, 255, 511, 512, 513, 1000, 2047, 2048, 2049, 4095, 4097, 33000]
+
+
+def long_text(rng, n, dirty):
+    """Pets whose strings and lists are as long as what warps take over, and a byte more or less."""
+    word = lambda k: "".join(rng.choice(['\\"', "\\n", "\\u0001", "x"]) if rng.random() < dirty else "abcdefg"[j % 7] for j in range(k))
+    out = []
+    for i in range(n):
+        urls = ",".join('"%s"' % word(rng.choice([0, 3, 30, 300, 1100])) for _ in range(rng.choice([0, 1, 7, 8, 9, 32, 33, 70])))
+        tags = ",".join(rng.choice(["{}", '{"id":%d}' % j, '{"id":%d,"name":"%s"}' % (j, word(rng.choice([0, 9, 512, 2100])))]) for j in range(rng.choice([0, 1, 7, 8, 9, 40])))
+        out.append('{"id":%d,"category":{"id":1,"name":"%s"},"name":"%s","photoUrls":[%s],"tags":[%s]}' % (i, word(rng.choice(SIZES[:-1])), word(rng.choice(SIZES)), urls, tags))
+    return as_u8("\n".join(out).encode())
+
+
+@pytest.mark.parametrize("dirty", [0, 0.002, 0.5])
+@pytest.mark.parametrize("seed", range(3))
+def test_long_strings_and_lists(writer, oracle, seed, dirty):
+    """In the window, beyond it (one record after the other) and on the general road (no room to stage a tile, a record map of the caller's own)."""
+    rng = random.Random(seed)
+    cols = oracle.parse(PET, long_text(rng, 24, dirty))
+    assert cols.n_errors == 0
+    want = oracle.write(PET, cols, NDJSON, abi.PJ_INCLUDE_NON_NULL)
+    for shape in [dict(recs=24, shared=131072), dict(recs=3, shared=100 * 1024, mis=3, order=5), dict(recs=1, shared=65536, mis=15), dict(recs=1, shared=131072, mis=1), dict(recs=24, shared=16384, mis=7), dict(recs=2, shared=8192)]:
+        write(writer, PET, cols, want, **shape)
+    mixed = oracle.parse(MIXED, np.concatenate([long_text(rng, 40, dirty), as_u8(b"\n"), pj.gen_text(MIXED, seed, 0, 40, ESC if dirty else 0)]))
+    n = mixed.n_records
+    kind, row = mixed.arrays[COL["rec_type"]][:n], mixed.arrays[COL["rec_row"]].view(np.uint32)[:n]
+    kind[:], row[:] = kind[::-1].copy(), row[::-1].copy()
+    want = oracle.write(MIXED, mixed, NDJSON, abi.PJ_INCLUDE_NON_NULL)
+    for shape in [dict(recs=80, shared=100 * 1024, mis=5), dict(recs=16, shared=8192, order=3)]:
+        write(writer, MIXED, mixed, want, **shape)
+
+
+@pytest.mark.parametrize("length, esc", [(511, 0), (512, 0), (512, 40), (1000, 0), (5000, 30)])
+def test_more_long_strings_than_a_tile_keeps(writer, oracle, length, esc):
+    text = "".join('\\"' if esc and k % esc == 3 else "q" for k in range(length))
+    line = lambda i: ('{"id":%d,' % i + ",".join('"%s":"%s%s"' % (k, text, "z" * (i % 5)) for k in ("username", "firstName", "lastName", "email", "password", "phone")) + "}").encode()
+    cols = oracle.parse(USER, as_u8(b"\n".join(line(i) for i in range(70))))
+    want = oracle.write(USER, cols, NDJSON, abi.PJ_INCLUDE_NON_NULL)
+    for shape in [dict(recs=70, shared=131072), dict(recs=70, shared=16384, mis=9), dict(recs=40, shared=131072, mis=2, order=7), dict(recs=2, shared=80 * 1024), dict(recs=2, shared=65536)]:
+        write(writer, USER, cols, want, **shape)
+
+
 def fall(off, row, by):
     """The range of string `row` goes back by `by` bytes: the string behind it shares them."""
     off[row + 1] = off[row] - by
