@@ -189,6 +189,20 @@ def test_more_long_strings_than_a_tile_keeps(writer, oracle, length, esc):
         write(writer, USER, cols, want, **shape)
 
 
+def test_a_window_holds_a_record(writer):
+    """Of the average size, and one and a half; else the tile is made for the general road."""
+    out = (C.c_uint32 * 2)()
+    for per in [60, 300, 1800, 5000, 9000, 16000, 30000, 38000, 43000, 60000, 10 ** 6]:
+        for model in (0, 2):
+            for items in (0, 10, 200):
+                rows = [0, 0, 0]
+                rows[model] = n = 50_000
+                writer.emu_write_shape(C.c_uint64(n), (C.c_uint64 * 3)(*rows), C.c_uint64(n * per), C.c_uint64(n * items if model == 0 else 0), C.c_uint64(0), out)
+                staged, text = per + 40 + 8 * (items if model == 0 else 0), per + 130 + 3 * (items if model == 0 else 0)
+                fits = staged * 1.04 + 1024 + 1.5 * text + 300 <= (128 if model == 0 and items > 16 else 100 if model == 0 else 64) * 1024
+                assert out[1] >= out[0] * staged + 1.4 * text if fits else out[0] >= 16, (per, model, items, out[0], out[1])
+
+
 def fall(off, row, by):
     """The range of string `row` goes back by `by` bytes: the string behind it shares them."""
     off[row + 1] = off[row] - by
