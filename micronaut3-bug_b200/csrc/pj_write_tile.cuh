@@ -1386,6 +1386,28 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
 }
 
 /* ---- host: the schema's columns as the tiles stage them ---------------------------------------------------------------- */
+/* How many wt_add_columns() makes of OBJ's properties from I on: with an element per row of the root's (ROWS), or the others. */
+template <int OBJ, int LEVEL, bool ROWS, int I = -1>
+PJ_CX uint32_t wt_count_columns() {
+  constexpr uint32_t own = (LEVEL == 0) == ROWS; /* a column that has an element wherever OBJ has one */
+  if constexpr (I < 0) return own + wt_count_columns<OBJ, LEVEL, ROWS, 0>(); /* presence */
+  else if constexpr (I >= CObj<OBJ>::N) return 0;
+  else {
+    constexpr uint32_t kind = CObj<OBJ>::f[I].kind;
+    uint32_t n = 0;
+    if constexpr (kind == K_DATETIME) n = 3u * own;
+    else if constexpr (kind == K_STR) n = own + !ROWS;
+    else if constexpr (kind == K_OBJ) n = wt_count_columns<CObj<OBJ>::f[I].child, LEVEL, ROWS>();
+    else if constexpr (kind == K_LIST_STR) n = own + 2u * !ROWS;
+    else if constexpr (kind == K_LIST_OBJ) n = own + wt_count_columns<CObj<OBJ>::f[I].child, 2, ROWS>();
+    else n = own;
+    return n + wt_count_columns<OBJ, LEVEL, ROWS, I + 1>();
+  }
+}
+static constexpr uint32_t WT_ROW_COLS = wt_count_columns<OBJ_PET, 0, true>() + wt_count_columns<OBJ_ORDER, 0, true>() + wt_count_columns<OBJ_USER, 0, true>();
+static constexpr uint32_t WT_OTHER_COLS = wt_count_columns<OBJ_PET, 0, false>() + wt_count_columns<OBJ_ORDER, 0, false>() + wt_count_columns<OBJ_USER, 0, false>();
+static_assert(WT_ROW_COLS <= 32u && WT_OTHER_COLS <= 32u, "wt_stage() takes a column per lane");
+static_assert(WT_ROW_COLS + WT_OTHER_COLS <= WT_COLS, "room for the columns");
 inline void wt_add_columns(const Schema& S, const ObjDesc& O, const DevCols& cols, uint32_t model, uint32_t level, bool rows, WTileArgs* a) {
   auto add = [&](uint32_t col, uint32_t shift, uint32_t lev, uint32_t plus, int off) {
     if ((lev == 0 && off < 0) != rows) return;

@@ -74,6 +74,15 @@ extern "C" int emu_write_tiles(uint32_t schema, uint32_t array, int inclusion, u
   *out_len = res.out_bytes;
   return res.ok ? 0 : 1;
 }
+/* Columns of a stream of several models, as the tiles stage them and as the limits count them: with an element per row, others, the same two. */
+extern "C" void emu_write_columns(uint32_t* out) {
+  Schema S;
+  build_schema(&S);
+  WTileArgs a;
+  memset((void*)&a, 0, sizeof a);
+  wt_columns(S, PJ_SCHEMA_MIXED, a.w.cols, &a);
+  out[0] = a.nrow; out[1] = a.ncol - a.nrow; out[2] = WT_ROW_COLS; out[3] = WT_OTHER_COLS;
+}
 extern "C" void emu_write_shape(uint64_t n, const uint64_t* rows, uint64_t arena, uint64_t strs, uint64_t objs, uint32_t* out) {
   WriteShapeIn in{n, {rows[0], rows[1], rows[2]}, arena, strs, objs, 148};
   const WriteShape s = write_shape(in, WT_MAX_RECS, WT_MAX_SMEM);

@@ -259,6 +259,13 @@ def test_no_records(writer, oracle):
     assert writer.emu_write_tiles(PET, 0, 0, 0, C.byref(cols.raw), None, C.c_uint64(0), 32, 8192, 0, C.byref(n)) == 0 and n.value == 0
 
 
+def test_columns_are_counted(writer):
+    """The limits of the staging (a column per lane) are checked when the kernel is compiled, on a count of what it is given."""
+    out = (C.c_uint32 * 4)()
+    writer.emu_write_columns(out)
+    assert tuple(out[:2]) == tuple(out[2:]) and 0 < out[0] <= 32 and 0 < out[1] <= 32 and out[0] + out[1] == len(abi.schema_columns(MIXED)) - 5
+
+
 def test_shapes_fit(writer):
     out = (C.c_uint32 * 2)()
     for n in (0, 1, 20, 5000, 10 ** 6, 10 ** 8):
