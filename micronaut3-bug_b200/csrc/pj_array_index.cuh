@@ -162,7 +162,7 @@ __device__ __forceinline__ bool arr_blank(uint32_t x) { return x == ' ' || x == 
 
 /* Separators of one word that starts at depth d outside (in: inside strings) ...; bytes [lo, hi) are input. bad, opener: lowest byte that breaks
  * `ws [ ... ] ws`, lowest `[` at depth 0 (64: none). */
-__device__ __forceinline__ uint64_t arr_mark(const uint8_t* p, const ArrWord& m, uint64_t quotes, uint64_t in, int32_t d, int32_t lo, int32_t hi, uint32_t* bad, uint32_t* opener, uint32_t* openers) {
+__device__ __forceinline__ uint64_t arr_mark(const uint8_t* p, const ArrWord& m, uint64_t quotes, uint64_t in, int32_t d, int32_t lo, int32_t hi, uint32_t* bad, uint32_t* opener) {
   const uint64_t valid = (hi >= 64 ? ~0ull : (1ull << hi) - 1u) & (lo > 0 ? ~0ull << lo : ~0ull);
   const uint64_t outside = ~in & ~quotes & valid, strange = (~in | quotes) & valid; /* not inside a string: quotes count there */
   uint64_t sep = 0, ev = (m.O | m.C) & outside;
@@ -179,7 +179,7 @@ __device__ __forceinline__ uint64_t arr_mark(const uint8_t* p, const ArrWord& m,
     const uint64_t bit = 1ull << b;
     ev &= ev - 1u;
     if (m.O & bit) {
-      if (d == 0 && p[b] == '[') { sep |= bit; if (*opener == 64u) *opener = b; ++*openers; }
+      if (d == 0 && p[b] == '[') { sep |= bit; if (*opener == 64u) *opener = b; }
       else if (d <= 0 && *bad == 64u) *bad = b;
       ++d;
     } else {
@@ -282,11 +282,11 @@ __global__ void __launch_bounds__(AI_THREADS, 4) k_arr_index(const __grid_consta
     const uint32_t up = popc64(m[k].O & ~in & ~q[k]), down = popc64(m[k].C & ~in & ~q[k]);
     sep[k] = 0;
     if (v < end && d - (int32_t)down <= 1) { /* (deeper all through: no separator) */
-      uint32_t bad = 64u, opener = 64u, openers = 0;
+      uint32_t bad = 64u, opener = 64u;
       const int32_t hi = end - v >= 64u ? 64 : (int32_t)(end - v);
-      if (d < 2 || !arr_mark_deep(base + v, m[k], q[k], in, d, hi, &sep[k])) sep[k] = arr_mark(base + v, m[k], q[k], in, d, v ? 0 : (int32_t)mis, hi, &bad, &opener, &openers);
+      if (d < 2 || !arr_mark_deep(base + v, m[k], q[k], in, d, hi, &sep[k])) sep[k] = arr_mark(base + v, m[k], q[k], in, d, v ? 0 : (int32_t)mis, hi, &bad, &opener);
       if (ok && bad < 64u) atomicMin(&a.res->doc_err_off, (unsigned long long)(v + bad - mis));
-      if (ok && opener < 64u) { atomicMin(&a.res->first_opener, (unsigned long long)(v + opener - mis)); atomicAdd(&a.res->n_openers, openers); }
+      if (ok && opener < 64u) atomicMin(&a.res->first_opener, (unsigned long long)(v + opener - mis));
     }
     d += (int32_t)up - (int32_t)down;
     s = (uint32_t)(in >> 63);

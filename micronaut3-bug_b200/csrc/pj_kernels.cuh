@@ -3,9 +3,10 @@
  *
  * JSON is parsed by k_parse_stream (pj_stream_kernel.cuh) and k_parse_items (pj_item.cuh), which build their own line index. This
  * header holds
- *   - the NDJSON record index on its own (k_nd_index<false> / k_scan_single / k_nd_index<true>: pj_index_records and
- *     its allocation-free variant);
- *   - what runs before and behind the writer's tiles (k_write_tile: pj_write_tile.cuh): k_reset and k_write_close.
+ *   - the NDJSON record index on its own: k_nd_records (pj_index_records), and k_nd_index<false> / k_scan_single / k_nd_index<true> (its
+ *     allocation-free variant);
+ *   - what runs before and behind a call's kernels: k_reset, k_fetch, and k_write_close behind the writer's tiles (pj_write_tile.cuh);
+ *   - the checksums of columns.
  *
  * Kernels that wait on other blocks (the look-backs) take their tile from an atomic ticket, so every block they
  * wait for is running or done, and every wait is bounded (the spin limit of the kernel's arguments ->
@@ -14,7 +15,9 @@
 #ifndef PJ_KERNELS_CUH
 #define PJ_KERNELS_CUH
 
+#if defined(__CUDACC__)
 #include <cuda_runtime.h>
+#endif
 #include <stddef.h>
 
 #include "pj_core.cuh"

@@ -29,7 +29,6 @@ struct DevResult {
   unsigned long long n_dense; /* k_parse_items: lines that hold no blank between tokens and no null */
   uint32_t max_rec;  /* bytes of the longest record, as far as the tiles saw its end */
   uint32_t strs_per_kb; /* k_parse_items: strings per 1024 bytes, of the tile with the most */
-  uint32_t n_openers;              /* array framing: `[` at depth 0 (a clean document has one) */
   unsigned long long first_opener; /* array framing: offset of the first `[` at depth 0 */
   uint32_t arr_final_s;            /* array framing: the input ends inside a string */
   int32_t arr_final_d;             /* array framing: nesting depth at the end of the input */

@@ -317,7 +317,7 @@ extern "C" int emu_parse_fast(uint32_t schema, uint32_t framing, const uint8_t* 
   }
 }
 
-#include "pj_array.cuh"
+#include "pj_array_ref.h"
 extern "C" int emu_array_index(const uint8_t* in, uint64_t len, uint64_t* s_out, uint64_t* e_out, uint8_t* blank_out, uint64_t cap,
                                uint64_t* n_out, uint32_t* doc_kind, uint64_t* doc_off) {
   uint64_t nwords = (len + 63) >> 6;

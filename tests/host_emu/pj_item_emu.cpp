@@ -9,6 +9,7 @@
 #include "pj_item.cuh"
 #include "pj_item_shape.h"
 #include "pj_choice.h"
+#include "pj_array_ref.h"
 
 using namespace pj;
 
@@ -41,7 +42,7 @@ void array_index(const uint8_t* in, uint64_t len, std::vector<uint64_t>& sep, De
     const WordMarks k = mark_word(m, e, st.d);
     sep[w] = k.sep;
     if (k.doc_bit < 64) res.doc_err_off = std::min<unsigned long long>(res.doc_err_off, w * 64 + k.doc_bit);
-    if (k.opener_bit < 64) { res.first_opener = std::min<unsigned long long>(res.first_opener, w * 64 + k.opener_bit); res.n_openers += k.n_openers; }
+    if (k.opener_bit < 64) res.first_opener = std::min<unsigned long long>(res.first_opener, w * 64 + k.opener_bit);
     st = e.out;
   }
   res.arr_final_s = st.s; res.arr_final_d = st.d;
