@@ -259,9 +259,10 @@ enum {
   PJ_OPT_HEX_LOWER = 1u << 3,              /* W3: \u00xx escapes are written with lower-case hex digits                    */
   PJ_OPT_TEST_RECORDS = 1u << 29, /* test hooks: the context's NDJSON calls all take the parse kernel with a record per thread / the one */
   PJ_OPT_TEST_ITEMS = 1u << 30,   /* that spreads a tile over strings, instead of the one its earlier calls speak for */
-  PJ_OPT_TEST_STALL_ONCE = 1u << 31 /* test hook for the time-out path: in the context's FIRST NDJSON parse call the first
-                                       tile is never handed out, so every other tile's bounded wait for it runs out
-                                       (after spin_limit_us) and the call answers PJ_ERR_TIMEOUT; later calls are normal */
+  PJ_OPT_TEST_STALL_ONCE = 1u << 31 /* test hook for the time-out path: in the context's FIRST call (pj_parse, pj_write or
+                                       pj_index_records) the first tile is never handed out, so every other tile's bounded
+                                       wait for it runs out (after spin_limit_us) and the call answers PJ_ERR_TIMEOUT; later
+                                       calls are normal */
 };
 
 typedef struct pj_options {

@@ -356,6 +356,13 @@ bool take_columns(pj_ctx* c, const ParsePlan& pp, const FetchArgs& fa, pj_column
   }
   return true;
 }
+/* Test hook (PJ_OPT_TEST_STALL_ONCE): of the context's first call tickets start at 1, tile 0 is never processed, the waits for it run out. */
+bool take_stall(pj_ctx* c) {
+  const bool s = c->stall_once;
+  c->stall_once = false;
+  return s;
+}
+cudaError_t stall_tile_0(pj_ctx* c, void* ticket) { return cudaMemsetAsync(ticket, 1, 1, c->stream); }
 /* the same look as the device's, for input that is in host memory and on its way in pieces */
 bool nd_host_looks_long(const uint8_t* in, uint64_t len) {
   uint32_t n = 0;
@@ -474,10 +481,7 @@ pj_status parse_stream(pj_ctx* c, uint32_t schema, const uint8_t* in, uint64_t l
       count_launch(c, 0);
     }
   }
-  if (c->stall_once) { /* test hook: tickets start at 1, tile 0 is never processed, the waits for it run out */
-    c->stall_once = false;
-    for (int p = 0; p < np; ++p) PJ_CUDA(c, cudaMemsetAsync((uint8_t*)c->tiles.p + (size_t)p * 256, 1, 1, c->stream));
-  }
+  if (take_stall(c)) for (int p = 0; p < np; ++p) PJ_CUDA(c, stall_tile_0(c, (uint8_t*)c->tiles.p + (size_t)p * 256));
   c->stats.tile_records = items ? IT_THREADS : ST_THREADS;
   uint64_t tiles_at = 0;
   for (int p = 0; p < np; ++p) {
@@ -614,8 +618,11 @@ pj_status array_index_plan(pj_ctx* c, const uint8_t* in, uint64_t len, size_t be
   ix->reset.res = c->d_res;
   return PJ_OK;
 }
-cudaError_t array_index_launch(pj_ctx* c, const ArrIndex& ix) {
+cudaError_t array_index_launch(pj_ctx* c, ArrIndex& ix) {
+  const bool stall = take_stall(c);
+  if (stall) ix.reset.more_words = ((ix.a.len + 63) >> 6) + 1; /* (the words of the tile that nobody writes) */
   k_reset<<<persistent_grid(c, ix.reset.words + ix.reset.more_words, 256), 256, 0, c->stream>>>(ix.reset);
+  if (stall) { const cudaError_t e = stall_tile_0(c, ix.a.ticket); if (e != cudaSuccess) return e; }
   if (ix.words == 4u) k_arr_index<4><<<ix.a.ntiles, AI_THREADS, 0, c->stream>>>(ix.a);
   else k_arr_index<1><<<ix.a.ntiles, AI_THREADS, 0, c->stream>>>(ix.a);
   count_launch(c, 0, 2);
@@ -927,6 +934,7 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   Stage stage(c);
   if (!array) {
     k_reset<<<persistent_grid(c, ix.reset.words, 256), 256, 0, c->stream>>>(ix.reset);
+    if (take_stall(c)) PJ_CUDA(c, stall_tile_0(c, rt.ticket));
     IndexArgs ia;
     ia.in = d_in; ia.len = len; ia.limit = len; ia.is_first = 1; ia.is_last = 1;
     ia.tile = nullptr; ia.rec_start = d_rs; ia.cap = cap; ia.goff = 0;
@@ -1106,6 +1114,7 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
   Stage stage(c);
   k_reset<<<persistent_grid(c, ra.words, 256), 256, 0, c->stream>>>(ra);
   count_launch(c, 0);
+  if (take_stall(c)) PJ_CUDA(c, stall_tile_0(c, ta.ticket));
   stage.next();
   cudaEvent_t ev_tile0 = c->ev[8], ev_tile1 = c->ev[9];
   PJ_CUDA(c, cudaEventRecord(ev_tile0, c->stream));
