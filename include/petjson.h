@@ -298,8 +298,9 @@ typedef struct pj_call_stats {
   uint32_t pieces;          /* pj_parse: pieces the input was parsed in (see pj_options.host_piece_bytes) */
   float device_ms;          /* CUDA-event time from first launch to last, on the call's stream  */
   float main_kernel_ms;     /* CUDA-event time of the dominant kernel(s) of the call            */
-  float stage_ms[8];        /* CUDA-event time per stage. parse, NDJSON: [2] the parse kernel(s), nothing else
-                               runs; parse, array framing: [0] separator index, [1] state reset, [2] the
+  float stage_ms[8];        /* CUDA-event time per stage. parse, NDJSON: [2] the parse kernel(s); what resets the
+                               state before them and brings the result to host memory behind them is in no stage;
+                               parse, array framing: [0] state reset and separators, [1] nothing, [2] the
                                parse kernel; write: [0] state reset, [1] the closing
                                kernel, [2] the tile kernel */
   uint32_t stage_launches[8]; /* kernels launched per stage; [4]: small calls, the kernel that brings the result to host memory
@@ -407,7 +408,9 @@ pj_status pj_index_records_static(const uint8_t* in, uint64_t len, uint64_t* rec
  * for a whole table: serialises rows [0, cols->n_rows[type]) of the model table(s) of `schema`
  * (for PJ_SCHEMA_MIXED: records in PJ_COL_REC_TYPE / PJ_COL_REC_ROW order, PJ_TYPE_NONE skipped).
  * `out` (cap bytes, `out_kind` memory) receives the JSON; *out_len the byte count, also on
- * PJ_ERR_CAPACITY. Columns live in cols->mem_kind memory. */
+ * PJ_ERR_CAPACITY. Columns live in cols->mem_kind memory; device columns and arenas are read in aligned blocks of
+ * 16 bytes, so up to 15 bytes before and behind a buffer may be read along with it (never across a block that holds
+ * none of its bytes); what they hold does not matter. */
 pj_status pj_write(pj_ctx* ctx, uint32_t schema, uint32_t framing, const pj_columns* cols,
                    uint8_t* out, uint64_t cap, uint32_t out_kind, uint64_t* out_len);
 

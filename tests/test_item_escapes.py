@@ -1,5 +1,5 @@
-"""Strings with escapes and UTF-8 in k_parse_items, decoded by a warp 32 bytes a step: every kind of character at every place around a step's edges,
-whole and broken, against the checker (on the CPU: tests/host_emu)."""
+"""Strings with escapes and UTF-8 in k_parse_items, decoded by a thread each, four bytes a step: every kind of character at every place in a word and around
+the 32nd and 64th byte, whole and broken, against the checker (on the CPU: tests/host_emu)."""
 import random
 
 import pytest
