@@ -5,15 +5,17 @@
  *
  *  1. The rows of a tile are consecutive in every model's table, so what it reads is ONE piece of every column and arena: bulk copies
  *     (cp.async.bulk) bring them to shared memory, and nothing is read from global memory after that. All threads look the strings over
- *     for bytes that have to be escaped, 16 bytes at a time; the few blocks that hold one are looked at again, a lane each, and their
- *     escapes counted for the strings they lie in.
+ *     for bytes that have to be escaped, 16 bytes at a time; the few blocks that hold one are looked at again, a byte per lane, and their
+ *     escapes counted for the strings they lie in. Where more than WT_HITS blocks hold one, all strings are looked over instead, one per
+ *     lane (200 k Pets with two quotes a name, kernel, us: every block by a warp 138, strings by lanes 84, and the short ones written by the lanes that
+ *     meet them 74; 100 k Users with four paths 107 / 66 / 48).
  *  2. Sizes: first the elements of the lists, an element per lane, with running sums; then the records, a record per lane, 32 of one
  *     model at a time.
  *  3. One decoupled look-back over the earlier tiles gives the tile's place in the output.
  *  4. Text: the first half of a record's properties, the second half, the strings of its list and the objects of its list are units
  *     of their own, each a lane's, so that the lanes of a warp do the same and long lists are spread over lanes. A lane puts its text
  *     together in a register and stores whole words into a window in shared memory; words that two units share are or-ed.
- *     Strings with a byte to escape and strings of 512 bytes and more are left out and written afterwards, a warp per string or per 2 KB of it (by the
+ *     Strings with a byte to escape (but short ones where most are) and strings of 512 bytes and more are left out and written afterwards, a warp per string or per 2 KB of it (by the
  *     lane that meets them, 300 MB of Users: strings of 300 bytes 780 us with it, 940 without; of 1000 bytes 666 and 440).
  *  5. The window leaves with one bulk copy. Text longer than the window goes in several rounds of 4 and 5.
  *
@@ -62,6 +64,7 @@ static constexpr uint32_t WT_MIN_WINDOW = 2048;
 static constexpr uint32_t WT_ESC = 160;             /* strings with escapes, and long ones, a round keeps for later */
 static constexpr uint32_t WT_LONG = 512;            /* bytes of a string that a warp copies */
 static constexpr uint32_t WT_LONG_LIST = 8;         /* elements of a list that a warp writes on the general road */
+static constexpr uint32_t WT_SHORT = 48;            /* bytes up to which a lane escapes a string where the tile has many of them */
 static constexpr uint32_t WT_PART = 2048;           /* bytes of a long string a warp takes at a time */
 static constexpr uint32_t WT_HITS = 192;            /* 16-byte blocks with a byte to escape that are kept in a list */
 static constexpr uint32_t WT_BACK = 4;              /* tiles a lane looks back at per round */
@@ -214,6 +217,7 @@ __device__ __forceinline__ uint32_t wt_extra(const WtShared& sh, const uint8_t* 
 struct WtRead { /* what the units of a tile read */
   int incl;
   bool dirty; /* some string of the tile has to be escaped */
+  bool many;  /* most of them: short ones are the lanes' that meet them */
   bool later; /* ... or is long: not all are written where they are met */
   uint32_t hexa;
 };
@@ -479,18 +483,6 @@ __device__ __forceinline__ void wt_put_enum(WtOut& e, uint32_t k) { /* behind it
   wt_put(e, w1, n >= 8u ? 32u : 8u * (n - 4u));
   wt_put(e, w2, n > 8u ? 8u * (n - 8u) : 0u);
 }
-/* n bytes at byte s, escaped */
-static __device__ __noinline__ WtOut wt_put_escaped(WtOut e, uint32_t s, uint32_t n, uint32_t hexa) {
-  for (uint32_t i = 0; i < n; ++i) {
-    const uint32_t c = e.w8[s + i];
-    if (!escape_extra_byte(c)) { wt_put(e, c, 8); continue; }
-    const uint32_t y = c == 8 ? 'b' : (c == 9 ? 't' : (c == 10 ? 'n' : (c == 12 ? 'f' : (c == 13 ? 'r' : c))));
-    if (y >= 0x20) { wt_put(e, '\\' | (y << 8), 16); continue; }
-    wt_put4(e, '\\' | ('u' << 8) | ('0' << 16) | ('0' << 24));
-    wt_put(e, ('0' + (c >> 4)) | (((c & 15) < 10 ? '0' + (c & 15) : hexa + (c & 15) - 10) << 8), 16);
-  }
-  return e;
-}
 __device__ __forceinline__ uint32_t wt_peek4(const uint8_t* w8, uint32_t s) {
   return __funnelshift_r(wt_ld(w8, s & ~3u), wt_ld(w8, (s & ~3u) + 4u), (s & 3u) * 8u);
 }
@@ -507,6 +499,27 @@ __device__ __forceinline__ uint64_t wt_escaped(uint32_t c, uint32_t hexa, uint32
 __device__ __forceinline__ uint32_t wt_word_extra(uint32_t x, uint32_t have) {
   if (have < 4u) x |= 0x61616161u << (8u * have); /* (letters) */
   return word_needs_escape(x) ? word_escape_extra(x) : 0u;
+}
+/* n bytes at byte s, escaped */
+static __device__ __noinline__ WtOut wt_put_escaped(WtOut e, uint32_t s, uint32_t n, uint32_t hexa) {
+  for (uint32_t i = 0, left = 0; i < n; ++i) {
+    if (left == 0) { /* four bytes that stay as they are, or these four one by one */
+      const uint32_t have = n - i < 4u ? n - i : 4u, x = wt_low(wt_peek4(e.w8, s + i), have);
+      if (!wt_word_extra(x, have)) {
+        if (have == 4u) wt_put4(e, x); else wt_put(e, x, 8u * have);
+        i += have - 1u;
+        continue;
+      }
+      left = have;
+    }
+    --left;
+    uint32_t len;
+    const uint64_t v = wt_escaped(e.w8[s + i], hexa, &len);
+    if (len <= 2u) { wt_put(e, (uint32_t)v, 8u * len); continue; }
+    wt_put4(e, (uint32_t)v);
+    wt_put(e, (uint32_t)(v >> 32), 16);
+  }
+  return e;
 }
 /* the len (1 .. 6) bytes of v to byte p of the window */
 __device__ __forceinline__ void wt_or_bytes(uint8_t* w8, uint32_t p, uint64_t v, uint32_t len) {
@@ -585,7 +598,7 @@ __device__ __forceinline__ void wt_put_str(const WtRead& r, WtShared& sh, WtOut&
   if (r.later) {
     const uint32_t extra = r.dirty ? wt_extra(sh, e.w8, col, index) : 0u;
     if (extra || n >= WT_LONG) {
-      const uint32_t k = atomicAdd(&sh.nesc, 1u);
+      const uint32_t k = r.many && n < WT_SHORT ? WT_ESC : atomicAdd(&sh.nesc, 1u);
       if (k < WT_ESC) { /* later, by a warp */
         const uint32_t pos = wt_pos(e);
         sh.esc[k].at = s; sh.esc[k].n = n | (extra ? 0x80000000u : 0u); sh.esc[k].dst = pos;
@@ -894,6 +907,18 @@ __device__ __forceinline__ void wt_stage(const WTileArgs& a, WtShared& sh, uint8
   if (extra + 4u * strs + 16u + WT_MIN_WINDOW > a.smem) bad = true;
   if (lane == 0) { sh.stage = at; sh.sums = sums; sh.extra = sh.win = extra; sh.nstr = strs; if (bad) sh.odd = 1; }
 }
+/* bytes the escapes of the n bytes at s add, all lanes of a warp: 16-byte blocks, looked at again where there is one */
+__device__ __forceinline__ uint32_t wt_warp_extra(const uint8_t* s, uint32_t n, uint32_t lane) {
+  const uintptr_t from = reinterpret_cast<uintptr_t>(s), to = from + n;
+  uint32_t extra = 0;
+  for (uintptr_t p = (from & ~(uintptr_t)15) + 16u * lane; p < to; p += 512u) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+    if (word_needs_escape(x[0]) | word_needs_escape(x[1]) | word_needs_escape(x[2]) | word_needs_escape(x[3]))
+      for (uint32_t k = 0; k < 16u; ++k) if (p + k >= from && p + k < to) extra += escape_extra_byte((x[k >> 2] >> (8u * (k & 3u))) & 0xFFu);
+  }
+  return __reduce_add_sync(0xFFFFFFFFu, extra);
+}
 /* a 16-byte block with a byte to escape: counted for the strings it lies in, by a warp */
 __device__ __forceinline__ void wt_count_block(WtShared& sh, uint8_t* w8, uint32_t block, uint32_t lane) {
   const uint32_t who = __ballot_sync(0xFFFFFFFFu, block - sh.ar0[lane] < (uint32_t)sh.ar1[lane] - sh.ar0[lane]);
@@ -906,6 +931,35 @@ __device__ __forceinline__ void wt_count_block(WtShared& sh, uint8_t* w8, uint32
   uint32_t lo = 0, hi = level == 0 ? sh.cnt[model] : sh.itemn[level - 1u]; /* the last string that begins at or before it */
   while (lo + 1u < hi) { const uint32_t mid = (lo + hi) >> 1; if (o[mid] <= x) lo = mid; else hi = mid; }
   atomicAdd(wt_extras(sh, w8) + sh.str0[col] + lo, extra);
+}
+/* All strings of the tile that are staged, one per lane: their escapes. For text with many bytes to escape; bad: one lies outside its arena. */
+__device__ __forceinline__ bool wt_count_strings(WtShared& sh, uint8_t* w8, uint32_t warp, uint32_t warps, uint32_t lane) {
+  uint32_t todo = __ballot_sync(0xFFFFFFFFu, sh.ar1[lane] > sh.ar0[lane]), turn = 0; /* the first group of 32 goes to this warp */
+  bool bad = false;
+  for (; todo; todo &= todo - 1u) {
+    const uint32_t c = (uint32_t)__ffs((int)todo) - 1u, col = sh.arcol[c], level = sh.arlevel[c], model = sh.armodel[c];
+    const uint32_t first = level == 0 ? (uint32_t)sh.row0[model] : sh.item0[level - 1u], n = level == 0 ? sh.cnt[model] : sh.itemn[level - 1u], groups = (n + 31u) / 32u;
+    const uint32_t* o = wt_at<uint32_t>(sh, w8, col - 1u, first); /* (an arena's column follows its offsets') */
+    for (uint32_t g = (warp + warps - turn) % warps; g < groups; g += warps) {
+      const uint32_t k = 32u * g + lane;
+      uint32_t a = 0, len = 0;
+      if (k < n) {
+        const uint32_t b = o[k + 1u];
+        a = o[k];
+        if (a > b || a < sh.lo[col] || b - sh.lo[col] > sh.span[col]) bad = true;
+        else len = b - a;
+      }
+      const uint8_t* s = w8 + (sh.at[col] + a);
+      if (len && len < WT_LONG) wt_extras(sh, w8)[sh.str0[col] + k] = str_escape_extra(s, len);
+      for (uint32_t longs = __ballot_sync(0xFFFFFFFFu, len >= WT_LONG); longs; longs &= longs - 1u) { /* those are a warp's, one after the other */
+        const int who = __ffs((int)longs) - 1;
+        const uint32_t m = __shfl_sync(0xFFFFFFFFu, len, who), from = sh.at[col] + __shfl_sync(0xFFFFFFFFu, a, who), extra = wt_warp_extra(w8 + from, m, lane);
+        if (lane == 0) wt_extras(sh, w8)[sh.str0[col] + 32u * g + (uint32_t)who] = extra;
+      }
+    }
+    turn = (turn + groups) % warps;
+  }
+  return bad;
 }
 /* Mixed streams: the tile's records by model, in order; odd when the rows of a model do not follow each other. */
 __device__ __forceinline__ void wt_sort(const WTileArgs& a, WtShared& sh, uint64_t rec0, uint32_t nrec, uint32_t tid) {
@@ -992,18 +1046,6 @@ __device__ __forceinline__ unsigned long long wt_general_any(const DevCols* c, u
   if constexpr (SCHEMA == PJ_SCHEMA_USER || SCHEMA == PJ_SCHEMA_MIXED)
     if (model == 2) return WR && plain ? wt_general<OBJ_USER, WR, WR>(c, row, incl, hexa, dst, after, sh, e, cap, rec) : wt_general<OBJ_USER, WR, false>(c, row, incl, hexa, dst, after, sh, e, cap, rec);
   return 0;
-}
-/* bytes the escapes of the n bytes at s add, all lanes of a warp: 16-byte blocks, looked at again where there is one */
-__device__ __forceinline__ uint32_t wt_warp_extra(const uint8_t* s, uint32_t n, uint32_t lane) {
-  const uintptr_t from = reinterpret_cast<uintptr_t>(s), to = from + n;
-  uint32_t extra = 0;
-  for (uintptr_t p = (from & ~(uintptr_t)15) + 16u * lane; p < to; p += 512u) {
-    const uint4 v = *reinterpret_cast<const uint4*>(p);
-    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
-    if (word_needs_escape(x[0]) | word_needs_escape(x[1]) | word_needs_escape(x[2]) | word_needs_escape(x[3]))
-      for (uint32_t k = 0; k < 16u; ++k) if (p + k >= from && p + k < to) extra += escape_extra_byte((x[k >> 2] >> (8u * (k & 3u))) & 0xFFu);
-  }
-  return __reduce_add_sync(0xFFFFFFFFu, extra);
 }
 /* the n bytes at s to d, as they are, all lanes of a warp: 16-byte blocks of d */
 __device__ __forceinline__ void wt_warp_copy(uint8_t* d, const uint8_t* s, uint32_t n, uint32_t lane) {
@@ -1261,7 +1303,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
   if (warp == 0) wt_stage<SCHEMA>(a, sh, smem, lane);
   __syncthreads();
   WtRead x;
-  x.incl = a.w.inclusion; x.hexa = a.w.hexa; x.dirty = x.later = false;
+  x.incl = a.w.inclusion; x.hexa = a.w.hexa; x.dirty = x.later = x.many = false;
   bool odd = sh.odd != 0;
   const uint32_t ngroups = wt_groups<SCHEMA>(sh);
   if (sh.flight) {
@@ -1278,6 +1320,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
   }
   if (!odd) {
     const uint32_t b0 = sh.text >> 4, b1 = sh.stage >> 4;
+    bool bad = false;
     uint32_t any = 0;
     for (uint32_t b = b0 + tid; b < b1; b += THREADS) {
       const uint4 v = *reinterpret_cast<const uint4*>(smem + 16u * b);
@@ -1293,11 +1336,11 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
       if (tid == 0) sh.win = (sh.extra + 4u * sh.nstr + 15u) & ~15u;
       for (uint32_t k = tid; k < sh.nstr; k += THREADS) ex[k] = 0;
       __syncthreads();
-      const bool all = sh.nhit > WT_HITS; /* (more than the list holds: every block) */
-      for (uint32_t k = warp; k < (all ? b1 - b0 : sh.nhit); k += WARPS) wt_count_block(sh, smem, all ? b0 + k : sh.hit[k], lane);
+      x.many = sh.nhit > WT_HITS;
+      if (x.many) bad = wt_count_strings(sh, smem, warp, WARPS, lane);
+      else for (uint32_t k = warp; k < sh.nhit; k += WARPS) wt_count_block(sh, smem, sh.hit[k], lane);
       __syncthreads();
     }
-    bool bad = false;
     if constexpr (SCHEMA == PJ_SCHEMA_PET || SCHEMA == PJ_SCHEMA_MIXED) {
       const uint32_t npet = (sh.cnt[0] + 31u) / 32u;
       for (uint32_t u = warp; u < 2u * npet; u += WARPS) {

@@ -39,6 +39,15 @@ def test_long_strings(ctx, oracle, size, esc):
     check(ctx, oracle, USER, oracle.parse(USER, users(400 if size < 4000 else 40, size, esc)))
 
 
+@pytest.mark.parametrize("size, esc", [(5, 2), (20, 7), (47, 3), (48, 3), (70, 60), (520, 9)])
+def test_many_bytes_to_escape(ctx, oracle, size, esc):
+    """Strings looked over one per lane; those shorter than 48 bytes escaped by the lanes that meet them."""
+    check(ctx, oracle, USER, oracle.parse(USER, users(3000 if size < 500 else 300, size, esc)))
+    line = '{"id":%d,"category":{"name":"%s"},"name":"%s","photoUrls":["%s",""],"tags":[{"name":"%s"}]}'
+    text = lambda i: "".join('\\n' if (j + i) % esc == 1 else "p" for j in range(size))
+    check(ctx, oracle, PET, oracle.parse(PET, as_u8("\n".join(line % (i, text(i), text(i + 1), text(i + 2), text(i + 3)) for i in range(1500 if size < 500 else 200)))))
+
+
 @pytest.mark.parametrize("dirty", [0, 0.01])
 def test_long_lists_and_records_of_all_sizes(ctx, oracle, dirty):
     rng = random.Random(3)

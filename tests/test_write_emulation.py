@@ -253,6 +253,30 @@ def test_offsets_that_fall_where_no_string_is(writer, oracle, recs):
             write(writer, PET, cols, oracle.write(PET, cols, NDJSON, inclusion), inclusion=inclusion, recs=recs)
 
 
+@pytest.mark.parametrize("recs", [40, 128])
+@pytest.mark.parametrize("falls", [False, True])
+def test_tiles_with_many_bytes_to_escape(writer, oracle, falls, recs):
+    """More 16-byte blocks with one than a tile keeps: its strings are looked over one per lane. Whole words and ends of strings, plain and not."""
+    rng = random.Random(recs)
+    word = lambda k: "".join(rng.choice(['\\"', "\\n", "\\u0001", "\\\\"]) if rng.random() < 0.2 else "abcdefg"[j % 7] for j in range(k))
+    length = lambda: rng.choice([0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 33, 63] + [511, 512, 513] * (recs < 100))
+    users = ['{"id":%d,%s}' % (i, ",".join('"%s":"%s"' % (k, word(length())) for k in ("username", "firstName", "lastName", "email", "password", "phone"))) for i in range(150)]
+    pets = ['{"id":%d,"category":{"id":1,"name":"%s"},"name":"%s","photoUrls":["%s","%s"],"tags":[{"id":2,"name":"%s"},{"name":"%s"}]}' % ((i,) + tuple(word(length()) for _ in range(6))) for i in range(150)]
+    mixed = [x for pair in zip(users, pets) for x in pair]
+    for schema, lines in ((USER, users), (PET, pets), (MIXED, mixed)):
+        cols = oracle.parse(schema, as_u8("\n".join(lines)))
+        assert cols.n_errors == 0
+        if falls and schema != PET:
+            for row in range(1, 149, 9):
+                cols.arrays[COL["usr_present"]][row] &= ~2 & 0xFF
+                off = cols.arrays[COL["usr_username_off"]].view(np.uint32)
+                off[row + 1] = max(int(off[row]) - 5, 0)
+        for inclusion in INCLUSIONS:
+            want = oracle.write(schema, cols, NDJSON, inclusion)
+            for shape in (dict(shared=131072), dict(shared=100 * 1024, mis=7, order=3)):
+                write(writer, schema, cols, want, inclusion=inclusion, recs=recs, **shape)
+
+
 def test_no_records(writer, oracle):
     cols = abi.HostColumns(PET, abi.default_caps(PET, 1, 16))
     n = C.c_uint64()
