@@ -375,6 +375,19 @@ def test_choice_of_the_kernel(emu):
     assert choose(emu, ["spaced"] * 5, size=20_000) == [0, 1, 1, 1, 1]  # too short to be timed: by the spelling alone
 
 
+@pytest.mark.parametrize("first, later, other, best", [(0.255, 0.113, 0.172, 0), (0.255, 0.113, 0.080, 1), (0.60, 0.46, 0.35, 1)])
+def test_a_handles_first_call_does_not_decide_alone(emu, first, later, other, best):
+    """k_parse_stream's first call on a handle takes longer: where it loses narrowly it has a second one, then the faster kernel stays."""
+    lib, size, took, now, runs = emu[USER], 5_000_000, [], 0, 0
+    lib.emu_choice_reset()
+    for _ in range(40):
+        took.append(now)
+        ms = other if now else (later if runs else first)
+        runs += not now
+        now = lib.emu_choice_note(C.c_uint64(size), C.c_float(ms), C.c_uint64(50_000), C.c_uint64(0), C.c_uint64(0), C.c_uint64(0), C.c_uint32(110))
+    assert took[:3] == [0, 1, 0 if first - other < 0.2 else 1] and took[3:] == [best] * 37, took
+
+
 def test_under_sanitizers():
     asan = subprocess.run(["gcc", "-print-file-name=libasan.so"], capture_output=True, text=True).stdout.strip()
     if not os.path.isabs(asan) or not os.path.exists(asan):
