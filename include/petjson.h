@@ -260,7 +260,7 @@ enum {
   PJ_OPT_TEST_RECORDS = 1u << 29, /* test hooks: the context's NDJSON calls all take the parse kernel with a record per thread / the one */
   PJ_OPT_TEST_ITEMS = 1u << 30,   /* that spreads a tile over strings, instead of the one its earlier calls speak for */
   PJ_OPT_TEST_STALL_ONCE = 1u << 31 /* test hook for the time-out path: in the context's FIRST call (pj_parse, pj_write or
-                                       pj_index_records) the first tile is never handed out, so every other tile's bounded
+                                       pj_index_records) whose tiles wait for one another the first one is never handed out, so every other tile's bounded
                                        wait for it runs out (after spin_limit_us) and the call answers PJ_ERR_TIMEOUT; later
                                        calls are normal */
 };

@@ -893,6 +893,11 @@ pj_status pj_parse_shard(pj_ctx* ctx, uint32_t schema, const uint8_t* in, uint64
   return parse_impl(ctx, schema, PJ_FRAMING_NDJSON, in, len, slack, is_first != 0, is_last != 0, global_offset, in_kind, out);
 }
 
+/* NDJSON whose second reading comes from L2 (126 MB) is read twice, by kernels without a wait between tiles; less is not worth three launches, and more
+ * is read once. A call, us, twice / once with one word of 64 bytes a thread / with four: 8 MB 50 / 48 / -, 15 MB 51 / 55 / -, 19 MB 52 / 60 / -, 20 MB
+ * 52 / - / 52, 30 MB 56 / - / 58, 50 MB 62 / - / 68, 100 MB 93 / - / 83, 300 MB 184 / - / 174. */
+static constexpr uint64_t ND_TWICE_FROM = 8u << 20, ND_TWICE_TO = 64u << 20;
+
 pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint64_t len, uint32_t kind, uint64_t* rec_start,
                            uint64_t cap, uint64_t* n) {
   if (!c) return PJ_ERR_ARG;
@@ -905,7 +910,8 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   const uint8_t* d_in = in;
   uint64_t* d_rs = rec_start;
   const uint64_t nwords = (len + 63) >> 6;
-  const uint32_t words = !array && len >= (uint64_t)c->sms * 2u * 64u * 1024u ? 4u : 1u; /* of 64 bytes per thread, as in array_index_plan() */
+  const bool twice = !array && len >= ND_TWICE_FROM && len < ND_TWICE_TO;
+  const uint32_t words = !array && len >= ND_TWICE_TO ? 4u : 1u; /* of 64 bytes per thread */
   const uint64_t ntiles = array ? (nwords ? (nwords + ARR_THREADS - 1) / ARR_THREADS : 1) : (len + 15 + (uint64_t)INDEX_TILE * words) / ((uint64_t)INDEX_TILE * words);
   const size_t off_rs = align_up(array ? (nwords + 1) * 8 : 0, 256);
   { pj_status st = ensure(c, &c->scratch, off_rs + (kind == PJ_MEM_HOST ? cap * 8 : 0) + 256); if (st) return st; }
@@ -920,13 +926,13 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
     d_rs = (uint64_t*)((uint8_t*)c->scratch.p + off_rs);
   }
   RecordTiles rt;
-  const size_t state = align_up(256 + ntiles * 16, 256);
+  const size_t state = align_up(256 + (twice ? ntiles * 4 + 4 : ntiles * 16), 256);
   ArrIndex ix;
   if (array) { pj_status st = array_index_plan(c, d_in, len, state, 0, &ix); if (st) return st; }
   else {
     pj_status st = ensure(c, &c->tiles, state); if (st) return st;
     memset(&ix, 0, sizeof ix);
-    ix.reset.state = (unsigned long long*)c->tiles.p; ix.reset.words = state / 8; ix.reset.res = c->d_res;
+    ix.reset.state = (unsigned long long*)c->tiles.p; ix.reset.words = twice ? 0 : state / 8; ix.reset.res = c->d_res;
   }
   rt.ticket = (uint32_t*)c->tiles.p;
   rt.agg = (unsigned long long*)((uint8_t*)c->tiles.p + 256); rt.inc = rt.agg + ntiles;
@@ -934,13 +940,18 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   Stage stage(c);
   if (!array) {
     k_reset<<<persistent_grid(c, ix.reset.words, 256), 256, 0, c->stream>>>(ix.reset);
-    if (take_stall(c)) PJ_CUDA(c, stall_tile_0(c, rt.ticket));
+    if (!twice && take_stall(c)) PJ_CUDA(c, stall_tile_0(c, rt.ticket));
     IndexArgs ia;
     ia.in = d_in; ia.len = len; ia.limit = len; ia.is_first = 1; ia.is_last = 1;
     ia.tile = nullptr; ia.rec_start = d_rs; ia.cap = cap; ia.goff = 0;
-    if (words == 4u) k_nd_records<4><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia, rt);
+    if (twice) {
+      ia.tile = (uint32_t*)((uint8_t*)c->tiles.p + 256);
+      k_nd_index<false><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia);
+      k_scan_single<uint32_t><<<1, 1024, 0, c->stream>>>(ia.tile, ntiles, &c->d_res->n_records);
+      k_nd_index<true><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia);
+    } else if (words == 4u) k_nd_records<4><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia, rt);
     else k_nd_records<1><<<(unsigned)ntiles, INDEX_THREADS, 0, c->stream>>>(ia, rt);
-    count_launch(c, 0, 2);
+    count_launch(c, 0, twice ? 4 : 2);
   } else {
     PJ_CUDA(c, array_index_launch(c, ix));
     ArrArgs aa;
@@ -955,8 +966,7 @@ pj_status pj_index_records(pj_ctx* c, uint32_t framing, const uint8_t* in, uint6
   stage.next();
   FetchArgs fa;
   fa.n = 0;
-  if (len <= SMALL_CALL) PJ_CUDA(c, launch_fetch(c, fa));
-  else PJ_CUDA(c, cudaMemcpyAsync(c->h_res, c->d_res, sizeof(DevResult), cudaMemcpyDeviceToHost, c->stream));
+  PJ_CUDA(c, launch_fetch(c, fa));
   PJ_CUDA(c, cudaStreamSynchronize(c->stream));
   collect_times(c, 1);
   c->stats.main_kernel_ms = c->stats.stage_ms[0];

@@ -3,8 +3,8 @@
  *
  * JSON is parsed by k_parse_stream (pj_stream_kernel.cuh) and k_parse_items (pj_item.cuh), which build their own line index. This
  * header holds
- *   - the NDJSON record index on its own: k_nd_records (pj_index_records), and k_nd_index<false> / k_scan_single / k_nd_index<true> (its
- *     allocation-free variant);
+ *   - the NDJSON record index on its own: k_nd_records (pj_index_records), and k_nd_index<false> / k_scan_single / k_nd_index<true> (the
+ *     same for inputs that L2 holds, and its allocation-free variant);
  *   - what runs before and behind a call's kernels: k_reset, k_fetch, and k_write_close behind the writer's tiles (pj_write_tile.cuh);
  *   - the checksums of columns.
  *
@@ -141,8 +141,8 @@ __device__ __forceinline__ bool records_before(const RecordTiles& t, uint32_t ti
   return sh[1] != 0;
 }
 /* The NDJSON record index in one pass: W words of 64 bytes per thread, a tile's place by look-back. (In two passes and
- * three launches before: 1000 Pets 38 -> 31 us a call; 1 M Pets 157 -> 147, where the look-back takes a third.)
- * k_nd_index stays for callers without memory for the tiles' states. */
+ * three launches: 1000 Pets 38 -> 31 us a call; 1 M Pets 157 -> 147, where the look-back takes a third.)
+ * k_nd_index stays for inputs that it reads from L2 the second time, and for callers without memory for the tiles' states. */
 template <int W>
 __global__ void __launch_bounds__(INDEX_THREADS) k_nd_records(const __grid_constant__ IndexArgs a, const __grid_constant__ RecordTiles t) {
   __shared__ uint32_t sh[33], sh_tile;

@@ -140,3 +140,22 @@ def test_a_bounded_wait_that_runs_out(native, oracle, what):
             call()
         assert e.value.status == abi.PJ_ERR_TIMEOUT
         assert call() and call()
+
+
+@pytest.mark.parametrize("edge", [8 << 20, 64 << 20])
+def test_record_index_where_the_input_is_read_twice(ctx, oracle, edge):
+    """Between 8 and 64 MB two passes, else one."""
+    import torch
+
+    body = text_of(edge + 1, False)
+    buf = torch.empty(body.size + 16, dtype=torch.uint8, device="cuda")
+    for size in (edge - 1, edge, edge + 1):
+        want = oracle.index(body[:size], NDJSON)
+        for off in (0, 5):
+            buf[off:off + size].copy_(torch.from_numpy(body[:size]))
+            starts = torch.zeros(want.size + 1, dtype=torch.int64, device="cuda")
+            torch.cuda.synchronize()
+            assert ctx.index_records(buf[off:off + size], starts, NDJSON) == want.size
+            got = starts.cpu().numpy().view(np.uint64)
+            assert np.array_equal(got[:-1], want) and got[-1] == 0
+        assert ctx.index_records(buf[5:5 + size], starts[:10], NDJSON, allow_capacity=True) == want.size
