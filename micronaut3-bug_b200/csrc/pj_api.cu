@@ -322,7 +322,8 @@ uint32_t pick_stream_tile(const pj_ctx* c, uint32_t schema) {
   return (uint32_t)tb;
 }
 /* Calls of up to so many bytes are told their result by a kernel (k_fetch) and reset by one (k_reset): a copy engine and a memset each cost 4 - 6 us, of
- * the 40 that a small call takes. Above, that does not matter, and an NDJSON call stays one launch. */
+ * the 40 that a small call takes. Larger calls of the parse kernels still go without, though 30 to 45 of their 150 to 600 us are outside the main
+ * kernel: an NDJSON call of one model stays one launch there. */
 static constexpr uint64_t SMALL_CALL = 16u << 20;
 /* Columns of a small call that go to host memory with the result: none when `out` lies on the device or the input suggests more than there is room for. */
 void fetch_columns(const ParsePlan& pp, const pj_columns* out, uint64_t len, FetchArgs* fa) {
