@@ -816,6 +816,7 @@ pj_status pj_create(const pj_options* opt, pj_ctx** out) {
   if (e == cudaSuccess) e = stream_init_3(&c->schema);
   if (e == cudaSuccess) e = stream_init_4(&c->schema);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_PET>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_PET, WT_SHORT_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_USER>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_write_tile<PJ_SCHEMA_MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, WT_MAX_SMEM);
@@ -1130,7 +1131,10 @@ pj_status pj_write(pj_ctx* c, uint32_t schema, uint32_t framing, const pj_column
   cudaEvent_t ev_tile0 = c->ev[8], ev_tile1 = c->ev[9];
   PJ_CUDA(c, cudaEventRecord(ev_tile0, c->stream));
   switch (schema) {
-    case PJ_SCHEMA_PET: k_write_tile<PJ_SCHEMA_PET><<<(unsigned)ntiles, WtT<PJ_SCHEMA_PET>::threads, shape.smem, c->stream>>>(ta); break;
+    case PJ_SCHEMA_PET:
+      if (wt_short(shape.smem, ntiles, (uint32_t)c->sms)) k_write_tile<PJ_SCHEMA_PET, WT_SHORT_THREADS><<<(unsigned)ntiles, WT_SHORT_THREADS, shape.smem, c->stream>>>(ta);
+      else k_write_tile<PJ_SCHEMA_PET><<<(unsigned)ntiles, WtT<PJ_SCHEMA_PET>::threads, shape.smem, c->stream>>>(ta);
+      break;
     case PJ_SCHEMA_ORDER: k_write_tile<PJ_SCHEMA_ORDER><<<(unsigned)ntiles, WtT<PJ_SCHEMA_ORDER>::threads, shape.smem, c->stream>>>(ta); break;
     case PJ_SCHEMA_USER: k_write_tile<PJ_SCHEMA_USER><<<(unsigned)ntiles, WtT<PJ_SCHEMA_USER>::threads, shape.smem, c->stream>>>(ta); break;
     default: k_write_tile<PJ_SCHEMA_MIXED><<<(unsigned)ntiles, WtT<PJ_SCHEMA_MIXED>::threads, shape.smem, c->stream>>>(ta); break;

@@ -57,6 +57,7 @@ template <int SCHEMA> struct WtT {
   static constexpr uint32_t warps = threads / 32u;
 };
 static_assert(WT_MAX_RECS <= 256, "a record per thread");
+static constexpr uint32_t WT_SHORT_THREADS = 256, WT_SHORT_BLOCKS = 4; /* tables of short Pets, see wt_short() */
 inline uint32_t wt_threads(uint32_t schema) { return schema == PJ_SCHEMA_PET ? WtT<1>::threads : (schema == PJ_SCHEMA_ORDER ? WtT<2>::threads : (schema == PJ_SCHEMA_USER ? WtT<3>::threads : WtT<4>::threads)); }
 static constexpr uint32_t WT_MOST_WARPS = 16;
 static constexpr uint32_t WT_MAX_SMEM = 128 * 1024;
@@ -214,6 +215,12 @@ __device__ __forceinline__ uint32_t wt_extra(const WtShared& sh, const uint8_t* 
 }
 
 /* ---- sizes ----------------------------------------------------------------------------------------------------------- */
+/* Pets whose tiles leave four blocks room on an SM, and more tiles than two blocks of it take at once: a short tile is three trips of its staging and a
+ * look-back, and four of them wait in turn. 1 M Pets, 512 threads / 256, us of the kernel: {} 143 / 95, an id and a name of two bytes 167 / 113, 64 bytes of
+ * text 197 / 146; 200 k 42 / 30, 46 / 34, 50 / 42. 60 k are one wave either way (22 / 23; with a name of 64 bytes and escapes 40 k 33 / 41). */
+inline bool wt_short(uint32_t smem, uint64_t ntiles, uint32_t sms) {
+  return smem <= 228u * 1024u / WT_SHORT_BLOCKS - 1024u - (uint32_t)sizeof(WtShared) && ntiles > 2u * (uint64_t)sms;
+}
 struct WtRead { /* what the units of a tile read */
   int incl;
   bool dirty; /* some string of the tile has to be escaped */
@@ -1210,9 +1217,9 @@ __device__ __forceinline__ void wt_note_cycles(DevResult* res, long long c0, lon
  * 300 MB against a record per thread with all of its strings (kernel, us): Users of 72 KB 30 200 -> 430, of 1.2 MB 67 600 -> 425, Pets of 3000 short
  * strings 31 700 -> 1 230; 100 k Users of which one in a thousand has 96 KB 6 270 -> 117; 300 k records of three models in the caller's own order 490 -> 260, with escapes 590 -> 355 (and 240 and 435 in tiles of 128
  * records of 128 threads, five to an SM, whose strings were looked over for escapes by a kernel of their own, 40 us more). */
-template <int SCHEMA>
+template <int SCHEMA, uint32_t THREADS>
 __device__ __noinline__ void wt_general_tile(const WTileArgs& a, WtShared& sh, uint8_t* smem, uint64_t rec0, uint32_t nrec, uint32_t tile, long long c0) {
-  constexpr uint32_t THREADS = WtT<SCHEMA>::threads, WARPS = WtT<SCHEMA>::warps;
+  constexpr uint32_t WARPS = THREADS / 32u;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, ngroups = wt_groups<SCHEMA>(sh);
   WtLater* const e = reinterpret_cast<WtLater*>(smem);
   if (tid < nrec) sh.bytes[tid] = 0;
@@ -1262,9 +1269,8 @@ __device__ __noinline__ void wt_general_tile(const WTileArgs& a, WtShared& sh, u
   if (tid == 0) wt_note_cycles(a.w.res, c0, c1, c2, c3);
 }
 /* One record of a staged tile whose text has no window: the same steps, straight to dst. w8: `bytes` of shared memory that are free. */
-template <int SCHEMA>
+template <int SCHEMA, uint32_t WARPS>
 __device__ __noinline__ void wt_general_one(const WTileArgs& a, WtShared& sh, uint8_t* w8, uint32_t bytes, uint64_t i, uint32_t rec, uint8_t* dst) {
-  constexpr uint32_t WARPS = WtT<SCHEMA>::warps;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, most = bytes / (uint32_t)sizeof(WtLater), cap = most < WT_LATERS ? most : WT_LATERS;
   WtLater* const e = reinterpret_cast<WtLater*>(w8);
   uint32_t model = SCHEMA - 1u; /* thread 0's */
@@ -1284,9 +1290,9 @@ __device__ __noinline__ void wt_general_one(const WTileArgs& a, WtShared& sh, ui
   __syncthreads();
 }
 
-template <int SCHEMA>
-__global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_write_tile(const __grid_constant__ WTileArgs a) {
-  constexpr uint32_t THREADS = WtT<SCHEMA>::threads, WARPS = WtT<SCHEMA>::warps;
+template <int SCHEMA, uint32_t THREADS = WtT<SCHEMA>::threads>
+__global__ void __launch_bounds__(THREADS, THREADS == WtT<SCHEMA>::threads ? WtT<SCHEMA>::blocks : WT_SHORT_BLOCKS) k_write_tile(const __grid_constant__ WTileArgs a) {
+  constexpr uint32_t WARPS = THREADS / 32u;
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) WtShared sh;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -1358,7 +1364,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
     odd = __syncthreads_or((int)bad) != 0;
     x.later = x.dirty || sh.longs;
   }
-  if (odd) { wt_general_tile<SCHEMA>(a, sh, smem, rec0, nrec, tile, c0); return; }
+  if (odd) { wt_general_tile<SCHEMA, THREADS>(a, sh, smem, rec0, nrec, tile, c0); return; }
   /* where the records start */
   const uint32_t len = tid < nrec ? sh.pos[tid] : 0u;
   uint32_t at = warp_incl_scan(len);
@@ -1390,7 +1396,7 @@ __global__ void __launch_bounds__(WtT<SCHEMA>::threads, WtT<SCHEMA>::blocks) k_w
       rb = lo - ra > 32u ? lo - (lo - ra) % 32u : lo; /* whole groups */
     }
     uint8_t* const dst0 = out0 + start;
-    if (rb == ra) { wt_general_one<SCHEMA>(a, sh, smem + win, room + 48u, rec0 + ra, ra, dst0); ++ra; continue; } /* no window for this one */
+    if (rb == ra) { wt_general_one<SCHEMA, WARPS>(a, sh, smem + win, room + 48u, rec0 + ra, ra, dst0); ++ra; continue; } /* no window for this one */
     const uint32_t pad = (uint32_t)(reinterpret_cast<uintptr_t>(dst0) & 15u), bytes = sh.pos[rb] - start;
     /* the window mirrors the output's alignment: window byte k goes to (dst0 - pad)[k] */
     if (ra) { wt_zero(smem, win, win + 32u + bytes, tid, THREADS); if (tid == 0) sh.nesc = 0; __syncthreads(); }

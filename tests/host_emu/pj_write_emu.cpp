@@ -27,11 +27,12 @@ thread_local __attribute__((aligned(16))) uint8_t smem[228 * 1024];
 }
 
 namespace {
+static bool g_short = false;
 WTileArgs g_args;
 uint32_t g_schema;
 void one_thread(void*) {
   switch (g_schema) {
-    case PJ_SCHEMA_PET: k_write_tile<PJ_SCHEMA_PET>(g_args); break;
+    case PJ_SCHEMA_PET: if (g_short) k_write_tile<PJ_SCHEMA_PET, WT_SHORT_THREADS>(g_args); else k_write_tile<PJ_SCHEMA_PET>(g_args); break;
     case PJ_SCHEMA_ORDER: k_write_tile<PJ_SCHEMA_ORDER>(g_args); break;
     case PJ_SCHEMA_USER: k_write_tile<PJ_SCHEMA_USER>(g_args); break;
     default: k_write_tile<PJ_SCHEMA_MIXED>(g_args); break;
@@ -39,6 +40,8 @@ void one_thread(void*) {
 }
 }  // namespace
 
+/* Pets by blocks of WT_SHORT_THREADS, from now on. */
+extern "C" void emu_write_short(int on) { g_short = on != 0; }
 extern "C" const char* emu_write_error() { return emu_block::error; }
 /* The records' text without the brackets of an array. recs, shared: records per tile, bytes of shared memory. Returns 0, 1 (no room) or -1. */
 extern "C" int emu_write_tiles(uint32_t schema, uint32_t array, int inclusion, uint32_t lower, const pj_columns* cols, uint8_t* out, uint64_t cap, uint32_t recs, uint32_t shared,
@@ -66,7 +69,7 @@ extern "C" int emu_write_tiles(uint32_t schema, uint32_t array, int inclusion, u
   for (uint32_t t = 0; t < a.ntiles && fine; ++t) {
     memset(smem, 0xC3, shared);
     EMU_POISON(smem + shared, sizeof smem - shared);
-    fine = emu_block::run(wt_threads(schema), one_thread, nullptr, order + t);
+    fine = emu_block::run(g_short && schema == PJ_SCHEMA_PET ? WT_SHORT_THREADS : wt_threads(schema), one_thread, nullptr, order + t);
     EMU_UNPOISON(smem + shared, sizeof smem - shared);
   }
   if (fine && res.timeout) { snprintf(emu_block::error, sizeof emu_block::error, "a bounded wait ran out"); fine = false; }

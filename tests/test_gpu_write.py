@@ -48,6 +48,13 @@ def test_many_bytes_to_escape(ctx, oracle, size, esc):
     check(ctx, oracle, PET, oracle.parse(PET, as_u8("\n".join(line % (i, text(i), text(i + 1), text(i + 2), text(i + 3)) for i in range(1500 if size < 500 else 200)))))
 
 
+@pytest.mark.parametrize("text", ['{"name":"","photoUrls":[]}', '{"id":%d,"name":"ab","photoUrls":[]}', '{"id":%d,"name":"say \\"%d\\"","photoUrls":["u","\\n"],"tags":[{"id":%d}],"status":"sold"}'])
+def test_many_short_pets(ctx, oracle, text):
+    """Tables of four blocks to an SM; and of few tiles, which are not."""
+    for n in (150_001, 2000):
+        check(ctx, oracle, PET, oracle.parse(PET, as_u8("\n".join(text.replace("%d", str(i)) for i in range(n)))))
+
+
 @pytest.mark.parametrize("dirty", [0, 0.01])
 def test_long_lists_and_records_of_all_sizes(ctx, oracle, dirty):
     rng = random.Random(3)

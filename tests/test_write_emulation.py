@@ -277,6 +277,23 @@ def test_tiles_with_many_bytes_to_escape(writer, oracle, falls, recs):
                 write(writer, schema, cols, want, inclusion=inclusion, recs=recs, **shape)
 
 
+@pytest.mark.parametrize("flags", [0, ESC | SPARSE, ZIPF | ESC])
+def test_blocks_of_short_pets(writer, oracle, flags):
+    """Half as many threads to a tile: whole tiles, lists, windows in rounds, the general road."""
+    rng = random.Random(7)
+    cols = oracle.parse(PET, pj.gen_text(PET, 12, 0, 300, flags))
+    edges, long_ = oracle.parse(PET, edge_text(rng, 300)), oracle.parse(PET, long_text(rng, 12, 0.1))
+    short = oracle.parse(PET, as_u8("\n".join('{"id":%d,"name":"%s","photoUrls":[]}' % (i, "ab"[: i % 3]) for i in range(600))))
+    writer.emu_write_short(1)
+    try:
+        for c in (cols, edges, long_, short):
+            want = oracle.write(PET, c, NDJSON, abi.PJ_INCLUDE_NON_NULL)
+            for shape in (dict(recs=256, shared=131072), dict(recs=96, shared=28 * 1024, mis=9, order=3), dict(recs=5, shared=8192, mis=1)):
+                write(writer, PET, c, want, **shape)
+    finally:
+        writer.emu_write_short(0)
+
+
 def test_no_records(writer, oracle):
     cols = abi.HostColumns(PET, abi.default_caps(PET, 1, 16))
     n = C.c_uint64()
